@@ -65,6 +65,23 @@ int upload(qgw_run* r, T** out, const std::vector<double>& host) {
   return cudaStreamSynchronize(r->stream) == cudaSuccess ? QGW_OK : QGW_ERR_CUDA;
 }
 
+int upload_fx(qgw_run* r, qgw::FxTables* out, const qgw::FxTablesHost& h) {
+  auto put = [&](auto** dst, const auto& v) -> int {
+    int rc = dalloc(r, dst, v.size());
+    if (rc) return rc;
+    CK(cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, r->stream));
+    return QGW_OK;
+  };
+  qgw::Q4 *tw, *sp;
+  qgw::Q2* sj;
+  int rc;
+  if ((rc = put(&tw, h.twq)) || (rc = put(&sp, h.spq)) || (rc = put(&sj, h.nsj))) return rc;
+  out->twq = tw;
+  out->spq = sp;
+  out->nsj = sj;
+  return cudaStreamSynchronize(r->stream) == cudaSuccess ? QGW_OK : QGW_ERR_CUDA;
+}
+
 // choose the modes per row block and the columns per column block so that
 // each block's two work buffers stay within the shared-memory budget
 // Shared-memory budget of the row kernels' work buffers.  Measured at
@@ -234,6 +251,9 @@ int setup_args(qgw_run* r, StepArgs<T>& a) {
     t.sjp = (const qgw::C2<T>*)sjp;
     t.bc = (const qgw::C2<T>*)bc;
     t.bz = (const qgw::C2<T>*)bz;
+    qgw::FxTables& f = dim == 0 ? a.fx : a.fy;
+    f = qgw::FxTables{};
+    if (sizeof(T) == 8 && !per && !g.blue && (rc = upload_fx(r, &f, qgw::build_fx_tables(g)))) return rc;
   }
   T *cl, *cm;
   if ((rc = upload<T>(r, &cl, r->cl2m))) return rc;

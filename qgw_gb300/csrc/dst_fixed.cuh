@@ -1,13 +1,11 @@
 // dst_fixed.cuh -- the batched DST-I of dst_core.h specialised at compile
-// time for one transform length (M = 2H = 2^(LGH+1)), used by the step
-// kernels for the common lengths, and its complex FFT alone (the periodic
-// transforms).  Same arithmetic as the generic block DST (step_device.cuh),
+// time for one transform length (M = 2H = 2^(LGH+1)), used by the FP32 step
+// kernels for the common lengths (FP64: dst_fx.cuh), and its complex FFT
+// alone (the periodic transforms of both precisions).  Same arithmetic as the generic block DST (step_device.cuh),
 // with phases merged where the data allow it:
 //   [pre-processing + first radix-8 pass] -> later Stockham passes
 //   -> [split + prefix sum of the odd outputs]
-// (FP32; the FP64 kernels, bound by their FP64 pipe and short of registers
-// for the merged phases, keep the pre-processing and the split and prefix
-// sum as phases of their own).  The merged first pass reads the four raw
+// (rows of H = 64 keep the pre-processing as a phase of its own).  The merged first pass reads the four raw
 // values each complex input needs (x_{2m}, x_{2m+1}, x_{M-2m}, x_{M-2m-1}),
 // so the pre-processed row is never stored.  With the geometry fixed, a
 // padded shared-memory index is one base computation plus compile-time
@@ -437,9 +435,7 @@ __device__ T* dst_block_fixed(T* A, T* B, int nrows, int ld, const DstTables<T>&
     src = cfft_passes_fixed<T, LGH, 1>(B, A, nrows, ld, tb.twp);
   } else {
     // pre-processing as its own phase, A -> B (dst_pre_item's arithmetic):
-    // doubles (the merged phase's 16 live complex values and their table
-    // entries exceed the FP64 kernels' register bound; those kernels are
-    // bound by the FP64 pipe, not by barriers) and short float rows (H = 64)
+    // short rows (H = 64)
     for (int w = tid; w < nrows * H; w += DST_NT) {
       const int r = w >> LGH, j = (w & (H - 1)) + 1;
       const T* x = A + r * ld;
@@ -510,39 +506,8 @@ __device__ T* dst_block_fixed(T* A, T* B, int nrows, int ld, const DstTables<T>&
   __syncthreads();
   // phase 4: prefix sum of the odd outputs (indices 1, 3, 5, ...), one warp
   // per row.
-  if constexpr (sizeof(T) == 8) {
-    // FP64 (the FP64 pipe bounds these kernels, so the fewest additions):
-    // lane c scans chunk c sequentially, the chunk totals are scanned by
-    // shuffles and added back -- two additions per value
-    constexpr int CH = H >= 256 ? H / 32 : 8, NC = H / CH;
-    static_assert((2 * CH) % (2 * Pad<T>::P) == 0, "chunk start must be pad-aligned");
-    const int warp = tid >> 5, lane = tid & 31, nwarp = DST_NT >> 5;
-    for (int r = warp; r < nrows; r += nwarp) {
-      // odd index 2k + 1 of the chunk: o[pr(2t)] (2t and 2t + 1 share a pad period)
-      T* o = dst + r * ld + pr<T>(2 * CH * lane) + 1;
-      T acc = T(0);
-      if (lane < NC) {
-        acc = o[0];
-#pragma unroll
-        for (int t = 1; t < CH; ++t) {
-          acc = acc + o[pr<T>(2 * t)];
-          o[pr<T>(2 * t)] = acc;
-        }
-      }
-      T incl = acc;
-#pragma unroll
-      for (int of = 1; of < 32; of <<= 1) {
-        const T u = __shfl_up_sync(0xffffffffu, incl, of);
-        if (lane >= of) incl += u;
-      }
-      T ex = __shfl_up_sync(0xffffffffu, incl, 1);
-      if (lane > 0 && lane < NC) {
-#pragma unroll
-        for (int t = 0; t < CH; ++t) o[pr<T>(2 * t)] += ex;
-      }
-    }
-  } else {
-    // FP32 (rows of other lengths): each lane scans NV consecutive 16-byte
+  {
+    // (rows of other lengths): each lane scans NV consecutive 16-byte
     // vectors (4 NV reals, 2 NV odd outputs, the .y and .w members) in
     // registers, the lane totals are scanned by shuffles, and a running
     // carry joins the 128 NV reals of one round to the next:  out = (carry +

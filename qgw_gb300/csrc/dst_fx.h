@@ -1,0 +1,344 @@
+// dst_fx.h -- the FP64 path's DST-I in 64-bit block fixed point: the same
+// half-length transform as dst_core.h, with every value of a row an integer
+// times one power of two that the row's own data set.
+//
+// Why: this chip issues two FP64 operations per clock and SM, but 64-128
+// integer ones.  A 1024-point DST is 18 FP64 operations per point; in
+// integers its additions cost two instructions each on the wide pipes and
+// its products six (fx_mul), and none runs on the FP64 pipe.
+//
+// Accuracy: a row enters at 59 bits below its largest value, additions are
+// exact, and before each pass's twiddle products the row is shifted to 2^61
+// by its measured magnitude (the bitwise OR of |v| over the row), so each
+// pass's products round at about 2^-57 of the row's rms, and the tables hold
+// 62 bits.  The prefix sum of the odd outputs, which multiplies the
+// roundings before it by about sqrt(M) and in floating point adds one per
+// term, adds none.  The error against exact arithmetic is below the FP64
+// transform's (tests/test_host.py).
+//
+// A value v of a row stands for v 2^e, e the row's exponent.  A row whose
+// largest magnitude is infinite or NaN has every output NaN, a row of zeros
+// every output zero; magnitudes
+// below 2^-957 round to multiples of 2^-1015.
+//
+// Work items as in dst_core.h: one item of one phase, any order within a
+// phase.  Buffers hold 8-byte values in the padded layout of doubles.
+#pragma once
+
+#include "dst_core.h"
+
+namespace qgw {
+
+typedef long long fx_t;
+template <> struct QGW_ALIGN(16) C2<fx_t> { fx_t x, y; };
+
+// A fixed-point constant h 2^32 + l, both halves signed, so that a product
+// takes signed 32-bit multiplies only.
+struct QGW_ALIGN(8) Q2 { int h, l; };
+struct QGW_ALIGN(16) Q4 { Q2 x, y; };
+
+QGW_HD Q2 q2_split(fx_t w) {
+  Q2 q;
+  q.l = (int)w;
+  q.h = (int)(w >> 32) - (q.l >> 31);
+  return q;
+}
+
+// Tables: twq the pass twiddles (cos, -sin) scaled by 2^62, in the order of
+// fill_pass_twiddles; nsj -s_j scaled by 2^63, j <= H (s_H = 1 has no
+// positive 2^63); spq (cos, -sin)(2 pi k / M) scaled by 2^63, 1 <= k <= H/2.
+struct FxTables {
+  const Q4* twq;
+  const Q2* nsj;
+  const Q4* spq;
+};
+
+QGW_HD int fx_mh(int a, int b) {
+#ifdef __CUDA_ARCH__
+  return __mulhi(a, b);
+#else
+  return (int)(((long long)a * b) >> 32);
+#endif
+}
+QGW_HD int fx_clz(unsigned int v) {
+#ifdef __CUDA_ARCH__
+  return __clz((int)v);
+#else
+  return v ? __builtin_clz(v) : 32;
+#endif
+}
+
+// v w / 2^64 to within one unit: one 32 x 32 -> 64 product and the high
+// words of the two cross products (their truncations, half a unit each on
+// average, are added back).  |v| < 2^61.5.
+QGW_HD fx_t fx_mul(fx_t v, Q2 w) {
+  const Q2 a = q2_split(v);
+  return (fx_t)a.h * w.h + (fx_t)(fx_mh(a.h, w.l) + fx_mh(a.l, w.h) + 1);
+}
+// (x + iy) w / 2^64, |w| components at most 2^62
+QGW_HD void fx_cmul(fx_t& x, fx_t& y, const Q4& w) {
+  const Q2 a = q2_split(x), b = q2_split(y);
+  const int t1 = fx_mh(a.h, w.x.l) + fx_mh(a.l, w.x.h), t2 = fx_mh(b.h, w.y.l) + fx_mh(b.l, w.y.h);
+  const int t3 = fx_mh(a.h, w.y.l) + fx_mh(a.l, w.y.h) + fx_mh(b.h, w.x.l) + fx_mh(b.l, w.x.h) + 2;
+  x = ((fx_t)a.h * w.x.h + (fx_t)(t1 - t2)) - (fx_t)b.h * w.y.h;
+  y = (fx_t)b.h * w.x.h + ((fx_t)a.h * w.y.h + (fx_t)t3);
+}
+// v c for a constant c = B + f, |f| < 1/2, f scaled by 2^64
+template <int B> QGW_HD fx_t fx_mulc(fx_t v, int h, int l) {
+  Q2 f;
+  f.h = h;
+  f.l = l;
+  const fx_t p = fx_mul(v, f);
+  return B == 1 ? v + p : B == -1 ? p - v : p;
+}
+
+QGW_HD fx_t fx_shl(fx_t v, int s) { return (fx_t)((unsigned long long)v << s); }
+// v / 2^n rounded, ties to even: the roundings of a row must not share a
+// sign, or the prefix sum would add M of them up
+QGW_HD fx_t fx_shr(fx_t v, int n) { return (v + ((((fx_t)1 << n) >> 1) - 1 + ((v >> n) & 1))) >> n; }
+QGW_HD fx_t fx_shift(fx_t v, int s) { return s >= 0 ? fx_shl(v, s > 63 ? 63 : s) : s < -62 ? 0 : fx_shr(v, -s); }
+QGW_HD unsigned int fx_mag(fx_t v) {  // OR of these over values: their magnitude's bits above 2^32
+  const int h = (int)(v >> 32);
+  return (unsigned int)(h ^ (h >> 31));
+}
+
+// ---- doubles in and out
+constexpr int FX_EMIN = 66;    // smallest biased exponent a row is scaled to
+constexpr int FX_EOFF = 1081;  // X = x 2^(FX_EOFF - E) < 2^59, E the row's largest biased exponent
+constexpr int FX_NAN = 1 << 20;  // row exponent of a non-finite row
+constexpr int FX_ZERO = -FX_NAN;  // and of a row of zeros (v 2^e is 0)
+// the scale's biased exponent of a row from its largest high word
+QGW_HD int fx_scale(unsigned int mx) { return (int)(mx >> 20) < FX_EMIN ? FX_EMIN : (int)(mx >> 20); }
+
+QGW_HD fx_t fx_from_bits(unsigned long long b, int E) {
+  const unsigned int hi = (unsigned int)(b >> 32);
+  int sh = E - (int)((hi >> 20) & 0x7ffu);
+  sh = sh > 63 ? 63 : sh;
+  const unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | (b & 0xffffffffull)) << 6;
+  const fx_t v = (fx_t)(m >> sh);
+  return (int)hi < 0 ? -v : v;
+}
+// v 2^e rounded to a double; e from fx_exp_ok's range (fx_to_bits) or any
+QGW_HD bool fx_exp_ok(int e) { return e >= -1020 && e <= 900; }
+QGW_HD unsigned long long fx_to_bits(fx_t v, int e) {
+  const unsigned long long sg = (unsigned long long)v & 0x8000000000000000ull;
+  unsigned long long m = (unsigned long long)(v < 0 ? -v : v);
+  unsigned int hi = (unsigned int)(m >> 32);
+  int n = fx_clz(hi);
+  if (hi == 0) {
+    hi = (unsigned int)m;
+    n = 32 + fx_clz(hi);
+  }
+  m <<= (n & 63);
+  m = (m >> 11) + ((m >> 10) & 1);  // 53 bits, rounded; a carry moves into the exponent
+  return (hi == 0 ? 0 : ((unsigned long long)(1085 + e - n) << 52) + m) | sg;
+}
+
+// ---- phase 1: pre-processing of raw doubles, items j = 1..H.  y_j / 2 =
+// (x_j - x_{M-j}) / 4 + s_j (x_j + x_{M-j}) / 2; returns the item's part of
+// sum |X| in units of 2^41, rounded up.
+QGW_HD unsigned int fx_pre_item(const unsigned long long* x, fx_t* y, int j, int M, int E, const Q2* nsj) {
+  const fx_t a = fx_from_bits(x[pr<double>(j)], E), b = fx_from_bits(x[pr<double>(M - j)], E);
+  const fx_t p = fx_mul(a + b, nsj[j]);
+  const fx_t d = fx_shr(a - b, 2);
+  y[pr<double>(j)] = d - p;
+  if (2 * j != M) y[pr<double>(M - j)] = -d - p;
+  if (j == 1) y[0] = 0;
+  const unsigned int la = (fx_mag(a) >> 9) + 1, lb = (fx_mag(b) >> 9) + 1;
+  return 2 * j != M ? la + lb : la;
+}
+
+// ---- phase 2: forward DFTs (exact but for the products)
+QGW_HD void fx_dft2(C2<fx_t>* v) { dft2<fx_t>(v); }
+QGW_HD fx_t fx_hs(fx_t v) { return fx_mulc<1>(v, -1257966796, -102865788); }  // v sqrt(1/2)
+QGW_HD void fx_dft8(C2<fx_t>* v) {
+  C2<fx_t> a[4], b[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) { a[r] = cadd(v[r], v[r + 4]); b[r] = csub(v[r], v[r + 4]); }
+  dft4<fx_t>(a);
+  v[0] = a[0]; v[2] = a[1]; v[4] = a[2]; v[6] = a[3];
+  // odd outputs: DFT4(b0, W b1, W^2 b2, W^3 b3), W = (1 - i)/sqrt 2
+  const fx_t p1x = fx_hs(b[1].x + b[1].y), p1y = fx_hs(b[1].y - b[1].x);
+  const fx_t p3x = fx_hs(b[3].y - b[3].x), p3y = -fx_hs(b[3].x + b[3].y);
+  b[1].x = p1x; b[1].y = p1y;
+  b[2] = cmi(b[2]);
+  b[3].x = p3x; b[3].y = p3y;
+  dft4<fx_t>(b);
+  v[1] = b[0]; v[3] = b[1]; v[5] = b[2]; v[7] = b[3];
+}
+QGW_HD void fx_dft3(C2<fx_t>* v) {
+  const C2<fx_t> t = cadd(v[1], v[2]), d = csub(v[1], v[2]);
+  C2<fx_t> m, p;
+  m.x = v[0].x - ((t.x + 1) >> 1); m.y = v[0].y - ((t.y + 1) >> 1);
+  p.x = fx_mulc<1>(d.x, -575416509, -1033546850); p.y = fx_mulc<1>(d.y, -575416509, -1033546850);  // sin(2 pi/3)
+  v[0] = cadd(v[0], t);
+  v[1].x = m.x + p.y; v[1].y = m.y - p.x;
+  v[2].x = m.x - p.y; v[2].y = m.y + p.x;
+}
+QGW_HD fx_t fx_c51(fx_t v) { return fx_mulc<0>(v, 1327217885, -1079689717); }   // cos(2 pi/5)
+QGW_HD fx_t fx_c52(fx_t v) { return fx_mulc<-1>(v, 820265763, 1079689717); }    // cos(4 pi/5)
+QGW_HD fx_t fx_s51(fx_t v) { return fx_mulc<1>(v, -210210662, 581434099); }     // sin(2 pi/5)
+QGW_HD fx_t fx_s52(fx_t v) { return fx_mulc<1>(v, -1770448860, -1429016722); }  // sin(4 pi/5)
+QGW_HD void fx_dft5(C2<fx_t>* v) {
+  const C2<fx_t> t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]);
+  const C2<fx_t> d1 = csub(v[1], v[4]), d2 = csub(v[2], v[3]);
+  C2<fx_t> a, b, p, q;
+  a.x = v[0].x + fx_c51(t1.x) + fx_c52(t2.x); a.y = v[0].y + fx_c51(t1.y) + fx_c52(t2.y);
+  b.x = v[0].x + fx_c52(t1.x) + fx_c51(t2.x); b.y = v[0].y + fx_c52(t1.y) + fx_c51(t2.y);
+  p.x = fx_s51(d1.x) + fx_s52(d2.x); p.y = fx_s51(d1.y) + fx_s52(d2.y);
+  q.x = fx_s52(d1.x) - fx_s51(d2.x); q.y = fx_s52(d1.y) - fx_s51(d2.y);
+  v[0] = cadd(v[0], cadd(t1, t2));
+  v[1].x = a.x + p.y; v[1].y = a.y - p.x;
+  v[4].x = a.x - p.y; v[4].y = a.y + p.x;
+  v[2].x = b.x + q.y; v[2].y = b.y - q.x;
+  v[3].x = b.x - q.y; v[3].y = b.y + q.x;
+}
+// cos, sin of 2 pi e / 7, e = 1, 2, 3
+QGW_HD fx_t fx_c7(fx_t v, int e) {
+  return e == 1 ? fx_mulc<1>(v, -1617098988, 1601080166)
+       : e == 2 ? fx_mulc<0>(v, -955720134, -76219603)
+                : fx_mulc<-1>(v, 425335474, -1524860563);
+}
+QGW_HD fx_t fx_s7(fx_t v, int e) {
+  return e == 1 ? fx_mulc<1>(v, -937026648, 787634270)
+       : e == 2 ? fx_mulc<1>(v, -107683797, -951367907)
+                : fx_mulc<0>(v, 1863516470, -961608703);
+}
+QGW_HD void fx_dft7(C2<fx_t>* v) {
+  C2<fx_t> t[3], d[3], y[7];
+  for (int n = 0; n < 3; ++n) { t[n] = cadd(v[n + 1], v[6 - n]); d[n] = csub(v[n + 1], v[6 - n]); }
+  y[0] = cadd(v[0], cadd(t[0], cadd(t[1], t[2])));
+  for (int k = 1; k <= 3; ++k) {
+    C2<fx_t> a = v[0], p;
+    p.x = 0; p.y = 0;
+    for (int n = 1; n <= 3; ++n) {
+      const int e = (n * k) % 7, f = e <= 3 ? e : 7 - e;
+      a.x += fx_c7(t[n - 1].x, f); a.y += fx_c7(t[n - 1].y, f);
+      const fx_t sx = fx_s7(d[n - 1].x, f), sy = fx_s7(d[n - 1].y, f);
+      p.x += e <= 3 ? sx : -sx; p.y += e <= 3 ? sy : -sy;
+    }
+    y[k].x = a.x + p.y; y[k].y = a.y - p.x;
+    y[7 - k].x = a.x - p.y; y[7 - k].y = a.y + p.x;
+  }
+  for (int k = 0; k < 7; ++k) v[k] = y[k];
+}
+template <int R> QGW_HD void fx_dft(C2<fx_t>* v) {
+  if (R == 8) fx_dft8(v);
+  else if (R == 4) dft4<fx_t>(v);
+  else if (R == 2) dft2<fx_t>(v);
+  else if (R == 3) fx_dft3(v);
+  else if (R == 5) fx_dft5(v);
+  else fx_dft7(v);
+}
+
+// The shift before a pass's twiddles, from the OR of fx_mag over the row:
+// |v| 2^s < 2^61.  The components of a product (/ 4) are below 2^59.5 and a
+// radix-8 butterfly's outputs below 2^62.5; so are the first pass's
+// (|y / 2| < 2^59).
+QGW_HD int fx_pass_shift(unsigned int mag) { return 29 - (32 - fx_clz(mag)); }
+
+// the members' twiddles w^(q k) (tw: the pass's table, entry (q-1) Ns + k)
+// on the row shifted by s; every member is divided by 4
+template <int R> QGW_HD void fx_twiddle(C2<fx_t>* v, int k, int Ns, int s, const Q4* tw) {
+  if (s >= 0) {
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      v[q].x = fx_shl(v[q].x, s);
+      v[q].y = fx_shl(v[q].y, s);
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      v[q].x = fx_shr(v[q].x, -s);
+      v[q].y = fx_shr(v[q].y, -s);
+    }
+  }
+  v[0].x = fx_shr(v[0].x, 2);
+  v[0].y = fx_shr(v[0].y, 2);
+#pragma unroll
+  for (int q = 1; q < R; ++q) fx_cmul(v[q].x, v[q].y, tw[(q - 1) * Ns + k]);
+}
+template <int R> QGW_HD unsigned int fx_mag_all(const C2<fx_t>* v) {
+  unsigned int m = 0;
+#pragma unroll
+  for (int q = 0; q < R; ++q) m |= fx_mag(v[q].x) | fx_mag(v[q].y);
+  return m;
+}
+// Stockham pass, item b (stockham_item_k's indices); returns the OR of its
+// outputs' magnitudes
+template <int R>
+QGW_HD unsigned int fx_stockham_item(const C2<fx_t>* src, C2<fx_t>* dst, int b, int k, int Ns, int H, int s,
+                                     const Q4* tw) {
+  const int stride = H / R;
+  C2<fx_t> v[R];
+#pragma unroll
+  for (int q = 0; q < R; ++q) v[q] = src[pc<double>(b + q * stride)];
+  if (Ns > 1) fx_twiddle<R>(v, k, Ns, s, tw);
+  fx_dft<R>(v);
+  const int base = (b - k) * R + k;
+#pragma unroll
+  for (int q = 0; q < R; ++q) dst[pc<double>(base + q * Ns)] = v[q];
+  return fx_mag_all<R>(v);
+}
+template <int R>
+QGW_HD_NOINLINE unsigned int fx_stockham_item_far(const C2<fx_t>* src, C2<fx_t>* dst, int b, int k, int Ns, int H,
+                                                  int s, const Q4* tw) {
+  return fx_stockham_item<R>(src, dst, b, k, Ns, H, s, tw);
+}
+// tw: the table of the pass (twq + Ns - R0)
+QGW_HD unsigned int fx_stockham_dispatch(int R, const C2<fx_t>* src, C2<fx_t>* dst, int b, int k, int Ns, int H, int s,
+                                         const Q4* tw) {
+  switch (R) {
+    case 8: return fx_stockham_item_far<8>(src, dst, b, k, Ns, H, s, tw);
+    case 4: return fx_stockham_item_far<4>(src, dst, b, k, Ns, H, s, tw);
+    case 2: return fx_stockham_item_far<2>(src, dst, b, k, Ns, H, s, tw);
+    case 3: return fx_stockham_item_far<3>(src, dst, b, k, Ns, H, s, tw);
+    case 5: return fx_stockham_item_far<5>(src, dst, b, k, Ns, H, s, tw);
+    default: return fx_stockham_item_far<7>(src, dst, b, k, Ns, H, s, tw);
+  }
+}
+
+// ---- phase 3: split.  Shift s of Z: below 2^59 (a doubled difference
+// enters a product), and so that |Y| <= 2 sum |X| stays below 2^62 (the
+// prefix sums of the odd outputs are outputs, and wrapped intermediate sums
+// of integers do no harm).  l1: sum of fx_pre_item's values; drop: the
+// passes' sum of 2 - shift.
+QGW_HD int fx_split_shift(unsigned int mag, unsigned int l1, int drop) {
+  const int a = 27 - (32 - fx_clz(mag)), b = 21 - (32 - fx_clz(l1)) + drop;
+  return a < b ? a : b;
+}
+// exponent of the row's outputs (mx: its largest high word)
+QGW_HD int fx_row_exp(unsigned int mx, int drop, int s) {
+  return mx == 0 ? FX_ZERO : mx >= 0x7ff00000u ? FX_NAN : fx_scale(mx) - FX_EOFF + 1 + drop - s;
+}
+
+QGW_HD void fx_split_pair(C2<fx_t> A, C2<fx_t> B, const Q4& cs, C2<fx_t>& lo, C2<fx_t>& hi) {
+  const fx_t sr = A.x + B.x, si = A.y - B.y, dr = 2 * (A.x - B.x), di = 2 * (A.y + B.y);
+  const fx_t P = fx_mul(di, cs.x) + fx_mul(dr, cs.y);  // c di - s dr
+  const fx_t Q = fx_mul(dr, cs.x) - fx_mul(di, cs.y);  // c dr + s di
+  lo.x = Q - si;  // Y_{2k}
+  lo.y = sr + P;  // 2 R_k
+  hi.x = Q + si;  // Y_{2(H-k)}
+  hi.y = sr - P;  // 2 R_{H-k}
+}
+QGW_HD C2<fx_t> fx_shift2(C2<fx_t> v, int s) {
+  v.x = fx_shift(v.x, s);
+  v.y = fx_shift(v.y, s);
+  return v;
+}
+QGW_HD void fx_split_item(const C2<fx_t>* Z, C2<fx_t>* o, int k, int H, int s, const Q4* spq) {
+  if (k == 0) {
+    const C2<fx_t> a = fx_shift2(Z[0], s);
+    C2<fx_t> z0;
+    z0.x = 0;
+    z0.y = a.x + a.y;  // R_0
+    o[0] = z0;
+    return;
+  }
+  C2<fx_t> lo, hi;
+  fx_split_pair(fx_shift2(Z[pc<double>(k)], s), fx_shift2(Z[pc<double>(H - k)], s), spq[k], lo, hi);
+  o[pc<double>(k)] = lo;
+  if (2 * k != H) o[pc<double>(H - k)] = hi;
+}
+
+}  // namespace qgw

@@ -22,7 +22,7 @@
 #include <cstring>
 
 #include "../../include/qgw_gpu.h"
-#include "dst_core.h"
+#include "dst_tables.h"
 #include "host.h"
 #include "kernels.h"
 #include "qgw_device.cuh"
@@ -33,9 +33,10 @@ constexpr size_t kFieldMax = (size_t)1 << 21;  // doubles: nl*(NX+1)*(NY+1) limi
 constexpr int kMMax = 1024;                     // NX, NY limit (DST length + 1)
 constexpr int kNlMax = 32;  // layers the shared scratch array holds
 constexpr int kDevMax = 16;
-// DST tables of one dimension: tw (H), pre (H+1), spl (H/2+1), twp (< H)
-// complex values
-constexpr size_t kTab = 2 * (2 * ((size_t)kMMax / 2) + ((size_t)kMMax / 2 + 1) + ((size_t)kMMax / 4 + 1));
+// DST tables of one dimension (dst_fx.h): twq (< H) and spq (H/2+1) pairs,
+// nsj (H+1) values, rounded to 16 bytes
+constexpr size_t kTwq = 2 * ((size_t)kMMax / 2), kSpq = 2 * ((size_t)kMMax / 4 + 1);
+constexpr size_t kTab = kTwq + kSpq + ((size_t)kMMax / 2 + 2);
 constexpr size_t kStateD = (sizeof(qgw::DevState) + 7) / 8;
 
 // offsets (in doubles) inside the scratch array
@@ -52,7 +53,7 @@ constexpr size_t oState = oKsq + kMMax;
 constexpr size_t kTotal = oState + kStateD;
 
 // host staging of the small tables (file scope: no heap use per call)
-double h_tab[oState - oTx];
+alignas(16) double h_tab[oState - oTx];
 double h_key[kDevMax][3 * kNlMax * kNlMax + 16];  // set-up held by each device
 bool h_key_valid[kDevMax];
 double* d_base[kDevMax];
@@ -102,35 +103,12 @@ __global__ void k_noalloc_ghosts(double* q, double* psi, int nx, int ny, int nl,
   }
 }
 
-double sinpi_r(long m, long N) {
-  long r = m % (2 * N);
-  if (r < 0) r += 2 * N;
-  double sg = 1.0;
-  if (r >= N) { r -= N; sg = -1.0; }
-  if (2 * r > N) r = N - r;
-  return sg * std::sin(M_PI * (double)r / (double)N);
-}
-
-// the DST tables of dst_core.h for length M into dst (tw | pre | spl)
+// the fixed-point DST's tables for length M into dst (twq | spq | nsj)
 void fill_tables(int M, double* dst) {
-  const int H = M / 2;
-  double* tw = dst;
-  double* pre = tw + 2 * H;
-  double* spl = pre + 2 * (H + 1);
-  for (int m = 0; m < H; ++m) {
-    tw[2 * m] = sinpi_r(4L * m + H, 2L * H);
-    tw[2 * m + 1] = -sinpi_r(2L * m, H);
-  }
-  for (int j = 0; j <= H; ++j) {
-    const double s = sinpi_r(j, M);
-    pre[2 * j] = s + 0.5;
-    pre[2 * j + 1] = s - 0.5;
-  }
-  for (int k = 0; k <= H / 2; ++k) {
-    spl[2 * k] = sinpi_r(4L * k + M, 2L * M);
-    spl[2 * k + 1] = sinpi_r(2L * k, M);
-  }
-  qgw::fill_pass_twiddles(qgw::make_geom(M), tw, spl + 2 * (H / 2 + 1));
+  qgw::fill_fx_tables(qgw::make_geom(M), (qgw::Q4*)dst, (qgw::Q4*)(dst + kTwq), (qgw::Q2*)(dst + kTwq + kSpq));
+}
+qgw::FxTables tables_at(const double* p) {
+  return qgw::FxTables{(const qgw::Q4*)p, (const qgw::Q2*)(p + kTwq + kSpq), (const qgw::Q4*)(p + kTwq)};
 }
 
 // a grid size of a closed basin the transforms take (the run path's rule:
@@ -214,15 +192,8 @@ extern "C" int qgw_invert_pv_noalloc(const qgw_params* p, const double* cl2m, co
   a.lstride = lstride;
   a.gx = qgw::make_geom(nx + 1);
   a.gy = qgw::make_geom(ny + 1);
-  const int Hx = (nx + 1) / 2, Hy = (ny + 1) / 2;
-  a.tx.tw = (const qgw::C2<double>*)(base + oTx);
-  a.tx.pre = (const qgw::C2<double>*)(base + oTx + 2 * Hx);
-  a.tx.spl = (const qgw::C2<double>*)(base + oTx + 2 * Hx + 2 * (Hx + 1));
-  a.tx.twp = (const qgw::C2<double>*)(base + oTx + 2 * Hx + 2 * (Hx + 1) + 2 * (Hx / 2 + 1));
-  a.ty.tw = (const qgw::C2<double>*)(base + oTy);
-  a.ty.pre = (const qgw::C2<double>*)(base + oTy + 2 * Hy);
-  a.ty.spl = (const qgw::C2<double>*)(base + oTy + 2 * Hy + 2 * (Hy + 1));
-  a.ty.twp = (const qgw::C2<double>*)(base + oTy + 2 * Hy + 2 * (Hy + 1) + 2 * (Hy / 2 + 1));
+  a.fx = tables_at(base + oTx);
+  a.fy = tables_at(base + oTy);
   a.cl2m = base + oCl;
   a.cm2l = base + oCm;
   a.iRd2 = base + oIrd;

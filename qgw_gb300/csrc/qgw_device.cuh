@@ -23,6 +23,7 @@
 #include <stdint.h>
 
 #include "dst_core.h"
+#include "dst_fx.h"
 #include "glibc_rand.h"
 
 namespace qgw {
@@ -83,6 +84,7 @@ template <typename T> struct StepArgs {
   long long lstride;               // ny * pitch
   DstGeom gx, gy;
   DstTables<T> tx, ty;
+  FxTables fx, fy;                 // FP64 closed basins: the fixed-point transforms' tables
   // vertical modes (FP64 master copies and T copies)
   const T* cl2m;                   // nl*nl row-major, mode m row: cl2m[m*nl+l]
   const T* cm2l;                   // cm2l[l*nl+m]

@@ -30,6 +30,7 @@
 
 #include "dst_blue.h"
 #include "dst_fixed.cuh"
+#include "dst_fx.cuh"
 #include "periodic.cuh"
 #include "kernels.h"
 #include "qgw_device.cuh"
@@ -127,10 +128,11 @@ __device__ __forceinline__ T* dst_block_blue(T* A, T* B, int nrows, int ld, cons
   return out;
 }
 
-// Block DST of any supported length: the power-of-two lengths M = 128..2048
-// use the compile-time specialisations of dst_fixed.cuh (FP32 M = 512 and
-// 1024: one warp per row, in place, the result in A), others (mixed radix
-// 2, 3, 5, 7) the generic loops.
+// Block DST of FP32 rows of any supported length, and the chirp-z form of
+// both precisions (FP64 rows of the other lengths: dst_fx).  The power-of-two
+// lengths M = 128..2048 use the compile-time specialisations of
+// dst_fixed.cuh (M = 512 and 1024: one warp per row, in place, the result in
+// A), others (mixed radix 2, 3, 5, 7) the generic loops.
 // HL != 0: a kernel specialised for half-length HL (its launcher checked the
 // run's length), whose code then holds that transform alone -- the step
 // kernels of the common lengths keep their instruction stream small; HL = -1:
@@ -138,22 +140,35 @@ __device__ __forceinline__ T* dst_block_blue(T* A, T* B, int nrows, int ld, cons
 template <typename T, int HL = 0>
 __device__ __forceinline__ T* dst_block(T* A, T* B, int nrows, int ld, const DstGeom& g, const DstTables<T>& tb,
                                         T* tot) {
-  if constexpr (HL == 512) {
-    if constexpr (sizeof(T) == 4) return dst_block_warp_f32<9>(A, nrows, ld, tb);
-    else return dst_block_fixed<T, 9>(A, B, nrows, ld, tb);
+  if constexpr (HL == -1) {
+    return dst_block_blue<T>(A, B, nrows, ld, g, tb);
+  } else if constexpr (sizeof(T) == 8) {
+    return A;
+  } else if constexpr (HL == 512) {
+    return dst_block_warp_f32<9>(A, nrows, ld, tb);
+  } else {
+    switch (g.H) {
+      case 64: return dst_block_fixed<T, 6>(A, B, nrows, ld, tb);
+      case 128: return dst_block_fixed<T, 7>(A, B, nrows, ld, tb);
+      case 256: return dst_block_warp_f32<8>(A, nrows, ld, tb);
+      case 512: return dst_block_warp_f32<9>(A, nrows, ld, tb);
+      case 1024: return dst_block_fixed<T, 10>(A, B, nrows, ld, tb);
+      default: return dst_block_generic<T>(A, B, nrows, ld, g, tb, tot);
+    }
   }
-  if constexpr (HL == -1) return dst_block_blue<T>(A, B, nrows, ld, g, tb);
-  switch (g.H) {
-    case 64: return dst_block_fixed<T, 6>(A, B, nrows, ld, tb);
-    case 128: return dst_block_fixed<T, 7>(A, B, nrows, ld, tb);
-    case 256:
-      if constexpr (sizeof(T) == 4) return dst_block_warp_f32<8>(A, nrows, ld, tb);
-      else return dst_block_fixed<T, 8>(A, B, nrows, ld, tb);
-    case 512:
-      if constexpr (sizeof(T) == 4) return dst_block_warp_f32<9>(A, nrows, ld, tb);
-      else return dst_block_fixed<T, 9>(A, B, nrows, ld, tb);
-    case 1024: return dst_block_fixed<T, 10>(A, B, nrows, ld, tb);
-    default: return dst_block_generic<T>(A, B, nrows, ld, g, tb, tot);
+}
+
+// The FP64 closed-basin transforms other than the chirp-z ones run in fixed
+// point (dst_fx.cuh); the block's scratch for them lies in tot.
+template <typename T, bool PER, int HL> constexpr bool fx_path = sizeof(T) == 8 && !PER && HL != -1;
+static_assert(2 * sizeof(FxScratch) <= sizeof(double) * GMAX * 32 && GMAX <= FX_ROWS && NT == FX_NT, "tot holds two");
+// the largest high words of the rows this thread and its warp have written
+// to A (x_{i+1} at index i + 1, i = threadIdx.x, + NT, ...)
+__device__ __forceinline__ void fx_note_rows(FxScratch* sc, const double* A, int nrows, int ld, int nx) {
+  for (int g = 0; g < nrows; ++g) {
+    unsigned int m = 0;
+    for (int i = threadIdx.x; i < nx; i += NT) m = max(m, fx_hi(A[g * ld + pr<double>(i + 1)]));
+    fx_note_max(sc, g, m);
   }
 }
 
@@ -462,6 +477,8 @@ __device__ __forceinline__ void project_fwd(const StepArgs<T>& a, int j, bool up
 template <typename T, bool COMP, bool PER, int HL = 0>
 __device__ __forceinline__ void body_rows_fwd(const StepArgs<T>& a, int step_mode, int j, unsigned char* smem_raw,
                                               T* tot, T* cst) {
+  constexpr bool FX = fx_path<T, PER, HL>;
+  FxScratch* sc = (FxScratch*)tot;
   DevState* st = a.state;
   if (step_mode && !st->active) return;
   const int ld = row_len<T>(a.gx);
@@ -479,7 +496,7 @@ __device__ __forceinline__ void body_rows_fwd(const StepArgs<T>& a, int step_mod
   // FP32 groups of 9..12 modes run at width 12 (three 16-byte coefficient
   // vectors), the common 10-layer case without six idle accumulators
   const int GB = (sizeof(T) == 4 && a.G1 > 8 && a.G1 <= 12) ? 12 : group_width(a.G1);
-  if (!PER) prefetch_tables_l1(a.tx, a.gx.M);
+  if (!PER && !FX) prefetch_tables_l1(a.tx, a.gx.M);
   const T* frow = (ab3 && a.fr.on) ? a.fr.field + (size_t)j * a.pitch : nullptr;
   const T sqdt = frow ? (T)sqrt(st->dt) : T(0);
   const T* r1 = nullptr;
@@ -499,6 +516,7 @@ __device__ __forceinline__ void body_rows_fwd(const StepArgs<T>& a, int step_mod
   for (int gi = 0, m0 = 0; gi < ng; m0 += gq + (gi < gr), ++gi) {
     const int G = gq + (gi < gr);
     const bool upd = ab3 && m0 == 0;
+    if constexpr (FX) fx_clear(sc);
     for (int w = tid; w < a.nl * GMAX; w += NT) {
       const int l = w / GMAX, g = w - l * GMAX;
       cst[w] = g < G ? a.cl2m[(size_t)(m0 + g) * a.nl + l] : T(0);
@@ -533,6 +551,18 @@ __device__ __forceinline__ void body_rows_fwd(const StepArgs<T>& a, int step_mod
     }
 #undef QGW_PF_GB
 #undef QGW_PF
+    if constexpr (FX) {
+      fx_note_rows(sc, A, G, ld, a.nx);
+      __syncthreads();
+      const fx_t* O = dst_fx<HL>(A, B, G, ld, a.gx, a.fx, sc);
+      for (int gg = 0; gg < G; ++gg) {
+        T* dstrow = a.spec + (size_t)(m0 + gg) * a.lstride + (size_t)j * a.pitch;
+        const int ex = sc->ex[gg];
+        for (int i = threadIdx.x; i < a.nx; i += NT) dstrow[i] = fx_out(O[gg * ld + pr<T>(i + 1)], ex);
+      }
+      __syncthreads();
+      continue;
+    }
     __syncthreads();
     T* O = PER ? rfft_block<T>(A, B, G, ld, a.gx, a.tx) : dst_block<T, HL>(A, B, G, ld, a.gx, a.tx, tot);
     // spectral row: the real FFT's X_0..X_H as (re, im) pairs from index 0,
@@ -591,6 +621,58 @@ __device__ __forceinline__ void store_cols(T* __restrict__ dst, const T* v) {
   }
 }
 
+// The rest of body_cols in fixed point: forward DST of the tile in A, the
+// Helmholtz factors in FP64 (the one FP64 operation per point; the outputs
+// go back to doubles anyway, since a column's new scale is not known before
+// its largest product), inverse DST, store.  sc[0]'s largest high words are
+// noted and the block is synchronised.
+template <int CT, int HL>
+__device__ __forceinline__ void body_cols_fx(const StepArgs<double>& a, int k0, int CTb, int m, double* A, double* B,
+                                             int ld, bool vec, FxScratch* sc) {
+  const int ny = a.ny;
+  fx_t* O = dst_fx<HL>(A, B, CT, ld, a.gy, a.fy, &sc[0]);
+  unsigned int hmax[CT];
+  int ex[CT];
+#pragma unroll
+  for (int c = 0; c < CT; ++c) {
+    hmax[c] = 0;
+    ex[c] = sc[0].ex[c];
+  }
+  for (int jj = (int)threadIdx.x - 1; jj < ny; jj += NT) {
+    if (jj < 0) continue;
+    const double* hrow = a.hinv + (size_t)m * a.lstride + (size_t)jj * a.pitch + k0;
+    double h[CT];
+    if (vec) load_cols<double, CT>(hrow, h);
+    else
+      for (int c = 0; c < CT; ++c) h[c] = c < CTb ? hrow[c] : 0.0;
+    const int pj = pr<double>(jj + 1);
+#pragma unroll
+    for (int c = 0; c < CT; ++c) {
+      const double x = fx_out(O[c * ld + pj], ex[c]) * h[c];
+      O[c * ld + pj] = __double_as_longlong(x);
+      hmax[c] = max(hmax[c], fx_hi(x));
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < CT; ++c) fx_note_max(&sc[1], c, hmax[c]);
+  __syncthreads();
+  fx_t* Oth = O == (fx_t*)A ? (fx_t*)B : (fx_t*)A;
+  const fx_t* O2 = dst_fx<HL>((double*)O, (double*)Oth, CT, ld, a.gy, a.fy, &sc[1]);
+#pragma unroll
+  for (int c = 0; c < CT; ++c) ex[c] = sc[1].ex[c];
+  for (int jj = (int)threadIdx.x - 1; jj < ny; jj += NT) {
+    if (jj < 0) continue;
+    const int pj = pr<double>(jj + 1);
+    double v[CT];
+#pragma unroll
+    for (int c = 0; c < CT; ++c) v[c] = c < CTb ? fx_out(O2[c * ld + pj], ex[c]) : 0.0;
+    double* dst = a.spec + (size_t)m * a.lstride + (size_t)jj * a.pitch + k0;
+    if (vec) store_cols<double, CT>(dst, v);
+    else
+      for (int c = 0; c < CTb; ++c) dst[c] = v[c];
+  }
+}
+
 template <typename T, bool COMP, int CT, int HL = 0>
 __device__ __forceinline__ void body_cols(const StepArgs<T>& a, int step_mode, int bx, int m, unsigned char* smem_raw,
                                           T* tot) {
@@ -609,7 +691,18 @@ __device__ __forceinline__ void body_cols(const StepArgs<T>& a, int step_mode, i
   T* B = A + (size_t)(zm ? 2 : 1) * CT * ld;
   T* S = a.spec + (size_t)m * a.lstride;
   const int ny = a.ny;
-  prefetch_tables_l1(a.ty, a.gy.M);
+  constexpr bool FX = fx_path<T, false, HL>;
+  FxScratch* sc = (FxScratch*)tot;  // [0] the forward, [1] the inverse transform's
+  unsigned int hmax[FX ? CT : 1];
+  if constexpr (FX) {
+    fx_clear(&sc[0]);
+    fx_clear(&sc[1]);
+#pragma unroll
+    for (int c = 0; c < CT; ++c) hmax[c] = 0;
+    __syncthreads();
+  } else {
+    prefetch_tables_l1(a.ty, a.gy.M);
+  }
   // 16-byte vectors need 16-byte aligned rows (vec_cols); the last tile then
   // reads the padding column (index nx < pitch), never past the row.  RB
   // rows per pass, all their loads in flight before any store (two 32-byte
@@ -644,11 +737,22 @@ __device__ __forceinline__ void body_cols(const StepArgs<T>& a, int step_mode, i
       if (jj >= 0 && jj < ny) {
         const int pj = pr<T>(jj + 1);
 #pragma unroll
-        for (int c = 0; c < CT; ++c) A[c * ld + pj] = vv[u][c];
+        for (int c = 0; c < CT; ++c) {
+          A[c * ld + pj] = vv[u][c];
+          if constexpr (FX) hmax[c] = max(hmax[c], fx_hi(vv[u][c]));
+        }
       }
     }
   }
+  if constexpr (FX) {
+#pragma unroll
+    for (int c = 0; c < CT; ++c) fx_note_max(&sc[0], c, hmax[c]);
+  }
   __syncthreads();
+  if constexpr (FX) {
+    body_cols_fx<CT, HL>(a, k0, CTb, m, A, B, ld, vec, sc);
+    return;
+  }
   T* O = dst_block<T, HL>(A, B, CT, ld, a.gy, a.ty, tot);
   T* C = O + (size_t)CT * ld;  // the second field's rows (zeta mode)
   const double iRd2 = a.iRd2[m];
@@ -920,6 +1024,8 @@ __device__ __forceinline__ void project_spec(const StepArgs<T>& a, int j, int G,
 template <typename T, bool COMP, bool PER, int HL = 0>
 __device__ __forceinline__ void body_rows_inv(const StepArgs<T>& a, int step_mode, int j, unsigned char* smem_raw,
                                               T* tot, T* cst, int only = -1) {
+  constexpr bool FX = fx_path<T, PER, HL>;
+  FxScratch* sc = (FxScratch*)tot;
   DevState* st = a.state;
   if (step_mode && !st->active) return;
   const int ld = row_len<T>(a.gx);
@@ -928,7 +1034,7 @@ __device__ __forceinline__ void body_rows_inv(const StepArgs<T>& a, int step_mod
   T* A = (T*)smem_raw;
   T* B = A + (size_t)(zm ? 2 * Gb : Gb) * ld;
   const int GB = group_width(Gb);
-  if (!PER) prefetch_tables_l1(a.tx, a.gx.M);
+  if (!PER && !FX) prefetch_tables_l1(a.tx, a.gx.M);
   // ceil(nl / Gb) layer groups of balanced sizes (at most Gb each)
   const int ng = (a.nl + Gb - 1) / Gb, gq = a.nl / ng, gr = a.nl - gq * ng;
   const int g_begin = only < 0 ? 0 : only, g_end = only < 0 ? ng : min(only + 1, ng);
@@ -938,6 +1044,7 @@ __device__ __forceinline__ void body_rows_inv(const StepArgs<T>& a, int step_mod
       const int m = w / GMAX, g = w - m * GMAX;
       cst[w] = g < G ? a.cm2l[(size_t)(l0 + g) * a.nl + m] : T(0);
     }
+    if constexpr (FX) fx_clear(sc);
     __syncthreads();
     const int ncols = PER ? a.nx + 2 : a.nx, xo = PER ? 0 : 1;
     if (zm) {
@@ -955,6 +1062,18 @@ __device__ __forceinline__ void body_rows_inv(const StepArgs<T>& a, int step_mod
         case 8: project_spec<T, false, 8>(a, j, G, A, ld, cst, ncols, xo); break;
         default: project_spec<T, false, 16>(a, j, G, A, ld, cst, ncols, xo); break;
       }
+    }
+    if constexpr (FX) {
+      fx_note_rows(sc, A, G, ld, a.nx);
+      __syncthreads();
+      const fx_t* O = dst_fx<HL>(A, B, G, ld, a.gx, a.fx, sc);
+      for (int g = 0; g < G; ++g) {
+        T* prow = a.psi + (size_t)(l0 + g) * a.lstride + (size_t)j * a.pitch;
+        const int ex = sc->ex[g];
+        for (int i = threadIdx.x; i < a.nx; i += NT) prow[i] = fx_out(O[g * ld + pr<T>(i + 1)], ex);
+      }
+      __syncthreads();
+      continue;
     }
     __syncthreads();
     const int nrow = zm ? 2 * G : G;

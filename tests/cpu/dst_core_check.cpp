@@ -124,6 +124,85 @@ static void run_warp(int howmany, float* data) {
 }
 
 // the one-warp transform for M = 512 and 1024; returns 0 for other lengths
+// The fixed-point transform (dst_fx.h): raw doubles in, doubles out.
+static void run_fx(int M, int howmany, double* data) {
+  DstGeom g = make_geom(M);
+  FxTablesHost fx = build_fx_tables(g);
+  const int L = padded_len<double>(M), H = g.H;
+  std::vector<fx_t> A(L), B(L);
+  for (int r = 0; r < howmany; ++r) {
+    double* x = data + (size_t)r * (M - 1);
+    for (int j = 0; j < L; ++j) A[j] = B[j] = 777;  // pad slots must never be read
+    unsigned int mx = 0;
+    for (int j = 1; j < M; ++j) {
+      std::memcpy(&A[pr<double>(j)], &x[j - 1], 8);
+      const unsigned int h = (unsigned int)((unsigned long long)A[pr<double>(j)] >> 32) & 0x7fffffffu;
+      mx = h > mx ? h : mx;
+    }
+    const int E = fx_scale(mx);
+    unsigned int l1 = 0;
+    for (int j = 1; j <= H; ++j)
+      l1 += fx_pre_item((const unsigned long long*)A.data(), B.data(), j, M, E, fx.nsj.data());
+    C2<fx_t>* src = (C2<fx_t>*)B.data();
+    C2<fx_t>* dst = (C2<fx_t>*)A.data();
+    int Ns = 1, drop = 0;
+    unsigned int mag = 0;
+    for (int p = 0; p < g.npass; ++p) {
+      const int R = g.radix[p], s = p ? fx_pass_shift(mag) : 0;
+      if (p) drop += 2 - s;
+      mag = 0;
+      for (int b = 0; b < H / R; ++b)
+        mag |= fx_stockham_dispatch(R, src, dst, b, b % Ns, Ns, H, s, fx.twq.data() + (p ? Ns - g.radix[0] : 0));
+      Ns *= R;
+      C2<fx_t>* t = src; src = dst; dst = t;
+    }
+    const int s = fx_split_shift(mag, l1, drop), e = fx_row_exp(mx, drop, s);
+    for (int k = 0; k <= H / 2; ++k) fx_split_item(src, dst, k, H, s, fx.spq.data());
+    fx_t* o = (fx_t*)dst;
+    for (int k = 1; k < H; ++k) o[pr<double>(2 * k + 1)] += o[pr<double>(2 * k - 1)];
+    for (int j = 1; j < M; ++j) {
+      const fx_t v = o[pr<double>(j)];
+      if (e == FX_NAN) x[j - 1] = std::nan("");
+      else if (fx_exp_ok(e)) { const unsigned long long b = fx_to_bits(v, e); std::memcpy(&x[j - 1], &b, 8); }
+      else x[j - 1] = std::ldexp((double)v, e);
+    }
+  }
+}
+// DST-I by its definition in long double (at least 64 bits), one row
+static void run_exact(int M, const double* x, long double* y) {
+  std::vector<long double> s(2 * (size_t)M);
+  const long double pi = 3.14159265358979323846264338327950288L;
+  for (int m = 0; m < 2 * M; ++m) {
+    int r = m % M;
+    if (2 * r > M) r = M - r;
+    s[m] = (m < M ? 1 : -1) * sinl(pi * r / M);
+  }
+  for (int k = 1; k < M; ++k) {
+    long double t = 0;
+    for (int j = 1; j < M; ++j) t += x[j - 1] * s[(long)j * k % (2 * M)];
+    y[k - 1] = 2 * t;
+  }
+}
+
+// relative errors (2-norm, in units of 2^-53) of the FP64 and the fixed-point
+// transform of one row
+extern "C" void dst_fx_errors(int M, const double* x, double* err) {
+  std::vector<long double> e(M - 1);
+  run_exact(M, x, e.data());
+  for (int f = 0; f < 2; ++f) {
+    std::vector<double> y(x, x + M - 1);
+    if (f) run_fx(M, 1, y.data());
+    else run<double>(M, 1, y.data());
+    long double d = 0, n = 0;
+    for (int k = 0; k < M - 1; ++k) {
+      d += (y[k] - e[k]) * (y[k] - e[k]);
+      n += e[k] * e[k];
+    }
+    err[f] = (double)(sqrtl(d / n) * 9007199254740992.0L);
+  }
+}
+extern "C" void dst_fx_run(int M, int howmany, double* data) { run_fx(M, howmany, data); }
+
 extern "C" int dst_warp_run_f32(int M, int howmany, float* data) {
   if (M == 512) run_warp<8>(howmany, data);
   else if (M == 1024) run_warp<9>(howmany, data);

@@ -19,7 +19,7 @@ namespace qgw {
 
 constexpr int FX_NT = 256;    // threads per block
 constexpr int FX_ROWS = 16;   // rows of one batched transform, at most
-constexpr int FX_PASSES = 12; // Stockham passes, at most (DstGeom::radix)
+constexpr int FX_PASSES = 8;  // Stockham passes, at most (H <= 4096: 2 3^6)
 
 struct FxScratch {
   unsigned int mx[FX_ROWS];               // largest |x|'s high word

@@ -19,7 +19,7 @@ namespace qgw {
 template <typename T, bool COMP, bool PER, int HL>
 __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) k_rows_fwd(StepArgs<T> a, int step_mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ T tot[GMAX * 32];
+  __shared__ __align__(16) T tot[tot_len<T, PER, HL>];
   body_rows_fwd<T, COMP, PER, HL>(a, step_mode, blockIdx.x, smem_raw + cst_bytes<T>(a.nl), tot, (T*)smem_raw);
 }
 // CT: columns per tile (closed basin; the periodic kernel takes two complex
@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) k_rows_fwd(StepArg
 template <typename T, bool COMP, bool PER, int CT, int HL>
 __global__ void __launch_bounds__(NT, 3) k_cols(StepArgs<T> a, int step_mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ T tot[GMAX * 32];
+  __shared__ __align__(16) T tot[tot_len<T, PER, HL>];
   if (PER) body_cols_per<T, COMP>(a, step_mode, blockIdx.x, blockIdx.y, smem_raw);
   else body_cols<T, COMP, CT, HL>(a, step_mode, blockIdx.x, blockIdx.y, smem_raw, tot);
 }
@@ -37,7 +37,7 @@ template <typename T> constexpr int CTD = ColsPer<T>::value;
 template <typename T, bool COMP, bool PER, int HL>
 __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) k_rows_inv(StepArgs<T> a, int step_mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ T tot[GMAX * 32];
+  __shared__ __align__(16) T tot[tot_len<T, PER, HL>];
   body_rows_inv<T, COMP, PER, HL>(a, step_mode, blockIdx.x, smem_raw + cst_bytes<T>(a.nl), tot, (T*)smem_raw,
                                   gridDim.y > 1 ? (int)blockIdx.y : -1);
 }

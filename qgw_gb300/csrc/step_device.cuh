@@ -161,7 +161,12 @@ __device__ __forceinline__ T* dst_block(T* A, T* B, int nrows, int ld, const Dst
 // The FP64 closed-basin transforms other than the chirp-z ones run in fixed
 // point (dst_fx.cuh); the block's scratch for them lies in tot.
 template <typename T, bool PER, int HL> constexpr bool fx_path = sizeof(T) == 8 && !PER && HL != -1;
-static_assert(2 * sizeof(FxScratch) <= sizeof(double) * GMAX * 32 && GMAX <= FX_ROWS && NT == FX_NT, "tot holds two");
+// values of tot: two scratches (the column kernel's two transforms), which
+// leaves room for a third 1024-point column block per SM, or the chunk totals
+// of the generic transform
+template <typename T, bool PER, int HL>
+constexpr int tot_len = fx_path<T, PER, HL> ? (int)(2 * sizeof(FxScratch) / sizeof(T)) : GMAX * 32;
+static_assert(GMAX <= FX_ROWS && NT == FX_NT, "a scratch holds every row");
 // the largest high words of the rows this thread and its warp have written
 // to A (x_{i+1} at index i + 1, i = threadIdx.x, + NT, ...)
 __device__ __forceinline__ void fx_note_rows(FxScratch* sc, const double* A, int nrows, int ld, int nx) {
@@ -1192,7 +1197,8 @@ template <typename T> __host__ __device__ constexpr int tile_round(int n) {
 // for FP64, the centred differences).  Every array starts 128-byte aligned.
 template <typename T, int R, int TY> struct RhsShape {
   static constexpr int HH = TY + 2 * R, QH = TY + 2, QW = TX + 2;
-  static constexpr int TS = tile_round<T>(TW * HH), QS = tile_round<T>(TW * QH), ZS = tile_round<T>(TW * (HH - 2));
+  static constexpr int TS = tile_round<T>(TW * HH), QS = tile_round<T>(TW * QH);
+  static constexpr int ZS = sizeof(T) == 4 ? tile_round<T>(TW * (HH - 2)) : 0;
   static constexpr int IS = TS + QS + ZS;  // one input buffer
   static constexpr int DIFFS = sizeof(T) == 8 ? tile_round<T>(2 * QW * TY + 2 * TX * QH) : 0;
   static constexpr int WS = 2 * TS + DIFFS;  // work buffers
@@ -1615,6 +1621,48 @@ __device__ __forceinline__ decltype(absbits_native(T(0))) rhs_tile_compute(const
   return mymax_n;
 }
 
+}  // namespace qgw
+#include "rhs_fx.cuh"
+namespace qgw {
+
+// the tile at (i0, j0) plus its psi halo R touches a wall (or wraps)
+__device__ __forceinline__ bool rhs_edge_tile(int i0, int j0, int R, int ty, int nx, int ny) {
+  return i0 < R || j0 < R || i0 + TX + R > nx || j0 + ty + R > ny;
+}
+
+// One RHS tile of TX x TY points whose inputs have arrived (the block is
+// synchronised since).  FP64: bands of TYF rows, each in fixed point where
+// rhs_fx_ok, else in FP64.
+template <typename T, bool COMP, int R, int TY>
+__device__ __forceinline__ decltype(absbits_native(T(0))) rhs_tile(const StepArgs<T>& a, int i0, int j0, int k,
+                                                                    int step_index, const RhsIn<T>& in, T* wk) {
+  if constexpr (sizeof(T) == 8) {
+    unsigned long long m = 0;
+#pragma unroll 1
+    for (int b = 0; b < TY && j0 + b < a.ny; b += TYF) {
+      const bool edge = rhs_edge_tile(i0, j0 + b, R, TYF, a.nx, a.ny);
+      const RhsIn<T> band{in.ps + b * TW, in.qs + b * TW, nullptr};
+      if (b > 0) __syncthreads();
+      unsigned long long v;
+      if (rhs_fx_ok(a, edge, k))
+        v = edge ? rhs_tile_fx<R, true>(a, i0, j0 + b, k, step_index, band, wk)
+                 : rhs_tile_fx<R, false>(a, i0, j0 + b, k, step_index, band, wk);
+      else
+        v = edge ? rhs_tile_compute<T, COMP, R, TYF, true>(a, i0, j0 + b, k, step_index, band, wk)
+                 : rhs_tile_compute<T, COMP, R, TYF, false>(a, i0, j0 + b, k, step_index, band, wk);
+      m = v > m ? v : m;
+    }
+    return m;
+  } else {
+    const bool edge = rhs_edge_tile(i0, j0, R, TY, a.nx, a.ny);
+    // interior tiles of zeta mode 1 with R sweeps run the compile-time form
+    const bool z1 = COMP && a.zeta_mode == 1 && a.nsweep == R;
+    return edge ? rhs_tile_compute<T, COMP, R, TY, true>(a, i0, j0, k, step_index, in, wk)
+           : z1 ? rhs_tile_compute<T, COMP, R, TY, false, true>(a, i0, j0, k, step_index, in, wk)
+                : rhs_tile_compute<T, COMP, R, TY, false>(a, i0, j0, k, step_index, in, wk);
+  }
+}
+
 // End of a block's RHS work: the block's CFL maximum joins the run's
 // (atomicMax on the bits), and the last of `total` blocks to finish runs
 // the time-step update (adjust_timestep, src/timestep.h:74-87).
@@ -1642,11 +1690,6 @@ __device__ __forceinline__ void rhs_block_done(DevState* st, unsigned long long 
     __threadfence();
     scalar_update(st, Delta, cfl);
   }
-}
-
-// the tile at (i0, j0) plus its psi halo R touches a wall (or wraps)
-__device__ __forceinline__ bool rhs_edge_tile(int i0, int j0, int R, int ty, int nx, int ny) {
-  return i0 < R || j0 < R || i0 + TX + R > nx || j0 + ty + R > ny;
 }
 
 // The RHS stage of one run: tiles t = blockIdx.x, blockIdx.x + gridDim.x,
@@ -1704,9 +1747,6 @@ __device__ __forceinline__ void body_rhs_tiles(const StepArgs<T>& a, int ntx, in
     for (int p = 0; p < NB - 1; ++p, c = advance(c))
       if ((int)blockIdx.x + p * step < ntiles) issue(c, p);
   }
-  // interior tiles of the compensated path's zeta mode 1 with R sweeps run
-  // the compile-time form
-  const bool z1 = COMP && a.zeta_mode == 1 && a.nsweep == R;
   decltype(absbits_native(T(0))) mymax = 0;
   int it = 0;
   for (int t = (int)blockIdx.x; t < ntiles; t += step, ++it, cur_c = advance(cur_c)) {
@@ -1735,9 +1775,7 @@ __device__ __forceinline__ void body_rhs_tiles(const StepArgs<T>& a, int ntx, in
     }
     __syncthreads();
     if (ok) {
-      const auto m = edge ? rhs_tile_compute<T, COMP, R, TY, true>(a, i0, j0, k, si, in, wk)
-                     : z1 ? rhs_tile_compute<T, COMP, R, TY, false, true>(a, i0, j0, k, si, in, wk)
-                          : rhs_tile_compute<T, COMP, R, TY, false>(a, i0, j0, k, si, in, wk);
+      const auto m = rhs_tile<T, COMP, R, TY>(a, i0, j0, k, si, in, wk);
       mymax = m > mymax ? m : mymax;
     }
     __syncthreads();
@@ -1771,8 +1809,7 @@ __device__ __forceinline__ void body_rhs(const StepArgs<T>& a, int bx, int by, i
   __syncthreads();
   decltype(absbits_native(T(0))) mymax = 0;
   if (ok) {
-    mymax = edge ? rhs_tile_compute<T, COMP, R, TY, true>(a, i0, j0, k, si, in, wk)
-                 : rhs_tile_compute<T, COMP, R, TY, false>(a, i0, j0, k, si, in, wk);
+    mymax = rhs_tile<T, COMP, R, TY>(a, i0, j0, k, si, in, wk);
   }
   rhs_block_done(st, widen_absbits<T>(mymax), total, a.Delta, a.cfl);
 }

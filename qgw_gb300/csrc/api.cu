@@ -65,20 +65,18 @@ int upload(qgw_run* r, T** out, const std::vector<double>& host) {
   return cudaStreamSynchronize(r->stream) == cudaSuccess ? QGW_OK : QGW_ERR_CUDA;
 }
 
-int upload_fx(qgw_run* r, qgw::FxTables* out, const qgw::FxTablesHost& h) {
-  auto put = [&](auto** dst, const auto& v) -> int {
-    int rc = dalloc(r, dst, v.size());
-    if (rc) return rc;
-    CK(cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, r->stream));
-    return QGW_OK;
-  };
-  qgw::Q4 *tw, *sp;
-  qgw::Q2* sj;
-  int rc;
-  if ((rc = put(&tw, h.twq)) || (rc = put(&sp, h.spq)) || (rc = put(&sj, h.nsj))) return rc;
-  out->twq = tw;
-  out->spq = sp;
-  out->nsj = sj;
+// the fixed-point transform's tables in one allocation (twq | spq | nsj)
+int upload_fx(qgw_run* r, qgw::FxTables* out, const qgw::DstGeom& g) {
+  const size_t ntw = qgw::fx_twq_len(g), nsp = (size_t)g.H / 2 + 1, nsj = ((size_t)g.H + 2) / 2;
+  std::vector<qgw::Q4> h(ntw + nsp + nsj);
+  qgw::fill_fx_tables(g, h.data(), h.data() + ntw, (qgw::Q2*)(h.data() + ntw + nsp));
+  qgw::Q4* d;
+  int rc = dalloc(r, &d, h.size());
+  if (rc) return rc;
+  CK(cudaMemcpyAsync(d, h.data(), h.size() * sizeof(h[0]), cudaMemcpyHostToDevice, r->stream));
+  out->twq = d;
+  out->spq = d + ntw;
+  out->nsj = (const qgw::Q2*)(d + ntw + nsp);
   return cudaStreamSynchronize(r->stream) == cudaSuccess ? QGW_OK : QGW_ERR_CUDA;
 }
 
@@ -226,6 +224,12 @@ int setup_args(qgw_run* r, StepArgs<T>& a) {
   // transform tables for x and y
   for (int dim = 0; dim < 2; ++dim) {
     const qgw::DstGeom& g = dim == 0 ? a.gx : a.gy;
+    qgw::FxTables& f = dim == 0 ? a.fx : a.fy;
+    f = qgw::FxTables{};
+    if (sizeof(T) == 8 && !per && !g.blue) {
+      if ((rc = upload_fx(r, &f, g))) return rc;
+      continue;
+    }
     // the chirp-z form's FFT is L = g.H points: its tables are those of a
     // half-length FFT of L (the DST tables of 2L), plus the chirp tables
     qgw::DstTablesHost th = qgw::build_dst_tables(g.blue ? 2 * g.H : g.M);
@@ -251,9 +255,6 @@ int setup_args(qgw_run* r, StepArgs<T>& a) {
     t.sjp = (const qgw::C2<T>*)sjp;
     t.bc = (const qgw::C2<T>*)bc;
     t.bz = (const qgw::C2<T>*)bz;
-    qgw::FxTables& f = dim == 0 ? a.fx : a.fy;
-    f = qgw::FxTables{};
-    if (sizeof(T) == 8 && !per && !g.blue && (rc = upload_fx(r, &f, qgw::build_fx_tables(g)))) return rc;
   }
   T *cl, *cm;
   if ((rc = upload<T>(r, &cl, r->cl2m))) return rc;

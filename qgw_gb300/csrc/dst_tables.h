@@ -84,20 +84,21 @@ inline DstTablesHost build_dst_tables(int M) {
   return t;
 }
 
-// sin and cos of pi m / N by their Taylor series in 64-bit fixed point, N up
-// to 2^14, to 2^-61: the fixed-point transform (dst_fx.h) rounds at 2^-57, so
-// it would feel the rounding of a double.
-inline void sincospi_fixed(long m, long N, long double* sn, long double* cs) {
+// cos and -sin of pi m / N scaled by 2^b, b = 62 or 63, N up to 2^14, by
+// their Taylor series in 64-bit fixed point to 2^-61: the fixed-point
+// transform (dst_fx.h) rounds at 2^-57, so it would feel the rounding of a
+// double.  At b = 63 a value of +1 does not fit (no table holds one).
+inline Q4 sincospi_fixed(long m, long N, int b) {
   typedef unsigned long long u64;
-  auto hi = [](u64 a, u64 b) { return (u64)(((unsigned __int128)a * b) >> 64); };
+  auto hi = [](u64 a, u64 c) { return (u64)(((unsigned __int128)a * c) >> 64); };
   long r = m % (2 * N);
   if (r < 0) r += 2 * N;
-  const int half = r >= N;  // sign of both
+  const bool half = r >= N;  // both signs change
   if (half) r -= N;
-  const bool refl = 2 * r > N;  // cos changes sign
+  const bool refl = 2 * r > N;  // the cosine's changes
   if (refl) r = N - r;
   const bool swap = 4 * r > N;
-  const long a = swap ? N - 2 * r : 2 * r;  // angle pi a / (2 N), at most pi / 4
+  const long a = swap ? N - 2 * r : 2 * r;  // the angle is pi a / (2 N), at most pi / 4
   // pi / 4 in units of 2^-64, times 2 a / N <= 1
   const u64 pi4 = 0xC90FDAA22168C235ull;
   const u64 t = (u64)(((unsigned __int128)pi4 * (u64)(2 * a)) / (u64)N);
@@ -107,41 +108,33 @@ inline void sincospi_fixed(long m, long N, long double* sn, long double* cs) {
     s = ~0ull - hi(t2 / (u64)((2 * k) * (2 * k + 1)), s);
     c = ~0ull - hi(t2 / (u64)((2 * k - 1) * (2 * k)), c);
   }
-  long double S = (long double)hi(t, s), C = (long double)c;
-  S = a == 0 ? 0.0L : S / 18446744073709551616.0L;
-  C = a == 0 ? 1.0L : C / 18446744073709551616.0L;
+  s = hi(t, s);
+  // round from 2^-64 to 2^-b
+  const int n = 64 - b;
+  u64 S = a == 0 ? 0 : (s >> n) + ((s >> (n - 1)) & 1), C = a == 0 ? 1ull << b : (c >> n) + ((c >> (n - 1)) & 1);
   if (swap) std::swap(S, C);
-  *sn = half ? -S : S;
-  *cs = (half != refl) ? -C : C;
+  // two's complement negation carries 2^63 to the value -1 has
+  Q4 w;
+  w.x = q2_split((fx_t)(half != refl ? 0 - C : C));
+  w.y = q2_split((fx_t)(half ? S : 0 - S));
+  return w;
 }
 
 // The tables of the fixed-point transform (dst_fx.h) of geometry g, into
 // arrays of fx_twq_len, H/2 + 1 and H + 1 entries.
-inline Q2 fx_const(long double v, long double scale) { return q2_split((fx_t)std::nearbyintl(v * scale)); }
 inline size_t fx_twq_len(const DstGeom& g) { return (size_t)(g.npass ? g.H - g.radix[0] : 0) + 1; }
 inline void fill_fx_tables(const DstGeom& g, Q4* twq, Q4* spq, Q2* nsj) {
-  constexpr long double S62 = 4611686018427387904.0L, S63 = 9223372036854775808.0L;
   const int H = g.H, M = g.M;
-  long double s, c;
   int Ns = g.radix[0];
   for (int p = 1; p < g.npass; ++p) {
     const int R = g.radix[p];
     for (int q = 1; q < R; ++q)
-      for (int k = 0; k < Ns; ++k) {
-        sincospi_fixed(2L * q * k, (long)Ns * R, &s, &c);
-        twq[(Ns - g.radix[0]) + (q - 1) * Ns + k] = Q4{fx_const(c, S62), fx_const(-s, S62)};
-      }
+      for (int k = 0; k < Ns; ++k) twq[(Ns - g.radix[0]) + (q - 1) * Ns + k] = sincospi_fixed(2L * q * k, (long)Ns * R, 62);
     Ns *= R;
   }
   spq[0] = Q4{};
-  for (int k = 1; k <= H / 2; ++k) {
-    sincospi_fixed(2L * k, M, &s, &c);
-    spq[k] = Q4{fx_const(c, S63), fx_const(-s, S63)};
-  }
-  for (int j = 0; j <= H; ++j) {
-    sincospi_fixed(j, M, &s, &c);
-    nsj[j] = fx_const(-s, S63);
-  }
+  for (int k = 1; k <= H / 2; ++k) spq[k] = sincospi_fixed(2L * k, M, 63);
+  for (int j = 0; j <= H; ++j) nsj[j] = sincospi_fixed(j, M, 63).y;
 }
 struct FxTablesHost {
   std::vector<Q4> twq, spq;

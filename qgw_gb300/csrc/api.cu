@@ -80,22 +80,32 @@ int upload_fx(qgw_run* r, qgw::FxTables* out, const qgw::DstGeom& g) {
   return cudaStreamSynchronize(r->stream) == cudaSuccess ? QGW_OK : QGW_ERR_CUDA;
 }
 
-// choose the modes per row block and the columns per column block so that
-// each block's two work buffers stay within the shared-memory budget
-// Shared-memory budget of the row kernels' work buffers.  Measured at
-// 1024^2 x 10 on GB300: 64 KiB (3 blocks/SM) is fastest for FP64 and 40 KiB
-// (4-5 blocks/SM) for FP32; QGW_ROW_SMEM_KB overrides it (tuning knob).
-// Shared-memory budget of the work buffers of the forward rows kernel (K1):
-// 48 KiB (FP64) / 56 KiB (FP32), which keeps four blocks per SM, and 40 KiB
-// for FP32 rows of 2048 and more or more than 10 layers; measured at 512^2,
-// 1024^2 and 2048^2 with 10, 16 and 20 layers on GB300 (1024^2 x 16 FP32:
-// 0.254 -> 0.197 ms).  QGW_ROW_SMEM_KB overrides it.
+// a projection matrix in fixed point, in one allocation (c | e)
+int upload_modes(qgw_run* r, qgw::ModeTable* out, const std::vector<double>& mat) {
+  const size_t nc = (size_t)r->nl * r->nl;
+  std::vector<qgw::Q2> h(nc + ((size_t)r->nl + 1) / 2);
+  qgw::fill_mode_table(r->nl, mat.data(), h.data(), (int*)(h.data() + nc));
+  qgw::Q2* d;
+  int rc = dalloc(r, &d, h.size());
+  if (rc) return rc;
+  CK(cudaMemcpyAsync(d, h.data(), h.size() * sizeof(h[0]), cudaMemcpyHostToDevice, r->stream));
+  out->c = d;
+  out->e = (const int*)(d + nc);
+  return cudaStreamSynchronize(r->stream) == cudaSuccess ? QGW_OK : QGW_ERR_CUDA;
+}
+
+// Shared-memory budget of the row kernels' work buffers.  FP64: 74 KiB (three
+// blocks per SM; four rows of 1024).  FP32, the forward rows kernel: 56 KiB,
+// which keeps four blocks per SM, and 40 KiB for rows of 2048 and more or more
+// than 10 layers; measured at 512^2, 1024^2 and 2048^2 with 10, 16 and 20
+// layers on GB300 (1024^2 x 16: 0.254 -> 0.197 ms).  QGW_ROW_SMEM_KB
+// overrides it.
 size_t row_budget(size_t elem, int M, int nl) {
   const char* e = std::getenv("QGW_ROW_SMEM_KB");
   const long v = e ? std::atol(e) : 0;
   if (v >= 16 && v <= 220) return (size_t)v * 1024;
   if (elem == 4 && (M >= 2048 || nl > 10)) return (size_t)40 * 1024;
-  return (size_t)(elem == 8 ? 48 : 56) * 1024;
+  return (size_t)(elem == 8 ? 74 : 56) * 1024;
 }
 
 // Layers per block of the inverse rows kernel (K3): the measured optimum is
@@ -124,27 +134,6 @@ int mode_group(int nl, int M, size_t elem, size_t budget, int rows_per_mode, int
   if (g < 1) g = 1;
   const int ngroups = (nl + g - 1) / g;
   return (nl + ngroups - 1) / ngroups;
-}
-
-// The same for a kernel bound by its projection FMAs (the FP64 forward rows
-// kernel): each group's loop runs at the compile-time width GB = the power
-// of two at or above its size, so a group of 5 costs 8 FMAs per layer and
-// point, and each group costs about 1.5 such FMAs more in fixed work (its
-// pass over the layers, its barriers).  Among the sizes the budget allows,
-// take the one of least groups x (GB + 1.5), then the fewest groups
-// (fitted to GB300 sweeps of 256^2 and 512^2 x 5, 10, 20 layers: groups of
-// 4 for 10 and 20 layers, one group for 5; 512^2 x 20: 0.579 -> 0.461 ms).
-int mode_group_fma(int nl, int M, size_t elem, size_t budget, int gmax) {
-  const int gfit = mode_group(1 << 30, M, elem, budget, 1, gmax, gmax);  // largest size that fits
-  int best = 1, best_cost = 1 << 30, best_ng = 1 << 30;
-  for (int g = 1; g <= gfit; ++g) {
-    const int ng = (nl + g - 1) / g, s = (nl + ng - 1) / ng;
-    int gb = 1;
-    while (gb < s) gb <<= 1;
-    const int cost = ng * (2 * gb + 3);
-    if (cost < best_cost || (cost == best_cost && ng < best_ng)) { best = s; best_cost = cost; best_ng = ng; }
-  }
-  return best;
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no
@@ -256,6 +245,10 @@ int setup_args(qgw_run* r, StepArgs<T>& a) {
     t.bc = (const qgw::C2<T>*)bc;
     t.bz = (const qgw::C2<T>*)bz;
   }
+  if (sizeof(T) == 8) {
+    a.modes_fx = qgw::modes_fixed_ok(r->nl, r->cl2m.data()) && qgw::modes_fixed_ok(r->nl, r->cm2l.data());
+    if ((rc = upload_modes(r, &a.l2m, r->cl2m)) || (rc = upload_modes(r, &a.m2l, r->cm2l))) return rc;
+  }
   T *cl, *cm;
   if ((rc = upload<T>(r, &cl, r->cl2m))) return rc;
   if ((rc = upload<T>(r, &cm, r->cm2l))) return rc;
@@ -355,10 +348,16 @@ int setup_args(qgw_run* r, StepArgs<T>& a) {
     const int want = e ? std::atoi(e) : 0;
     const size_t budget = row_budget(sizeof(T), Mrow, r->nl);
     if (want >= 1 && want <= 16) a.G1 = mode_group(r->nl, Mrow, sizeof(T), budget, 1, 16, want, bufs_x);
-    else if (sizeof(T) == 8) a.G1 = mode_group_fma(r->nl, Mrow, sizeof(T), budget, 16);
     else a.G1 = mode_group(r->nl, Mrow, sizeof(T), budget, 1, 16, 16, bufs_x);
   }
   a.G3 = mode_group(r->nl, Mrow, sizeof(T), 110 * 1024, 1, 16, inv_group(0, Mrow, r->nl, bufs_x), bufs_x);
+  if (sizeof(T) == 8) {
+    // FP64 row kernels take rows of any layer: as many as the budget holds,
+    // but on small grids no more than leave every SM two blocks
+    a.G3 = a.G1;
+    const int fit = mode_group(1 << 20, Mrow, sizeof(T), row_budget(sizeof(T), Mrow, r->nl), 1, 16, 16);
+    a.RB1 = a.RB3 = std::max(1, std::min(fit, r->nl * r->ny / 304));
+  }
   a.CT = 0;
   a.low_k64 = 8;
   // 16-byte column vectors: rows 16-byte aligned and a whole number of
@@ -552,11 +551,13 @@ int set_shape(qgw_run* r, StepArgs<T>& a, const qgw_shape& sh) {
   if (sh.row_group_fwd) {
     if (sh.row_group_fwd < 1 || sh.row_group_fwd > 16) return QGW_ERR_PARAM;
     b.G1 = mode_group(r->nl, Mx, sizeof(T), any, 1, 16, sh.row_group_fwd, bufs_x);
+    b.RB1 = b.G1;
   }
   if (sh.row_group_inv) {
     if (sh.row_group_inv < 1 || sh.row_group_inv > 16) return QGW_ERR_PARAM;
     const bool zm = a.zeta_mode != 0;
     b.G3 = mode_group(r->nl, Mx, sizeof(T), any, zm ? 2 : 1, zm ? 8 : 16, sh.row_group_inv, bufs_x);
+    b.RB3 = b.G3;
   }
   if (b.rhs_ty != a.rhs_ty) encode_rhs_maps<T>(r, b);
   cudaError_t e;
@@ -760,7 +761,7 @@ void qgw_destroy(qgw_run* r) {
 }
 
 void* qgw_stream(qgw_run* r) { return r ? (void*)r->stream : nullptr; }
-int qgw_kernels_per_step(qgw_run* r) { return r ? 4 : 0; }
+int qgw_kernels_per_step(qgw_run* r) { return !r ? 0 : r->precision == QGW_FP64 ? 6 : 4; }
 
 static int reset_history(qgw_run* r) {
   const size_t field = (size_t)r->nl * r->lstride;

@@ -39,7 +39,9 @@ __device__ __forceinline__ void fx_note_max(FxScratch* sc, int row, unsigned int
   const unsigned int m = __reduce_max_sync(0xffffffffu, hi);
   if ((threadIdx.x & 31) == 0) atomicMax(&sc->mx[row], m);
 }
-// an output as a double; ex the row's exponent
+// an output as a double; ex the row's exponent.  (The hardware's 64-bit
+// conversion runs at the FP64 rate of two a clock and SM: no faster in the
+// transforms, and the RHS kernel went from 0.30 to 0.36 ms with it.)
 static __device__ __noinline__ double fx_out_far(fx_t v, int ex) {
   return ex == FX_NAN ? __longlong_as_double(0x7ff8000000000000ll) : ldexp((double)v, ex);
 }

@@ -47,6 +47,12 @@ QGW_HD Q2 q2_split(fx_t w) {
 // Tables: twq the pass twiddles (cos, -sin) scaled by 2^62, in the order of
 // fill_pass_twiddles; nsj -s_j scaled by 2^63, j <= H (s_H = 1 has no
 // positive 2^63); spq (cos, -sin)(2 pi k / M) scaled by 2^63, 1 <= k <= H/2.
+// A projection's constants (modes_fx.cuh): c = (h 2^32 + l) 2^(e - 60) < 2^e,
+// e per row of the matrix.
+struct ModeTable {
+  const Q2* c;   // nl x nl, row m: output m
+  const int* e;  // nl
+};
 struct FxTables {
   const Q4* twq;
   const Q2* nsj;
@@ -97,6 +103,7 @@ QGW_HD fx_t fx_shl(fx_t v, int s) { return (fx_t)((unsigned long long)v << s); }
 // sign, or the prefix sum would add M of them up
 QGW_HD fx_t fx_shr(fx_t v, int n) { return (v + ((((fx_t)1 << n) >> 1) - 1 + ((v >> n) & 1))) >> n; }
 QGW_HD fx_t fx_shift(fx_t v, int s) { return s >= 0 ? fx_shl(v, s > 63 ? 63 : s) : s < -62 ? 0 : fx_shr(v, -s); }
+QGW_HD fx_t fx_shr0(fx_t v, int n) { return n > 0 ? fx_shr(v, n) : v; }
 QGW_HD unsigned int fx_mag(fx_t v) {  // OR of these over values: their magnitude's bits above 2^32
   const int h = (int)(v >> 32);
   return (unsigned int)(h ^ (h >> 31));
@@ -110,11 +117,13 @@ constexpr int FX_ZERO = -FX_NAN;  // and of a row of zeros (v 2^e is 0)
 // the scale's biased exponent of a row from its largest high word
 QGW_HD int fx_scale(unsigned int mx) { return (int)(mx >> 20) < FX_EMIN ? FX_EMIN : (int)(mx >> 20); }
 
-QGW_HD fx_t fx_from_bits(unsigned long long b, int E) {
+// x 2^(1075 + UP - E) of a double's bits, truncated; E at least its biased
+// exponent
+template <int UP = 6> QGW_HD fx_t fx_from_bits(unsigned long long b, int E) {
   const unsigned int hi = (unsigned int)(b >> 32);
   int sh = E - (int)((hi >> 20) & 0x7ffu);
   sh = sh > 63 ? 63 : sh;
-  const unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | (b & 0xffffffffull)) << 6;
+  const unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | (b & 0xffffffffull)) << UP;
   const fx_t v = (fx_t)(m >> sh);
   return (int)hi < 0 ? -v : v;
 }

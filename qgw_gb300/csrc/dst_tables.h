@@ -149,4 +149,28 @@ inline FxTablesHost build_fx_tables(const DstGeom& g) {
   return t;
 }
 
+// Whether a projection runs in fixed point (modes_fx.cuh): at most 32 terms,
+// and the largest entries of the matrix's columns within a factor of 64.
+inline bool modes_fixed_ok(int nl, const double* mat) {
+  if (nl > 32) return false;
+  double lo = 0, hi = 0;
+  for (int l = 0; l < nl; ++l) {
+    double mx = 0;
+    for (int m = 0; m < nl; ++m) mx = std::fmax(mx, std::fabs(mat[(size_t)m * nl + l]));
+    lo = l ? std::fmin(lo, mx) : mx;
+    hi = std::fmax(hi, mx);
+  }
+  return lo > 0 && hi <= 64 * lo && hi < 1e150 && lo > 1e-150;
+}
+// A projection matrix (nl x nl, row m: output m) in fixed point: every row by
+// its largest entry.
+inline void fill_mode_table(int nl, const double* mat, Q2* c, int* e) {
+  for (int m = 0; m < nl; ++m) {
+    double mx = 0;
+    for (int l = 0; l < nl; ++l) mx = std::fmax(mx, std::fabs(mat[(size_t)m * nl + l]));
+    std::frexp(mx, &e[m]);
+    for (int l = 0; l < nl; ++l) c[m * nl + l] = q2_split((fx_t)std::nearbyint(std::ldexp(mat[(size_t)m * nl + l], 60 - e[m])));
+  }
+}
+
 }  // namespace qgw

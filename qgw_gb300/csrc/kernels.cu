@@ -19,7 +19,7 @@ namespace qgw {
 template <typename T, bool COMP, bool PER, int HL>
 __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) k_rows_fwd(StepArgs<T> a, int step_mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ __align__(16) T tot[tot_len<T, PER, HL>];
+  __shared__ __align__(16) T tot[tot_len<T>];
   body_rows_fwd<T, COMP, PER, HL>(a, step_mode, blockIdx.x, smem_raw + cst_bytes<T>(a.nl), tot, (T*)smem_raw);
 }
 // CT: columns per tile (closed basin; the periodic kernel takes two complex
@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) k_rows_fwd(StepArg
 template <typename T, bool COMP, bool PER, int CT, int HL>
 __global__ void __launch_bounds__(NT, 3) k_cols(StepArgs<T> a, int step_mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ __align__(16) T tot[tot_len<T, PER, HL>];
+  __shared__ __align__(16) T tot[tot_len<T>];
   if (PER) body_cols_per<T, COMP>(a, step_mode, blockIdx.x, blockIdx.y, smem_raw);
   else body_cols<T, COMP, CT, HL>(a, step_mode, blockIdx.x, blockIdx.y, smem_raw, tot);
 }
@@ -37,7 +37,7 @@ template <typename T> constexpr int CTD = ColsPer<T>::value;
 template <typename T, bool COMP, bool PER, int HL>
 __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) k_rows_inv(StepArgs<T> a, int step_mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ __align__(16) T tot[tot_len<T, PER, HL>];
+  __shared__ __align__(16) T tot[tot_len<T>];
   body_rows_inv<T, COMP, PER, HL>(a, step_mode, blockIdx.x, smem_raw + cst_bytes<T>(a.nl), tot, (T*)smem_raw,
                                   gridDim.y > 1 ? (int)blockIdx.y : -1);
 }
@@ -56,6 +56,34 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 4) k_rhs(const __grid
     for (int b = 0; b < 4; ++b) mbar_init(&bar[b]);
   __syncthreads();
   body_rhs_tiles<T, COMP, R, TY, rhs_nbuf<T>()>(a, ntx, nty, base, a.use_tma ? &a.tm[0] : nullptr, bar);
+}
+
+// FP64: the projections, one thread per point (NL: layers in registers, 0:
+// any number), and the row transforms (modes_fx.cuh)
+template <int NL, bool FWD>
+__global__ void __launch_bounds__(NT, 2) k_modes(const __grid_constant__ StepArgs<double> a, int step_mode) {
+  if (step_mode && !a.state->active) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Q2* cs = (Q2*)smem_raw;
+  const ModeTable& tb = FWD ? a.l2m : a.m2l;
+  __shared__ QUpdate u;
+  if (FWD && threadIdx.x == 0) u = q_update(a, step_mode);
+  if constexpr (NL > 0) modes_stage<NL>(tb, cs);
+  __syncthreads();
+  const int np = !FWD && a.periodic ? a.nx + 2 : a.nx;
+  const int w = blockIdx.x * NT + threadIdx.x, j = w / np, i = w - j * np;
+  if constexpr (NL == 0) modes_point_any<FWD>(a, tb, u, j, i, j < a.ny, cs);
+  else if (j < a.ny) modes_point<NL, FWD>(a, tb, u, j, i, cs);
+}
+template <bool PER, int HL, bool INV>
+__global__ void __launch_bounds__(NT, 3) k_rows_f64(StepArgs<double> a, int step_mode) {
+  if (step_mode && !a.state->active) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(16) double tot[tot_len<double>];
+  const int rows = INV ? a.RB3 : a.RB1, r0 = blockIdx.x * rows;
+  double* A = (double*)smem_raw;
+  rows_f64<PER, HL, INV>(a, INV ? a.psi : a.spec, r0, min(rows, a.nl * a.ny - r0), -1, A,
+                         A + (size_t)rows * row_len<double>(a.gx), tot);
 }
 
 // ------------------------------------------------------- small kernels
@@ -324,6 +352,8 @@ static __global__ void k_budget_final(const double* part, int nblk, double scale
 // The dynamic shared-memory limit is a process-wide attribute of each kernel,
 // shared by every run in the process; it is set to the device's opt-in
 // maximum (never lowered) so that runs of different sizes can coexist.
+[[maybe_unused]] static size_t rows_bytes(const StepArgs<double>& a) { return smem_rows_f64(a, std::max(a.RB1, a.RB3)); }
+[[maybe_unused]] static size_t rows_bytes(const StepArgs<float>&) { return 0; }
 template <typename T, bool COMP>
 static cudaError_t set_attrs(const StepArgs<T>& a) {
   int dev = 0, optin = 0;
@@ -334,20 +364,32 @@ static cudaError_t set_attrs(const StepArgs<T>& a) {
   const size_t static_tot = sizeof(T) * GMAX * 32 + 64;
   if (smem_rows<T, COMP>(a) + static_tot > (size_t)optin || smem_cols<T, COMP>(a) + static_tot > (size_t)optin ||
       smem_rows_inv<T, COMP>(a) + static_tot > (size_t)optin || rhs_halo(a) > RHS_RMAX ||
+      (sizeof(T) == 8 && rows_bytes(a) + static_tot > (size_t)optin) ||
       smem_rhs<T>(a) + 1024 > (size_t)optin || smem_rhs_tiles<T>(a) + 1024 > (size_t)optin)
     return cudaErrorInvalidValue;
   const int lim = optin - (int)static_tot;
-  const void* transforms[] = {
-      (const void*)k_rows_fwd<T, COMP, false, 0>,         (const void*)k_rows_fwd<T, COMP, false, 512>,
-      (const void*)k_rows_inv<T, COMP, false, 0>,         (const void*)k_rows_inv<T, COMP, false, 512>,
+  const void* columns[] = {
       (const void*)k_cols<T, COMP, false, CTD<T>, 0>,     (const void*)k_cols<T, COMP, false, CTD<T>, 512>,
       (const void*)k_cols<T, COMP, false, CTD<T> / 2, 0>, (const void*)k_cols<T, COMP, false, CTD<T> / 2, 512>,
-      (const void*)k_rows_fwd<T, COMP, false, -1>,        (const void*)k_rows_inv<T, COMP, false, -1>,
       (const void*)k_cols<T, COMP, false, CTD<T> / 2, -1>, (const void*)k_cols<T, COMP, false, 1, -1>,
-      (const void*)k_rows_fwd<T, COMP, true, 0>,          (const void*)k_rows_inv<T, COMP, true, 0>,
       (const void*)k_cols<T, COMP, true, CTD<T>, 0>};
-  for (const void* f : transforms)
+  for (const void* f : columns)
     if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, lim))) return e;
+  if constexpr (sizeof(T) == 8) {
+    const void* rows[] = {(const void*)k_rows_f64<false, 0, false>,   (const void*)k_rows_f64<false, 0, true>,
+                          (const void*)k_rows_f64<false, 512, false>, (const void*)k_rows_f64<false, 512, true>,
+                          (const void*)k_rows_f64<false, -1, false>,  (const void*)k_rows_f64<false, -1, true>,
+                          (const void*)k_rows_f64<true, 0, false>,    (const void*)k_rows_f64<true, 0, true>};
+    for (const void* f : rows)
+      if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, lim))) return e;
+  } else {
+    const void* rows[] = {(const void*)k_rows_fwd<T, COMP, false, 0>,   (const void*)k_rows_inv<T, COMP, false, 0>,
+                          (const void*)k_rows_fwd<T, COMP, false, 512>, (const void*)k_rows_inv<T, COMP, false, 512>,
+                          (const void*)k_rows_fwd<T, COMP, false, -1>,  (const void*)k_rows_inv<T, COMP, false, -1>,
+                          (const void*)k_rows_fwd<T, COMP, true, 0>,    (const void*)k_rows_inv<T, COMP, true, 0>};
+    for (const void* f : rows)
+      if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, lim))) return e;
+  }
   if ((e = cudaFuncSetAttribute(k_forc_cols<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim))) return e;
   if ((e = cudaFuncSetAttribute(k_forc_rows<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim))) return e;
   const int rl = optin - 1024;
@@ -360,13 +402,41 @@ static cudaError_t set_attrs(const StepArgs<T>& a) {
   return cudaSuccess;
 }
 
+// FP64: a projection and the row transforms after it
+template <bool FWD> static void launch_modes(const StepArgs<double>& a, int step_mode, cudaStream_t s) {
+  const size_t n = (size_t)a.ny * (!FWD && a.periodic ? a.nx + 2 : a.nx);
+  const dim3 grid((unsigned int)((n + NT - 1) / NT));
+  switch (a.modes_fx ? a.nl : 0) {
+#define QGW_MODES(N) \
+  case N: k_modes<N, FWD><<<grid, NT, sizeof(Q2) * ModeShape<N>::len, s>>>(a, step_mode); break;
+    QGW_MODES(1) QGW_MODES(2) QGW_MODES(3) QGW_MODES(4) QGW_MODES(5) QGW_MODES(6) QGW_MODES(7) QGW_MODES(8)
+    QGW_MODES(9) QGW_MODES(10) QGW_MODES(11) QGW_MODES(12) QGW_MODES(13) QGW_MODES(14) QGW_MODES(15) QGW_MODES(16)
+#undef QGW_MODES
+    default: k_modes<0, FWD><<<grid, NT, sizeof(Q2) * 8 * a.nl, s>>>(a, step_mode); break;
+  }
+}
+template <bool INV> static void launch_rows(const StepArgs<double>& a, int step_mode, cudaStream_t s) {
+  const int rows = INV ? a.RB3 : a.RB1;
+  const size_t sm = smem_rows_f64(a, rows);
+  const dim3 grid((a.nl * a.ny + rows - 1) / rows);
+  if (a.periodic) k_rows_f64<true, 0, INV><<<grid, NT, sm, s>>>(a, step_mode);
+  else if (a.gx.blue) k_rows_f64<false, -1, INV><<<grid, NT, sm, s>>>(a, step_mode);
+  else if (a.gx.H == 512) k_rows_f64<false, 512, INV><<<grid, NT, sm, s>>>(a, step_mode);
+  else k_rows_f64<false, 0, INV><<<grid, NT, sm, s>>>(a, step_mode);
+}
+
 template <typename T, bool COMP>
 static void launch_k1(const StepArgs<T>& a, int step_mode, cudaStream_t s) {
-  const size_t sm = smem_rows<T, COMP>(a);
-  if (a.periodic) k_rows_fwd<T, COMP, true, 0><<<dim3(a.ny), NT, sm, s>>>(a, step_mode);
-  else if (a.gx.blue) k_rows_fwd<T, COMP, false, -1><<<dim3(a.ny), NT, sm, s>>>(a, step_mode);
-  else if (a.gx.H == 512) k_rows_fwd<T, COMP, false, 512><<<dim3(a.ny), NT, sm, s>>>(a, step_mode);
-  else k_rows_fwd<T, COMP, false, 0><<<dim3(a.ny), NT, sm, s>>>(a, step_mode);
+  if constexpr (sizeof(T) == 8) {
+    launch_modes<true>(a, step_mode, s);
+    launch_rows<false>(a, step_mode, s);
+  } else {
+    const size_t sm = smem_rows<T, COMP>(a);
+    if (a.periodic) k_rows_fwd<T, COMP, true, 0><<<dim3(a.ny), NT, sm, s>>>(a, step_mode);
+    else if (a.gx.blue) k_rows_fwd<T, COMP, false, -1><<<dim3(a.ny), NT, sm, s>>>(a, step_mode);
+    else if (a.gx.H == 512) k_rows_fwd<T, COMP, false, 512><<<dim3(a.ny), NT, sm, s>>>(a, step_mode);
+    else k_rows_fwd<T, COMP, false, 0><<<dim3(a.ny), NT, sm, s>>>(a, step_mode);
+  }
 }
 template <typename T, bool COMP>
 static void launch_k2(const StepArgs<T>& a, int step_mode, cudaStream_t s) {
@@ -383,14 +453,19 @@ static void launch_k2(const StepArgs<T>& a, int step_mode, cudaStream_t s) {
 }
 template <typename T, bool COMP>
 static void launch_k3(const StepArgs<T>& a, int step_mode, cudaStream_t s) {
-  const size_t sm = smem_rows_inv<T, COMP>(a);
-  // rows x layer groups: a row's groups read the same spectral rows, so
-  // splitting them over blocks adds no traffic and evens out the SMs' loads
-  const dim3 grid(a.ny, a.inv_split ? (a.nl + a.G3 - 1) / a.G3 : 1);
-  if (a.periodic) k_rows_inv<T, COMP, true, 0><<<grid, NT, sm, s>>>(a, step_mode);
-  else if (a.gx.blue) k_rows_inv<T, COMP, false, -1><<<grid, NT, sm, s>>>(a, step_mode);
-  else if (a.gx.H == 512) k_rows_inv<T, COMP, false, 512><<<grid, NT, sm, s>>>(a, step_mode);
-  else k_rows_inv<T, COMP, false, 0><<<grid, NT, sm, s>>>(a, step_mode);
+  if constexpr (sizeof(T) == 8) {
+    launch_modes<false>(a, step_mode, s);
+    launch_rows<true>(a, step_mode, s);
+  } else {
+    const size_t sm = smem_rows_inv<T, COMP>(a);
+    // rows x layer groups: a row's groups read the same spectral rows, so
+    // splitting them over blocks adds no traffic and evens out the SMs' loads
+    const dim3 grid(a.ny, a.inv_split ? (a.nl + a.G3 - 1) / a.G3 : 1);
+    if (a.periodic) k_rows_inv<T, COMP, true, 0><<<grid, NT, sm, s>>>(a, step_mode);
+    else if (a.gx.blue) k_rows_inv<T, COMP, false, -1><<<grid, NT, sm, s>>>(a, step_mode);
+    else if (a.gx.H == 512) k_rows_inv<T, COMP, false, 512><<<grid, NT, sm, s>>>(a, step_mode);
+    else k_rows_inv<T, COMP, false, 0><<<grid, NT, sm, s>>>(a, step_mode);
+  }
 }
 // tiles of the RHS kernel along x and y
 template <typename T> static int rhs_ntx(const StepArgs<T>& a) { return (a.nx + TX - 1) / TX; }

@@ -46,8 +46,11 @@ constexpr size_t oTx = oHinv + kFieldMax;
 constexpr size_t oTy = oTx + kTab;
 constexpr size_t oCl = oTy + kTab;
 constexpr size_t oCm = oCl + (size_t)kNlMax * kNlMax;
-constexpr size_t oIrd = oCm + (size_t)kNlMax * kNlMax;
-constexpr size_t oLsq = oIrd + kNlMax;
+constexpr size_t oClq = oCm + (size_t)kNlMax * kNlMax;
+constexpr size_t oCmq = oClq + (size_t)kNlMax * kNlMax;
+constexpr size_t oIrd = oCmq + (size_t)kNlMax * kNlMax;
+constexpr size_t oExp = oIrd + kNlMax;  // the projections' exponents (2 x kNlMax ints)
+constexpr size_t oLsq = oExp + kNlMax;
 constexpr size_t oKsq = oLsq + kMMax;
 constexpr size_t oState = oKsq + kMMax;
 constexpr size_t kTotal = oState + kStateD;
@@ -170,6 +173,8 @@ extern "C" int qgw_invert_pv_noalloc(const qgw_params* p, const double* cl2m, co
     fill_tables(ny + 1, h_tab + (oTy - oTx));
     std::memcpy(h_tab + (oCl - oTx), kcl, sizeof(double) * nl * nl);
     std::memcpy(h_tab + (oCm - oTx), kcm, sizeof(double) * nl * nl);
+    qgw::fill_mode_table(nl, kcl, (qgw::Q2*)(h_tab + (oClq - oTx)), (int*)(h_tab + (oExp - oTx)));
+    qgw::fill_mode_table(nl, kcm, (qgw::Q2*)(h_tab + (oCmq - oTx)), (int*)(h_tab + (oExp - oTx)) + kNlMax);
     std::memcpy(h_tab + (oIrd - oTx), kir, sizeof(double) * nl);
     for (int k = 0; k < nx; ++k) { const double L = M_PI * (k + 1) / p->Lx; h_tab[oLsq - oTx + k] = L * L; }
     for (int j = 0; j < ny; ++j) { const double K = M_PI * (j + 1) / p->Lx; h_tab[oKsq - oTx + j] = K * K; }
@@ -196,6 +201,9 @@ extern "C" int qgw_invert_pv_noalloc(const qgw_params* p, const double* cl2m, co
   a.fy = tables_at(base + oTy);
   a.cl2m = base + oCl;
   a.cm2l = base + oCm;
+  a.modes_fx = qgw::modes_fixed_ok(nl, cl2m) && qgw::modes_fixed_ok(nl, cm2l);
+  a.l2m = qgw::ModeTable{(const qgw::Q2*)(base + oClq), (const int*)(base + oExp)};
+  a.m2l = qgw::ModeTable{(const qgw::Q2*)(base + oCmq), (const int*)(base + oExp) + kNlMax};
   a.iRd2 = base + oIrd;
   a.q = q_dev + pitch + 1;
   a.psi = psi_dev + pitch + 1;
@@ -214,6 +222,7 @@ extern "C" int qgw_invert_pv_noalloc(const qgw_params* p, const double* cl2m, co
   const int ngroups = (nl + g - 1) / g;
   a.G1 = (nl + ngroups - 1) / ngroups;
   a.G3 = a.G1;
+  a.RB1 = a.RB3 = g < 4 ? g : 4;
   int ct = (int)(budget / (2 * (size_t)(ny + 1) * sizeof(double)));
   a.CT = ct < 1 ? 1 : (ct > 16 ? 16 : ct);
   qgw::enqueue_invert_f64(a, s);

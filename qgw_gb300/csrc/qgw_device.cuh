@@ -85,6 +85,9 @@ template <typename T> struct StepArgs {
   DstGeom gx, gy;
   DstTables<T> tx, ty;
   FxTables fx, fy;                 // FP64 closed basins: the fixed-point transforms' tables
+  ModeTable l2m, m2l;              // FP64: the projections' constants
+  int modes_fx;                    // FP64: 1 projects in fixed point, 0 in FP64 (cl2m, cm2l)
+  int RB1, RB3;                    // FP64: rows per block of the forward and inverse row kernels
   // vertical modes (FP64 master copies and T copies)
   const T* cl2m;                   // nl*nl row-major, mode m row: cl2m[m*nl+l]
   const T* cm2l;                   // cm2l[l*nl+m]

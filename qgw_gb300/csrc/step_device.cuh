@@ -161,22 +161,11 @@ __device__ __forceinline__ T* dst_block(T* A, T* B, int nrows, int ld, const Dst
 // The FP64 closed-basin transforms other than the chirp-z ones run in fixed
 // point (dst_fx.cuh); the block's scratch for them lies in tot.
 template <typename T, bool PER, int HL> constexpr bool fx_path = sizeof(T) == 8 && !PER && HL != -1;
-// values of tot: two scratches (the column kernel's two transforms), which
-// leaves room for a third 1024-point column block per SM, or the chunk totals
-// of the generic transform
-template <typename T, bool PER, int HL>
-constexpr int tot_len = fx_path<T, PER, HL> ? (int)(2 * sizeof(FxScratch) / sizeof(T)) : GMAX * 32;
+// values of tot: FP64 two scratches (the column kernel's two transforms),
+// which leaves room for a third 1024-point column block per SM; FP32 the
+// chunk totals of the generic transform
+template <typename T> constexpr int tot_len = sizeof(T) == 8 ? (int)(2 * sizeof(FxScratch) / sizeof(T)) : GMAX * 32;
 static_assert(GMAX <= FX_ROWS && NT == FX_NT, "a scratch holds every row");
-// the largest high words of the rows this thread and its warp have written
-// to A (x_{i+1} at index i + 1, i = threadIdx.x, + NT, ...)
-__device__ __forceinline__ void fx_note_rows(FxScratch* sc, const double* A, int nrows, int ld, int nx) {
-  for (int g = 0; g < nrows; ++g) {
-    unsigned int m = 0;
-    for (int i = threadIdx.x; i < nx; i += NT) m = max(m, fx_hi(A[g * ld + pr<double>(i + 1)]));
-    fx_note_max(sc, g, m);
-  }
-}
-
 __device__ __forceinline__ void slabs(int si, int& s0, int& s1, int& s2) {
   const int m = si % 3;
   s0 = (3 - m) % 3;
@@ -482,8 +471,6 @@ __device__ __forceinline__ void project_fwd(const StepArgs<T>& a, int j, bool up
 template <typename T, bool COMP, bool PER, int HL = 0>
 __device__ __forceinline__ void body_rows_fwd(const StepArgs<T>& a, int step_mode, int j, unsigned char* smem_raw,
                                               T* tot, T* cst) {
-  constexpr bool FX = fx_path<T, PER, HL>;
-  FxScratch* sc = (FxScratch*)tot;
   DevState* st = a.state;
   if (step_mode && !st->active) return;
   const int ld = row_len<T>(a.gx);
@@ -501,7 +488,7 @@ __device__ __forceinline__ void body_rows_fwd(const StepArgs<T>& a, int step_mod
   // FP32 groups of 9..12 modes run at width 12 (three 16-byte coefficient
   // vectors), the common 10-layer case without six idle accumulators
   const int GB = (sizeof(T) == 4 && a.G1 > 8 && a.G1 <= 12) ? 12 : group_width(a.G1);
-  if (!PER && !FX) prefetch_tables_l1(a.tx, a.gx.M);
+  if (!PER) prefetch_tables_l1(a.tx, a.gx.M);
   const T* frow = (ab3 && a.fr.on) ? a.fr.field + (size_t)j * a.pitch : nullptr;
   const T sqdt = frow ? (T)sqrt(st->dt) : T(0);
   const T* r1 = nullptr;
@@ -521,7 +508,6 @@ __device__ __forceinline__ void body_rows_fwd(const StepArgs<T>& a, int step_mod
   for (int gi = 0, m0 = 0; gi < ng; m0 += gq + (gi < gr), ++gi) {
     const int G = gq + (gi < gr);
     const bool upd = ab3 && m0 == 0;
-    if constexpr (FX) fx_clear(sc);
     for (int w = tid; w < a.nl * GMAX; w += NT) {
       const int l = w / GMAX, g = w - l * GMAX;
       cst[w] = g < G ? a.cl2m[(size_t)(m0 + g) * a.nl + l] : T(0);
@@ -556,18 +542,6 @@ __device__ __forceinline__ void body_rows_fwd(const StepArgs<T>& a, int step_mod
     }
 #undef QGW_PF_GB
 #undef QGW_PF
-    if constexpr (FX) {
-      fx_note_rows(sc, A, G, ld, a.nx);
-      __syncthreads();
-      const fx_t* O = dst_fx<HL>(A, B, G, ld, a.gx, a.fx, sc);
-      for (int gg = 0; gg < G; ++gg) {
-        T* dstrow = a.spec + (size_t)(m0 + gg) * a.lstride + (size_t)j * a.pitch;
-        const int ex = sc->ex[gg];
-        for (int i = threadIdx.x; i < a.nx; i += NT) dstrow[i] = fx_out(O[gg * ld + pr<T>(i + 1)], ex);
-      }
-      __syncthreads();
-      continue;
-    }
     __syncthreads();
     T* O = PER ? rfft_block<T>(A, B, G, ld, a.gx, a.tx) : dst_block<T, HL>(A, B, G, ld, a.gx, a.tx, tot);
     // spectral row: the real FFT's X_0..X_H as (re, im) pairs from index 0,
@@ -1029,8 +1003,6 @@ __device__ __forceinline__ void project_spec(const StepArgs<T>& a, int j, int G,
 template <typename T, bool COMP, bool PER, int HL = 0>
 __device__ __forceinline__ void body_rows_inv(const StepArgs<T>& a, int step_mode, int j, unsigned char* smem_raw,
                                               T* tot, T* cst, int only = -1) {
-  constexpr bool FX = fx_path<T, PER, HL>;
-  FxScratch* sc = (FxScratch*)tot;
   DevState* st = a.state;
   if (step_mode && !st->active) return;
   const int ld = row_len<T>(a.gx);
@@ -1039,7 +1011,7 @@ __device__ __forceinline__ void body_rows_inv(const StepArgs<T>& a, int step_mod
   T* A = (T*)smem_raw;
   T* B = A + (size_t)(zm ? 2 * Gb : Gb) * ld;
   const int GB = group_width(Gb);
-  if (!PER && !FX) prefetch_tables_l1(a.tx, a.gx.M);
+  if (!PER) prefetch_tables_l1(a.tx, a.gx.M);
   // ceil(nl / Gb) layer groups of balanced sizes (at most Gb each)
   const int ng = (a.nl + Gb - 1) / Gb, gq = a.nl / ng, gr = a.nl - gq * ng;
   const int g_begin = only < 0 ? 0 : only, g_end = only < 0 ? ng : min(only + 1, ng);
@@ -1049,7 +1021,6 @@ __device__ __forceinline__ void body_rows_inv(const StepArgs<T>& a, int step_mod
       const int m = w / GMAX, g = w - m * GMAX;
       cst[w] = g < G ? a.cm2l[(size_t)(l0 + g) * a.nl + m] : T(0);
     }
-    if constexpr (FX) fx_clear(sc);
     __syncthreads();
     const int ncols = PER ? a.nx + 2 : a.nx, xo = PER ? 0 : 1;
     if (zm) {
@@ -1067,18 +1038,6 @@ __device__ __forceinline__ void body_rows_inv(const StepArgs<T>& a, int step_mod
         case 8: project_spec<T, false, 8>(a, j, G, A, ld, cst, ncols, xo); break;
         default: project_spec<T, false, 16>(a, j, G, A, ld, cst, ncols, xo); break;
       }
-    }
-    if constexpr (FX) {
-      fx_note_rows(sc, A, G, ld, a.nx);
-      __syncthreads();
-      const fx_t* O = dst_fx<HL>(A, B, G, ld, a.gx, a.fx, sc);
-      for (int g = 0; g < G; ++g) {
-        T* prow = a.psi + (size_t)(l0 + g) * a.lstride + (size_t)j * a.pitch;
-        const int ex = sc->ex[g];
-        for (int i = threadIdx.x; i < a.nx; i += NT) prow[i] = fx_out(O[g * ld + pr<T>(i + 1)], ex);
-      }
-      __syncthreads();
-      continue;
     }
     __syncthreads();
     const int nrow = zm ? 2 * G : G;
@@ -1103,6 +1062,10 @@ __device__ __forceinline__ void body_rows_inv(const StepArgs<T>& a, int step_mod
     __syncthreads();
   }
 }
+
+}  // namespace qgw
+#include "modes_fx.cuh"
+namespace qgw {
 
 // ------------------------------------------------------------------ K4
 __device__ __forceinline__ unsigned long long absbits(double v) {
@@ -1834,6 +1797,10 @@ static int dst_bufs(const StepArgs<T>& a, const DstGeom& g) {
 template <typename T, bool COMP>
 static size_t smem_rows(const StepArgs<T>& a) {
   return cst_bytes<T>(a.nl) + (size_t)dst_bufs(a, a.gx) * a.G1 * row_len<T>(a.gx) * sizeof(T);
+}
+// FP64: rows per block rows in two buffers each
+static inline size_t smem_rows_f64(const StepArgs<double>& a, int rows) {
+  return (size_t)2 * rows * row_len<double>(a.gx) * sizeof(double);
 }
 template <typename T, bool COMP>
 static size_t smem_cols(const StepArgs<T>& a) {

@@ -920,8 +920,8 @@ int qgw_set_time(qgw_run* r, const qgw_time* in) {
 }
 
 static void enqueue_invert(qgw_run* r) {
-  if (r->precision == QGW_FP64) qgw::enqueue_invert_f64(r->a64, r->stream);
-  else qgw::enqueue_invert_f32c(r->a32, r->stream);
+  if (r->precision == QGW_FP64) qgw::enqueue_invert_f64(r->a64, true, r->stream);
+  else qgw::enqueue_invert_f32c(r->a32, true, r->stream);
 }
 
 int qgw_step(qgw_run* r, int nsteps, double t_out, double tend, qgw_step_info* info) {

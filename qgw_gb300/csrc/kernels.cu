@@ -20,6 +20,7 @@ template <typename T, bool COMP, bool PER, int HL>
 __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) k_rows_fwd(StepArgs<T> a, int step_mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(16) T tot[tot_len<T>];
+  grid_wait();
   body_rows_fwd<T, COMP, PER, HL>(a, step_mode, blockIdx.x, smem_raw + cst_bytes<T>(a.nl), tot, (T*)smem_raw);
 }
 // CT: columns per tile (closed basin; the periodic kernel takes two complex
@@ -28,6 +29,7 @@ template <typename T, bool COMP, bool PER, int CT, int HL>
 __global__ void __launch_bounds__(NT, 3) k_cols(StepArgs<T> a, int step_mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(16) T tot[tot_len<T>];
+  grid_wait();
   if (PER) body_cols_per<T, COMP>(a, step_mode, blockIdx.x, blockIdx.y, smem_raw);
   else body_cols<T, COMP, CT, HL>(a, step_mode, blockIdx.x, blockIdx.y, smem_raw, tot);
 }
@@ -38,6 +40,7 @@ template <typename T, bool COMP, bool PER, int HL>
 __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) k_rows_inv(StepArgs<T> a, int step_mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(16) T tot[tot_len<T>];
+  grid_wait();
   body_rows_inv<T, COMP, PER, HL>(a, step_mode, blockIdx.x, smem_raw + cst_bytes<T>(a.nl), tot, (T*)smem_raw,
                                   gridDim.y > 1 ? (int)blockIdx.y : -1);
 }
@@ -54,6 +57,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 4) k_rhs(const __grid
   unsigned char* base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
   if (threadIdx.x == 0 && threadIdx.y == 0)
     for (int b = 0; b < 4; ++b) mbar_init(&bar[b]);
+  grid_wait();
   __syncthreads();
   body_rhs_tiles<T, COMP, R, TY, rhs_nbuf<T>()>(a, ntx, nty, base, a.use_tma ? &a.tm[0] : nullptr, bar);
 }
@@ -62,6 +66,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 4) k_rhs(const __grid
 // any number), and the row transforms (modes_fx.cuh)
 template <int NL, bool FWD>
 __global__ void __launch_bounds__(NT, 2) k_modes(const __grid_constant__ StepArgs<double> a, int step_mode) {
+  grid_wait();
   if (step_mode && !a.state->active) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Q2* cs = (Q2*)smem_raw;
@@ -77,6 +82,7 @@ __global__ void __launch_bounds__(NT, 2) k_modes(const __grid_constant__ StepArg
 }
 template <bool PER, int HL, bool INV>
 __global__ void __launch_bounds__(NT, 3) k_rows_f64(StepArgs<double> a, int step_mode) {
+  grid_wait();
   if (step_mode && !a.state->active) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(16) double tot[tot_len<double>];
@@ -402,69 +408,88 @@ static cudaError_t set_attrs(const StepArgs<T>& a) {
   return cudaSuccess;
 }
 
+// A step kernel's launch.  pdl: the kernel before it in the stream is one of
+// a step too (or anything else: it then just completes first), and this one
+// may be placed on the SMs before that has drained (grid_wait).  Kernels of
+// small grids run 5-20 us, of which the launch gap was 2-3.
+template <typename... P, typename... A>
+static void launch(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool pdl, const A&... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = pdl ? 1 : 0;
+  cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
+}
+
 // FP64: a projection and the row transforms after it
-template <bool FWD> static void launch_modes(const StepArgs<double>& a, int step_mode, cudaStream_t s) {
+template <bool FWD> static void launch_modes(const StepArgs<double>& a, int step_mode, bool pdl, cudaStream_t s) {
   const size_t n = (size_t)a.ny * (!FWD && a.periodic ? a.nx + 2 : a.nx);
   const dim3 grid((unsigned int)((n + NT - 1) / NT));
   switch (a.modes_fx ? a.nl : 0) {
 #define QGW_MODES(N) \
-  case N: k_modes<N, FWD><<<grid, NT, sizeof(Q2) * ModeShape<N>::len, s>>>(a, step_mode); break;
+  case N: launch(k_modes<N, FWD>, grid, dim3(NT), sizeof(Q2) * ModeShape<N>::len, s, pdl, a, step_mode); break;
     QGW_MODES(1) QGW_MODES(2) QGW_MODES(3) QGW_MODES(4) QGW_MODES(5) QGW_MODES(6) QGW_MODES(7) QGW_MODES(8)
     QGW_MODES(9) QGW_MODES(10) QGW_MODES(11) QGW_MODES(12) QGW_MODES(13) QGW_MODES(14) QGW_MODES(15) QGW_MODES(16)
 #undef QGW_MODES
-    default: k_modes<0, FWD><<<grid, NT, sizeof(Q2) * 8 * a.nl, s>>>(a, step_mode); break;
+    default: launch(k_modes<0, FWD>, grid, dim3(NT), sizeof(Q2) * 8 * a.nl, s, pdl, a, step_mode); break;
   }
 }
-template <bool INV> static void launch_rows(const StepArgs<double>& a, int step_mode, cudaStream_t s) {
+template <bool INV> static void launch_rows(const StepArgs<double>& a, int step_mode, bool pdl, cudaStream_t s) {
   const int rows = INV ? a.RB3 : a.RB1;
   const size_t sm = smem_rows_f64(a, rows);
   const dim3 grid((a.nl * a.ny + rows - 1) / rows);
-  if (a.periodic) k_rows_f64<true, 0, INV><<<grid, NT, sm, s>>>(a, step_mode);
-  else if (a.gx.blue) k_rows_f64<false, -1, INV><<<grid, NT, sm, s>>>(a, step_mode);
-  else if (a.gx.H == 512) k_rows_f64<false, 512, INV><<<grid, NT, sm, s>>>(a, step_mode);
-  else k_rows_f64<false, 0, INV><<<grid, NT, sm, s>>>(a, step_mode);
+  if (a.periodic) launch(k_rows_f64<true, 0, INV>, grid, dim3(NT), sm, s, pdl, a, step_mode);
+  else if (a.gx.blue) launch(k_rows_f64<false, -1, INV>, grid, dim3(NT), sm, s, pdl, a, step_mode);
+  else if (a.gx.H == 512) launch(k_rows_f64<false, 512, INV>, grid, dim3(NT), sm, s, pdl, a, step_mode);
+  else launch(k_rows_f64<false, 0, INV>, grid, dim3(NT), sm, s, pdl, a, step_mode);
 }
 
 template <typename T, bool COMP>
-static void launch_k1(const StepArgs<T>& a, int step_mode, cudaStream_t s) {
+static void launch_k1(const StepArgs<T>& a, int step_mode, bool pdl, cudaStream_t s) {
   if constexpr (sizeof(T) == 8) {
-    launch_modes<true>(a, step_mode, s);
-    launch_rows<false>(a, step_mode, s);
+    launch_modes<true>(a, step_mode, pdl, s);
+    launch_rows<false>(a, step_mode, pdl, s);
   } else {
     const size_t sm = smem_rows<T, COMP>(a);
-    if (a.periodic) k_rows_fwd<T, COMP, true, 0><<<dim3(a.ny), NT, sm, s>>>(a, step_mode);
-    else if (a.gx.blue) k_rows_fwd<T, COMP, false, -1><<<dim3(a.ny), NT, sm, s>>>(a, step_mode);
-    else if (a.gx.H == 512) k_rows_fwd<T, COMP, false, 512><<<dim3(a.ny), NT, sm, s>>>(a, step_mode);
-    else k_rows_fwd<T, COMP, false, 0><<<dim3(a.ny), NT, sm, s>>>(a, step_mode);
+    if (a.periodic) launch(k_rows_fwd<T, COMP, true, 0>, dim3(a.ny), dim3(NT), sm, s, pdl, a, step_mode);
+    else if (a.gx.blue) launch(k_rows_fwd<T, COMP, false, -1>, dim3(a.ny), dim3(NT), sm, s, pdl, a, step_mode);
+    else if (a.gx.H == 512) launch(k_rows_fwd<T, COMP, false, 512>, dim3(a.ny), dim3(NT), sm, s, pdl, a, step_mode);
+    else launch(k_rows_fwd<T, COMP, false, 0>, dim3(a.ny), dim3(NT), sm, s, pdl, a, step_mode);
   }
 }
 template <typename T, bool COMP>
-static void launch_k2(const StepArgs<T>& a, int step_mode, cudaStream_t s) {
+static void launch_k2(const StepArgs<T>& a, int step_mode, bool pdl, cudaStream_t s) {
   const dim3 grid(col_tiles(a), a.nl);
   const size_t sm = smem_cols<T, COMP>(a);
   const bool wide = col_width(a) == CTD<T>, h512 = a.gy.H == 512 && !a.gy.blue;
-  if (a.periodic) k_cols<T, COMP, true, CTD<T>, 0><<<grid, NT, sm, s>>>(a, step_mode);
-  else if (a.gy.blue && col_width(a) == 1) k_cols<T, COMP, false, 1, -1><<<grid, NT, sm, s>>>(a, step_mode);
-  else if (a.gy.blue) k_cols<T, COMP, false, CTD<T> / 2, -1><<<grid, NT, sm, s>>>(a, step_mode);
-  else if (wide && h512) k_cols<T, COMP, false, CTD<T>, 512><<<grid, NT, sm, s>>>(a, step_mode);
-  else if (wide) k_cols<T, COMP, false, CTD<T>, 0><<<grid, NT, sm, s>>>(a, step_mode);
-  else if (h512) k_cols<T, COMP, false, CTD<T> / 2, 512><<<grid, NT, sm, s>>>(a, step_mode);
-  else k_cols<T, COMP, false, CTD<T> / 2, 0><<<grid, NT, sm, s>>>(a, step_mode);
+  if (a.periodic) launch(k_cols<T, COMP, true, CTD<T>, 0>, grid, dim3(NT), sm, s, pdl, a, step_mode);
+  else if (a.gy.blue && col_width(a) == 1) launch(k_cols<T, COMP, false, 1, -1>, grid, dim3(NT), sm, s, pdl, a, step_mode);
+  else if (a.gy.blue) launch(k_cols<T, COMP, false, CTD<T> / 2, -1>, grid, dim3(NT), sm, s, pdl, a, step_mode);
+  else if (wide && h512) launch(k_cols<T, COMP, false, CTD<T>, 512>, grid, dim3(NT), sm, s, pdl, a, step_mode);
+  else if (wide) launch(k_cols<T, COMP, false, CTD<T>, 0>, grid, dim3(NT), sm, s, pdl, a, step_mode);
+  else if (h512) launch(k_cols<T, COMP, false, CTD<T> / 2, 512>, grid, dim3(NT), sm, s, pdl, a, step_mode);
+  else launch(k_cols<T, COMP, false, CTD<T> / 2, 0>, grid, dim3(NT), sm, s, pdl, a, step_mode);
 }
 template <typename T, bool COMP>
-static void launch_k3(const StepArgs<T>& a, int step_mode, cudaStream_t s) {
+static void launch_k3(const StepArgs<T>& a, int step_mode, bool pdl, cudaStream_t s) {
   if constexpr (sizeof(T) == 8) {
-    launch_modes<false>(a, step_mode, s);
-    launch_rows<true>(a, step_mode, s);
+    launch_modes<false>(a, step_mode, pdl, s);
+    launch_rows<true>(a, step_mode, pdl, s);
   } else {
     const size_t sm = smem_rows_inv<T, COMP>(a);
     // rows x layer groups: a row's groups read the same spectral rows, so
     // splitting them over blocks adds no traffic and evens out the SMs' loads
     const dim3 grid(a.ny, a.inv_split ? (a.nl + a.G3 - 1) / a.G3 : 1);
-    if (a.periodic) k_rows_inv<T, COMP, true, 0><<<grid, NT, sm, s>>>(a, step_mode);
-    else if (a.gx.blue) k_rows_inv<T, COMP, false, -1><<<grid, NT, sm, s>>>(a, step_mode);
-    else if (a.gx.H == 512) k_rows_inv<T, COMP, false, 512><<<grid, NT, sm, s>>>(a, step_mode);
-    else k_rows_inv<T, COMP, false, 0><<<grid, NT, sm, s>>>(a, step_mode);
+    if (a.periodic) launch(k_rows_inv<T, COMP, true, 0>, grid, dim3(NT), sm, s, pdl, a, step_mode);
+    else if (a.gx.blue) launch(k_rows_inv<T, COMP, false, -1>, grid, dim3(NT), sm, s, pdl, a, step_mode);
+    else if (a.gx.H == 512) launch(k_rows_inv<T, COMP, false, 512>, grid, dim3(NT), sm, s, pdl, a, step_mode);
+    else launch(k_rows_inv<T, COMP, false, 0>, grid, dim3(NT), sm, s, pdl, a, step_mode);
   }
 }
 // tiles of the RHS kernel along x and y
@@ -472,7 +497,7 @@ template <typename T> static int rhs_ntx(const StepArgs<T>& a) { return (a.nx + 
 template <typename T> static int rhs_nty(const StepArgs<T>& a) { return (a.ny + rhs_ty(a) - 1) / rhs_ty(a); }
 
 template <typename T, bool COMP>
-static void launch_rhs(const StepArgs<T>& a, cudaStream_t s) {
+static void launch_rhs(const StepArgs<T>& a, bool pdl, cudaStream_t s) {
   const int ntx = rhs_ntx(a), nty = rhs_nty(a), ntiles = ntx * nty * a.nl;
   const int grid = (a.rhs_grid > 0 && a.rhs_grid < ntiles) ? a.rhs_grid : ntiles;
   const dim3 blk(32, 8);
@@ -480,20 +505,20 @@ static void launch_rhs(const StepArgs<T>& a, cudaStream_t s) {
   const bool t32 = rhs_ty(a) == 32;
   switch (rhs_halo(a)) {
     case 1:
-      if (t32) k_rhs<T, COMP, 1, 32><<<grid, blk, sm, s>>>(a, ntx, nty);
-      else k_rhs<T, COMP, 1, 16><<<grid, blk, sm, s>>>(a, ntx, nty);
+      if (t32) launch(k_rhs<T, COMP, 1, 32>, grid, blk, sm, s, pdl, a, ntx, nty);
+      else launch(k_rhs<T, COMP, 1, 16>, grid, blk, sm, s, pdl, a, ntx, nty);
       break;
     case 2:
-      if (t32) k_rhs<T, COMP, 2, 32><<<grid, blk, sm, s>>>(a, ntx, nty);
-      else k_rhs<T, COMP, 2, 16><<<grid, blk, sm, s>>>(a, ntx, nty);
+      if (t32) launch(k_rhs<T, COMP, 2, 32>, grid, blk, sm, s, pdl, a, ntx, nty);
+      else launch(k_rhs<T, COMP, 2, 16>, grid, blk, sm, s, pdl, a, ntx, nty);
       break;
     case 3:
-      if (t32) k_rhs<T, COMP, 3, 32><<<grid, blk, sm, s>>>(a, ntx, nty);
-      else k_rhs<T, COMP, 3, 16><<<grid, blk, sm, s>>>(a, ntx, nty);
+      if (t32) launch(k_rhs<T, COMP, 3, 32>, grid, blk, sm, s, pdl, a, ntx, nty);
+      else launch(k_rhs<T, COMP, 3, 16>, grid, blk, sm, s, pdl, a, ntx, nty);
       break;
     default:
-      if (t32) k_rhs<T, COMP, 4, 32><<<grid, blk, sm, s>>>(a, ntx, nty);
-      else k_rhs<T, COMP, 4, 16><<<grid, blk, sm, s>>>(a, ntx, nty);
+      if (t32) launch(k_rhs<T, COMP, 4, 32>, grid, blk, sm, s, pdl, a, ntx, nty);
+      else launch(k_rhs<T, COMP, 4, 16>, grid, blk, sm, s, pdl, a, ntx, nty);
       break;
   }
 }
@@ -516,10 +541,10 @@ static int rhs_grid(const StepArgs<T>& a) {
 }
 
 template <typename T, bool COMP>
-static void launch_invert(const StepArgs<T>& a, int step_mode, cudaStream_t s) {
-  launch_k1<T, COMP>(a, step_mode, s);
-  launch_k2<T, COMP>(a, step_mode, s);
-  launch_k3<T, COMP>(a, step_mode, s);
+static void launch_invert(const StepArgs<T>& a, int step_mode, bool pdl, cudaStream_t s) {
+  launch_k1<T, COMP>(a, step_mode, pdl, s);
+  launch_k2<T, COMP>(a, step_mode, pdl, s);
+  launch_k3<T, COMP>(a, step_mode, pdl, s);
 }
 
 template <typename T, bool COMP>
@@ -533,10 +558,10 @@ static void launch_flush(const StepArgs<T>& a, cudaStream_t s) {
 
 template <typename T, bool COMP>
 static void launch_one(const StepArgs<T>& a, int which, cudaStream_t s) {
-  if (which == 0) launch_k1<T, COMP>(a, 1, s);
-  if (which == 1) launch_k2<T, COMP>(a, 1, s);
-  if (which == 2) launch_k3<T, COMP>(a, 1, s);
-  if (which == 3) launch_rhs<T, COMP>(a, s);
+  if (which == 0) launch_k1<T, COMP>(a, 1, false, s);
+  if (which == 1) launch_k2<T, COMP>(a, 1, false, s);
+  if (which == 2) launch_k3<T, COMP>(a, 1, false, s);
+  if (which == 3) launch_rhs<T, COMP>(a, false, s);
 }
 
 // ---- entry points used by api.cu (see kernels.h)
@@ -569,14 +594,14 @@ cudaError_t prepare_f64(const StepArgs<double>& a) { return set_attrs<double, fa
 int rhs_grid_f64(const StepArgs<double>&) { return 0; }  // one block per tile
 
 void enqueue_step_f64(const StepArgs<double>& a, cudaStream_t s) {
-  launch_invert<double, false>(a, 1, s);
-  launch_rhs<double, false>(a, s);
+  launch_invert<double, false>(a, 1, true, s);
+  launch_rhs<double, false>(a, true, s);
   launch_forcing<double>(a, s);
 }
 
 void enqueue_forcing_f64(const StepArgs<double>& a, cudaStream_t s) { launch_forcing<double>(a, s); }
 
-void enqueue_invert_f64(const StepArgs<double>& a, cudaStream_t s) { launch_invert<double, false>(a, 0, s); }
+void enqueue_invert_f64(const StepArgs<double>& a, bool pdl, cudaStream_t s) { launch_invert<double, false>(a, 0, pdl, s); }
 
 void enqueue_flush_f64(const StepArgs<double>& a, cudaStream_t s) { launch_flush<double, false>(a, s); }
 
@@ -616,14 +641,14 @@ cudaError_t prepare_f32c(const StepArgs<float>& a) { return set_attrs<float, tru
 int rhs_grid_f32c(const StepArgs<float>& a) { return rhs_grid<float, true>(a); }
 
 void enqueue_step_f32c(const StepArgs<float>& a, cudaStream_t s) {
-  launch_invert<float, true>(a, 1, s);
-  launch_rhs<float, true>(a, s);
+  launch_invert<float, true>(a, 1, true, s);
+  launch_rhs<float, true>(a, true, s);
   launch_forcing<float>(a, s);
 }
 
 void enqueue_forcing_f32c(const StepArgs<float>& a, cudaStream_t s) { launch_forcing<float>(a, s); }
 
-void enqueue_invert_f32c(const StepArgs<float>& a, cudaStream_t s) { launch_invert<float, true>(a, 0, s); }
+void enqueue_invert_f32c(const StepArgs<float>& a, bool pdl, cudaStream_t s) { launch_invert<float, true>(a, 0, pdl, s); }
 
 void enqueue_flush_f32c(const StepArgs<float>& a, cudaStream_t s) { launch_flush<float, true>(a, s); }
 

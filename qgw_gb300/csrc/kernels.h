@@ -18,8 +18,10 @@ int rhs_grid_f32c(const StepArgs<float>& a);
 void enqueue_begin(DevState* st, double t_out, double tend, cudaStream_t s);
 void enqueue_step_f64(const StepArgs<double>& a, cudaStream_t s);
 void enqueue_step_f32c(const StepArgs<float>& a, cudaStream_t s);
-void enqueue_invert_f64(const StepArgs<double>& a, cudaStream_t s);
-void enqueue_invert_f32c(const StepArgs<float>& a, cudaStream_t s);
+// pdl: programmatic dependent launches (not on a caller's stream, which may
+// be capturing)
+void enqueue_invert_f64(const StepArgs<double>& a, bool pdl, cudaStream_t s);
+void enqueue_invert_f32c(const StepArgs<float>& a, bool pdl, cudaStream_t s);
 // the stochastic forcing kernels of one step (ensembles launch them per member)
 void enqueue_forcing_f64(const StepArgs<double>& a, cudaStream_t s);
 void enqueue_forcing_f32c(const StepArgs<float>& a, cudaStream_t s);

@@ -172,6 +172,7 @@ __device__ __forceinline__ void modes_point(const StepArgs<double>& a, const Mod
     q_case(a, u, [&](auto fk) { load([&](int l, size_t ol) { return q_value<decltype(fk)::value>(a, u, l, j, i, ol); }); });
   else
     load([&](int, size_t ol) { return src[ol]; });
+  grid_next();
   const int E = fx_scale(h);
   fx_t x[NL];
 #pragma unroll
@@ -287,6 +288,7 @@ __device__ __forceinline__ void rows_f64(const StepArgs<double>& a, double* F, i
   else if constexpr (!PER) O = dst_block<double, HL>(A, B, nr, ld, a.gx, a.tx, tot);
   else if constexpr (INV) O = irfft_block<double>(A, B, nr, ld, a.gx, a.tx);
   else O = rfft_block<double>(A, B, nr, ld, a.gx, a.tx);
+  grid_next();
   for (int r = 0; r < nr; ++r) {
     double* dst = row(r);
     const int ex = FX ? sc->ex[r] : 0;

@@ -225,7 +225,7 @@ extern "C" int qgw_invert_pv_noalloc(const qgw_params* p, const double* cl2m, co
   a.RB1 = a.RB3 = g < 4 ? g : 4;
   int ct = (int)(budget / (2 * (size_t)(ny + 1) * sizeof(double)));
   a.CT = ct < 1 ? 1 : (ct > 16 ? 16 : ct);
-  qgw::enqueue_invert_f64(a, s);
+  qgw::enqueue_invert_f64(a, false, s);
   const double c = 2 * p->bc_fac / (a.Delta * a.Delta);
   k_noalloc_ghosts<<<64, 256, 0, s>>>(q_dev, psi_dev, nx, ny, nl, c);
   return cudaGetLastError() == cudaSuccess ? QGW_OK : QGW_ERR_CUDA;

@@ -200,6 +200,16 @@ template <typename T> __device__ __forceinline__ T pick(double d, float f);
 template <> __device__ __forceinline__ double pick<double>(double d, float) { return d; }
 template <> __device__ __forceinline__ float pick<float>(double, float f) { return f; }
 
+// Programmatic dependent launch (launch(), kernels.cu): a step kernel may be
+// placed on the SMs while the one before it drains.  Every such kernel first
+// waits for its predecessor to complete -- before it reads anything, returns
+// included, so that a kernel's completion implies its predecessor's -- and
+// lets its successor be placed (grid_next) only as it comes to its last
+// stores: placed from the start, the successor's blocks crowd the SMs that
+// the running kernel leaves idle, which cost small grids up to a tenth.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void grid_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 // Asynchronous global -> shared element copies (no register staging), so the
 // independent tile loads of a block are all in flight at once.
 template <typename T>
@@ -544,6 +554,7 @@ __device__ __forceinline__ void body_rows_fwd(const StepArgs<T>& a, int step_mod
 #undef QGW_PF
     __syncthreads();
     T* O = PER ? rfft_block<T>(A, B, G, ld, a.gx, a.tx) : dst_block<T, HL>(A, B, G, ld, a.gx, a.tx, tot);
+    if (gi == ng - 1) grid_next();
     // spectral row: the real FFT's X_0..X_H as (re, im) pairs from index 0,
     // or the DST's Y_1..Y_{M-1} from index 1
     const int nout = PER ? a.nx + 2 : a.nx, yo = PER ? 0 : 1;
@@ -639,6 +650,7 @@ __device__ __forceinline__ void body_cols_fx(const StepArgs<double>& a, int k0, 
   const fx_t* O2 = dst_fx<HL>((double*)O, (double*)Oth, CT, ld, a.gy, a.fy, &sc[1]);
 #pragma unroll
   for (int c = 0; c < CT; ++c) ex[c] = sc[1].ex[c];
+  grid_next();
   for (int jj = (int)threadIdx.x - 1; jj < ny; jj += NT) {
     if (jj < 0) continue;
     const int pj = pr<double>(jj + 1);
@@ -811,6 +823,7 @@ __device__ __forceinline__ void body_cols(const StepArgs<T>& a, int step_mode, i
   T* Oth = (O == A) ? B : A;
   T* O2 = dst_block<T, HL>(O, Oth, zm ? 2 * CT : CT, ld, a.gy, a.ty, tot);
   T* S2 = zm ? a.spec2 + (size_t)m * a.lstride : nullptr;
+  grid_next();
   T v[CT];
   for (int jj = threadIdx.x - 1; jj < ny; jj += NT) {
     if (jj < 0) continue;
@@ -915,6 +928,7 @@ __device__ __forceinline__ void body_cols_per(const StepArgs<T>& a, int step_mod
   __syncthreads();
   T* Oth = (O == A) ? B : A;
   T* O2 = cfft_block<T>(O, Oth, CC, ld, a.gy, a.ty.tw, a.ty.twp);
+  if (!zm) grid_next();
   for (int jj = tid; jj < ny; jj += NT) {
     const int pj = pc<T>(jj);
     const C2<T> z0 = ((const C2<T>*)O2)[pj];
@@ -1042,6 +1056,7 @@ __device__ __forceinline__ void body_rows_inv(const StepArgs<T>& a, int step_mod
     __syncthreads();
     const int nrow = zm ? 2 * G : G;
     T* O = PER ? irfft_block<T>(A, B, nrow, ld, a.gx, a.tx) : dst_block<T, HL>(A, B, nrow, ld, a.gx, a.tx, tot);
+    if (gi == g_end - 1) grid_next();
     // periodic: x_{2m+1} is minus the imaginary part of the backward FFT
     // (x_i at index i); DST: x_{i+1} at index i + 1
     const T odd = PER ? T(-1) : T(1);
@@ -1634,6 +1649,7 @@ __device__ __forceinline__ void rhs_block_done(DevState* st, unsigned long long 
   __shared__ unsigned long long wmax[NT / 32];
   __shared__ int is_last;
   const int tid = threadIdx.x + threadIdx.y * 32;
+  grid_next();
   for (int o = 16; o > 0; o >>= 1) {
     const unsigned long long u = __shfl_xor_sync(0xffffffffu, mymax, o);
     mymax = u > mymax ? u : mymax;

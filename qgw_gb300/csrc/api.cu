@@ -65,18 +65,26 @@ int upload(qgw_run* r, T** out, const std::vector<double>& host) {
   return cudaStreamSynchronize(r->stream) == cudaSuccess ? QGW_OK : QGW_ERR_CUDA;
 }
 
-// the fixed-point transform's tables in one allocation (twq | spq | nsj)
+// the fixed-point transform's tables in one allocation (twq | spq | nsj, or
+// twq | bc | bz)
 int upload_fx(qgw_run* r, qgw::FxTables* out, const qgw::DstGeom& g) {
-  const size_t ntw = qgw::fx_twq_len(g), nsp = (size_t)g.H / 2 + 1, nsj = ((size_t)g.H + 2) / 2;
-  std::vector<qgw::Q4> h(ntw + nsp + nsj);
-  qgw::fill_fx_tables(g, h.data(), h.data() + ntw, (qgw::Q2*)(h.data() + ntw + nsp));
+  const qgw::FxTablesHost t = qgw::build_fx_tables(g);
+  const size_t ntw = t.twq.size(), n2 = g.blue ? t.bc.size() : t.spq.size(), n3 = g.blue ? t.bz.size() : (t.nsj.size() + 1) / 2;
+  std::vector<qgw::Q4> h(ntw + n2 + n3);
+  std::copy(t.twq.begin(), t.twq.end(), h.begin());
+  std::copy((g.blue ? t.bc : t.spq).begin(), (g.blue ? t.bc : t.spq).end(), h.begin() + ntw);
+  if (g.blue) std::copy(t.bz.begin(), t.bz.end(), h.begin() + ntw + n2);
+  else std::copy(t.nsj.begin(), t.nsj.end(), (qgw::Q2*)(h.data() + ntw + n2));
   qgw::Q4* d;
   int rc = dalloc(r, &d, h.size());
   if (rc) return rc;
   CK(cudaMemcpyAsync(d, h.data(), h.size() * sizeof(h[0]), cudaMemcpyHostToDevice, r->stream));
+  *out = qgw::FxTables{};
   out->twq = d;
-  out->spq = d + ntw;
-  out->nsj = (const qgw::Q2*)(d + ntw + nsp);
+  (g.blue ? out->bc : out->spq) = d + ntw;
+  if (g.blue) out->bz = d + ntw + n2;
+  else out->nsj = (const qgw::Q2*)(d + ntw + n2);
+  out->be = t.be;
   return cudaStreamSynchronize(r->stream) == cudaSuccess ? QGW_OK : QGW_ERR_CUDA;
 }
 
@@ -215,7 +223,7 @@ int setup_args(qgw_run* r, StepArgs<T>& a) {
     const qgw::DstGeom& g = dim == 0 ? a.gx : a.gy;
     qgw::FxTables& f = dim == 0 ? a.fx : a.fy;
     f = qgw::FxTables{};
-    if (sizeof(T) == 8 && !per && !g.blue) {
+    if (sizeof(T) == 8) {
       if ((rc = upload_fx(r, &f, g))) return rc;
       continue;
     }

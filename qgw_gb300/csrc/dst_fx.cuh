@@ -79,7 +79,7 @@ __device__ __forceinline__ void fx_row_add(unsigned int* slot, int r, unsigned i
   }
 }
 
-// The row's sum of 2 - shift over the passes, and the split's shift
+// The row's sum of 2 - shift over the passes
 __device__ __forceinline__ int fx_drop(const FxScratch* sc, int r, int npass) {
   int d = 0;
   for (int p = 1; p < npass; ++p) d += 2 - fx_pass_shift(sc->mag[p - 1][r]);
@@ -87,8 +87,9 @@ __device__ __forceinline__ int fx_drop(const FxScratch* sc, int r, int npass) {
 }
 
 // ---- compile-time lengths H = 2^LGH >= 64
-// One Stockham pass (StockhamItem's indices, dst_fixed.cuh) over all rows.
-template <int R, int NS, int H>
+// One Stockham pass (StockhamItem's indices, dst_fixed.cuh) over all rows;
+// RAW (the first pass): of raw doubles, whose largest high words mag_in holds.
+template <int R, int NS, int H, bool RAW = false>
 __device__ __forceinline__ void fx_pass_fixed(const fx_t* src, fx_t* dst, int nrows, int ld, const Q4* tw,
                                               const unsigned int* mag_in, unsigned int* mag_out) {
   constexpr int NB = H / R, S = H / R;
@@ -102,6 +103,14 @@ __device__ __forceinline__ void fx_pass_fixed(const fx_t* src, fx_t* dst, int nr
     C2<fx_t> v[R];
 #pragma unroll
     for (int q = 0; q < R; ++q) v[q] = in[pco(q * S)];
+    if constexpr (RAW) {
+      const int E = fx_scale(mag_in[r]);
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        v[q].x = fx_from_bits((unsigned long long)v[q].x, E);
+        v[q].y = fx_from_bits((unsigned long long)v[q].y, E);
+      }
+    }
     if constexpr (NS > 1) fx_twiddle<R>(v, k, NS, fx_pass_shift(mag_in[r]), tw);
     fx_dft<R>(v);
 #pragma unroll
@@ -110,10 +119,42 @@ __device__ __forceinline__ void fx_pass_fixed(const fx_t* src, fx_t* dst, int nr
   }
 }
 
+// The passes of the complex FFT of 2^LGH points from src, dst the second
+// buffer; returns the buffer of the result, whose magnitudes are in
+// sc->mag[passes - 1].  Ends with the block synchronised.
+template <int LGH, bool RAW>
+__device__ __forceinline__ fx_t* fx_passes_fixed(fx_t* src, fx_t* dst, int nrows, int ld, const Q4* tw, FxScratch* sc) {
+  constexpr int H = 1 << LGH, NP8 = LGH / 3, RL = 1 << (LGH % 3);
+  static_assert(LGH >= 6 && NP8 <= 4, "two to four radix-8 passes");
+  auto turn = [&] {
+    __syncthreads();
+    fx_t* t = src;
+    src = dst;
+    dst = t;
+  };
+  fx_pass_fixed<8, 1, H, RAW>(src, dst, nrows, ld, nullptr, sc->mx, sc->mag[0]);
+  turn();
+  fx_pass_fixed<8, 8, H>(src, dst, nrows, ld, tw, sc->mag[0], sc->mag[1]);
+  turn();
+  if constexpr (NP8 >= 3) {
+    fx_pass_fixed<8, 64, H>(src, dst, nrows, ld, tw + 56, sc->mag[1], sc->mag[2]);
+    turn();
+  }
+  if constexpr (NP8 >= 4) {
+    fx_pass_fixed<8, 512, H>(src, dst, nrows, ld, tw + 504, sc->mag[2], sc->mag[3]);
+    turn();
+  }
+  if constexpr (RL > 1) {
+    constexpr int NS = 1 << (3 * NP8);
+    fx_pass_fixed<RL, NS, H>(src, dst, nrows, ld, tw + NS - 8, sc->mag[NP8 - 1], sc->mag[NP8]);
+    turn();
+  }
+  return src;
+}
+
 template <int LGH>
 __device__ fx_t* dst_fx_fixed(double* A, double* B, int nrows, int ld, const FxTables& tb, FxScratch* sc) {
-  constexpr int H = 1 << LGH, M = 2 * H, NP8 = LGH / 3, RL = 1 << (LGH % 3), NP = NP8 + (RL > 1 ? 1 : 0);
-  static_assert(LGH >= 6 && NP8 <= 3, "two or three radix-8 passes");
+  constexpr int H = 1 << LGH, M = 2 * H, NP = LGH / 3 + (LGH % 3 ? 1 : 0);
   const int tid = threadIdx.x, lane = tid & 31;
   // pre-processing, A -> B
   for (int w = tid; w < nrows * H; w += FX_NT) {
@@ -124,27 +165,8 @@ __device__ fx_t* dst_fx_fixed(double* A, double* B, int nrows, int ld, const FxT
     if (lane == 0) atomicAdd(&sc->l1[r], t);
   }
   __syncthreads();
-  fx_t* src = (fx_t*)B;
-  fx_t* dst = (fx_t*)A;
-  auto turn = [&] {
-    __syncthreads();
-    fx_t* t = src;
-    src = dst;
-    dst = t;
-  };
-  fx_pass_fixed<8, 1, H>(src, dst, nrows, ld, nullptr, nullptr, sc->mag[0]);
-  turn();
-  fx_pass_fixed<8, 8, H>(src, dst, nrows, ld, tb.twq, sc->mag[0], sc->mag[1]);
-  turn();
-  if constexpr (NP8 == 3) {
-    fx_pass_fixed<8, 64, H>(src, dst, nrows, ld, tb.twq + 56, sc->mag[1], sc->mag[2]);
-    turn();
-  }
-  if constexpr (RL > 1) {
-    constexpr int NS = 1 << (3 * NP8);
-    fx_pass_fixed<RL, NS, H>(src, dst, nrows, ld, tb.twq + NS - 8, sc->mag[NP8 - 1], sc->mag[NP8]);
-    turn();
-  }
+  fx_t* src = fx_passes_fixed<LGH, false>((fx_t*)B, (fx_t*)A, nrows, ld, tb.twq, sc);
+  fx_t* dst = src == (fx_t*)A ? (fx_t*)B : (fx_t*)A;
   // split: items k = 0..H/2-1, item 0 also k = H/2 (and R_0)
   {
     constexpr int KI = H / 2;
@@ -199,31 +221,35 @@ __device__ fx_t* dst_fx_fixed(double* A, double* B, int nrows, int ld, const FxT
 }
 
 // ---- any half-length that is a product of 2, 3, 5 and 7
-static __device__ __noinline__ fx_t* dst_fx_any(double* A, double* B, int nrows, int ld, const DstGeom& g, const FxTables& tb,
-                                                FxScratch* sc) {
-  const int H = g.H, M = g.M, tid = threadIdx.x, lane = tid & 31;
-  // items w of a phase with n items a row, whole warps at a time: f(row,
-  // item, whether the lane has one)
-  auto items = [&](int n, auto f) {
-    for (int w0 = tid - lane; w0 < nrows * n; w0 += FX_NT) {
-      const int w = min(w0 + lane, nrows * n - 1), r = w / n;
-      f(r, w - r * n, w0 + lane < nrows * n);
-    }
-  };
-  items(H, [&](int r, int i, bool on) {
-    unsigned int l = 0;
-    if (on)
-      l = fx_pre_item((const unsigned long long*)A + r * ld, (fx_t*)B + r * ld, i + 1, M, fx_scale(sc->mx[r]), tb.nsj);
-    fx_row_add(sc->l1, r, l);
-  });
-  __syncthreads();
-  fx_t* src = (fx_t*)B;
-  fx_t* dst = (fx_t*)A;
+// items w of a phase with n items a row, whole warps at a time: f(row, item,
+// whether the lane has one)
+template <typename F> __device__ __forceinline__ void fx_items(int nrows, int n, F f) {
+  const int lane = threadIdx.x & 31;
+  const unsigned int inv = 0xffffffffu / (unsigned int)n + 1;  // w / n exactly, w n < 2^32
+  for (int w0 = threadIdx.x - lane; w0 < nrows * n; w0 += FX_NT) {
+    const int w = min(w0 + lane, nrows * n - 1), r = n == 1 ? w : (int)__umulhi((unsigned int)w, inv);
+    f(r, w - r * n, w0 + lane < nrows * n);
+  }
+}
+template <bool RAW>
+__device__ __forceinline__ fx_t* fx_passes_any(fx_t* src, fx_t* dst, int nrows, int ld, const DstGeom& g, const Q4* twq,
+                                               FxScratch* sc) {
+  const int H = g.H;
+  if constexpr (RAW) {
+    fx_items(nrows, H, [&](int r, int e, bool on) {
+      if (!on) return;
+      fx_t* p = src + r * ld + 2 * pc<double>(e);
+      const int E = fx_scale(sc->mx[r]);
+      p[0] = fx_from_bits((unsigned long long)p[0], E);
+      p[1] = fx_from_bits((unsigned long long)p[1], E);
+    });
+    __syncthreads();
+  }
   int Ns = 1;
   for (int p = 0; p < g.npass; ++p) {
     const int R = g.radix[p];
-    const Q4* tw = tb.twq + (p ? Ns - g.radix[0] : 0);
-    items(H / R, [&](int r, int b, bool on) {
+    const Q4* tw = twq + (p ? Ns - g.radix[0] : 0);
+    fx_items(nrows, H / R, [&](int r, int b, bool on) {
       unsigned int m = 0;
       if (on)
         m = fx_stockham_dispatch(R, (const C2<fx_t>*)(src + r * ld), (C2<fx_t>*)(dst + r * ld), b, b % Ns, Ns, H,
@@ -236,7 +262,21 @@ static __device__ __noinline__ fx_t* dst_fx_any(double* A, double* B, int nrows,
     src = dst;
     dst = t;
   }
-  items(H / 2 + 1, [&](int r, int k, bool on) {
+  return src;
+}
+static __device__ __noinline__ fx_t* dst_fx_any(double* A, double* B, int nrows, int ld, const DstGeom& g, const FxTables& tb,
+                                                FxScratch* sc) {
+  const int H = g.H, M = g.M, tid = threadIdx.x, lane = tid & 31;
+  fx_items(nrows, H, [&](int r, int i, bool on) {
+    unsigned int l = 0;
+    if (on)
+      l = fx_pre_item((const unsigned long long*)A + r * ld, (fx_t*)B + r * ld, i + 1, M, fx_scale(sc->mx[r]), tb.nsj);
+    fx_row_add(sc->l1, r, l);
+  });
+  __syncthreads();
+  fx_t* src = fx_passes_any<false>((fx_t*)B, (fx_t*)A, nrows, ld, g, tb.twq, sc);
+  fx_t* dst = src == (fx_t*)A ? (fx_t*)B : (fx_t*)A;
+  fx_items(nrows, H / 2 + 1, [&](int r, int k, bool on) {
     if (!on) return;
     const int drop = fx_drop(sc, r, g.npass), s = fx_split_shift(sc->mag[g.npass - 1][r], sc->l1[r], drop);
     fx_split_item((const C2<fx_t>*)(src + r * ld), (C2<fx_t>*)(dst + r * ld), k, H, s, tb.spq);
@@ -264,15 +304,108 @@ static __device__ __noinline__ fx_t* dst_fx_any(double* A, double* B, int nrows,
   return dst;
 }
 
+// The complex FFT of g.H points (a power of two from 64 to 1024, or any
+// supported length) of nrows rows: src raw doubles (RAW) or integers.
+template <bool RAW>
+__device__ __forceinline__ fx_t* fx_cfft(fx_t* src, fx_t* dst, int nrows, int ld, const DstGeom& g, const Q4* twq,
+                                         FxScratch* sc) {
+  switch (g.H) {
+    case 64: return fx_passes_fixed<6, RAW>(src, dst, nrows, ld, twq, sc);
+    case 128: return fx_passes_fixed<7, RAW>(src, dst, nrows, ld, twq, sc);
+    case 256: return fx_passes_fixed<8, RAW>(src, dst, nrows, ld, twq, sc);
+    case 512: return fx_passes_fixed<9, RAW>(src, dst, nrows, ld, twq, sc);
+    case 1024: return fx_passes_fixed<10, RAW>(src, dst, nrows, ld, twq, sc);
+    default: return fx_passes_any<RAW>(src, dst, nrows, ld, g, twq, sc);
+  }
+}
+// Real FFT of raw rows (x_i at index i): 2 X_k, k = 0..H, as complex values at
+// index k, with the rows' exponents (of X_k) in sc->ex; and the inverse, c2r,
+// of raw spectral rows: x_{2m} = Re, x_{2m+1} = -Im of the value at index m.
+__device__ __forceinline__ fx_t* fx_rfft(double* A, double* B, int nrows, int ld, const DstGeom& g, const FxTables& tb,
+                                         FxScratch* sc) {
+  const int H = g.H;
+  fx_t* src = fx_cfft<true>((fx_t*)A, (fx_t*)B, nrows, ld, g, tb.twq, sc);
+  fx_t* dst = src == (fx_t*)A ? (fx_t*)B : (fx_t*)A;
+  fx_items(nrows, H / 2 + 1, [&](int r, int k, bool on) {
+    if (!on) return;
+    const int s = fx_rsplit_shift(sc->mag[g.npass - 1][r]);
+    fx_rsplit_item((const C2<fx_t>*)(src + r * ld), (C2<fx_t>*)(dst + r * ld), k, H, s, tb.spq);
+    // (fx_row_exp's exponent is one more than X's, and 2 X two: 2 X lies at
+    // fx_row_exp - 1, X one below)
+    if (k == 0) sc->ex[r] = fx_exp_add(fx_row_exp(sc->mx[r], fx_drop(sc, r, g.npass), s), -2);
+  });
+  __syncthreads();
+  return dst;
+}
+__device__ __forceinline__ fx_t* fx_irfft(double* A, double* B, int nrows, int ld, const DstGeom& g, const FxTables& tb,
+                                          FxScratch* sc) {
+  const int H = g.H;
+  fx_items(nrows, H / 2 + 1, [&](int r, int k, bool on) {
+    if (on) fx_rjoin_item((const C2<double>*)(A + r * ld), (C2<fx_t>*)(B + r * ld), k, H, fx_scale(sc->mx[r]), tb.spq);
+  });
+  __syncthreads();
+  fx_t* src = fx_cfft<false>((fx_t*)B, (fx_t*)A, nrows, ld, g, tb.twq, sc);
+  if (threadIdx.x < nrows) {
+    const int r = threadIdx.x;
+    sc->ex[r] = fx_exp_add(fx_row_exp(sc->mx[r], fx_drop(sc, r, g.npass), 0), 2);
+  }
+  __syncthreads();
+  return src;
+}
+// Chirp-z DST-I of raw rows (dst_blue.h), rows of L complex values, g.H = L;
+// sc: two scratches.  The result Y_k at index k.
+__device__ __forceinline__ fx_t* dst_fx_blue(double* A, double* B, int nrows, int ld, const DstGeom& g, const FxTables& tb,
+                                             FxScratch* sc) {
+  const int M = g.M, L = g.H;
+  auto passes = [&](fx_t* src, fx_t* dst, FxScratch* s) {
+    switch (L) {
+      case 64: return fx_passes_fixed<6, false>(src, dst, nrows, ld, tb.twq, s);
+      case 128: return fx_passes_fixed<7, false>(src, dst, nrows, ld, tb.twq, s);
+      case 256: return fx_passes_fixed<8, false>(src, dst, nrows, ld, tb.twq, s);
+      case 512: return fx_passes_fixed<9, false>(src, dst, nrows, ld, tb.twq, s);
+      case 1024: return fx_passes_fixed<10, false>(src, dst, nrows, ld, tb.twq, s);
+      case 2048: return fx_passes_fixed<11, false>(src, dst, nrows, ld, tb.twq, s);
+      case 4096: return fx_passes_fixed<12, false>(src, dst, nrows, ld, tb.twq, s);
+      default: return fx_passes_any<false>(src, dst, nrows, ld, g, tb.twq, s);
+    }
+  };
+  fx_items(nrows, L, [&](int r, int m, bool on) {
+    if (on)
+      fx_chirp_item((const unsigned long long*)A + r * ld, (C2<fx_t>*)((fx_t*)B + r * ld), m, M, fx_scale(sc->mx[r]), tb.bc);
+  });
+  __syncthreads();
+  fx_t* O = passes((fx_t*)B, (fx_t*)A, &sc[0]);
+  fx_items(nrows, L, [&](int r, int k, bool on) {
+    if (on) fx_chirp_mul_item((C2<fx_t>*)(O + r * ld), k, fx_pass_shift(sc[0].mag[g.npass - 1][r]), tb.bz);
+  });
+  __syncthreads();
+  fx_t* D = passes(O, O == (fx_t*)A ? (fx_t*)B : (fx_t*)A, &sc[1]);
+  fx_t* out = D == (fx_t*)A ? (fx_t*)B : (fx_t*)A;
+  fx_items(nrows, M, [&](int r, int k, bool on) {
+    if (!on) return;
+    const int s = fx_pass_shift(sc[1].mag[g.npass - 1][r]);
+    fx_chirp_out_item((const C2<fx_t>*)(D + r * ld), out + r * ld, k, s, tb.bc);
+    if (k == 0) {
+      // passes, product, passes, output (each product by a table / 4), 2 / L
+      const int drop = fx_drop(&sc[0], r, g.npass) + (2 - fx_pass_shift(sc[0].mag[g.npass - 1][r])) + tb.be +
+                       fx_drop(&sc[1], r, g.npass) + 2 + 1 - (31 - __clz(L));
+      sc->ex[r] = fx_exp_add(fx_row_exp(sc->mx[r], drop, s), -1);
+    }
+  });
+  __syncthreads();
+  return out;
+}
+
 // DST-I of nrows raw rows in A (x_j at index j; the block synchronised since
 // they were written, their largest high words noted), B the second buffer:
 // returns the buffer that holds Y_k at index k as integers of the rows'
 // exponents sc->ex.  HL: the half-length whose transform alone the kernel
-// holds, or 0.
+// holds, 0, or -1 for the chirp-z lengths.
 template <int HL>
 __device__ __forceinline__ fx_t* dst_fx(double* A, double* B, int nrows, int ld, const DstGeom& g, const FxTables& tb,
                                         FxScratch* sc) {
   if constexpr (HL == 512) return dst_fx_fixed<9>(A, B, nrows, ld, tb, sc);
+  if constexpr (HL == -1) return dst_fx_blue(A, B, nrows, ld, g, tb, sc);
   switch (g.H) {
     case 64: return dst_fx_fixed<6>(A, B, nrows, ld, tb, sc);
     case 128: return dst_fx_fixed<7>(A, B, nrows, ld, tb, sc);

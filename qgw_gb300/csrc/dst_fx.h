@@ -43,6 +43,8 @@ QGW_HD Q2 q2_split(fx_t w) {
   q.h = (int)(w >> 32) - (q.l >> 31);
   return q;
 }
+// of a constant: l is never -2^31 (fx_mul negates it)
+QGW_HD Q2 q2_const(fx_t w) { return q2_split((int)w == (int)0x80000000 ? w + 1 : w); }
 
 // Tables: twq the pass twiddles (cos, -sin) scaled by 2^62, in the order of
 // fill_pass_twiddles; nsj -s_j scaled by 2^63, j <= H (s_H = 1 has no
@@ -53,10 +55,14 @@ struct ModeTable {
   const Q2* c;   // nl x nl, row m: output m
   const int* e;  // nl
 };
+// Chirp-z lengths (dst_blue.h): twq of the L-point FFT, bc the chirp c_m
+// scaled by 2^62, m < M, bz the transform of its conjugate scaled by 2^(62 - be).
 struct FxTables {
   const Q4* twq;
   const Q2* nsj;
   const Q4* spq;
+  const Q4 *bc, *bz;
+  int be;
 };
 
 QGW_HD int fx_mh(int a, int b) {
@@ -75,19 +81,33 @@ QGW_HD int fx_clz(unsigned int v) {
 }
 
 // v w / 2^64 to within one unit: one 32 x 32 -> 64 product and the high
-// words of the two cross products (their truncations, half a unit each on
-// average, are added back).  |v| < 2^61.5.
+// words of the two cross products, one truncated down and the other, of the
+// negated constant, up: the errors cancel on average and a zero gives zero
+// (a constant added against two truncations down would be an error of one
+// sign wherever a product is exact -- zeros, or a factor of one -- and a
+// transform adds those up in one bin).  |v| < 2^61.5; no constant has l =
+// -2^31.
 QGW_HD fx_t fx_mul(fx_t v, Q2 w) {
   const Q2 a = q2_split(v);
-  return (fx_t)a.h * w.h + (fx_t)(fx_mh(a.h, w.l) + fx_mh(a.l, w.h) + 1);
+  return (fx_t)a.h * w.h + (fx_t)(fx_mh(a.l, w.h) - fx_mh(a.h, -w.l));
 }
-// (x + iy) w / 2^64, |w| components at most 2^62
-QGW_HD void fx_cmul(fx_t& x, fx_t& y, const Q4& w) {
+// (x + iy) w / 2^64, |w| components at most 2^62.  UP: the truncations the
+// other way round, which matters for a factor of one (l = 0), whose remaining
+// one is then up instead of down: the members of a butterfly alternate.
+template <bool UP = false> QGW_HD void fx_cmul(fx_t& x, fx_t& y, const Q4& w) {
   const Q2 a = q2_split(x), b = q2_split(y);
-  const int t1 = fx_mh(a.h, w.x.l) + fx_mh(a.l, w.x.h), t2 = fx_mh(b.h, w.y.l) + fx_mh(b.l, w.y.h);
-  const int t3 = fx_mh(a.h, w.y.l) + fx_mh(a.l, w.y.h) + fx_mh(b.h, w.x.l) + fx_mh(b.l, w.x.h) + 2;
-  x = ((fx_t)a.h * w.x.h + (fx_t)(t1 - t2)) - (fx_t)b.h * w.y.h;
-  y = (fx_t)b.h * w.x.h + ((fx_t)a.h * w.y.h + (fx_t)t3);
+  int t1, t2;
+  if (UP) {
+    const int nx = -w.x.h, ny = -w.y.h;
+    t1 = fx_mh(a.h, w.x.l) + fx_mh(b.l, ny) - fx_mh(a.l, nx) - fx_mh(b.h, w.y.l);
+    t2 = fx_mh(a.h, w.y.l) + fx_mh(b.h, w.x.l) - fx_mh(a.l, ny) - fx_mh(b.l, nx);
+  } else {
+    const int nx = -w.x.l, ny = -w.y.l;
+    t1 = fx_mh(a.l, w.x.h) + fx_mh(b.h, ny) - fx_mh(a.h, nx) - fx_mh(b.l, w.y.h);
+    t2 = fx_mh(a.l, w.y.h) + fx_mh(b.l, w.x.h) - fx_mh(a.h, ny) - fx_mh(b.h, nx);
+  }
+  x = ((fx_t)a.h * w.x.h + (fx_t)t1) - (fx_t)b.h * w.y.h;
+  y = (fx_t)b.h * w.x.h + ((fx_t)a.h * w.y.h + (fx_t)t2);
 }
 // v c for a constant c = B + f, |f| < 1/2, f scaled by 2^64
 template <int B> QGW_HD fx_t fx_mulc(fx_t v, int h, int l) {
@@ -265,7 +285,10 @@ template <int R> QGW_HD void fx_twiddle(C2<fx_t>* v, int k, int Ns, int s, const
   v[0].x = fx_shr(v[0].x, 2);
   v[0].y = fx_shr(v[0].y, 2);
 #pragma unroll
-  for (int q = 1; q < R; ++q) fx_cmul(v[q].x, v[q].y, tw[(q - 1) * Ns + k]);
+  for (int q = 1; q < R; ++q) {
+    if (q & 1) fx_cmul<true>(v[q].x, v[q].y, tw[(q - 1) * Ns + k]);
+    else fx_cmul<false>(v[q].x, v[q].y, tw[(q - 1) * Ns + k]);
+  }
 }
 template <int R> QGW_HD unsigned int fx_mag_all(const C2<fx_t>* v) {
   unsigned int m = 0;
@@ -321,6 +344,8 @@ QGW_HD int fx_row_exp(unsigned int mx, int drop, int s) {
   return mx == 0 ? FX_ZERO : mx >= 0x7ff00000u ? FX_NAN : fx_scale(mx) - FX_EOFF + 1 + drop - s;
 }
 
+QGW_HD int fx_exp_add(int ex, int d) { return ex == FX_NAN || ex == FX_ZERO ? ex : ex + d; }
+
 QGW_HD void fx_split_pair(C2<fx_t> A, C2<fx_t> B, const Q4& cs, C2<fx_t>& lo, C2<fx_t>& hi) {
   const fx_t sr = A.x + B.x, si = A.y - B.y, dr = 2 * (A.x - B.x), di = 2 * (A.y + B.y);
   const fx_t P = fx_mul(di, cs.x) + fx_mul(dr, cs.y);  // c di - s dr
@@ -348,6 +373,93 @@ QGW_HD void fx_split_item(const C2<fx_t>* Z, C2<fx_t>* o, int k, int H, int s, c
   fx_split_pair(fx_shift2(Z[pc<double>(k)], s), fx_shift2(Z[pc<double>(H - k)], s), spq[k], lo, hi);
   o[pc<double>(k)] = lo;
   if (2 * k != H) o[pc<double>(H - k)] = hi;
+}
+
+// ---- real FFT of N = 2H reals (periodic.cuh's forms), scaled by 2: the split
+// of Z (below 2^59) into 2 X_k, 2 X_{H-k}, 1 <= k <= H/2, cs = spq[k]
+QGW_HD int fx_rsplit_shift(unsigned int mag) { return 27 - (32 - fx_clz(mag)); }
+QGW_HD void fx_rsplit_pair(C2<fx_t> A, C2<fx_t> B, const Q4& cs, C2<fx_t>& xk, C2<fx_t>& xh) {
+  const fx_t Pr = A.x + B.x, Pi = A.y - B.y, Qr = 2 * (A.x - B.x), Qi = 2 * (A.y + B.y);
+  const fx_t Vr = fx_mul(Qi, cs.x) + fx_mul(Qr, cs.y);  // c Qi - s Qr
+  const fx_t Vi = fx_mul(Qi, cs.y) - fx_mul(Qr, cs.x);  // -(c Qr + s Qi)
+  xk.x = Pr + Vr; xk.y = Pi + Vi;
+  xh.x = Pr - Vr; xh.y = Vi - Pi;
+}
+// and its inverse: conj Z'_k, conj Z'_{H-k} of X_k, X_{H-k} (below 2^59),
+// divided by 8 (below 2^59 again)
+QGW_HD void fx_rjoin_pair(C2<fx_t> a, C2<fx_t> b, const Q4& cs, C2<fx_t>& zk, C2<fx_t>& zh) {
+  const fx_t Pr = a.x + b.x, Pi = a.y - b.y, Qr = 2 * (a.x - b.x), Qi = 2 * (a.y + b.y);
+  const fx_t Ui = fx_mul(Qr, cs.x) + fx_mul(Qi, cs.y);  // c Qr - s Qi
+  const fx_t Ur = fx_mul(Qr, cs.y) - fx_mul(Qi, cs.x);  // -(c Qi + s Qr)
+  zk.x = fx_shr(Pr + Ur, 3); zk.y = -fx_shr(Pi + Ui, 3);
+  zh.x = fx_shr(Pr - Ur, 3); zh.y = fx_shr(Pi - Ui, 3);
+}
+// item k = 0..H/2 of the join from raw doubles X (k complex values) to Z
+QGW_HD C2<fx_t> fx_raw2(const C2<double>* x, int k, int E) {
+  const unsigned long long* p = (const unsigned long long*)(x + pc<double>(k));
+  C2<fx_t> v;
+  v.x = fx_from_bits(p[0], E);
+  v.y = fx_from_bits(p[1], E);
+  return v;
+}
+QGW_HD void fx_rjoin_item(const C2<double>* X, C2<fx_t>* Z, int k, int H, int E, const Q4* spq) {
+  C2<fx_t> a = fx_raw2(X, k, E), b = fx_raw2(X, H - k, E), zk, zh;
+  if (k == 0) {
+    // X_0 and X_H are real: Z'_0 = (X_0 + X_H) + i (X_0 - X_H)
+    zk.x = fx_shr(a.x + b.x, 3);
+    zk.y = -fx_shr(a.x - b.x, 3);
+    Z[0] = zk;
+    return;
+  }
+  fx_rjoin_pair(a, b, spq[k], zk, zh);
+  Z[pc<double>(k)] = zk;
+  if (2 * k != H) Z[pc<double>(H - k)] = zh;
+}
+QGW_HD void fx_rsplit_item(const C2<fx_t>* Z, C2<fx_t>* X, int k, int H, int s, const Q4* spq) {
+  if (k == 0) {
+    const C2<fx_t> a = fx_shift2(Z[0], s);
+    C2<fx_t> x0, xH;
+    x0.x = 2 * (a.x + a.y); x0.y = 0;
+    xH.x = 2 * (a.x - a.y); xH.y = 0;
+    X[0] = x0;
+    X[pc<double>(H)] = xH;
+    return;
+  }
+  C2<fx_t> xk, xh;
+  fx_rsplit_pair(fx_shift2(Z[pc<double>(k)], s), fx_shift2(Z[pc<double>(H - k)], s), spq[k], xk, xh);
+  X[pc<double>(k)] = xk;
+  if (2 * k != H) X[pc<double>(H - k)] = xh;
+}
+
+// ---- chirp-z DST-I (dst_blue.h)
+// z_m = x_m c_m (the value below 2^61, its product / 4), zero outside 1 <= m <
+// M, of a raw row
+QGW_HD void fx_chirp_item(const unsigned long long* x, C2<fx_t>* z, int m, int M, int E, const Q4* bc) {
+  C2<fx_t> v;
+  v.x = v.y = 0;
+  if (m >= 1 && m < M) {
+    const fx_t X = fx_from_bits<8>(x[pr<double>(m)], E);
+    v.x = fx_mul(X, bc[m].x);
+    v.y = fx_mul(X, bc[m].y);
+  }
+  z[pc<double>(m)] = v;
+}
+// conj(z_k bz_k) / 4 of the row shifted by s to below 2^61, in place
+QGW_HD void fx_chirp_mul_item(C2<fx_t>* z, int k, int s, const Q4* bz) {
+  C2<fx_t> v = fx_shift2(z[pc<double>(k)], s);
+  fx_cmul(v.x, v.y, bz[k]);
+  v.y = -v.y;
+  z[pc<double>(k)] = v;
+}
+// Im(c_k conj d_k) / 4 of the row shifted by s, into y (index k); Y_k is 2 / L
+// times it
+QGW_HD void fx_chirp_out_item(const C2<fx_t>* d, fx_t* y, int k, int s, const Q4* bc) {
+  if (k == 0) {
+    y[0] = 0;
+    return;
+  }
+  const C2<fx_t> v = fx_shift2(d[pc<double>(k)], s);
+  y[pr<double>(k)] = fx_mul(v.x, bc[k].y) - fx_mul(v.y, bc[k].x);
 }
 
 }  // namespace qgw

@@ -84,7 +84,7 @@ inline DstTablesHost build_dst_tables(int M) {
   return t;
 }
 
-// cos and -sin of pi m / N scaled by 2^b, b = 62 or 63, N up to 2^14, by
+// cos and -sin of pi m / N scaled by 2^b, b <= 63, N up to 2^14, by
 // their Taylor series in 64-bit fixed point to 2^-61: the fixed-point
 // transform (dst_fx.h) rounds at 2^-57, so it would feel the rounding of a
 // double.  At b = 63 a value of +1 does not fit (no table holds one).
@@ -115,16 +115,15 @@ inline Q4 sincospi_fixed(long m, long N, int b) {
   if (swap) std::swap(S, C);
   // two's complement negation carries 2^63 to the value -1 has
   Q4 w;
-  w.x = q2_split((fx_t)(half != refl ? 0 - C : C));
-  w.y = q2_split((fx_t)(half ? S : 0 - S));
+  w.x = q2_const((fx_t)(half != refl ? 0 - C : C));
+  w.y = q2_const((fx_t)(half ? S : 0 - S));
   return w;
 }
 
 // The tables of the fixed-point transform (dst_fx.h) of geometry g, into
 // arrays of fx_twq_len, H/2 + 1 and H + 1 entries.
 inline size_t fx_twq_len(const DstGeom& g) { return (size_t)(g.npass ? g.H - g.radix[0] : 0) + 1; }
-inline void fill_fx_tables(const DstGeom& g, Q4* twq, Q4* spq, Q2* nsj) {
-  const int H = g.H, M = g.M;
+inline void fill_fx_twiddles(const DstGeom& g, Q4* twq) {
   int Ns = g.radix[0];
   for (int p = 1; p < g.npass; ++p) {
     const int R = g.radix[p];
@@ -132,20 +131,70 @@ inline void fill_fx_tables(const DstGeom& g, Q4* twq, Q4* spq, Q2* nsj) {
       for (int k = 0; k < Ns; ++k) twq[(Ns - g.radix[0]) + (q - 1) * Ns + k] = sincospi_fixed(2L * q * k, (long)Ns * R, 62);
     Ns *= R;
   }
+}
+inline void fill_fx_tables(const DstGeom& g, Q4* twq, Q4* spq, Q2* nsj) {
+  const int H = g.H, M = g.M;
+  fill_fx_twiddles(g, twq);
   spq[0] = Q4{};
   for (int k = 1; k <= H / 2; ++k) spq[k] = sincospi_fixed(2L * k, M, 63);
   for (int j = 0; j <= H; ++j) nsj[j] = sincospi_fixed(j, M, 63).y;
 }
+// The chirp-z tables of g (g.blue): bc (M entries), bz (L = g.H entries) and
+// bz's exponent.  bz is the transform's own FFT of the conjugate chirp, run
+// with the device's work items; twq: g's pass twiddles.
+inline int fill_fx_blue(const DstGeom& g, const Q4* twq, Q4* bc, Q4* bz) {
+  const int M = g.M, L = g.H;
+  std::vector<C2<fx_t>> a((size_t)pc<double>(L) + 1, C2<fx_t>{0, 0}), b(a.size());
+  auto join = [](Q2 q) { return ((fx_t)q.h << 32) + q.l; };
+  for (int m = 0; m < M; ++m) {
+    const long e = ((long)m * m) % (4L * M);  // exp(i pi e / 2M)
+    bc[m] = sincospi_fixed(-e, 2L * M, 62);
+    // b at d mod L, d in (-M, M): conj(c_|d|)
+    const Q4 w = sincospi_fixed(e, 2L * M, 58);
+    a[pc<double>(m)].x = a[pc<double>((L - m) % L)].x = join(w.x);
+    a[pc<double>(m)].y = a[pc<double>((L - m) % L)].y = join(w.y);
+  }
+  C2<fx_t>*src = a.data(), *dst = b.data();
+  int Ns = 1, drop = 0;
+  unsigned int mag = 0;
+  for (int p = 0; p < g.npass; ++p) {
+    const int R = g.radix[p], s = p ? fx_pass_shift(mag) : 0;
+    if (p) drop += 2 - s;
+    mag = 0;
+    for (int i = 0; i < L / R; ++i)
+      mag |= fx_stockham_dispatch(R, src, dst, i, i % Ns, Ns, L, s, twq + (p ? Ns - g.radix[0] : 0));
+    Ns *= R;
+    std::swap(src, dst);
+  }
+  double mx = 0;
+  for (int k = 0; k < L; ++k) mx = std::fmax(mx, std::hypot((double)src[pc<double>(k)].x, (double)src[pc<double>(k)].y));
+  int e;
+  std::frexp(mx, &e);  // modulus < 2^e: up to 2^62
+  const int up = 62 - e;
+  for (int k = 0; k < L; ++k) {
+    const C2<fx_t> v = fx_shift2(src[pc<double>(k)], up);
+    bz[k] = Q4{q2_const(v.x), q2_const(v.y)};
+  }
+  return 62 - 58 + drop - up;  // value = bz 2^(drop - 58 - up)
+}
 struct FxTablesHost {
-  std::vector<Q4> twq, spq;
+  std::vector<Q4> twq, spq, bc, bz;
   std::vector<Q2> nsj;
+  int be = 0;
 };
 inline FxTablesHost build_fx_tables(const DstGeom& g) {
   FxTablesHost t;
   t.twq.resize(fx_twq_len(g));
   t.spq.resize((size_t)g.H / 2 + 1);
   t.nsj.resize((size_t)g.H + 1);
-  fill_fx_tables(g, t.twq.data(), t.spq.data(), t.nsj.data());
+  if (g.blue) {
+    fill_fx_twiddles(g, t.twq.data());
+    t.bc.resize(g.M);
+    t.bz.resize(g.H);
+    t.be = fill_fx_blue(g, t.twq.data(), t.bc.data(), t.bz.data());
+  } else {
+    fill_fx_tables(g, t.twq.data(), t.spq.data(), t.nsj.data());
+  }
   return t;
 }
 
@@ -169,7 +218,7 @@ inline void fill_mode_table(int nl, const double* mat, Q2* c, int* e) {
     double mx = 0;
     for (int l = 0; l < nl; ++l) mx = std::fmax(mx, std::fabs(mat[(size_t)m * nl + l]));
     std::frexp(mx, &e[m]);
-    for (int l = 0; l < nl; ++l) c[m * nl + l] = q2_split((fx_t)std::nearbyint(std::ldexp(mat[(size_t)m * nl + l], 60 - e[m])));
+    for (int l = 0; l < nl; ++l) c[m * nl + l] = q2_const((fx_t)std::nearbyint(std::ldexp(mat[(size_t)m * nl + l], 60 - e[m])));
   }
 }
 

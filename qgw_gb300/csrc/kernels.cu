@@ -23,14 +23,15 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) k_rows_fwd(StepArg
   grid_wait();
   body_rows_fwd<T, COMP, PER, HL>(a, step_mode, blockIdx.x, smem_raw + cst_bytes<T>(a.nl), tot, (T*)smem_raw);
 }
-// CT: columns per tile (closed basin; the periodic kernel takes two complex
-// columns whatever CT)
+// CT: columns per tile (closed basin, and complex columns in FP64; the FP32
+// periodic kernel takes two complex columns whatever CT)
 template <typename T, bool COMP, bool PER, int CT, int HL>
-__global__ void __launch_bounds__(NT, 3) k_cols(StepArgs<T> a, int step_mode) {
+__global__ void __launch_bounds__(NT, 3) k_cols(const __grid_constant__ StepArgs<T> a, int step_mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ __align__(16) T tot[tot_len<T>];
+  __shared__ __align__(16) T tot[tot_len<T, HL>];
   grid_wait();
-  if (PER) body_cols_per<T, COMP>(a, step_mode, blockIdx.x, blockIdx.y, smem_raw);
+  if constexpr (PER && sizeof(T) == 8) body_cols_per_fx<CT>(a, step_mode, blockIdx.x, blockIdx.y, smem_raw, tot);
+  else if constexpr (PER) body_cols_per<T, COMP>(a, step_mode, blockIdx.x, blockIdx.y, smem_raw);
   else body_cols<T, COMP, CT, HL>(a, step_mode, blockIdx.x, blockIdx.y, smem_raw, tot);
 }
 template <typename T> constexpr int CTD = ColsPer<T>::value;
@@ -81,11 +82,11 @@ __global__ void __launch_bounds__(NT, 2) k_modes(const __grid_constant__ StepArg
   else if (j < a.ny) modes_point<NL, FWD>(a, tb, u, j, i, cs);
 }
 template <bool PER, int HL, bool INV>
-__global__ void __launch_bounds__(NT, 3) k_rows_f64(StepArgs<double> a, int step_mode) {
+__global__ void __launch_bounds__(NT, 3) k_rows_f64(const __grid_constant__ StepArgs<double> a, int step_mode) {
   grid_wait();
   if (step_mode && !a.state->active) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ __align__(16) double tot[tot_len<double>];
+  __shared__ __align__(16) double tot[tot_len<double, HL>];
   const int rows = INV ? a.RB3 : a.RB1, r0 = blockIdx.x * rows;
   double* A = (double*)smem_raw;
   rows_f64<PER, HL, INV>(a, INV ? a.psi : a.spec, r0, min(rows, a.nl * a.ny - r0), -1, A,
@@ -378,7 +379,8 @@ static cudaError_t set_attrs(const StepArgs<T>& a) {
       (const void*)k_cols<T, COMP, false, CTD<T>, 0>,     (const void*)k_cols<T, COMP, false, CTD<T>, 512>,
       (const void*)k_cols<T, COMP, false, CTD<T> / 2, 0>, (const void*)k_cols<T, COMP, false, CTD<T> / 2, 512>,
       (const void*)k_cols<T, COMP, false, CTD<T> / 2, -1>, (const void*)k_cols<T, COMP, false, 1, -1>,
-      (const void*)k_cols<T, COMP, true, CTD<T>, 0>};
+      (const void*)k_cols<T, COMP, true, CTD<T>, 0>,
+      (const void*)k_cols<T, COMP, true, sizeof(T) == 8 ? 2 : CTD<T>, 0>};
   for (const void* f : columns)
     if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, lim))) return e;
   if constexpr (sizeof(T) == 8) {
@@ -468,6 +470,16 @@ static void launch_k2(const StepArgs<T>& a, int step_mode, bool pdl, cudaStream_
   const dim3 grid(col_tiles(a), a.nl);
   const size_t sm = smem_cols<T, COMP>(a);
   const bool wide = col_width(a) == CTD<T>, h512 = a.gy.H == 512 && !a.gy.blue;
+  if constexpr (sizeof(T) == 8) {
+    if (a.periodic) {
+      const int cc = per_cols(a);
+      const dim3 tiles((a.gx.H + cc) / cc, a.nl);
+      const size_t bytes = (size_t)2 * cc * row_len<T>(a.gy) * sizeof(T);
+      if (cc == 4) launch(k_cols<T, COMP, true, 4, 0>, tiles, dim3(NT), bytes, s, pdl, a, step_mode);
+      else launch(k_cols<T, COMP, true, 2, 0>, tiles, dim3(NT), bytes, s, pdl, a, step_mode);
+      return;
+    }
+  }
   if (a.periodic) launch(k_cols<T, COMP, true, CTD<T>, 0>, grid, dim3(NT), sm, s, pdl, a, step_mode);
   else if (a.gy.blue && col_width(a) == 1) launch(k_cols<T, COMP, false, 1, -1>, grid, dim3(NT), sm, s, pdl, a, step_mode);
   else if (a.gy.blue) launch(k_cols<T, COMP, false, CTD<T> / 2, -1>, grid, dim3(NT), sm, s, pdl, a, step_mode);

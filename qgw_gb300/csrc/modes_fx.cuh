@@ -260,7 +260,6 @@ __device__ __forceinline__ void modes_point_any(const StepArgs<double>& a, const
 template <bool PER, int HL, bool INV>
 __device__ __forceinline__ void rows_f64(const StepArgs<double>& a, double* F, int r0, int nr, int row_j, double* A,
                                          double* B, double* tot) {
-  constexpr bool FX = fx_path<double, PER, HL>;
   FxScratch* sc = (FxScratch*)tot;
   const int ld = row_len<double>(a.gx), xo = PER ? 0 : 1;
   const int nin = PER && INV ? a.nx + 2 : a.nx, nout = PER && !INV ? a.nx + 2 : a.nx;
@@ -268,35 +267,31 @@ __device__ __forceinline__ void rows_f64(const StepArgs<double>& a, double* F, i
     const int l = row_j >= 0 ? r0 + r : (r0 + r) / a.ny, j = row_j >= 0 ? row_j : r0 + r - l * a.ny;
     return F + (size_t)l * a.lstride + (size_t)j * a.pitch;
   };
-  if constexpr (FX) {
-    fx_clear(sc);
-    __syncthreads();
-  }
+  for (int n = 0; n < (HL == -1 ? 2 : 1); ++n) fx_clear(&sc[n]);
+  __syncthreads();
   for (int r = 0; r < nr; ++r) {
     const double* src = row(r);
     unsigned int h = 0;
     for (int i = threadIdx.x; i < nin; i += NT) {
       const double v = src[i];
       A[r * ld + pr<double>(i + xo)] = v;
-      if constexpr (FX) h = max(h, fx_hi(v));
+      h = max(h, fx_hi(v));
     }
-    if constexpr (FX) fx_note_max(sc, r, h);
+    fx_note_max(sc, r, h);
   }
   __syncthreads();
-  const double* O;
-  if constexpr (FX) O = (const double*)dst_fx<HL>(A, B, nr, ld, a.gx, a.fx, sc);
-  else if constexpr (!PER) O = dst_block<double, HL>(A, B, nr, ld, a.gx, a.tx, tot);
-  else if constexpr (INV) O = irfft_block<double>(A, B, nr, ld, a.gx, a.tx);
-  else O = rfft_block<double>(A, B, nr, ld, a.gx, a.tx);
+  const fx_t* O;
+  if constexpr (!PER) O = dst_fx<HL>(A, B, nr, ld, a.gx, a.fx, sc);
+  else if constexpr (INV) O = fx_irfft(A, B, nr, ld, a.gx, a.fx, sc);
+  else O = fx_rfft(A, B, nr, ld, a.gx, a.fx, sc);
   grid_next();
   for (int r = 0; r < nr; ++r) {
     double* dst = row(r);
-    const int ex = FX ? sc->ex[r] : 0;
+    const int ex = sc->ex[r];
     for (int i = threadIdx.x; i < nout; i += NT) {
-      const double v = O[r * ld + pr<double>(i + xo)];
-      if constexpr (FX) dst[i] = fx_out(__double_as_longlong(v), ex);
+      const double v = fx_out(O[r * ld + pr<double>(i + xo)], ex);
       // the backward FFT's x_{2m+1} is minus its imaginary part
-      else dst[i] = PER && INV && (i & 1) ? -v : v;
+      dst[i] = PER && INV && (i & 1) ? -v : v;
     }
   }
   __syncthreads();

@@ -111,7 +111,7 @@ void fill_tables(int M, double* dst) {
   qgw::fill_fx_tables(qgw::make_geom(M), (qgw::Q4*)dst, (qgw::Q4*)(dst + kTwq), (qgw::Q2*)(dst + kTwq + kSpq));
 }
 qgw::FxTables tables_at(const double* p) {
-  return qgw::FxTables{(const qgw::Q4*)p, (const qgw::Q2*)(p + kTwq + kSpq), (const qgw::Q4*)(p + kTwq)};
+  return qgw::FxTables{(const qgw::Q4*)p, (const qgw::Q2*)(p + kTwq + kSpq), (const qgw::Q4*)(p + kTwq), nullptr, nullptr, 0};
 }
 
 // a grid size of a closed basin the transforms take (the run path's rule:

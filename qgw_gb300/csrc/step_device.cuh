@@ -128,8 +128,7 @@ __device__ __forceinline__ T* dst_block_blue(T* A, T* B, int nrows, int ld, cons
   return out;
 }
 
-// Block DST of FP32 rows of any supported length, and the chirp-z form of
-// both precisions (FP64 rows of the other lengths: dst_fx).  The power-of-two
+// Block DST of FP32 rows of any supported length (FP64: dst_fx).  The power-of-two
 // lengths M = 128..2048 use the compile-time specialisations of
 // dst_fixed.cuh (M = 512 and 1024: one warp per row, in place, the result in
 // A), others (mixed radix 2, 3, 5, 7) the generic loops.
@@ -140,10 +139,10 @@ __device__ __forceinline__ T* dst_block_blue(T* A, T* B, int nrows, int ld, cons
 template <typename T, int HL = 0>
 __device__ __forceinline__ T* dst_block(T* A, T* B, int nrows, int ld, const DstGeom& g, const DstTables<T>& tb,
                                         T* tot) {
-  if constexpr (HL == -1) {
+  if constexpr (sizeof(T) == 8) {
+    return A;  // (never: body_cols has left through body_cols_fx)
+  } else if constexpr (HL == -1) {
     return dst_block_blue<T>(A, B, nrows, ld, g, tb);
-  } else if constexpr (sizeof(T) == 8) {
-    return A;
   } else if constexpr (HL == 512) {
     return dst_block_warp_f32<9>(A, nrows, ld, tb);
   } else {
@@ -160,11 +159,11 @@ __device__ __forceinline__ T* dst_block(T* A, T* B, int nrows, int ld, const Dst
 
 // The FP64 closed-basin transforms other than the chirp-z ones run in fixed
 // point (dst_fx.cuh); the block's scratch for them lies in tot.
-template <typename T, bool PER, int HL> constexpr bool fx_path = sizeof(T) == 8 && !PER && HL != -1;
-// values of tot: FP64 two scratches (the column kernel's two transforms),
-// which leaves room for a third 1024-point column block per SM; FP32 the
+// values of tot: FP64 two scratches (the column kernel's two transforms; the
+// chirp-z form, two FFTs a transform, four), which leaves room for a third 1024-point column block per SM; FP32 the
 // chunk totals of the generic transform
-template <typename T> constexpr int tot_len = sizeof(T) == 8 ? (int)(2 * sizeof(FxScratch) / sizeof(T)) : GMAX * 32;
+template <typename T, int HL = 0>
+constexpr int tot_len = sizeof(T) == 8 ? (int)((HL == -1 ? 4 : 2) * sizeof(FxScratch) / sizeof(T)) : GMAX * 32;
 static_assert(GMAX <= FX_ROWS && NT == FX_NT, "a scratch holds every row");
 __device__ __forceinline__ void slabs(int si, int& s0, int& s1, int& s2) {
   const int m = si % 3;
@@ -620,7 +619,9 @@ template <int CT, int HL>
 __device__ __forceinline__ void body_cols_fx(const StepArgs<double>& a, int k0, int CTb, int m, double* A, double* B,
                                              int ld, bool vec, FxScratch* sc) {
   const int ny = a.ny;
-  fx_t* O = dst_fx<HL>(A, B, CT, ld, a.gy, a.fy, &sc[0]);
+  constexpr bool VEC = CT * sizeof(double) % 16 == 0;
+  FxScratch* const sinv = sc + (HL == -1 ? 2 : 1);
+  fx_t* O = dst_fx<HL>(A, B, CT, ld, a.gy, a.fy, sc);
   unsigned int hmax[CT];
   int ex[CT];
 #pragma unroll
@@ -632,8 +633,10 @@ __device__ __forceinline__ void body_cols_fx(const StepArgs<double>& a, int k0, 
     if (jj < 0) continue;
     const double* hrow = a.hinv + (size_t)m * a.lstride + (size_t)jj * a.pitch + k0;
     double h[CT];
-    if (vec) load_cols<double, CT>(hrow, h);
-    else
+    if constexpr (VEC) {
+      if (vec) load_cols<double, CT>(hrow, h);
+    }
+    if (!vec)
       for (int c = 0; c < CT; ++c) h[c] = c < CTb ? hrow[c] : 0.0;
     const int pj = pr<double>(jj + 1);
 #pragma unroll
@@ -644,12 +647,12 @@ __device__ __forceinline__ void body_cols_fx(const StepArgs<double>& a, int k0, 
     }
   }
 #pragma unroll
-  for (int c = 0; c < CT; ++c) fx_note_max(&sc[1], c, hmax[c]);
+  for (int c = 0; c < CT; ++c) fx_note_max(sinv, c, hmax[c]);
   __syncthreads();
   fx_t* Oth = O == (fx_t*)A ? (fx_t*)B : (fx_t*)A;
-  const fx_t* O2 = dst_fx<HL>((double*)O, (double*)Oth, CT, ld, a.gy, a.fy, &sc[1]);
+  const fx_t* O2 = dst_fx<HL>((double*)O, (double*)Oth, CT, ld, a.gy, a.fy, sinv);
 #pragma unroll
-  for (int c = 0; c < CT; ++c) ex[c] = sc[1].ex[c];
+  for (int c = 0; c < CT; ++c) ex[c] = sinv->ex[c];
   grid_next();
   for (int jj = (int)threadIdx.x - 1; jj < ny; jj += NT) {
     if (jj < 0) continue;
@@ -658,8 +661,10 @@ __device__ __forceinline__ void body_cols_fx(const StepArgs<double>& a, int k0, 
 #pragma unroll
     for (int c = 0; c < CT; ++c) v[c] = c < CTb ? fx_out(O2[c * ld + pj], ex[c]) : 0.0;
     double* dst = a.spec + (size_t)m * a.lstride + (size_t)jj * a.pitch + k0;
-    if (vec) store_cols<double, CT>(dst, v);
-    else
+    if constexpr (VEC) {
+      if (vec) store_cols<double, CT>(dst, v);
+    }
+    if (!vec)
       for (int c = 0; c < CTb; ++c) dst[c] = v[c];
   }
 }
@@ -682,12 +687,11 @@ __device__ __forceinline__ void body_cols(const StepArgs<T>& a, int step_mode, i
   T* B = A + (size_t)(zm ? 2 : 1) * CT * ld;
   T* S = a.spec + (size_t)m * a.lstride;
   const int ny = a.ny;
-  constexpr bool FX = fx_path<T, false, HL>;
-  FxScratch* sc = (FxScratch*)tot;  // [0] the forward, [1] the inverse transform's
+  constexpr bool FX = sizeof(T) == 8;
+  FxScratch* sc = (FxScratch*)tot;  // the forward, then the inverse transform's
   unsigned int hmax[FX ? CT : 1];
   if constexpr (FX) {
-    fx_clear(&sc[0]);
-    fx_clear(&sc[1]);
+    for (int n = 0; n < (HL == -1 ? 4 : 2); ++n) fx_clear(&sc[n]);
 #pragma unroll
     for (int c = 0; c < CT; ++c) hmax[c] = 0;
     __syncthreads();
@@ -850,6 +854,89 @@ __device__ __forceinline__ void body_cols(const StepArgs<T>& a, int step_mode, i
 // per block: complex FFT along y, Helmholtz divide, backward FFT (as the
 // conjugate of the forward FFT of the conjugate), in zeta mode also the
 // spectral 5-point Laplacian of psi.  Columns k > nx/2 are padding.
+// FP64, in fixed point: CC complex columns, whose Helmholtz factors stay in
+// FP64 as in body_cols_fx.
+template <int CC>
+__device__ __forceinline__ void body_cols_per_fx(const StepArgs<double>& a, int step_mode, int bx, int m,
+                                                 unsigned char* smem_raw, double* tot) {
+  if (step_mode && !a.state->active) return;
+  FxScratch* sc = (FxScratch*)tot;
+  const int H = a.gx.H, k0 = bx * CC, ld = row_len<double>(a.gy), ny = a.ny;
+  double* A = (double*)smem_raw;
+  double* B = A + (size_t)CC * ld;
+  double* S = a.spec + (size_t)m * a.lstride + 2 * k0;
+  fx_clear(&sc[0]);
+  fx_clear(&sc[1]);
+  unsigned int hmax[CC];
+#pragma unroll
+  for (int c = 0; c < CC; ++c) hmax[c] = 0;
+  __syncthreads();
+  // columns past the row's pitch (a multiple of two complex values) are zero
+  for (int jj = threadIdx.x; jj < ny; jj += NT) {
+    const int pj = pr<double>(2 * jj);
+#pragma unroll
+    for (int c = 0; c < CC; c += 2) {
+      double v[4] = {};
+      if (2 * (k0 + c) < a.pitch) load_cols<double, 4>(S + (size_t)jj * a.pitch + 2 * c, v);
+#pragma unroll
+      for (int d = 0; d < 4; ++d) {
+        A[(c + d / 2) * ld + pj + d % 2] = v[d];
+        hmax[c + d / 2] = max(hmax[c + d / 2], fx_hi(v[d]));
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < CC; ++c) {
+    fx_note_max(&sc[0], c, hmax[c]);
+    hmax[c] = 0;
+  }
+  __syncthreads();
+  fx_t* O = fx_cfft<true>((fx_t*)A, (fx_t*)B, CC, ld, a.gy, a.fy.twq, &sc[0]);
+  int ex[CC];
+#pragma unroll
+  for (int c = 0; c < CC; ++c) ex[c] = fx_exp_add(fx_row_exp(sc[0].mx[c], fx_drop(&sc[0], c, a.gy.npass), 0), -1);
+  for (int jj = threadIdx.x; jj < ny; jj += NT) {
+    const int pj = pr<double>(2 * jj);
+    const double* hrow = a.hinv + (size_t)m * a.lstride + (size_t)jj * a.pitch + k0;
+#pragma unroll
+    for (int c = 0; c < CC; ++c) {
+      // padding columns; the mean is removed (src/elliptic.h:115-118)
+      const double h = k0 + c > H || (k0 + c == 0 && jj == 0) ? 0.0 : hrow[c];
+      fx_t* z = O + c * ld + pj;
+      // conjugate: backward FFT = conj(FFT(conj))
+      const double x = fx_out(z[0], ex[c]) * h, y = -(fx_out(z[1], ex[c]) * h);
+      z[0] = __double_as_longlong(x);
+      z[1] = __double_as_longlong(y);
+      hmax[c] = max(hmax[c], max(fx_hi(x), fx_hi(y)));
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < CC; ++c) fx_note_max(&sc[1], c, hmax[c]);
+  __syncthreads();
+  fx_t* O2 = fx_cfft<true>(O, O == (fx_t*)A ? (fx_t*)B : (fx_t*)A, CC, ld, a.gy, a.fy.twq, &sc[1]);
+#pragma unroll
+  for (int c = 0; c < CC; ++c) ex[c] = fx_exp_add(fx_row_exp(sc[1].mx[c], fx_drop(&sc[1], c, a.gy.npass), 0), -1);
+  grid_next();
+  for (int jj = threadIdx.x; jj < ny; jj += NT) {
+    const int pj = pr<double>(2 * jj);
+#pragma unroll
+    for (int c = 0; c < CC; c += 2) {
+      double v[4];
+#pragma unroll
+      for (int d = 0; d < 4; ++d) {
+        const double x = fx_out(O2[(c + d / 2) * ld + pj + d % 2], ex[c + d / 2]);
+        v[d] = d % 2 ? -x : x;
+      }
+      if (2 * (k0 + c) < a.pitch) store_cols<double, 4>(S + (size_t)jj * a.pitch + 2 * c, v);
+    }
+  }
+}
+// complex columns per tile of a single FP64 run: as many as leave three
+// blocks per SM
+static inline int per_cols(const StepArgs<double>& a) {
+  return (size_t)8 * row_len<double>(a.gy) * sizeof(double) <= (size_t)74 * 1024 ? 4 : 2;
+}
+
 template <typename T, bool COMP>
 __device__ __forceinline__ void body_cols_per(const StepArgs<T>& a, int step_mode, int bx, int m, unsigned char* smem_raw) {
   constexpr int CC = 2;

@@ -168,6 +168,53 @@ static void run_fx(int M, int howmany, double* data) {
     }
   }
 }
+// The fixed-point chirp-z form.
+static void run_fx_blue(int M, int howmany, double* data) {
+  DstGeom g = make_geom_blue(M);
+  FxTablesHost fx = build_fx_tables(g);
+  const int Lc = g.H, ld = padded_len<double>(2 * Lc);
+  std::vector<fx_t> A(ld), B(ld);
+  auto passes = [&](C2<fx_t>*& src, C2<fx_t>*& dst, int& drop, unsigned int& mag) {
+    int Ns = 1;
+    for (int p = 0; p < g.npass; ++p) {
+      const int R = g.radix[p], s = p ? fx_pass_shift(mag) : 0;
+      if (p) drop += 2 - s;
+      mag = 0;
+      for (int b = 0; b < Lc / R; ++b)
+        mag |= fx_stockham_dispatch(R, src, dst, b, b % Ns, Ns, Lc, s, fx.twq.data() + (p ? Ns - g.radix[0] : 0));
+      Ns *= R;
+      C2<fx_t>* t = src; src = dst; dst = t;
+    }
+  };
+  for (int r = 0; r < howmany; ++r) {
+    double* x = data + (size_t)r * (M - 1);
+    for (int j = 0; j < ld; ++j) A[j] = B[j] = 777;
+    unsigned int mx = 0;
+    for (int j = 1; j < M; ++j) {
+      std::memcpy(&A[pr<double>(j)], &x[j - 1], 8);
+      const unsigned int h = (unsigned int)((unsigned long long)A[pr<double>(j)] >> 32) & 0x7fffffffu;
+      mx = h > mx ? h : mx;
+    }
+    C2<fx_t>* src = (C2<fx_t>*)B.data();
+    C2<fx_t>* dst = (C2<fx_t>*)A.data();
+    for (int m = 0; m < Lc; ++m)
+      fx_chirp_item((const unsigned long long*)A.data(), src, m, M, fx_scale(mx), fx.bc.data());
+    int drop = 0;
+    unsigned int mag = 0;
+    passes(src, dst, drop, mag);
+    int s = fx_pass_shift(mag);
+    drop += 2 - s + fx.be;
+    for (int k = 0; k < Lc; ++k) fx_chirp_mul_item(src, k, s, fx.bz.data());
+    passes(src, dst, drop, mag);
+    s = fx_pass_shift(mag);
+    for (int k = 0; k < M; ++k) fx_chirp_out_item(src, (fx_t*)dst, k, s, fx.bc.data());
+    int lg = 0;
+    while ((1 << lg) < Lc) ++lg;
+    const int e = fx_exp_add(fx_row_exp(mx, drop + 2 + 1 - lg, s), -1);
+    for (int j = 1; j < M; ++j)
+      x[j - 1] = e == FX_NAN ? std::nan("") : std::ldexp((double)((const fx_t*)dst)[pr<double>(j)], e);
+  }
+}
 // DST-I by its definition in long double (at least 64 bits), one row
 static void run_exact(int M, const double* x, long double* y) {
   std::vector<long double> s(2 * (size_t)M);
@@ -183,25 +230,6 @@ static void run_exact(int M, const double* x, long double* y) {
     y[k - 1] = 2 * t;
   }
 }
-
-// relative errors (2-norm, in units of 2^-53) of the FP64 and the fixed-point
-// transform of one row
-extern "C" void dst_fx_errors(int M, const double* x, double* err) {
-  std::vector<long double> e(M - 1);
-  run_exact(M, x, e.data());
-  for (int f = 0; f < 2; ++f) {
-    std::vector<double> y(x, x + M - 1);
-    if (f) run_fx(M, 1, y.data());
-    else run<double>(M, 1, y.data());
-    long double d = 0, n = 0;
-    for (int k = 0; k < M - 1; ++k) {
-      d += (y[k] - e[k]) * (y[k] - e[k]);
-      n += e[k] * e[k];
-    }
-    err[f] = (double)(sqrtl(d / n) * 9007199254740992.0L);
-  }
-}
-extern "C" void dst_fx_run(int M, int howmany, double* data) { run_fx(M, howmany, data); }
 
 extern "C" int dst_warp_run_f32(int M, int howmany, float* data) {
   if (M == 512) run_warp<8>(howmany, data);
@@ -280,3 +308,25 @@ extern "C" int dst_core_check_twp(int M) {
 
 // the transform lengths the library accepts (M even, M/2 a product of 2, 3, 5, 7)
 extern "C" int dst_core_length_ok(int M) { return transform_length_ok(M) ? 1 : 0; }
+
+// relative errors (2-norm, in units of 2^-53) of the FP64 and the fixed-point
+// transform of one row
+extern "C" void dst_fx_errors(int M, const double* x, double* err) {
+  std::vector<long double> e(M - 1);
+  run_exact(M, x, e.data());
+  const bool blue = !transform_length_ok(M);
+  for (int f = 0; f < 2; ++f) {
+    std::vector<double> y(x, x + M - 1);
+    if (f) blue ? run_fx_blue(M, 1, y.data()) : run_fx(M, 1, y.data());
+    else blue ? run_blue<double>(M, 1, y.data()) : run<double>(M, 1, y.data());
+    long double d = 0, n = 0;
+    for (int k = 0; k < M - 1; ++k) {
+      d += (y[k] - e[k]) * (y[k] - e[k]);
+      n += e[k] * e[k];
+    }
+    err[f] = (double)(sqrtl(d / n) * 9007199254740992.0L);
+  }
+}
+extern "C" void dst_fx_run(int M, int howmany, double* data) {
+  transform_length_ok(M) ? run_fx(M, howmany, data) : run_fx_blue(M, howmany, data);
+}

@@ -24,10 +24,12 @@ def rows(M):
     yield rng.standard_normal(M - 1) * 1e200
 
 
-@pytest.mark.parametrize("M", [4, 6, 10, 14, 16, 30, 70, 128, 240, 256, 384, 486, 512, 1000, 1024, 2048, 2430, 4096])
+@pytest.mark.parametrize("M", [4, 6, 10, 14, 16, 30, 70, 128, 240, 256, 384, 486, 512, 1000, 1024, 2048, 2430, 4096,
+                               5, 9, 22, 33, 131, 207, 301, 514, 953, 1025, 2039])
 def test_error_no_larger_than_fp64(dstcore, M):  # noqa: F811
     """Against the DST-I by its definition in long double, over random,
-    smooth, peaked and decaying rows: no row further off than the worst of
+    smooth, peaked and decaying rows, the half-length forms and (from 5 on)
+    the chirp-z ones: no row further off than the worst of
     the floating-point transform's rows (or 2 units of 2^-53, the rounding
     of the results and tables themselves), and all together closer."""
     dstcore.dst_fx_errors.argtypes = [ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]

@@ -503,7 +503,9 @@ int setup_args(qgw_run* r, StepArgs<T>& a) {
     };
     const size_t limit = (size_t)200 * 1024;
     if (a.gy.blue) a.CT = (32 / (int)sizeof(T)) / 2;
-    if (need() > limit) a.CT = (32 / (int)sizeof(T)) / 2;
+    // FP64: 16-byte tiles already where 32-byte ones leave one block per SM
+    // (more than 113 KiB: NY > 1536)
+    if (need() > (sizeof(T) == 8 ? (size_t)113 * 1024 : limit)) a.CT = (32 / (int)sizeof(T)) / 2;
     if (a.gy.blue && need() > limit) a.CT = 1;
   }
   // TMA tensor maps of the RHS kernel's tiles (psi with halo R, q with halo

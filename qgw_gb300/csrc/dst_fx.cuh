@@ -249,10 +249,12 @@ __device__ __forceinline__ fx_t* fx_passes_any(fx_t* src, fx_t* dst, int nrows, 
   for (int p = 0; p < g.npass; ++p) {
     const int R = g.radix[p];
     const Q4* tw = twq + (p ? Ns - g.radix[0] : 0);
+    const unsigned int inv = 0xffffffffu / (unsigned int)Ns + 1;
     fx_items(nrows, H / R, [&](int r, int b, bool on) {
       unsigned int m = 0;
       if (on)
-        m = fx_stockham_dispatch(R, (const C2<fx_t>*)(src + r * ld), (C2<fx_t>*)(dst + r * ld), b, b % Ns, Ns, H,
+        m = fx_stockham_dispatch(R, (const C2<fx_t>*)(src + r * ld), (C2<fx_t>*)(dst + r * ld), b,
+                                 Ns == 1 ? 0 : b - Ns * (int)__umulhi((unsigned int)b, inv), Ns, H,
                                  p ? fx_pass_shift(sc->mag[p - 1][r]) : 0, tw);
       fx_row_or<0>(sc->mag[p], r, m);
     });
@@ -266,6 +268,9 @@ __device__ __forceinline__ fx_t* fx_passes_any(fx_t* src, fx_t* dst, int nrows, 
 }
 static __device__ __noinline__ fx_t* dst_fx_any(double* A, double* B, int nrows, int ld, const DstGeom& g, const FxTables& tb,
                                                 FxScratch* sc) {
+  __builtin_assume(__isShared(A));
+  __builtin_assume(__isShared(B));
+  __builtin_assume(__isShared(sc));
   const int H = g.H, M = g.M, tid = threadIdx.x, lane = tid & 31;
   fx_items(nrows, H, [&](int r, int i, bool on) {
     unsigned int l = 0;

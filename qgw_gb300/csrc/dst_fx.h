@@ -315,6 +315,11 @@ QGW_HD unsigned int fx_stockham_item(const C2<fx_t>* src, C2<fx_t>* dst, int b, 
 template <int R>
 QGW_HD_NOINLINE unsigned int fx_stockham_item_far(const C2<fx_t>* src, C2<fx_t>* dst, int b, int k, int Ns, int H,
                                                   int s, const Q4* tw) {
+#ifdef __CUDA_ARCH__
+  // a function of its own does not see that its rows lie in shared memory
+  __builtin_assume(__isShared(src));
+  __builtin_assume(__isShared(dst));
+#endif
   return fx_stockham_item<R>(src, dst, b, k, Ns, H, s, tw);
 }
 // tw: the table of the pass (twq + Ns - R0)

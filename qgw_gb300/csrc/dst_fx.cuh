@@ -288,21 +288,23 @@ static __device__ __noinline__ fx_t* dst_fx_any(double* A, double* B, int nrows,
     if (k == 0) sc->ex[r] = fx_row_exp(sc->mx[r], drop, s);
   });
   __syncthreads();
-  // prefix sum: one warp per row, chunk by chunk of 32 odd outputs
+  // prefix sum: one warp per row; a lane adds up its ceil(H / 32) odd outputs,
+  // then writes their running sums on top of the lanes' before it
+  const int ch = (H + 31) / 32, k0 = min(lane * ch, H), k1 = min(k0 + ch, H);
   for (int r = tid >> 5; r < nrows; r += FX_NT / 32) {
     fx_t* o = dst + r * ld;
-    fx_t carry = 0;
-    for (int k0 = 0; k0 < H; k0 += 32) {
-      const int k = k0 + lane;
-      fx_t v = k < H ? o[pr<double>(2 * k + 1)] : 0;
+    fx_t sum = 0;
+    for (int k = k0; k < k1; ++k) sum += o[pr<double>(2 * k + 1)];
+    fx_t incl = sum;
 #pragma unroll
-      for (int of = 1; of < 32; of <<= 1) {
-        const fx_t u = __shfl_up_sync(0xffffffffu, v, of);
-        if (lane >= of) v += u;
-      }
-      v += carry;
-      if (k < H) o[pr<double>(2 * k + 1)] = v;
-      carry = __shfl_sync(0xffffffffu, v, 31);
+    for (int of = 1; of < 32; of <<= 1) {
+      const fx_t u = __shfl_up_sync(0xffffffffu, incl, of);
+      if (lane >= of) incl += u;
+    }
+    fx_t run = incl - sum;
+    for (int k = k0; k < k1; ++k) {
+      run += o[pr<double>(2 * k + 1)];
+      o[pr<double>(2 * k + 1)] = run;
     }
   }
   __syncthreads();

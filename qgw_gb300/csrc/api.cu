@@ -361,12 +361,20 @@ int setup_args(qgw_run* r, StepArgs<T>& a) {
   a.G3 = mode_group(r->nl, Mrow, sizeof(T), 110 * 1024, 1, 16, inv_group(0, Mrow, r->nl, bufs_x), bufs_x);
   if (sizeof(T) == 8) {
     // FP64 row kernels take rows of any layer: as many as the budget holds,
-    // but on small grids no more than leave every SM two blocks
+    // but on small grids no more than leave every SM a few blocks
     a.G3 = a.G1;
+    // -- two blocks per SM (four for transforms of 256 points and more, whose
+    // phases fill a block with fewer rows) -- rounded down to a power of two,
+    // whose phases end in whole rounds of the block's threads.  384^2 x 8:
+    // ten rows 0.061 / 0.054 ms forward / inverse, eight 0.055 / 0.046; 512^2
+    // x 5: eight 0.048 / 0.041, four 0.044 / 0.038.
     const int fit = mode_group(1 << 20, Mrow, sizeof(T), row_budget(sizeof(T), Mrow, r->nl), 1, 16, 16);
-    a.RB1 = a.RB3 = std::max(1, std::min(fit, r->nl * r->ny / 304));
+    const int want = std::max(1, std::min(fit, r->nl * r->ny / (a.gx.H >= 256 ? 608 : 304)));
+    a.RB1 = 1;
+    while (2 * a.RB1 <= want) a.RB1 *= 2;
+    a.RB3 = a.RB1;
   }
-  a.CT = 0;
+  a.CT = a.CT1 = 0;
   a.low_k64 = 8;
   // 16-byte column vectors: rows 16-byte aligned and a whole number of
   // column tiles per row, so a tile never crosses into the next row
@@ -507,6 +515,16 @@ int setup_args(qgw_run* r, StepArgs<T>& a) {
     // (more than 113 KiB: NY > 1536)
     if (need() > (sizeof(T) == 8 ? (size_t)113 * 1024 : limit)) a.CT = (32 / (int)sizeof(T)) / 2;
     if (a.gy.blue && need() > limit) a.CT = 1;
+    // A single run's column kernel takes the narrower tiles too where the
+    // wider ones leave SMs idle -- FP32: fewer than two blocks per SM (128^2
+    // x 10, 160 blocks: 0.0165 -> 0.0124 ms; 384^2 x 8, 384 blocks: 0.041
+    // against 0.047 narrow), FP64: than one and a half (256^2 x 3, 192:
+    // 0.0195 -> 0.0181; 128^2 x 10, 320: 0.018 against 0.023) -- or, FP32,
+    // leave fewer than three resident (more than 75 KiB; 768^2 x 8: 0.162 ->
+    // 0.143 ms).  An ensemble fills the SMs with its members.
+    const int wide = 32 / (int)sizeof(T), blocks = (r->nx + wide - 1) / wide * r->nl;
+    const bool few = blocks < (sizeof(T) == 8 ? 228 : 304);
+    if (!per && !a.gy.blue && a.CT == 0 && (few || (sizeof(T) == 4 && need() > (size_t)75 * 1024))) a.CT1 = wide / 2;
   }
   // TMA tensor maps of the RHS kernel's tiles (psi with halo R, q with halo
   // 1, in zeta mode 1 zeta over the first sweep's region; zeta mode 2 reads
@@ -517,10 +535,11 @@ int setup_args(qgw_run* r, StepArgs<T>& a) {
   a.rhs_ty = 16;
   if (const char* e = std::getenv("QGW_RHS_TILE_ROWS")) a.rhs_ty = std::atoi(e) == 32 ? 32 : 16;
   encode_rhs_maps<T>(r, a);
-  // K3 over rows x layer groups in FP64 (measured at 1024^2 x 10: 0.575 ->
-  // 0.552 ms); the FP32c kernel keeps one block per row (0.109 against 0.123
-  // ms split).  QGW_INV_SPLIT=0/1 overrides.
-  a.inv_split = sizeof(T) == 8;
+  // FP32c K3: one block per row, or per (row, layer group) where the rows
+  // alone leave few blocks per SM: 128^2 x 10 0.0163 -> 0.0123 ms, 256^2 x 16
+  // 0.0287 -> 0.0226, 512^2 x 16 0.053 -> 0.049, 768^2 x 8 0.111 -> 0.094;
+  // 1024^2 x 10 0.109 against 0.123 split.  QGW_INV_SPLIT=0/1 overrides.
+  a.inv_split = r->ny < 900;
   if (const char* e = std::getenv("QGW_INV_SPLIT")) a.inv_split = std::atoi(e) != 0;
   // QGW_TEST_FIRST_WAIT_ITERS (tests of the timeout path only) lowers the
   // limit of the first wait for a tile's TMA bytes, down to 0 polls; the
@@ -552,6 +571,7 @@ int set_shape(qgw_run* r, StepArgs<T>& a, const qgw_shape& sh) {
     } else {
       if (sh.col_tile != ctd && sh.col_tile != ctd / 2) return QGW_ERR_PARAM;
       b.CT = sh.col_tile == ctd ? 0 : sh.col_tile;
+      b.CT1 = 0;
     }
   }
   const bool per = a.periodic != 0;
@@ -584,7 +604,7 @@ int set_shape(qgw_run* r, StepArgs<T>& a, const qgw_shape& sh) {
 template <typename T>
 void get_shape(const StepArgs<T>& a, qgw_shape* sh) {
   sh->rhs_tile_rows = a.rhs_ty == 32 ? 32 : 16;
-  sh->col_tile = a.CT ? a.CT : 32 / (int)sizeof(T);
+  sh->col_tile = a.CT1 ? a.CT1 : a.CT ? a.CT : 32 / (int)sizeof(T);
   sh->row_group_fwd = a.G1;
   sh->row_group_inv = a.G3;
 }

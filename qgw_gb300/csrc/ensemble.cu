@@ -239,6 +239,7 @@ void ens_core_free_tables(EnsembleCore* e) {
 static int uniform_shape(EnsembleCore* e) {
   if (e->members.empty()) return QGW_OK;
   qgw_shape first{};
+  for (qgw_run* r : e->members) r->a64.CT1 = r->a32.CT1 = 0;  // (a single run's choice)
   qgw_get_shape(e->members[0], &first);
   int ct = first.col_tile, ty = first.rhs_tile_rows;
   bool mixed = false;

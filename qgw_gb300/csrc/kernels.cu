@@ -467,9 +467,10 @@ static void launch_k1(const StepArgs<T>& a, int step_mode, bool pdl, cudaStream_
 }
 template <typename T, bool COMP>
 static void launch_k2(const StepArgs<T>& a, int step_mode, bool pdl, cudaStream_t s) {
-  const dim3 grid(col_tiles(a), a.nl);
-  const size_t sm = smem_cols<T, COMP>(a);
-  const bool wide = col_width(a) == CTD<T>, h512 = a.gy.H == 512 && !a.gy.blue;
+  const int width = a.CT1 ? a.CT1 : col_width(a);
+  const dim3 grid(a.periodic ? col_tiles(a) : (a.nx + width - 1) / width, a.nl);
+  const size_t sm = smem_cols<T, COMP>(a, width);
+  const bool wide = width == CTD<T>, h512 = a.gy.H == 512 && !a.gy.blue;
   if constexpr (sizeof(T) == 8) {
     if (a.periodic) {
       const int cc = per_cols(a);
@@ -481,7 +482,7 @@ static void launch_k2(const StepArgs<T>& a, int step_mode, bool pdl, cudaStream_
     }
   }
   if (a.periodic) launch(k_cols<T, COMP, true, CTD<T>, 0>, grid, dim3(NT), sm, s, pdl, a, step_mode);
-  else if (a.gy.blue && col_width(a) == 1) launch(k_cols<T, COMP, false, 1, -1>, grid, dim3(NT), sm, s, pdl, a, step_mode);
+  else if (a.gy.blue && width == 1) launch(k_cols<T, COMP, false, 1, -1>, grid, dim3(NT), sm, s, pdl, a, step_mode);
   else if (a.gy.blue) launch(k_cols<T, COMP, false, CTD<T> / 2, -1>, grid, dim3(NT), sm, s, pdl, a, step_mode);
   else if (wide && h512) launch(k_cols<T, COMP, false, CTD<T>, 512>, grid, dim3(NT), sm, s, pdl, a, step_mode);
   else if (wide) launch(k_cols<T, COMP, false, CTD<T>, 0>, grid, dim3(NT), sm, s, pdl, a, step_mode);

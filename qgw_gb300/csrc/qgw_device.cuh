@@ -141,7 +141,8 @@ template <typename T> struct StepArgs {
   // on the host: a double -> float conversion runs on the FP64 pipe
   float fc[24];
   const float* iRd2f;
-  int CT;                          // (unused by the kernels; kept for layout)
+  int CT;                          // columns per tile of the column kernels (0: 32-byte rows)
+  int CT1;                         // a single run's narrower tiles on a small grid (0: CT)
   int vec_cols;                    // rows are 16-byte aligned: 16-byte column loads
   int low_k64;                     // compensated: FP64 divide for mode 0, j,k < low_k64
   ForcArgs<T> fr;                  // stochastic forcing (fr.on = 0: none)
@@ -158,7 +159,7 @@ template <typename T> struct StepArgs {
   int use_tma;
   int rhs_grid;  // blocks of the persistent RHS kernel (0: one per tile)
   int rhs_ty;    // RHS tile height: 16 (default) or 32 rows
-  // K3 grid: 1 = one block per (row, layer group), 0 = one block per row
+  // FP32 K3 grid: 1 = one block per (row, layer group), 0 = one block per row
   // that runs the row's layer groups in turn (same arithmetic per layer)
   int inv_split;
   // iterations of the first bounded wait for a tile's TMA bytes (normally

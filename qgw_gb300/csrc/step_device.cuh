@@ -1906,13 +1906,13 @@ static inline size_t smem_rows_f64(const StepArgs<double>& a, int rows) {
   return (size_t)2 * rows * row_len<double>(a.gx) * sizeof(double);
 }
 template <typename T, bool COMP>
-static size_t smem_cols(const StepArgs<T>& a) {
+static size_t smem_cols(const StepArgs<T>& a, int width = 0) {
   // periodic: two complex columns of ny values (padded rows of 2 ny reals)
   // in two or three buffers; DST: the pairs [A | C] and [B | D] of CT rows
   // ([A] and [B] without the second field)
   const bool zm = COMP && a.zeta_mode;
   const size_t rows = a.periodic ? (size_t)(zm ? 3 : 2) * 2
-                                 : (size_t)(zm ? 2 : 1) * dst_bufs(a, a.gy) * col_width(a);
+                                 : (size_t)(zm ? 2 : 1) * dst_bufs(a, a.gy) * (width ? width : col_width(a));
   return rows * row_len<T>(a.gy) * sizeof(T);
 }
 // column tiles of one mode: four real columns (DST) or two complex columns

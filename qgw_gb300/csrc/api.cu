@@ -980,10 +980,9 @@ int qgw_step(qgw_run* r, int nsteps, double t_out, double tend, qgw_step_info* i
       if (!r->h_state->active) break;
     }
   }
-  if (r->precision == QGW_FP64) qgw::enqueue_flush_f64(r->a64, r->stream);
-  else qgw::enqueue_flush_f32c(r->a32, r->stream);
+  if (r->precision == QGW_FP64) qgw::enqueue_flush_f64(r->a64, r->h_state, r->stream);
+  else qgw::enqueue_flush_f32c(r->a32, r->h_state, r->stream);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(r->h_state, r->d_state, sizeof(DevState), cudaMemcpyDeviceToHost, r->stream));
   CK(cudaStreamSynchronize(r->stream));
   const DevState& s = *r->h_state;
   if (info) {
@@ -1169,8 +1168,8 @@ int qgw_profile_kernels(qgw_run* r, int nsteps, float* ms4) {
       CK(cudaEventRecord(ev[5 * s + k + 1], r->stream));
     }
   }
-  if (r->precision == QGW_FP64) qgw::enqueue_flush_f64(r->a64, r->stream);
-  else qgw::enqueue_flush_f32c(r->a32, r->stream);
+  if (r->precision == QGW_FP64) qgw::enqueue_flush_f64(r->a64, r->h_state, r->stream);
+  else qgw::enqueue_flush_f32c(r->a32, r->h_state, r->stream);
   CK(cudaStreamSynchronize(r->stream));
   for (int k = 0; k < 4; ++k) ms4[k] = 0;
   for (int s = 0; s < nsteps; ++s)

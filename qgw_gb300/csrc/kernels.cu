@@ -94,12 +94,16 @@ __global__ void __launch_bounds__(NT, 3) k_rows_f64(const __grid_constant__ Step
 }
 
 // ------------------------------------------------------- small kernels
-static __global__ void k_begin(DevState* st, double t_out, double tend) { begin_state(st, t_out, tend, 0); }
+static __global__ void k_begin(DevState* st, double t_out, double tend) {
+  grid_wait();
+  begin_state(st, t_out, tend, 0);
+}
 
 template <typename T, bool COMP>
 // (a.qout: also writes the final q, joined to FP64, into the caller's array
 // in the reference layout -- the interior; the host fills the ghost ring)
 __global__ void __launch_bounds__(NT) k_flush(StepArgs<T> a) {
+  grid_wait();
   DevState* st = a.state;
   const bool pend = st->pending != 0;
   if (!pend && !a.qout) return;
@@ -157,7 +161,15 @@ __global__ void __launch_bounds__(NT) k_flush(StepArgs<T> a) {
   }
 }
 
-static __global__ void k_end(DevState* st) { st->pending = 0; }
+// the end of a call: nothing pending, and the scalars into the host's pinned
+// copy (a copy of their own behind the kernels cost 5 us a call)
+static __global__ void k_end(DevState* st, DevState* host) {
+  grid_wait();
+  if (threadIdx.x == 0) st->pending = 0;
+  __syncthreads();
+  static_assert(sizeof(DevState) % 4 == 0 && sizeof(DevState) <= 4 * 64, "one word per thread");
+  if (threadIdx.x < sizeof(DevState) / 4) ((int*)host)[threadIdx.x] = ((const int*)st)[threadIdx.x];
+}
 
 // --------------------------------------------------- stochastic forcing
 // F1: new ring amplitudes after each completed step (calc_forc,
@@ -561,12 +573,12 @@ static void launch_invert(const StepArgs<T>& a, int step_mode, bool pdl, cudaStr
 }
 
 template <typename T, bool COMP>
-static void launch_flush(const StepArgs<T>& a, cudaStream_t s) {
+static void launch_flush(const StepArgs<T>& a, DevState* host, cudaStream_t s) {
   const size_t n = (size_t)a.nl * a.ny * a.nx;
   int blocks = (int)((n + NT - 1) / NT);
   if (blocks > 152 * 8) blocks = 152 * 8;
-  k_flush<T, COMP><<<blocks, NT, 0, s>>>(a);
-  k_end<<<1, 1, 0, s>>>(a.state);
+  launch(k_flush<T, COMP>, dim3(blocks), dim3(NT), 0, s, true, a);
+  launch(k_end, dim3(1), dim3(64), 0, s, true, a.state, host);
 }
 
 template <typename T, bool COMP>
@@ -586,7 +598,9 @@ static void budget_impl(const StepArgs<T>& a, const double* wts, double* part, i
 }
 
 #if QGW_KERNELS_PART == 1
-void enqueue_begin(DevState* st, double t_out, double tend, cudaStream_t s) { k_begin<<<1, 1, 0, s>>>(st, t_out, tend); }
+void enqueue_begin(DevState* st, double t_out, double tend, cudaStream_t s) {
+  launch(k_begin, dim3(1), dim3(1), 0, s, true, st, t_out, tend);
+}
 
 void enqueue_unpack_split(const double* full, float* hi, float* lo, int nx, int ny, int nl, int pitch,
                           cudaStream_t s) {
@@ -616,7 +630,7 @@ void enqueue_forcing_f64(const StepArgs<double>& a, cudaStream_t s) { launch_for
 
 void enqueue_invert_f64(const StepArgs<double>& a, bool pdl, cudaStream_t s) { launch_invert<double, false>(a, 0, pdl, s); }
 
-void enqueue_flush_f64(const StepArgs<double>& a, cudaStream_t s) { launch_flush<double, false>(a, s); }
+void enqueue_flush_f64(const StepArgs<double>& a, DevState* host, cudaStream_t s) { launch_flush<double, false>(a, host, s); }
 
 void enqueue_step_kernel_f64(const StepArgs<double>& a, int which, cudaStream_t s) { launch_one<double, false>(a, which, s); }
 
@@ -663,7 +677,7 @@ void enqueue_forcing_f32c(const StepArgs<float>& a, cudaStream_t s) { launch_for
 
 void enqueue_invert_f32c(const StepArgs<float>& a, bool pdl, cudaStream_t s) { launch_invert<float, true>(a, 0, pdl, s); }
 
-void enqueue_flush_f32c(const StepArgs<float>& a, cudaStream_t s) { launch_flush<float, true>(a, s); }
+void enqueue_flush_f32c(const StepArgs<float>& a, DevState* host, cudaStream_t s) { launch_flush<float, true>(a, host, s); }
 
 void enqueue_step_kernel_f32c(const StepArgs<float>& a, int which, cudaStream_t s) { launch_one<float, true>(a, which, s); }
 

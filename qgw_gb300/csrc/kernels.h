@@ -25,8 +25,9 @@ void enqueue_invert_f32c(const StepArgs<float>& a, bool pdl, cudaStream_t s);
 // the stochastic forcing kernels of one step (ensembles launch them per member)
 void enqueue_forcing_f64(const StepArgs<double>& a, cudaStream_t s);
 void enqueue_forcing_f32c(const StepArgs<float>& a, cudaStream_t s);
-void enqueue_flush_f64(const StepArgs<double>& a, cudaStream_t s);
-void enqueue_flush_f32c(const StepArgs<float>& a, cudaStream_t s);
+// host: pinned memory that receives the run's scalars
+void enqueue_flush_f64(const StepArgs<double>& a, DevState* host, cudaStream_t s);
+void enqueue_flush_f32c(const StepArgs<float>& a, DevState* host, cudaStream_t s);
 // which: 0 rows forward, 1 columns, 2 rows inverse, 3 RHS (step mode)
 void enqueue_step_kernel_f64(const StepArgs<double>& a, int which, cudaStream_t s);
 void enqueue_step_kernel_f32c(const StepArgs<float>& a, int which, cudaStream_t s);

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 4) k_rhs(const __grid
 // FP64: the projections, one thread per point (NL: layers in registers, 0:
 // any number), and the row transforms (modes_fx.cuh)
 template <int NL, bool FWD>
-__global__ void __launch_bounds__(NT, 2) k_modes(const __grid_constant__ StepArgs<double> a, int step_mode) {
+__global__ void __launch_bounds__(NT, NL <= 10 ? 4 : 2) k_modes(const __grid_constant__ StepArgs<double> a, int step_mode) {
   grid_wait();
   if (step_mode && !a.state->active) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];

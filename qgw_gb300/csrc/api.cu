@@ -999,8 +999,6 @@ int qgw_step(qgw_run* r, int nsteps, double t_out, double tend, qgw_step_info* i
   return s.nonfinite ? QGW_ERR_NAN : QGW_OK;
 }
 
-static void fill_ghosts(const qgw_run* r, double* psi, double* q, const double* ps);
-
 // qgw_step with the caller's q going in and out (the reference's
 // timestep(q) on a host array, n times): q_in replaces q keeping the AB3
 // history (as qgw_put_q), read by the first kernel of the call straight from
@@ -1015,7 +1013,7 @@ int qgw_step_host(qgw_run* r, int nsteps, double t_out, double tend, const doubl
   const bool direct = q_in && nsteps > 0 && t_out == 0 && tend == 0;
   const double* view = direct ? (const double*)device_view(r, q_in) : nullptr;
   if (q_in && !view && (rc = load_q(r, q_in, false))) return rc;
-  // q out: the end-of-call flush writes the interior into the caller's array
+  // q out: the end-of-call flush writes q into the caller's array
   // where the device can address it and the ghost ring needs no psi
   // (free-slip or periodic); otherwise as qgw_get
   double* oview = q_out && (r->p.bc_fac == 0 || r->p.bc_fac == -1) ? (double*)device_view(r, q_out) : nullptr;
@@ -1031,8 +1029,7 @@ int qgw_step_host(qgw_run* r, int nsteps, double t_out, double tend, const doubl
   r->a64.qout = r->a32.qout = nullptr;
   if (rc != QGW_OK && rc != QGW_ERR_NAN) return rc;
   int rc2 = QGW_OK;
-  if (oview) fill_ghosts(r, nullptr, q_out, nullptr);
-  else if (q_out) rc2 = qgw_get(r, nullptr, q_out);
+  if (q_out && !oview) rc2 = qgw_get(r, nullptr, q_out);
   return rc2 != QGW_OK ? rc2 : rc;
 }
 
@@ -1045,54 +1042,6 @@ int qgw_invert(qgw_run* r) {
   return QGW_OK;
 }
 
-// Ghost rings as adjust_bc leaves them after invert_pv (src/elliptic.h:152-153,
-// src/domain.h:308-348): periodic copies; at walls psi = 0 and
-// q = 2 bc_fac / Delta^2 * psi_adjacent (ps: psi, needed when bc_fac != 0).
-static void fill_ghosts(const qgw_run* r, double* psi, double* q, const double* ps) {
-  const int nxp2 = r->nx + 2, nyp2 = r->ny + 2;
-  const size_t L = (size_t)nxp2 * nyp2;
-  if (r->p.bc_fac == -1) {
-    // periodic copies, South, North, West, East in turn (src/domain.h:225-256)
-    for (double* F : {psi, q}) {
-      if (!F) continue;
-      for (int k = 0; k < r->nl; ++k) {
-        double* f = F + k * L;
-        for (int i = 0; i < nxp2; ++i) f[i] = f[(size_t)r->ny * nxp2 + i];
-        for (int i = 0; i < nxp2; ++i) f[(size_t)(nyp2 - 1) * nxp2 + i] = f[(size_t)nxp2 + i];
-        for (int j = 0; j < nyp2; ++j) f[(size_t)j * nxp2] = f[(size_t)j * nxp2 + r->nx];
-        for (int j = 0; j < nyp2; ++j) f[(size_t)j * nxp2 + nxp2 - 1] = f[(size_t)j * nxp2 + 1];
-      }
-    }
-    return;
-  }
-  const double c = 2 * r->p.bc_fac / (r->Delta * r->Delta);
-  for (int k = 0; k < r->nl; ++k) {
-    double* P = psi ? psi + k * L : nullptr;
-    double* Q = q ? q + k * L : nullptr;
-    const double* PS = ps ? ps + k * L : nullptr;
-    for (int i = 0; i < nxp2; ++i) {
-      for (int jj : {0, nyp2 - 1}) {
-        if (P) P[(size_t)jj * nxp2 + i] = 0.0;
-        if (Q) {
-          const int ja = jj == 0 ? 1 : nyp2 - 2;
-          const bool corner = (i == 0 || i == nxp2 - 1);
-          Q[(size_t)jj * nxp2 + i] = (corner || c == 0) ? 0.0 : c * PS[(size_t)ja * nxp2 + i];
-        }
-      }
-    }
-    for (int j = 0; j < nyp2; ++j) {
-      for (int ii : {0, nxp2 - 1}) {
-        if (P) P[(size_t)j * nxp2 + ii] = 0.0;
-        if (Q) {
-          const int ia = ii == 0 ? 1 : nxp2 - 2;
-          const bool corner = (j == 0 || j == nyp2 - 1);
-          Q[(size_t)j * nxp2 + ii] = (corner || c == 0) ? 0.0 : c * PS[(size_t)j * nxp2 + ia];
-        }
-      }
-    }
-  }
-}
-
 int qgw_get(qgw_run* r, double* psi, double* q) {
   if (!r) return QGW_ERR_PARAM;
   if (!r->has_q) return QGW_ERR_STATE;
@@ -1100,34 +1049,28 @@ int qgw_get(qgw_run* r, double* psi, double* q) {
   // ghost values of a no-slip or partial-slip wall
   if (psi || (r->p.bc_fac != 0 && r->p.bc_fac != -1)) enqueue_invert(r);
   const size_t nfull = (size_t)r->nl * (r->ny + 2) * (r->nx + 2);
-  // one field out through the staging buffer: pack (interior), contiguous copy
-  // (the pack kernel writes the caller's array directly where the device
-  // can address it)
+  const bool per = r->p.bc_fac == -1;
+  const double c = per ? 0.0 : 2 * r->p.bc_fac / (r->Delta * r->Delta);
+  // one field out, its ring included: packed straight into the caller's array
+  // where the device can address it, else into the staging buffer and copied
   auto fetch = [&](bool want_psi, double* host) -> int {
     double* view = (double*)device_view(r, host);
     double* dst = view ? view : r->d_full;
+    const bool ring = !want_psi && c != 0;
     if (r->precision == QGW_FP64)
-      qgw::enqueue_pack_f64(want_psi ? r->a64.psi : r->a64.q, dst, r->nx, r->ny, r->nl, r->pitch, r->stream);
+      qgw::enqueue_pack_f64(want_psi ? r->a64.psi : r->a64.q, ring ? r->a64.psi : nullptr, c, per, dst, r->nx, r->ny,
+                            r->nl, r->pitch, r->stream);
     else
-      qgw::enqueue_pack_join(want_psi ? r->a32.psi : r->a32.q, want_psi ? nullptr : r->a32.qlo, dst, r->nx, r->ny,
-                             r->nl, r->pitch, r->stream);
+      qgw::enqueue_pack_join(want_psi ? r->a32.psi : r->a32.q, want_psi ? nullptr : r->a32.qlo,
+                             ring ? r->a32.psi : nullptr, c, per, dst, r->nx, r->ny, r->nl, r->pitch, r->stream);
     if (!view) CK(cudaMemcpyAsync(host, r->d_full, sizeof(double) * nfull, cudaMemcpyDeviceToHost, r->stream));
-    CK(cudaStreamSynchronize(r->stream));
     return QGW_OK;
   };
   int rc;
   if (psi && (rc = fetch(true, psi))) return rc;
   if (q && (rc = fetch(false, q))) return rc;
+  CK(cudaStreamSynchronize(r->stream));
   CK(cudaGetLastError());
-  const double c = 2 * r->p.bc_fac / (r->Delta * r->Delta);
-  std::vector<double> psi_tmp;
-  const double* ps = psi;
-  if (r->p.bc_fac != -1 && q && !psi && c != 0) {
-    psi_tmp.resize((size_t)(r->nx + 2) * (r->ny + 2) * r->nl);
-    if ((rc = fetch(true, psi_tmp.data()))) return rc;
-    ps = psi_tmp.data();
-  }
-  fill_ghosts(r, psi, q, ps);
   return QGW_OK;
 }
 

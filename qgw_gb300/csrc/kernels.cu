@@ -101,7 +101,7 @@ static __global__ void k_begin(DevState* st, double t_out, double tend) {
 
 template <typename T, bool COMP>
 // (a.qout: also writes the final q, joined to FP64, into the caller's array
-// in the reference layout -- the interior; the host fills the ghost ring)
+// in the reference layout, its ring included)
 __global__ void __launch_bounds__(NT) k_flush(StepArgs<T> a) {
   grid_wait();
   DevState* st = a.state;
@@ -115,7 +115,6 @@ __global__ void __launch_bounds__(NT) k_flush(StepArgs<T> a) {
   const T* f0 = a.fab + s0 * fs;
   const T* f1 = a.fab + s1 * fs;
   const T* f2 = a.fab + s2 * fs;
-  const size_t n = (size_t)a.nl * a.ny * a.nx;
   const T* r1 = nullptr;
   const T* r2 = nullptr;
   T w1 = T(0), w2 = T(0);
@@ -126,37 +125,49 @@ __global__ void __launch_bounds__(NT) k_flush(StepArgs<T> a) {
     w1 = (T)fw.w1;
     w2 = (T)fw.w2;
   }
-  for (size_t w = blockIdx.x * (size_t)NT + threadIdx.x; w < n; w += (size_t)gridDim.x * NT) {
-    const size_t row = w / a.nx;
-    const int i = (int)(w - row * a.nx);
-    const size_t o = row * a.pitch + i;
-    // layer 0 also takes the stochastic forcing (src/timestep.h:143-150)
-    const T* fo = (a.fr.on && row < (size_t)a.ny) ? a.fr.field + o : nullptr;
-    double out;
-    if (COMP) {
-      float hi = (float)a.q[o], lo = (float)a.qlo[o];
-      if (pend) {
-        const float d = ab3_increment((float)c0, (float)c1, (float)c2, (float)f0[o], (float)f1[o], (float)f2[o]);
-        comp_add(hi, lo, d);
-        if (fo) comp_add(hi, lo, (float)*fo * (float)sqdt);
-        if (r1) comp_add(hi, lo, (float)forc4d_term<T>(r1, r2, o, w1, w2, (T)st->dt));
-        a.q[o] = (T)hi;
-        a.qlo[o] = (T)lo;
+  const int nxp2 = a.nx + 2;
+  for (int row = blockIdx.x; row < a.nl * a.ny; row += gridDim.x) {
+    const int l = row / a.ny, j = row - l * a.ny;
+    const size_t o0 = (size_t)l * a.lstride + (size_t)j * a.pitch;
+    // the caller's row, and the ring row that goes with the first and last:
+    // zero at walls (no-slip rings do not come this way), wrapped if periodic
+    double* out = a.qout ? a.qout + ((size_t)l * (a.ny + 2) + j + 1) * nxp2 : nullptr;
+    for (int i = threadIdx.x; i < a.nx; i += NT) {
+      const size_t o = o0 + i;
+      // layer 0 also takes the stochastic forcing (src/timestep.h:143-150)
+      const T* fo = (a.fr.on && l == 0) ? a.fr.field + o : nullptr;
+      double v;
+      if (COMP) {
+        float hi = (float)a.q[o], lo = (float)a.qlo[o];
+        if (pend) {
+          const float d = ab3_increment((float)c0, (float)c1, (float)c2, (float)f0[o], (float)f1[o], (float)f2[o]);
+          comp_add(hi, lo, d);
+          if (fo) comp_add(hi, lo, (float)*fo * (float)sqdt);
+          if (r1) comp_add(hi, lo, (float)forc4d_term<T>(r1, r2, o, w1, w2, (T)st->dt));
+          a.q[o] = (T)hi;
+          a.qlo[o] = (T)lo;
+        }
+        v = (double)hi + (double)lo;
+      } else {
+        T q = a.q[o];
+        if (pend) {
+          q = ab3_plain<T>(q, (T)c0, (T)c1, (T)c2, f0[o], f1[o], f2[o]);
+          if (fo) q = q + *fo * (T)sqdt;
+          if (r1) q = q + forc4d_term<T>(r1, r2, o, w1, w2, (T)st->dt);
+          a.q[o] = q;
+        }
+        v = (double)q;
       }
-      out = (double)hi + (double)lo;
-    } else {
-      T v = a.q[o];
-      if (pend) {
-        v = ab3_plain<T>(v, (T)c0, (T)c1, (T)c2, f0[o], f1[o], f2[o]);
-        if (fo) v = v + *fo * (T)sqdt;
-        if (r1) v = v + forc4d_term<T>(r1, r2, o, w1, w2, (T)st->dt);
-        a.q[o] = v;
+      if (out) {
+        auto put = [&](double* at, double x) {
+          at[i + 1] = x;
+          if (i == (a.periodic ? a.nx - 1 : 0)) at[0] = a.periodic ? x : 0.0;
+          if (i == (a.periodic ? 0 : a.nx - 1)) at[nxp2 - 1] = a.periodic ? x : 0.0;
+        };
+        put(out, v);
+        if (j == 0) put(out + (a.periodic ? a.ny : -1) * nxp2, a.periodic ? v : 0.0);
+        if (j == a.ny - 1) put(out + (a.periodic ? -a.ny : 1) * nxp2, a.periodic ? v : 0.0);
       }
-      out = (double)v;
-    }
-    if (a.qout) {
-      const size_t l = row / a.ny, jj = row - l * a.ny;
-      a.qout[(l * (a.ny + 2) + jj + 1) * (a.nx + 2) + i + 1] = out;
     }
   }
 }
@@ -275,37 +286,52 @@ static void launch_forcing(const StepArgs<T>& a, cudaStream_t s) {
 }
 
 // Boundary copies: the reference layout (nl, ny+2, nx+2) in one contiguous
-// device buffer <-> the interior-only run layout; a host array then crosses
-// the link in one contiguous copy instead of one row per DMA segment.
+// device buffer (or the caller's host array) <-> the interior-only run
+// layout, a row at a time.
 template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(256) k_unpack(const double* __restrict__ full, T* __restrict__ dst,
                                                 T* __restrict__ lo, int nx, int ny, int nl, int pitch) {
-  const size_t n = (size_t)nl * ny * nx;
-  for (size_t w = blockIdx.x * (size_t)blockDim.x + threadIdx.x; w < n; w += (size_t)gridDim.x * blockDim.x) {
-    const size_t row = w / nx;
-    const int i = (int)(w - row * nx);
-    const int l = (int)(row / ny), j = (int)(row - (size_t)l * ny);
-    const double v = full[((size_t)l * (ny + 2) + (j + 1)) * (nx + 2) + (i + 1)];
-    const size_t o = row * pitch + i;
-    if (SPLIT) {
-      const float h = (float)v;
-      dst[o] = (T)h;
-      lo[o] = (T)(float)(v - (double)h);
-    } else {
-      dst[o] = (T)v;
+  for (int row = blockIdx.x; row < nl * ny; row += gridDim.x) {
+    const int l = row / ny, j = row - l * ny;
+    const double* src = full + ((size_t)l * (ny + 2) + (j + 1)) * (nx + 2) + 1;
+    const size_t o0 = (size_t)row * pitch;
+    for (int i = threadIdx.x; i < nx; i += 256) {
+      const double v = src[i];
+      if (SPLIT) {
+        const float h = (float)v;
+        dst[o0 + i] = (T)h;
+        lo[o0 + i] = (T)(float)(v - (double)h);
+      } else {
+        dst[o0 + i] = (T)v;
+      }
     }
   }
 }
+// The ring is what adjust_bc leaves after invert_pv (src/elliptic.h:152-153,
+// src/domain.h:225-256,308-348): wrapped values in a periodic basin; at walls
+// 0 (psi null) or c psi at the adjacent interior point, corners 0.  (On the
+// host, its columns were one cache miss a point on memory the GPU had just
+// written: 2 of 5 ms for the fields of 16 small runs.)
 template <typename T>
 __global__ void __launch_bounds__(256) k_pack(const T* __restrict__ src, const T* __restrict__ lo,
+                                              const T* __restrict__ psi, double c, int periodic,
                                               double* __restrict__ full, int nx, int ny, int nl, int pitch) {
-  const size_t n = (size_t)nl * ny * nx;
-  for (size_t w = blockIdx.x * (size_t)blockDim.x + threadIdx.x; w < n; w += (size_t)gridDim.x * blockDim.x) {
-    const size_t row = w / nx;
-    const int i = (int)(w - row * nx);
-    const int l = (int)(row / ny), j = (int)(row - (size_t)l * ny);
-    const size_t o = row * pitch + i;
-    full[((size_t)l * (ny + 2) + (j + 1)) * (nx + 2) + (i + 1)] = (double)src[o] + (lo ? (double)lo[o] : 0.0);
+  for (int row = blockIdx.x; row < nl * (ny + 2); row += gridDim.x) {
+    const int l = row / (ny + 2), jj = row - l * (ny + 2) - 1;
+    // the interior row of the values (the adjacent one at walls)
+    const bool iny = jj >= 0 && jj < ny;
+    const int j = iny ? jj : periodic ? (jj < 0 ? ny - 1 : 0) : (jj < 0 ? 0 : ny - 1);
+    const size_t o0 = ((size_t)l * ny + j) * pitch;
+    double* dst = full + (size_t)row * (nx + 2);
+    for (int i = threadIdx.x; i < nx + 2; i += 256) {
+      const bool inx = i > 0 && i <= nx;
+      const int g = inx ? i - 1 : periodic ? (i ? 0 : nx - 1) : (i ? nx - 1 : 0);
+      const size_t o = o0 + g;
+      double v = 0.0;
+      if ((inx && iny) || periodic) v = (double)src[o] + (lo ? (double)lo[o] : 0.0);
+      else if (psi && (inx || iny)) v = c * (double)psi[o];
+      dst[i] = v;
+    }
   }
 }
 
@@ -574,9 +600,7 @@ static void launch_invert(const StepArgs<T>& a, int step_mode, bool pdl, cudaStr
 
 template <typename T, bool COMP>
 static void launch_flush(const StepArgs<T>& a, DevState* host, cudaStream_t s) {
-  const size_t n = (size_t)a.nl * a.ny * a.nx;
-  int blocks = (int)((n + NT - 1) / NT);
-  if (blocks > 152 * 8) blocks = 152 * 8;
+  const int blocks = std::min(a.nl * a.ny, 152 * 8);
   launch(k_flush<T, COMP>, dim3(blocks), dim3(NT), 0, s, true, a);
   launch(k_end, dim3(1), dim3(64), 0, s, true, a.state, host);
 }
@@ -604,12 +628,12 @@ void enqueue_begin(DevState* st, double t_out, double tend, cudaStream_t s) {
 
 void enqueue_unpack_split(const double* full, float* hi, float* lo, int nx, int ny, int nl, int pitch,
                           cudaStream_t s) {
-  k_unpack<float, true><<<152 * 8, 256, 0, s>>>(full, hi, lo, nx, ny, nl, pitch);
+  k_unpack<float, true><<<std::min(nl * ny, 152 * 8), 256, 0, s>>>(full, hi, lo, nx, ny, nl, pitch);
 }
 
-void enqueue_pack_join(const float* hi, const float* lo, double* full, int nx, int ny, int nl, int pitch,
-                       cudaStream_t s) {
-  k_pack<float><<<152 * 8, 256, 0, s>>>(hi, lo, full, nx, ny, nl, pitch);
+void enqueue_pack_join(const float* hi, const float* lo, const float* psi, double c, int periodic, double* full, int nx,
+                       int ny, int nl, int pitch, cudaStream_t s) {
+  k_pack<float><<<std::min(nl * (ny + 2), 152 * 8), 256, 0, s>>>(hi, lo, psi, c, periodic, full, nx, ny, nl, pitch);
 }
 
 int rhs_tile_x() { return TX; }
@@ -635,11 +659,12 @@ void enqueue_flush_f64(const StepArgs<double>& a, DevState* host, cudaStream_t s
 void enqueue_step_kernel_f64(const StepArgs<double>& a, int which, cudaStream_t s) { launch_one<double, false>(a, which, s); }
 
 void enqueue_unpack_f64(const double* full, double* q, int nx, int ny, int nl, int pitch, cudaStream_t s) {
-  k_unpack<double, false><<<152 * 8, 256, 0, s>>>(full, q, nullptr, nx, ny, nl, pitch);
+  k_unpack<double, false><<<std::min(nl * ny, 152 * 8), 256, 0, s>>>(full, q, nullptr, nx, ny, nl, pitch);
 }
 
-void enqueue_pack_f64(const double* src, double* full, int nx, int ny, int nl, int pitch, cudaStream_t s) {
-  k_pack<double><<<152 * 8, 256, 0, s>>>(src, nullptr, full, nx, ny, nl, pitch);
+void enqueue_pack_f64(const double* src, const double* psi, double c, int periodic, double* full, int nx, int ny, int nl,
+                      int pitch, cudaStream_t s) {
+  k_pack<double><<<std::min(nl * (ny + 2), 152 * 8), 256, 0, s>>>(src, nullptr, psi, c, periodic, full, nx, ny, nl, pitch);
 }
 
 void enqueue_split_f64(const double* src, float* hi, float* lo, size_t n, cudaStream_t s) {

@@ -84,3 +84,28 @@ def test_inversion_scales_with_q(qgwlib, e):
         out.append(r.get()[0] / f)
         r.close()
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("bc", [0.0, 1.0, -1.0])
+def test_rings(qgwlib, bc, prec):
+    """The ring of fields taken out: wrapped, or at walls psi = 0 and
+    q = 2 bc / Delta^2 psi at the adjacent point with corners of 0."""
+    p = dict(C.cfg1(40), NY=40 if bc < 0 else 24, bc_fac=bc)
+    r = qgwlib.Run(p, precision=prec)
+    r.set_q(C.noise_ic(p, 5))
+    psi, q = r.get()
+    out = np.full(r.shape, np.nan)
+    r.step_host(1, q, out)
+    again = r.get()
+    r.close()
+    c = 2 * bc / (p["Lx"] / 40) ** 2
+    for P, Q in ((psi, q), again, (again[0], out)):
+        eP, eQ = (np.pad(F[:, 1:-1, 1:-1], ((0, 0), (1, 1), (1, 1)), "wrap" if bc < 0 else "constant") for F in (P, Q))
+        if bc > 0:
+            eQ[:, 0], eQ[:, -1], eQ[:, 1:-1, 0], eQ[:, 1:-1, -1] = (c * F for F in (
+                P[:, 1], P[:, -2], P[:, 1:-1, 1], P[:, 1:-1, -2]))
+        assert np.array_equal(P, eP)
+        np.testing.assert_allclose(Q, eQ, rtol=1e-14, atol=0)
+    assert np.array_equal(again[1], out)

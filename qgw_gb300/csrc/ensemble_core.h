@@ -30,9 +30,11 @@ struct EnsembleCore {
   EnsSmem sm{};
   int total[4] = {0, 0, 0, 0};
   int rhs_total[5] = {0, 0, 0, 0, 0};
-  // persistent blocks per SM, per stage (tuned; capped by residency);
-  // 0: one block per work item
-  int bps[4] = {8, 8, 8, 8};
+  // persistent blocks per SM, per stage (tuned; capped by residency), or
+  // 0: one block per work item.  Items of one stage differ in length; a block
+  // that strides over several waits on its own latency where 8 independent
+  // ones overlap theirs: 16 members of 128^2 to 512^2, 505 against 448 us a step
+  int bps[4] = {0, 0, 0, 0};
   int grid[4] = {0, 0, 0, 0};
   int rhs_grid[5] = {0, 0, 0, 0, 0};
   cudaGraph_t graph = nullptr;

@@ -43,6 +43,7 @@ struct EnsembleCore {
 };
 
 // (re)build the device member table and work lists from e->members
+void ens_member_shape(qgw_run* r);  // the default shape of a new member
 int ens_core_build(EnsembleCore* e);
 void ens_core_free_tables(EnsembleCore* e);
 // enqueue up to nsteps steps for every member (max_steps[i] > 0 caps member

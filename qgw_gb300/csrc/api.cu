@@ -533,9 +533,16 @@ int setup_args(qgw_run* r, StepArgs<T>& a) {
   // 1, in zeta mode 1 zeta over the first sweep's region; zeta mode 2 reads
   // its field point by point)
   a.rhs_grid = 0;
-  // work-tile shape: RHS tiles of 16 rows (QGW_RHS_TILE_ROWS=32: 32 rows),
-  // the default column-tile width (a.CT = 0); qgw_set_shape changes them
+  // work-tile shape: the default column-tile width (a.CT = 0) and RHS tiles of
+  // 16 rows, or 32 in FP32c where the tiles carry no Laplacian sweep (halo 1:
+  // the ring of two tiles leaves the residency as it is) and are many: 1024^2 x
+  // 10 0.082 -> 0.066 ms, 2048^2 x 6 0.173 -> 0.130, 512^2 x 3 (1536 tiles of
+  // 16) 0.0205 -> 0.0197; 300^2 x 4 (760) 0.0168 against 0.0180; with sweeps
+  // 1024^2 x 10 0.103 against 0.125.  QGW_RHS_TILE_ROWS, qgw_set_shape change it.
   a.rhs_ty = 16;
+  if (sizeof(T) == 4 && (a.nsweep == 0 || a.zeta_mode == 2) &&
+      (r->nx + 31) / 32 * ((r->ny + 15) / 16) * r->nl >= 1500)
+    a.rhs_ty = 32;
   if (const char* e = std::getenv("QGW_RHS_TILE_ROWS")) a.rhs_ty = std::atoi(e) == 32 ? 32 : 16;
   encode_rhs_maps<T>(r, a);
   // FP32c K3: one block per row, or per (row, layer group) where the rows

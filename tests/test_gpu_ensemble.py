@@ -103,6 +103,25 @@ def test_shape_leaves_results_bitwise(qgwlib, prec):
         assert np.array_equal(psi, psi_a), (p["NX"], np.abs(psi - psi_a).max())
 
 
+@pytest.mark.parametrize("p", [dict(C.cfg1(512), NY=513), dict(C.cfg2(480, 4), hEkb=0.0)], ids=["viscosity", "chain"])
+def test_tall_rhs_tiles_by_default(qgwlib, p):
+    """FP32c without sweeps in its RHS tiles takes 32 rows from about 1500
+    16-row tiles on: bitwise the 16-row result."""
+    q0 = C.noise_ic(p, 43)
+    out = []
+    for rows in (32, 16):
+        r = qgwlib.Run(p, 1)
+        if rows == 16:
+            r.set_shape(rhs_tile_rows=16)
+        assert r.get_shape()["rhs_tile_rows"] == rows
+        r.set_q(q0)
+        r.fix_dt(p["dt"])
+        r.step(7)
+        out.append(r.get())
+        r.close()
+    assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][0], out[1][0])
+
+
 def test_shape_refuses_unknown_values(qgwlib):
     r = qgwlib.Run(C.cfg1(64), 1)
     before = r.get_shape()

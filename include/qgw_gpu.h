@@ -240,20 +240,21 @@ int qgw_footprint(const qgw_params* p, int precision, size_t* bytes);
 void* qgw_stream(qgw_run* run);
 int qgw_kernels_per_step(qgw_run* run);
 
-/* Run nsteps steps with CUDA events between the four kernels of each step
- * and return each kernel's mean duration in ms: ms4[0] rows forward
+/* Run nsteps steps with CUDA events between the four stages of each step
+ * and return each stage's mean duration in ms: ms4[0] rows forward
  * (AB3 + projection + x-DST), ms4[1] columns (y-DST, Helmholtz divide,
- * inverse y-DST), ms4[2] rows inverse (x-DST + back-projection), ms4[3] RHS. */
+ * inverse y-DST), ms4[2] rows inverse (x-DST + back-projection), ms4[3] RHS.
+ * (A stage is one kernel, in FP64 the row stages two: qgw_kernels_per_step.) */
 int qgw_profile_kernels(qgw_run* run, int nsteps, float* ms4);
 
 /* Work-tile shape of a run's step kernels (no counterpart in the
  * reference, which has no tiles): rhs_tile_rows, the RHS tile height (16 or
  * 32 rows); col_tile, columns per tile of the column transform (FP32: 8 or
  * 4, FP64: 4 or 2; a chirp-z NY keeps the width chosen at creation, 4 or 1
- * in FP32 and 2 or 1 in FP64); row_group_fwd and row_group_inv, modes (layers) per
- * block of the forward and inverse row kernels (1..16, balanced over the
- * run's layers; the inverse kernel takes at most 8 when it also transforms
- * zeta).  0 keeps a value.  No choice changes the arithmetic: a run's
+ * in FP32 and 2 or 1 in FP64); row_group_fwd and row_group_inv, rows per
+ * block of the forward and inverse row kernels (1..16; FP32: modes (layers) of
+ * one grid row, balanced over the run's, and at most 8 in an inverse kernel
+ * that also transforms zeta; FP64: rows of any layer).  0 keeps a value.  No choice changes the arithmetic: a run's
  * results are bitwise the same for every shape.  QGW_ERR_PARAM when a value
  * is not one of these or the shape needs more shared memory than the
  * device has (the run keeps its shape). */

@@ -9,8 +9,12 @@
 // phase before, so the shifts cost no barrier of their own.
 //
 // Measured at 1024^2 x 10 against the floating-point transforms (FP64 pipe
-// 83-88% busy): forward rows 0.64 -> 0.34 ms, columns 0.78 -> 0.28, inverse
-// rows 0.55 -> 0.28; rel-L2 error of q after 10 steps 1.7e-13 -> 2.3e-14.
+// 83-88% busy): columns 0.784 -> 0.255 ms; forward rows 0.640 -> 0.34 and
+// inverse rows 0.551 -> 0.28, and with the projections in kernels of their own
+// (modes_fx.cuh) 0.257 and 0.197 for both kernels; rel-L2 error of q after 10
+// steps 1.7e-13 -> 2.3e-14.  Bound by integer instructions: a product is six
+// (three multiplies, of which the wide one issues at 16 a clock and SM), a
+// double to fixed point and back a dozen each.
 #pragma once
 
 #include "dst_fx.h"

@@ -18,8 +18,7 @@
 //
 // A value v of a row stands for v 2^e, e the row's exponent.  A row whose
 // largest magnitude is infinite or NaN has every output NaN, a row of zeros
-// every output zero; magnitudes
-// below 2^-957 round to multiples of 2^-1015.
+// every output zero; magnitudes below 2^-957 round to multiples of 2^-1015.
 //
 // Work items as in dst_core.h: one item of one phase, any order within a
 // phase.  Buffers hold 8-byte values in the padded layout of doubles.
@@ -178,7 +177,6 @@ QGW_HD unsigned int fx_pre_item(const unsigned long long* x, fx_t* y, int j, int
 }
 
 // ---- phase 2: forward DFTs (exact but for the products)
-QGW_HD void fx_dft2(C2<fx_t>* v) { dft2<fx_t>(v); }
 QGW_HD fx_t fx_hs(fx_t v) { return fx_mulc<1>(v, -1257966796, -102865788); }  // v sqrt(1/2)
 QGW_HD void fx_dft8(C2<fx_t>* v) {
   C2<fx_t> a[4], b[4];

@@ -14,10 +14,11 @@
 namespace qgw {
 
 // ------------------------------------------------- single-run wrappers
+// The row kernels of the FP32c path (FP64: k_modes and k_rows_f64 below).
 // HL: 0, or the half-length whose transform alone the kernel holds (512:
 // the 1024-point rows and columns of the common grid)
 template <typename T, bool COMP, bool PER, int HL>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) k_rows_fwd(StepArgs<T> a, int step_mode) {
+__global__ void __launch_bounds__(NT, 4) k_rows_fwd(StepArgs<T> a, int step_mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(16) T tot[tot_len<T>];
   grid_wait();
@@ -35,10 +36,10 @@ __global__ void __launch_bounds__(NT, 3) k_cols(const __grid_constant__ StepArgs
   else body_cols<T, COMP, CT, HL>(a, step_mode, blockIdx.x, blockIdx.y, smem_raw, tot);
 }
 template <typename T> constexpr int CTD = ColsPer<T>::value;
-// FP32: four blocks per SM (64 registers; at 1024^2 x 10 the kernel drops
-// from 0.109 to 0.101 ms); FP64 keeps three (64 registers spill there)
+// four blocks per SM (64 registers; at 1024^2 x 10 the kernel drops from
+// 0.109 to 0.101 ms)
 template <typename T, bool COMP, bool PER, int HL>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) k_rows_inv(StepArgs<T> a, int step_mode) {
+__global__ void __launch_bounds__(NT, 4) k_rows_inv(StepArgs<T> a, int step_mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(16) T tot[tot_len<T>];
   grid_wait();
@@ -47,8 +48,8 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) k_rows_inv(StepArg
 }
 // The RHS of a step: a persistent grid (a.rhs_grid blocks) over the
 // ntx x nty x nl tiles (body_rhs_tiles); the FP64 path launches one block
-// per tile (its tiles keep the FP64 pipe busy, and blocks that each load
-// one tile overlap one another's loads without a second buffer).
+// per tile (bound by its integer instructions; blocks that each load one
+// tile overlap one another's loads without a second buffer).
 template <typename T, bool COMP, int R, int TY>
 __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 4) k_rhs(const __grid_constant__ StepArgs<T> a, int ntx,
                                                                     int nty) {
@@ -64,7 +65,10 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 4) k_rhs(const __grid
 }
 
 // FP64: the projections, one thread per point (NL: layers in registers, 0:
-// any number), and the row transforms (modes_fx.cuh)
+// any number), and the row transforms (modes_fx.cuh).  The projections wait
+// on their loads: four blocks per SM up to ten layers (64 registers; at three,
+// 1024^2 x 10 takes 0.267 ms for both forward kernels against 0.257, 768^2 x 8
+// 0.186 against 0.173), more layers need the registers.
 template <int NL, bool FWD>
 __global__ void __launch_bounds__(NT, NL <= 10 ? 4 : 2) k_modes(const __grid_constant__ StepArgs<double> a, int step_mode) {
   grid_wait();

@@ -12,7 +12,8 @@
 // where the floating-point form rounds at 2^-53 of |psi dq|, |psi| being tens
 // of |C| on any grid.  A point's few results become doubles at the end, for
 // the coefficients (3-4 FP64 operations a point instead of 34).  1024^2 x 10
-// with three sweeps: 0.767 -> 0.302 ms (FP64 pipe 86% busy before).
+// with three sweeps: 0.767 -> 0.303 ms (FP64 pipe 86% busy before; now about
+// 740 instructions a point, mostly integer).
 //
 // What stays in FP64 (rhs_tile_compute): edge tiles at walls with bc_fac !=
 // 0, whose ghost values (2 bc_fac / Delta^2 psi at every sweep) exceed the

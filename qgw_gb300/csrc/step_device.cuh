@@ -1,11 +1,11 @@
 // step_device.cuh -- the device side shared by the single-run kernels
 // (kernels.cu) and the ensemble kernels (kernels_ens.cu): the transforms,
-// the bodies of the four step kernels, the small device helpers and the
+// the bodies of the step kernels, the small device helpers and the
 // launch-size helpers.  Two translation units compile in parallel.
 #pragma once
-// The four kernels of one qgw time step on GB300 (sm_103a), for the plain
-// FP64 path (T = double) and the compensated FP32 path (T = float, q held
-// as hi + lo).
+// The kernels of one qgw time step on GB300 (sm_103a), for the plain FP64
+// path (T = double, in 64-bit block fixed point: dst_fx.cuh, modes_fx.cuh,
+// rhs_fx.cuh) and the compensated FP32 path (T = float, q held as hi + lo).
 //
 // One reference step (timestep, src/timestep.h:114-167) is
 //   K1 rows   : apply the pending AB3 update of the previous step, project
@@ -16,6 +16,8 @@
 //   K4 tiles  : RHS (Arakawa Jacobian, beta, viscosity, hyperviscosity,
 //               wind, bottom drag, topography) -> f0, CFL maximum; the last
 //               block advances dt/t and computes the AB3 coefficients
+// In FP64 the projections of K1 and K3 are kernels of their own, point by
+// point ahead of the forward and behind the column transforms: six a step.
 // The AB3 update q += c0 f0 + c1 f1 + c2 f2 needs the CFL-limited dt of the
 // same step, i.e. a reduction over all of psi, so it is applied by the next
 // step's K1 (or by the flush kernel at the end of a call), which saves one
@@ -157,11 +159,10 @@ __device__ __forceinline__ T* dst_block(T* A, T* B, int nrows, int ld, const Dst
   }
 }
 
-// The FP64 closed-basin transforms other than the chirp-z ones run in fixed
-// point (dst_fx.cuh); the block's scratch for them lies in tot.
-// values of tot: FP64 two scratches (the column kernel's two transforms; the
-// chirp-z form, two FFTs a transform, four), which leaves room for a third 1024-point column block per SM; FP32 the
-// chunk totals of the generic transform
+// Values of tot.  FP64: the scratch of the fixed-point transforms (dst_fx.cuh),
+// two for the column kernel's two transforms (the chirp-z form, two FFTs a
+// transform, four), which leaves room for a third 1024-point column block per
+// SM; FP32: the chunk totals of the generic transform.
 template <typename T, int HL = 0>
 constexpr int tot_len = sizeof(T) == 8 ? (int)((HL == -1 ? 4 : 2) * sizeof(FxScratch) / sizeof(T)) : GMAX * 32;
 static_assert(GMAX <= FX_ROWS && NT == FX_NT, "a scratch holds every row");
@@ -302,7 +303,7 @@ __device__ __forceinline__ T forc4d_term(const T* rec1, const T* rec2, size_t o,
   return (w1 * rec1[o] + w2 * rec2[o]) * dt;
 }
 
-// ------------------------------------------------------- mode projections
+// -------------------------------- mode projections (FP32; FP64: modes_fx.cuh)
 // The nl x G coefficients of one mode group are staged in shared memory as
 // cst[l * GMAX + gg] (zero for gg >= G), so one vector load serves a row of
 // the group and the group loops have a compile-time width GB >= G.  A padded
@@ -339,13 +340,13 @@ __device__ __forceinline__ int group_width(int G) { return G <= 1 ? 1 : G <= 2 ?
 // accumulates the G modes of its points in registers, layer by layer.
 // frow (optional): the stochastic forcing of row j, added to layer 0 as
 // frow * sqdt after the AB3 update (src/timestep.h:143-150)
-// FK: 0 no forcing, 1 stochastic forcing only (layer 0), 2 either or both
-// -- separate instantiations, so that each loop carries only the forcing it
-// applies; 3: no update pending, q comes from the caller's array a.qin
+// FK: 0 no forcing, 2 stochastic (layer 0), 4-D or both -- separate
+// instantiations, so that the common loop carries none; 3: no update
+// pending, q comes from the caller's array a.qin
 // (reference layout) and is stored into the run's field on the way.
 // Point i of the row goes to index i + xo of its mode row (xo = 1: the DST's
 // x_{i+1} at index i+1; xo = 0: the real FFT's x_i at index i).
-template <typename T, bool COMP, int GB, int FK>
+template <typename T, int GB, int FK>
 __device__ __forceinline__ void project_fwd(const StepArgs<T>& a, int j, bool upd, T c0, T c1, T c2, const T* f0,
                                             const T* f1, const T* f2, int G, T* A, int ld, const T* cst,
                                             const T* frow, T sqdt, const T* r1, const T* r2, T w1, T w2,
@@ -370,16 +371,9 @@ __device__ __forceinline__ void project_fwd(const StepArgs<T>& a, int j, bool up
           const int l = l0 + u;
           if (l >= a.nl) break;
           const size_t o = o0 + (size_t)l * a.lstride;
-          T v;
-          if constexpr (COMP) {
-            const float hi = (float)x[u];
-            a.q[o] = (T)hi;
-            a.qlo[o] = (T)(float)(x[u] - (double)hi);
-            v = (T)hi;
-          } else {
-            v = (T)x[u];
-            a.q[o] = v;
-          }
+          const T v = (T)x[u];
+          a.q[o] = v;
+          a.qlo[o] = (T)(x[u] - (double)v);
           T c[GB];
           ld_coefs<GB, T>(cst + l * GMAX, c);
 #pragma unroll
@@ -392,12 +386,10 @@ __device__ __forceinline__ void project_fwd(const StepArgs<T>& a, int j, bool up
         if (g < G) A[g * ld + pi] = acc[g];
     }
   } else {
-  // FP32: two points per pass (i and i + NT, the second absent past the
-  // row's end), every layer's loads of both issued before either is used:
-  // the fields stream from HBM/L2 and one point's chain of layers alone
-  // leaves the loads' latency exposed.  FP64 (bound by its FP64 pipe, and
-  // without registers for a second point's 16-wide groups): one point.
-  constexpr int PP = sizeof(T) == 4 ? 2 : 1;
+  // two points per pass (i and i + NT, the second absent past the row's
+  // end), every layer's loads of both issued before either is used: the
+  // fields stream from HBM/L2 and one point's chain of layers alone leaves
+  // the loads' latency exposed
   T* __restrict__ qh = a.q;
   T* __restrict__ ql = a.qlo;
   const T* __restrict__ g0 = f0;
@@ -406,38 +398,23 @@ __device__ __forceinline__ void project_fwd(const StepArgs<T>& a, int j, bool up
   // one layer of one point: the pending AB3 update (and forcing) of q,
   // stored back, and the value the projection takes
   auto layer = [&](int i, size_t o, int l, T qv, T lov, T a0, T a1, T a2) -> T {
-    if (COMP) {
-      float hi = (float)qv;
-      if (upd) {
-        float lo = (float)lov;
-        const float d = ab3_increment((float)c0, (float)c1, (float)c2, (float)a0, (float)a1, (float)a2);
-        comp_add(hi, lo, d);
-        if (FK == 1 && l == 0) comp_add(hi, lo, (float)frow[i] * (float)sqdt);
-        if (FK == 2) {
-          if (frow && l == 0) comp_add(hi, lo, (float)frow[i] * (float)sqdt);
-          if (r1) comp_add(hi, lo, (float)forc4d_term<T>(r1, r2, o, w1, w2, dtf));
-        }
-        qh[o] = (T)hi;
-        ql[o] = (T)lo;
+    float hi = (float)qv;
+    if (upd) {
+      float lo = (float)lov;
+      const float d = ab3_increment((float)c0, (float)c1, (float)c2, (float)a0, (float)a1, (float)a2);
+      comp_add(hi, lo, d);
+      if (FK == 2) {
+        if (frow && l == 0) comp_add(hi, lo, (float)frow[i] * (float)sqdt);
+        if (r1) comp_add(hi, lo, (float)forc4d_term<T>(r1, r2, o, w1, w2, dtf));
       }
-      return (T)hi;
-    } else {
-      T v = qv;
-      if (upd) {
-        v = ab3_plain<T>(v, c0, c1, c2, a0, a1, a2);
-        if (FK == 1 && l == 0) v = v + frow[i] * sqdt;
-        if (FK == 2) {
-          if (frow && l == 0) v = v + frow[i] * sqdt;
-          v = v + forc4d_term<T>(r1, r2, o, w1, w2, dtf);
-        }
-        qh[o] = v;
-      }
-      return v;
+      qh[o] = (T)hi;
+      ql[o] = (T)lo;
     }
+    return (T)hi;
   };
-  for (int i = threadIdx.x; i < a.nx; i += PP * NT) {
+  for (int i = threadIdx.x; i < a.nx; i += 2 * NT) {
     const int i2 = i + NT;
-    const bool two = PP == 2 && i2 < a.nx;
+    const bool two = i2 < a.nx;
     T acc[GB], acc2[GB];
 #pragma unroll
     for (int g = 0; g < GB; ++g) acc[g] = acc2[g] = T(0);
@@ -447,7 +424,8 @@ __device__ __forceinline__ void project_fwd(const StepArgs<T>& a, int j, bool up
       const T x = qh[o], x2 = two ? qh[o2] : T(0);
       T lo = T(0), lo2 = T(0), a0 = T(0), a1 = T(0), a2 = T(0), b0 = T(0), b1 = T(0), b2 = T(0);
       if (upd) {
-        if (COMP) { lo = ql[o]; if (two) lo2 = ql[o2]; }
+        lo = ql[o];
+        if (two) lo2 = ql[o2];
         a0 = g0[o]; a1 = g1[o]; a2 = g2[o];
         if (two) { b0 = g0[o2]; b1 = g1[o2]; b2 = g2[o2]; }
       }
@@ -494,9 +472,9 @@ __device__ __forceinline__ void body_rows_fwd(const StepArgs<T>& a, int step_mod
   const T* f1 = a.fab + s1 * fs;
   const T* f2 = a.fab + s2 * fs;
   const int tid = threadIdx.x;
-  // FP32 groups of 9..12 modes run at width 12 (three 16-byte coefficient
+  // groups of 9..12 modes run at width 12 (three 16-byte coefficient
   // vectors), the common 10-layer case without six idle accumulators
-  const int GB = (sizeof(T) == 4 && a.G1 > 8 && a.G1 <= 12) ? 12 : group_width(a.G1);
+  const int GB = (a.G1 > 8 && a.G1 <= 12) ? 12 : group_width(a.G1);
   if (!PER) prefetch_tables_l1(a.tx, a.gx.M);
   const T* frow = (ab3 && a.fr.on) ? a.fr.field + (size_t)j * a.pitch : nullptr;
   const T sqdt = frow ? (T)sqrt(st->dt) : T(0);
@@ -522,8 +500,8 @@ __device__ __forceinline__ void body_rows_fwd(const StepArgs<T>& a, int step_mod
       cst[w] = g < G ? a.cl2m[(size_t)(m0 + g) * a.nl + l] : T(0);
     }
     __syncthreads();
-    const int fk = (a.qin && m0 == 0) ? 3 : !upd ? 0 : r1 ? 2 : frow ? 1 : 0;
-#define QGW_PF(GBV, F) project_fwd<T, COMP, GBV, F>(a, j, upd, c0, c1, c2, f0, f1, f2, G, A, ld, cst, frow, sqdt, r1, \
+    const int fk = (a.qin && m0 == 0) ? 3 : upd && (r1 || frow) ? 2 : 0;
+#define QGW_PF(GBV, F) project_fwd<T, GBV, F>(a, j, upd, c0, c1, c2, f0, f1, f2, G, A, ld, cst, frow, sqdt, r1, \
                                                   r2, w1, w2, dtf, PER ? 0 : 1)
 #define QGW_PF_GB(F)                 \
   switch (GB) {                      \
@@ -531,21 +509,13 @@ __device__ __forceinline__ void body_rows_fwd(const StepArgs<T>& a, int step_mod
     case 2: QGW_PF(2, F); break;     \
     case 4: QGW_PF(4, F); break;     \
     case 8: QGW_PF(8, F); break;     \
-    case 12:                         \
-      if constexpr (sizeof(T) == 4) {\
-        QGW_PF(12, F);               \
-        break;                       \
-      }                              \
-      [[fallthrough]];               \
+    case 12: QGW_PF(12, F); break;   \
     default: QGW_PF(16, F); break;   \
   }
-    // the compensated path has registers for one forced loop only
     if (fk == 3) {
       QGW_PF_GB(3)
-    } else if (fk == 2 || (COMP && fk == 1)) {
+    } else if (fk == 2) {
       QGW_PF_GB(2)
-    } else if (fk == 1) {
-      if constexpr (!COMP) QGW_PF_GB(1)
     } else {
       QGW_PF_GB(0)
     }
@@ -1039,7 +1009,7 @@ __device__ __forceinline__ void body_cols_per(const StepArgs<T>& a, int step_mod
 
 // ------------------------------------------------------------------ K3
 // One block per row j with its LAYER groups in turn, or (a grid of rows x
-// groups, the FP64 default) one block per group of row j.  The mode -> layer
+// groups) one block per group of row j.  The mode -> layer
 // projection is linear and acts point by point, so it commutes with the
 // x-DST: each group first forms the spectral rows of its layers,
 // sum_m cm2l[l][m] * spec_m (and of zeta from spec2 in zeta mode), then
@@ -1050,14 +1020,12 @@ __device__ __forceinline__ void body_cols_per(const StepArgs<T>& a, int step_mod
 template <typename T, bool ZM, int GB>
 __device__ __forceinline__ void project_spec(const StepArgs<T>& a, int j, int G, T* A, int ld, const T* cst,
                                              int ncols, int xo) {
-  // FP32: two columns per pass (i and i + NT), each mode's loads of both
-  // issued before either is used (the spectral rows come from L2); FP64
-  // (FP64-pipe bound, registers for one column's groups): one column
-  constexpr int PP = sizeof(T) == 4 ? 2 : 1;
+  // two columns per pass (i and i + NT), each mode's loads of both issued
+  // before either is used (the spectral rows come from L2)
   const T* __restrict__ sp = a.spec;
   const T* __restrict__ sp2 = a.spec2;
-  for (int i = threadIdx.x; i < ncols; i += PP * NT) {
-    const bool two = PP == 2 && i + NT < ncols;
+  for (int i = threadIdx.x; i < ncols; i += 2 * NT) {
+    const bool two = i + NT < ncols;
     T acc[GB], zacc[ZM ? GB : 1], acc2[GB], zacc2[ZM ? GB : 1];
 #pragma unroll
     for (int g = 0; g < GB; ++g) {

@@ -5,8 +5,8 @@ commands of the profiles/ summaries run this file).
 
 The warm-up steps and the captured steps are separate qgw_step calls, so a
 profiler can skip the warm-up launches by count: each call launches one
-begin kernel, 4 kernels per step (7 with stochastic forcing), and a flush
-pair (2 kernels).
+begin kernel, 4 kernels per step (FP64: 6; 3 more with stochastic forcing),
+and a flush pair (2 kernels).
 """
 import argparse
 import os

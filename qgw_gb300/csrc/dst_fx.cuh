@@ -9,9 +9,9 @@
 // phase before, so the shifts cost no barrier of their own.
 //
 // Measured at 1024^2 x 10 against the floating-point transforms (FP64 pipe
-// 83-88% busy): columns 0.784 -> 0.255 ms; forward rows 0.640 -> 0.34 and
+// 83-88% busy): columns 0.784 -> 0.227 ms; forward rows 0.640 -> 0.34 and
 // inverse rows 0.551 -> 0.28, and with the projections in kernels of their own
-// (modes_fx.cuh) 0.257 and 0.197 for both kernels; rel-L2 error of q after 10
+// (modes_fx.cuh) 0.254 and 0.193 for both kernels; rel-L2 error of q after 10
 // steps 1.7e-13 -> 2.3e-14.  Bound by integer instructions: a product is six
 // (three multiplies, of which the wide one issues at 16 a clock and SM), a
 // double to fixed point and back a dozen each.
@@ -93,20 +93,29 @@ __device__ __forceinline__ int fx_drop(const FxScratch* sc, int r, int npass) {
 // ---- compile-time lengths H = 2^LGH >= 64
 // One Stockham pass (StockhamItem's indices, dst_fixed.cuh) over all rows;
 // RAW (the first pass): of raw doubles, whose largest high words mag_in holds.
-template <int R, int NS, int H, bool RAW = false>
+// ONE: in place -- the block's threads take one item each of whole rows, and
+// read all of them before any is written.
+template <int R, int NS, int H, bool RAW = false, bool ONE = false>
 __device__ __forceinline__ void fx_pass_fixed(const fx_t* src, fx_t* dst, int nrows, int ld, const Q4* tw,
                                               const unsigned int* mag_in, unsigned int* mag_out) {
   constexpr int NB = H / R, S = H / R;
   constexpr int LG = Pad<double>::LG, W = Pad<double>::W;
   auto pco = [](int e) { return e + W * (e >> LG); };
+  static_assert(!ONE || (FX_NT % NB == 0 && NB >= 32), "a round of items is whole rows, and whole warps have one");
   const int n = nrows * NB;
-  for (int w = threadIdx.x; w < n; w += FX_NT) {
+  for (int w = threadIdx.x; ONE ? w - (int)threadIdx.x < n : w < n; w += FX_NT) {
     const int r = w / NB, b = w & (NB - 1), k = b & (NS - 1);
     const C2<fx_t>* in = (const C2<fx_t>*)(src + r * ld) + pc<double>(b);
     C2<fx_t>* out = (C2<fx_t>*)(dst + r * ld) + pc<double>((b - k) * R + k);
     C2<fx_t> v[R];
+    if (!ONE || w < n) {
 #pragma unroll
-    for (int q = 0; q < R; ++q) v[q] = in[pco(q * S)];
+      for (int q = 0; q < R; ++q) v[q] = in[pco(q * S)];
+    }
+    if constexpr (ONE) {
+      __syncthreads();
+      if (w >= n) continue;
+    }
     if constexpr (RAW) {
       const int E = fx_scale(mag_in[r]);
 #pragma unroll
@@ -126,7 +135,7 @@ __device__ __forceinline__ void fx_pass_fixed(const fx_t* src, fx_t* dst, int nr
 // The passes of the complex FFT of 2^LGH points from src, dst the second
 // buffer; returns the buffer of the result, whose magnitudes are in
 // sc->mag[passes - 1].  Ends with the block synchronised.
-template <int LGH, bool RAW>
+template <int LGH, bool RAW, bool ONE = false>
 __device__ __forceinline__ fx_t* fx_passes_fixed(fx_t* src, fx_t* dst, int nrows, int ld, const Q4* tw, FxScratch* sc) {
   constexpr int H = 1 << LGH, NP8 = LGH / 3, RL = 1 << (LGH % 3);
   static_assert(LGH >= 6 && NP8 <= 4, "two to four radix-8 passes");
@@ -136,12 +145,12 @@ __device__ __forceinline__ fx_t* fx_passes_fixed(fx_t* src, fx_t* dst, int nrows
     src = dst;
     dst = t;
   };
-  fx_pass_fixed<8, 1, H, RAW>(src, dst, nrows, ld, nullptr, sc->mx, sc->mag[0]);
+  fx_pass_fixed<8, 1, H, RAW, ONE>(src, dst, nrows, ld, nullptr, sc->mx, sc->mag[0]);
   turn();
-  fx_pass_fixed<8, 8, H>(src, dst, nrows, ld, tw, sc->mag[0], sc->mag[1]);
+  fx_pass_fixed<8, 8, H, false, ONE>(src, dst, nrows, ld, tw, sc->mag[0], sc->mag[1]);
   turn();
   if constexpr (NP8 >= 3) {
-    fx_pass_fixed<8, 64, H>(src, dst, nrows, ld, tw + 56, sc->mag[1], sc->mag[2]);
+    fx_pass_fixed<8, 64, H, false, ONE>(src, dst, nrows, ld, tw + 56, sc->mag[1], sc->mag[2]);
     turn();
   }
   if constexpr (NP8 >= 4) {
@@ -156,10 +165,16 @@ __device__ __forceinline__ fx_t* fx_passes_fixed(fx_t* src, fx_t* dst, int nrows
   return src;
 }
 
-template <int LGH>
+// ONE (LGH = 9): all in A, B unused.  Apart from the passes every item writes
+// what it alone reads.  Half the shared memory, so a fourth block per SM at 64
+// registers, for one more barrier a pass: 1024^2 x 10 columns 0.257 -> 0.227
+// ms, rows 0.258 -> 0.254 and 0.197 -> 0.193.
+template <int LGH, bool ONE = false>
 __device__ fx_t* dst_fx_fixed(double* A, double* B, int nrows, int ld, const FxTables& tb, FxScratch* sc) {
   constexpr int H = 1 << LGH, M = 2 * H, NP = LGH / 3 + (LGH % 3 ? 1 : 0);
+  static_assert(!ONE || LGH == 9, "three radix-8 passes of 64 items a row");
   const int tid = threadIdx.x, lane = tid & 31;
+  if (ONE) B = A;
   // pre-processing, A -> B
   for (int w = tid; w < nrows * H; w += FX_NT) {
     const int r = w >> LGH, j = (w & (H - 1)) + 1;
@@ -169,8 +184,8 @@ __device__ fx_t* dst_fx_fixed(double* A, double* B, int nrows, int ld, const FxT
     if (lane == 0) atomicAdd(&sc->l1[r], t);
   }
   __syncthreads();
-  fx_t* src = fx_passes_fixed<LGH, false>((fx_t*)B, (fx_t*)A, nrows, ld, tb.twq, sc);
-  fx_t* dst = src == (fx_t*)A ? (fx_t*)B : (fx_t*)A;
+  fx_t* src = fx_passes_fixed<LGH, false, ONE>((fx_t*)B, (fx_t*)A, nrows, ld, tb.twq, sc);
+  fx_t* dst = ONE ? src : src == (fx_t*)A ? (fx_t*)B : (fx_t*)A;
   // split: items k = 0..H/2-1, item 0 also k = H/2 (and R_0)
   {
     constexpr int KI = H / 2;
@@ -415,7 +430,7 @@ __device__ __forceinline__ fx_t* dst_fx_blue(double* A, double* B, int nrows, in
 template <int HL>
 __device__ __forceinline__ fx_t* dst_fx(double* A, double* B, int nrows, int ld, const DstGeom& g, const FxTables& tb,
                                         FxScratch* sc) {
-  if constexpr (HL == 512) return dst_fx_fixed<9>(A, B, nrows, ld, tb, sc);
+  if constexpr (HL == 512) return dst_fx_fixed<9, true>(A, B, nrows, ld, tb, sc);
   if constexpr (HL == -1) return dst_fx_blue(A, B, nrows, ld, g, tb, sc);
   switch (g.H) {
     case 64: return dst_fx_fixed<6>(A, B, nrows, ld, tb, sc);

@@ -24,10 +24,11 @@ __global__ void __launch_bounds__(NT, 4) k_rows_fwd(StepArgs<T> a, int step_mode
   grid_wait();
   body_rows_fwd<T, COMP, PER, HL>(a, step_mode, blockIdx.x, smem_raw + cst_bytes<T>(a.nl), tot, (T*)smem_raw);
 }
+// FP64, HL = 512: in place, four blocks per SM at 64 registers (dst_fx_fixed).
 // CT: columns per tile (closed basin, and complex columns in FP64; the FP32
 // periodic kernel takes two complex columns whatever CT)
 template <typename T, bool COMP, bool PER, int CT, int HL>
-__global__ void __launch_bounds__(NT, 3) k_cols(const __grid_constant__ StepArgs<T> a, int step_mode) {
+__global__ void __launch_bounds__(NT, sizeof(T) == 8 && HL == 512 ? 4 : 3) k_cols(const __grid_constant__ StepArgs<T> a, int step_mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(16) T tot[tot_len<T, HL>];
   grid_wait();
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__(NT, NL <= 10 ? 4 : 2) k_modes(const __grid_con
   else if (j < a.ny) modes_point<NL, FWD>(a, tb, u, j, i, cs);
 }
 template <bool PER, int HL, bool INV>
-__global__ void __launch_bounds__(NT, 3) k_rows_f64(const __grid_constant__ StepArgs<double> a, int step_mode) {
+__global__ void __launch_bounds__(NT, HL == 512 ? 4 : 3) k_rows_f64(const __grid_constant__ StepArgs<double> a, int step_mode) {
   grid_wait();
   if (step_mode && !a.state->active) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -511,7 +512,8 @@ template <typename T, bool COMP>
 static void launch_k2(const StepArgs<T>& a, int step_mode, bool pdl, cudaStream_t s) {
   const int width = a.CT1 ? a.CT1 : col_width(a);
   const dim3 grid(a.periodic ? col_tiles(a) : (a.nx + width - 1) / width, a.nl);
-  const size_t sm = smem_cols<T, COMP>(a, width);
+  size_t sm = smem_cols<T, COMP>(a, width);
+  if constexpr (sizeof(T) == 8) sm = sm / 2 * fx_bufs(a, a.gy);
   const bool wide = width == CTD<T>, h512 = a.gy.H == 512 && !a.gy.blue;
   if constexpr (sizeof(T) == 8) {
     if (a.periodic) {

@@ -109,3 +109,27 @@ def test_rings(qgwlib, bc, prec):
         assert np.array_equal(P, eP)
         np.testing.assert_allclose(Q, eQ, rtol=1e-14, atol=0)
     assert np.array_equal(again[1], out)
+
+
+@pytest.mark.gpu
+def test_transforms_in_place(qgwlib):
+    """1024 points: the single run's transforms in one buffer, with blocks of
+    one to six rows and a last block of fewer, against the ensemble's in
+    two, bit for bit."""
+    p = C.cfg2(1024, 6)
+    q = C.noise_ic(p, 13)
+    ens = qgwlib.Ensemble([p], 0)
+    ens.set_q(0, q)
+    want = ens.get(0)[0]
+    ens.step(2)
+    want2 = ens.get(0)
+    ens.close()
+    for rows, cols in ((2, 4), (1, 2), (5, 4), (16, 4)):
+        r = qgwlib.Run(p)
+        r.set_shape(row_group_fwd=rows, row_group_inv=rows, col_tile=cols)
+        r.set_q(q)
+        assert np.array_equal(r.get()[0], want)
+        r.step(2)
+        psi, q2 = r.get()
+        r.close()
+        assert np.array_equal(psi, want2[0]) and np.array_equal(q2, want2[1]), rows

@@ -807,16 +807,9 @@ static int reset_history(qgw_run* r) {
   const size_t field = (size_t)r->nl * r->lstride;
   void* fab = r->precision == QGW_FP64 ? (void*)r->a64.fab : (void*)r->a32.fab;
   const size_t esz = r->precision == QGW_FP64 ? 8 : 4;
-  CK(cudaMemsetAsync(fab, 0, 3 * field * esz, r->stream));
-  // pending = 0, step_index = 0, maxbits = 0, done_blocks = 0
-  DevState* d = r->d_state;
-  CK(cudaMemsetAsync(&d->maxbits, 0, sizeof(unsigned long long), r->stream));
-  CK(cudaMemsetAsync(&d->done_blocks, 0, sizeof(unsigned int), r->stream));
-  CK(cudaMemsetAsync(&d->pending, 0, sizeof(int), r->stream));
-  CK(cudaMemsetAsync(&d->step_index, 0, sizeof(int), r->stream));
-  CK(cudaMemsetAsync(&d->forc_step, 0, sizeof(int), r->stream));
-  CK(cudaMemsetAsync(&d->nonfinite, 0, sizeof(int), r->stream));
-  CK(cudaMemsetAsync(&d->dev_error, 0, sizeof(int), r->stream));
+  // one launch in place of a memset for each counter: a set_q of a small run
+  // is mostly launches
+  qgw::enqueue_reset(r->d_state, fab, 3 * field * esz, r->stream);
   return QGW_OK;
 }
 

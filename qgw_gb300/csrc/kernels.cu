@@ -290,6 +290,25 @@ static void launch_forcing(const StepArgs<T>& a, cudaStream_t s) {
   k_forc_rows<T><<<a.ny, NT, (size_t)2 * padded_len<T>(f.gx.M) * sizeof(T), s>>>(a);
 }
 
+#if QGW_KERNELS_PART == 1
+// A new state's history: the three slabs of f (words: their 4-byte words) and
+// the counters of the step.
+static __global__ void __launch_bounds__(256) k_reset(DevState* st, unsigned int* fab, size_t words) {
+  uint4* f4 = reinterpret_cast<uint4*>(fab);
+  const size_t n4 = words / 4, t = (size_t)blockIdx.x * 256 + threadIdx.x;
+  for (size_t i = t; i < n4; i += (size_t)gridDim.x * 256) f4[i] = make_uint4(0, 0, 0, 0);
+  if (t < words - 4 * n4) fab[4 * n4 + t] = 0;
+  if (t == 0) {
+    st->maxbits = 0;
+    st->done_blocks = 0;
+    st->pending = 0;
+    st->step_index = 0;
+    st->forc_step = 0;
+    st->nonfinite = 0;
+    st->dev_error = 0;
+  }
+}
+#endif
 // Boundary copies: the reference layout (nl, ny+2, nx+2) in one contiguous
 // device buffer (or the caller's host array) <-> the interior-only run
 // layout, a row at a time.
@@ -664,6 +683,10 @@ void enqueue_flush_f64(const StepArgs<double>& a, DevState* host, cudaStream_t s
 
 void enqueue_step_kernel_f64(const StepArgs<double>& a, int which, cudaStream_t s) { launch_one<double, false>(a, which, s); }
 
+void enqueue_reset(DevState* st, void* fab, size_t bytes, cudaStream_t s) {
+  const size_t blocks = (bytes / 16 + 255) / 256 + 1;
+  k_reset<<<(int)std::min(blocks, (size_t)152 * 8), 256, 0, s>>>(st, (unsigned int*)fab, bytes / 4);
+}
 void enqueue_unpack_f64(const double* full, double* q, int nx, int ny, int nl, int pitch, cudaStream_t s) {
   k_unpack<double, false><<<std::min(nl * ny, 152 * 8), 256, 0, s>>>(full, q, nullptr, nx, ny, nl, pitch);
 }

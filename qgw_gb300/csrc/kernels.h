@@ -36,6 +36,8 @@ void enqueue_step_kernel_f32c(const StepArgs<float>& a, int which, cudaStream_t 
 void enqueue_unpack_f64(const double* full, double* q, int nx, int ny, int nl, int pitch, cudaStream_t s);
 void enqueue_unpack_split(const double* full, float* hi, float* lo, int nx, int ny, int nl, int pitch,
                           cudaStream_t s);
+// zero the slabs of f and the step's counters (one launch)
+void enqueue_reset(DevState* st, void* fab, size_t bytes, cudaStream_t s);
 // (the ring: wrapped, or at walls c psi at the adjacent point; psi null: zero)
 void enqueue_pack_f64(const double* src, const double* psi, double c, int periodic, double* full, int nx, int ny, int nl,
                       int pitch, cudaStream_t s);

@@ -177,8 +177,9 @@ def bytes_per_lgp(precision):
 
 
 def fp64_ops_per_lgp(nl, M, nsweep):
-    """FP64-pipe instructions (add, mul and fma each count one) per
-    layer-gridpoint of each kernel, from the kernels' arithmetic: DST-I of
+    """Floating-point operations (add, mul and fma each count one) per
+    layer-gridpoint of each stage done in FP64 -- what the fixed-point kernels
+    of the plain path stand in for, on the integer pipes: DST-I of
     length M-1 = pre-processing 2 + complex FFT of M/2 points (radix-8 first
     pass 52/8 per point, later passes 80/8, radix-4/2 tails) / 2 + split 3 +
     prefix sum 1."""
@@ -220,8 +221,9 @@ KERNEL_NAMES = ["rows_fwd (AB3 + projection + x-DST)", "cols (y-DST, Helmholtz, 
 def read_kernel_profile(precision, kernel):
     """ncu counters of one step kernel at this workload, from the committed
     summary profiles/traffic.json: per-launch DRAM bytes
-    (dram__bytes_read.sum + dram__bytes_write.sum) and, for the FP64 kernels,
-    the FP64 pipe's active share.  None when that kernel was not captured."""
+    (dram__bytes_read.sum + dram__bytes_write.sum; a stage of two kernels:
+    their sum) and the issue-active share.  None when that kernel was not
+    captured."""
     path = os.path.join(ROOT, "profiles", "traffic.json")
     try:
         with open(path) as f:
@@ -308,25 +310,26 @@ def run_ours(args, rank, world, local_rank):
     ops = fp64_ops_per_lgp(args.nl, M, nsweep)
     fp64_rate = ops[dom] * 2 * lgp / (kms64[dom] / 1e3) / 1e12  # one FMA slot = 2 flops
     prof64 = read_kernel_profile(0, dom) or {}
-    # The plain FP64 kernels are bound by the FP64 pipe, not by HBM: the
-    # headline roofline is that pipe (achieved = the kernel's FP64 operations
-    # from the instruction model, counted as FMA slots, over its CUDA-event
-    # time; peak = the FP64 FMA rate measured live on this GPU, which
-    # MEASURED_PEAKS.json does not carry), with ncu's FP64-pipe activity of
-    # the same kernel beside it and the HBM fraction as a secondary field.
-    roofline = {"bound": "fp64", "kernel": KERNEL_NAMES[dom], "achieved": fp64_rate, "peak": fp64_peak,
-                "unit": "TFLOP/s (FP64, FMA-slot equivalent)",
-                "frac": fp64_rate / fp64_peak if fp64_peak > 0 else None,
-                "peak_source": "measured live: qgw_probe_fp_rates (independent FP64 FMA chains)",
-                "ops_per_lgp_model": ops[dom],
-                "ncu_fp64_pipe_active_pct": prof64.get("fp64_pipe_active_pct"),
+    # The plain FP64 kernels compute in 64-bit fixed point and are bound by
+    # the issue of integer instructions (ncu's issue-active share beside it);
+    # the roofline is HBM's, over the algorithmic bytes, and fp64_pipe gives
+    # the rate the same arithmetic would need of the FP64 pipe against that
+    # pipe's FMA rate measured live on this GPU (above 1: beyond its roof).
+    step_bytes64 = sum(bpl) * lgp / (ms64 / K / 1e3) / 1e9
+    roofline = {"bound": "hbm", "limiter": "integer instruction issue (64-bit fixed point)",
+                "kernel": KERNEL_NAMES[dom], "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
+                "frac": achieved / hbm_peak, "peak_source": peak_kind, "bytes_per_lgp": bpl[dom],
                 "traffic": prof64.get("dram_bytes"),
-                "step_frac": sum(o * 2 * lgp for o in ops) / (ms64 / K / 1e3) / 1e12 / fp64_peak
-                if fp64_peak > 0 else None,
+                "ncu_issue_active_pct": prof64.get("issue_active_pct"),
+                "step_frac": step_bytes64 / hbm_peak,
                 "kernel_ms": kms64[dom], "all_kernels_ms": kms64,
-                "hbm": {"achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
-                        "peak_source": peak_kind, "bytes_per_lgp": bpl[dom],
-                        "traffic": prof64.get("dram_bytes")}}
+                "fp64_pipe": {"achieved": fp64_rate, "peak": fp64_peak,
+                              "unit": "TFLOP/s (FP64, FMA-slot equivalent)",
+                              "frac": fp64_rate / fp64_peak if fp64_peak > 0 else None,
+                              "peak_source": "measured live: qgw_probe_fp_rates (independent FP64 FMA chains)",
+                              "ops_per_lgp_model": ops[dom],
+                              "step_frac": sum(o * 2 * lgp for o in ops) / (ms64 / K / 1e3) / 1e12 / fp64_peak
+                              if fp64_peak > 0 else None}}
 
     # e2e: per step, q in from pinned host memory, one step, q out
     E = args.e2e_steps or K
@@ -385,7 +388,7 @@ def run_ours(args, rank, world, local_rank):
     cpu = None
     if getattr(args, "_cpu", None) is not None:
         cpu = args._cpu
-    launches = K * 4 + 3
+    launches = K * 6 + 3  # two kernels in each of the FP64 row stages; begin, flush, end
     out = {
         "metric": "layer-gridpoint-steps/s at 1024^2 x 10 layers (plain FP64 step)",
         "value": value, "unit": "lgp-steps/s", "n_gpus": world, "steps": K, "warmup": W,

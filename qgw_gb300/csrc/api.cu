@@ -106,7 +106,7 @@ int upload_modes(qgw_run* r, qgw::ModeTable* out, const std::vector<double>& mat
 }
 
 // Shared-memory budget of the row kernels' work buffers.  FP64: 74 KiB (three
-// blocks per SM; four rows of 1024).  FP32, the forward rows kernel: 56 KiB,
+// blocks per SM; four rows of 1024 in two buffers, half of it in place).  FP32, the forward rows kernel: 56 KiB,
 // which keeps four blocks per SM, and 40 KiB for rows of 2048 and more or more
 // than 10 layers; measured at 512^2, 1024^2 and 2048^2 with 10, 16 and 20
 // layers on GB300 (1024^2 x 16: 0.254 -> 0.197 ms).  QGW_ROW_SMEM_KB
@@ -515,7 +515,8 @@ int setup_args(qgw_run* r, StepArgs<T>& a) {
     const size_t limit = (size_t)200 * 1024;
     if (a.gy.blue) a.CT = (32 / (int)sizeof(T)) / 2;
     // FP64: 16-byte tiles already where 32-byte ones leave one block per SM
-    // (more than 113 KiB: NY > 1536)
+    // (more than 113 KiB in two buffers: NY > 1536; in place, 2048^2 x 6: 0.764
+    // ms against 0.619)
     if (need() > (sizeof(T) == 8 ? (size_t)113 * 1024 : limit)) a.CT = (32 / (int)sizeof(T)) / 2;
     if (a.gy.blue && need() > limit) a.CT = 1;
     // A single run's column kernel takes the narrower tiles too where the

@@ -11,7 +11,7 @@
 // Measured at 1024^2 x 10 against the floating-point transforms (FP64 pipe
 // 83-88% busy): columns 0.784 -> 0.227 ms; forward rows 0.640 -> 0.34 and
 // inverse rows 0.551 -> 0.28, and with the projections in kernels of their own
-// (modes_fx.cuh) 0.254 and 0.193 for both kernels; rel-L2 error of q after 10
+// (modes_fx.cuh) 0.249 and 0.191 for both kernels; rel-L2 error of q after 10
 // steps 1.7e-13 -> 2.3e-14.  Bound by integer instructions: a product is six
 // (three multiplies, of which the wide one issues at 16 a clock and SM), a
 // double to fixed point and back a dozen each.
@@ -93,15 +93,39 @@ __device__ __forceinline__ int fx_drop(const FxScratch* sc, int r, int npass) {
 // ---- compile-time lengths H = 2^LGH >= 64
 // One Stockham pass (StockhamItem's indices, dst_fixed.cuh) over all rows;
 // RAW (the first pass): of raw doubles, whose largest high words mag_in holds.
-// ONE: in place -- the block's threads take one item each of whole rows, and
-// read all of them before any is written.
+// ONE: in place -- the block's threads take items of whole rows, one each or U
+// of one row, and read all of them before any is written.
 template <int R, int NS, int H, bool RAW = false, bool ONE = false>
 __device__ __forceinline__ void fx_pass_fixed(const fx_t* src, fx_t* dst, int nrows, int ld, const Q4* tw,
                                               const unsigned int* mag_in, unsigned int* mag_out) {
   constexpr int NB = H / R, S = H / R;
   constexpr int LG = Pad<double>::LG, W = Pad<double>::W;
   auto pco = [](int e) { return e + W * (e >> LG); };
-  static_assert(!ONE || (FX_NT % NB == 0 && NB >= 32), "a round of items is whole rows, and whole warps have one");
+  static_assert(!ONE || ((FX_NT % NB == 0 || NB % FX_NT == 0) && NB >= 32), "a round is whole rows, and whole warps");
+  if constexpr (ONE && NB > FX_NT) {  // a row a round, U items a thread
+    constexpr int U = NB / FX_NT;
+    for (int r = 0; r < nrows; ++r) {
+      C2<fx_t>* row = (C2<fx_t>*)(src + r * ld);
+      C2<fx_t> v[U][R];
+      unsigned int m = 0;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int q = 0; q < R; ++q) v[u][q] = row[pc<double>((int)threadIdx.x + u * FX_NT) + pco(q * S)];
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int b = threadIdx.x + u * FX_NT, k = b & (NS - 1);
+        fx_twiddle<R>(v[u], k, NS, fx_pass_shift(mag_in[r]), tw);
+        fx_dft<R>(v[u]);
+#pragma unroll
+        for (int q = 0; q < R; ++q) row[pc<double>((b - k) * R + k) + pco(q * NS)] = v[u][q];
+        m |= fx_mag_all<R>(v[u]);
+      }
+      fx_row_or<NB>(mag_out, r, m);
+    }
+    return;
+  }
   const int n = nrows * NB;
   for (int w = threadIdx.x; ONE ? w - (int)threadIdx.x < n : w < n; w += FX_NT) {
     const int r = w / NB, b = w & (NB - 1), k = b & (NS - 1);
@@ -159,20 +183,20 @@ __device__ __forceinline__ fx_t* fx_passes_fixed(fx_t* src, fx_t* dst, int nrows
   }
   if constexpr (RL > 1) {
     constexpr int NS = 1 << (3 * NP8);
-    fx_pass_fixed<RL, NS, H>(src, dst, nrows, ld, tw + NS - 8, sc->mag[NP8 - 1], sc->mag[NP8]);
+    fx_pass_fixed<RL, NS, H, false, ONE>(src, dst, nrows, ld, tw + NS - 8, sc->mag[NP8 - 1], sc->mag[NP8]);
     turn();
   }
   return src;
 }
 
-// ONE (LGH = 9): all in A, B unused.  Apart from the passes every item writes
+// ONE (LGH = 9, 10): all in A, B unused.  Apart from the passes every item writes
 // what it alone reads.  Half the shared memory, so a fourth block per SM at 64
 // registers, for one more barrier a pass: 1024^2 x 10 columns 0.257 -> 0.227
-// ms, rows 0.258 -> 0.254 and 0.197 -> 0.193.
+// ms, rows 0.258 -> 0.254 and 0.197 -> 0.193; 2048^2 x 6 columns 0.782 ->
+// 0.619, rows 0.571 -> 0.557 and 0.443 -> 0.430.
 template <int LGH, bool ONE = false>
 __device__ fx_t* dst_fx_fixed(double* A, double* B, int nrows, int ld, const FxTables& tb, FxScratch* sc) {
   constexpr int H = 1 << LGH, M = 2 * H, NP = LGH / 3 + (LGH % 3 ? 1 : 0);
-  static_assert(!ONE || LGH == 9, "three radix-8 passes of 64 items a row");
   const int tid = threadIdx.x, lane = tid & 31;
   if (ONE) B = A;
   // pre-processing, A -> B
@@ -431,6 +455,7 @@ template <int HL>
 __device__ __forceinline__ fx_t* dst_fx(double* A, double* B, int nrows, int ld, const DstGeom& g, const FxTables& tb,
                                         FxScratch* sc) {
   if constexpr (HL == 512) return dst_fx_fixed<9, true>(A, B, nrows, ld, tb, sc);
+  if constexpr (HL == 1024) return dst_fx_fixed<10, true>(A, B, nrows, ld, tb, sc);
   if constexpr (HL == -1) return dst_fx_blue(A, B, nrows, ld, g, tb, sc);
   switch (g.H) {
     case 64: return dst_fx_fixed<6>(A, B, nrows, ld, tb, sc);

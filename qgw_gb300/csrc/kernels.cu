@@ -24,11 +24,11 @@ __global__ void __launch_bounds__(NT, 4) k_rows_fwd(StepArgs<T> a, int step_mode
   grid_wait();
   body_rows_fwd<T, COMP, PER, HL>(a, step_mode, blockIdx.x, smem_raw + cst_bytes<T>(a.nl), tot, (T*)smem_raw);
 }
-// FP64, HL = 512: in place, four blocks per SM at 64 registers (dst_fx_fixed).
+// FP64, HL = 512, 1024: in place, four blocks per SM at 64 registers (dst_fx_fixed).
 // CT: columns per tile (closed basin, and complex columns in FP64; the FP32
 // periodic kernel takes two complex columns whatever CT)
 template <typename T, bool COMP, bool PER, int CT, int HL>
-__global__ void __launch_bounds__(NT, sizeof(T) == 8 && HL == 512 ? 4 : 3) k_cols(const __grid_constant__ StepArgs<T> a, int step_mode) {
+__global__ void __launch_bounds__(NT, sizeof(T) == 8 && HL >= 512 ? 4 : 3) k_cols(const __grid_constant__ StepArgs<T> a, int step_mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(16) T tot[tot_len<T, HL>];
   grid_wait();
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(NT, NL > 10 ? 2 : NL == 8 ? 4 : 5) k_modes(con
   else if (j < a.ny) modes_point<NL, FWD>(a, tb, u, j, i, cs);
 }
 template <bool PER, int HL, bool INV>
-__global__ void __launch_bounds__(NT, HL == 512 ? 4 : 3) k_rows_f64(const __grid_constant__ StepArgs<double> a, int step_mode) {
+__global__ void __launch_bounds__(NT, HL >= 512 ? 4 : 3) k_rows_f64(const __grid_constant__ StepArgs<double> a, int step_mode) {
   grid_wait();
   if (step_mode && !a.state->active) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -448,7 +448,10 @@ static cudaError_t set_attrs(const StepArgs<T>& a) {
   for (const void* f : columns)
     if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, lim))) return e;
   if constexpr (sizeof(T) == 8) {
-    const void* rows[] = {(const void*)k_rows_f64<false, 0, false>,   (const void*)k_rows_f64<false, 0, true>,
+    const void* rows[] = {(const void*)k_cols<T, COMP, false, CTD<T>, 1024>,
+                          (const void*)k_cols<T, COMP, false, CTD<T> / 2, 1024>,
+                          (const void*)k_rows_f64<false, 1024, false>, (const void*)k_rows_f64<false, 1024, true>,
+                          (const void*)k_rows_f64<false, 0, false>,   (const void*)k_rows_f64<false, 0, true>,
                           (const void*)k_rows_f64<false, 512, false>, (const void*)k_rows_f64<false, 512, true>,
                           (const void*)k_rows_f64<false, -1, false>,  (const void*)k_rows_f64<false, -1, true>,
                           (const void*)k_rows_f64<true, 0, false>,    (const void*)k_rows_f64<true, 0, true>};
@@ -513,6 +516,7 @@ template <bool INV> static void launch_rows(const StepArgs<double>& a, int step_
   if (a.periodic) launch(k_rows_f64<true, 0, INV>, grid, dim3(NT), sm, s, pdl, a, step_mode);
   else if (a.gx.blue) launch(k_rows_f64<false, -1, INV>, grid, dim3(NT), sm, s, pdl, a, step_mode);
   else if (a.gx.H == 512) launch(k_rows_f64<false, 512, INV>, grid, dim3(NT), sm, s, pdl, a, step_mode);
+  else if (a.gx.H == 1024) launch(k_rows_f64<false, 1024, INV>, grid, dim3(NT), sm, s, pdl, a, step_mode);
   else launch(k_rows_f64<false, 0, INV>, grid, dim3(NT), sm, s, pdl, a, step_mode);
 }
 
@@ -543,6 +547,11 @@ static void launch_k2(const StepArgs<T>& a, int step_mode, bool pdl, cudaStream_
       const size_t bytes = (size_t)2 * cc * row_len<T>(a.gy) * sizeof(T);
       if (cc == 4) launch(k_cols<T, COMP, true, 4, 0>, tiles, dim3(NT), bytes, s, pdl, a, step_mode);
       else launch(k_cols<T, COMP, true, 2, 0>, tiles, dim3(NT), bytes, s, pdl, a, step_mode);
+      return;
+    }
+    if (a.gy.H == 1024 && !a.gy.blue) {
+      if (wide) launch(k_cols<T, COMP, false, CTD<T>, 1024>, grid, dim3(NT), sm, s, pdl, a, step_mode);
+      else launch(k_cols<T, COMP, false, CTD<T> / 2, 1024>, grid, dim3(NT), sm, s, pdl, a, step_mode);
       return;
     }
   }

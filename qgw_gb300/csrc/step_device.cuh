@@ -1869,10 +1869,10 @@ template <typename T, bool COMP>
 static size_t smem_rows(const StepArgs<T>& a) {
   return cst_bytes<T>(a.nl) + (size_t)dst_bufs(a, a.gx) * a.G1 * row_len<T>(a.gx) * sizeof(T);
 }
-// FP64: the buffers of a transform of the single-run kernels (1024 points: in
-// place)
+// FP64: the buffers of a transform of the single-run kernels (1024 and 2048
+// points: in place)
 static inline int fx_bufs(const StepArgs<double>& a, const DstGeom& g) {
-  return !a.periodic && !g.blue && g.H == 512 ? 1 : 2;
+  return !a.periodic && !g.blue && (g.H == 512 || g.H == 1024) ? 1 : 2;
 }
 static inline size_t smem_rows_f64(const StepArgs<double>& a, int rows) {
   return (size_t)fx_bufs(a, a.gx) * rows * row_len<double>(a.gx) * sizeof(double);

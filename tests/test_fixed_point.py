@@ -112,11 +112,12 @@ def test_rings(qgwlib, bc, prec):
 
 
 @pytest.mark.gpu
-def test_transforms_in_place(qgwlib):
-    """1024 points: the single run's transforms in one buffer, with blocks of
-    one to six rows and a last block of fewer, against the ensemble's in
-    two, bit for bit."""
-    p = C.cfg2(1024, 6)
+@pytest.mark.parametrize("N,nl", [(1024, 6), (2048, 3)])
+def test_transforms_in_place(qgwlib, N, nl):
+    """1024 and 2048 points: the single run's transforms in one buffer, with
+    blocks of one to six rows and a last block of fewer, against the
+    ensemble's in two, bit for bit."""
+    p = C.cfg2(N, nl)
     q = C.noise_ic(p, 13)
     ens = qgwlib.Ensemble([p], 0)
     ens.set_q(0, q)

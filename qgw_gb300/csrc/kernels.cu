@@ -67,13 +67,13 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 4) k_rhs(const __grid
 
 // FP64: the projections, one thread per point (NL: layers in registers, 0:
 // any number), and the row transforms (modes_fx.cuh).  The projections wait
-// on their loads: five blocks per SM up to ten layers (48 registers, few
-// spills; for eight layers four, where five spill and gain nothing).  Both
-// forward kernels, at three, four and five blocks: 1024^2 x 10 0.267, 0.255
-// and 0.249 ms, 2048^2 x 6 at four and five 0.591 and 0.571.  More layers
-// need the registers.
+// on their loads: five blocks per SM below eight layers (48 registers, few
+// spills), four up to ten.  Both forward kernels at three, four and five
+// blocks: 1024^2 x 10 0.265, 0.256 and 0.258 ms, 768^2 x 8 0.182, 0.173 and
+// 0.181, 1024^2 x 6 0.163, 0.157 and 0.155.  More layers need the registers
+// (any number, two and five blocks: 256^2 x 20 0.080 and 0.142).
 template <int NL, bool FWD>
-__global__ void __launch_bounds__(NT, NL > 10 ? 2 : NL == 8 ? 4 : 5) k_modes(const __grid_constant__ StepArgs<double> a, int step_mode) {
+__global__ void __launch_bounds__(NT, NL == 0 || NL > 10 ? 2 : NL >= 8 ? 4 : 5) k_modes(const __grid_constant__ StepArgs<double> a, int step_mode) {
   grid_wait();
   if (step_mode && !a.state->active) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];

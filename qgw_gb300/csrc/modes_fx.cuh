@@ -11,21 +11,17 @@
 // each pair of modes read the row's layers again.)  The extra pass over the
 // spectral field mostly stays in L2.
 //
-// A point's values become integers below 2^61 by the largest of them, the
-// coefficients integers below 2^60 by the largest of their row of the
-// matrix; products keep their high words (fx_mul's) and sums are exact, so
-// the result does not depend on how outputs are grouped: error about 2^-56 of
-// the largest term, below the FP64 sum's 2^-53.
-//
-// That holds while the inputs' columns of the matrix are of similar size: a
-// value is kept to 2^-61 of the point's largest, and a coefficient 2^k times
-// the others multiplies that.  So runs whose columns' largest entries differ
-// by more than 64 (strongly graded profiles of many layers, whose trapped
-// modes reach 1e6), or with more than 32 layers (the sums' headroom), keep
-// FP64 sums (a.modes_fx = 0).
+// The arithmetic is modes_core.h's.  It holds FP64's precision while the
+// inputs' columns of the matrix are of similar size: a value is kept to 2^-61
+// of the point's largest, and a coefficient 2^k times the others multiplies
+// that.  So runs whose columns' largest entries differ by more than 64
+// (strongly graded profiles of many layers, whose trapped modes reach 1e6), or
+// with more than 32 layers (the sums' headroom), keep FP64 sums (a.modes_fx = 0).
 #pragma once
 
 #include <type_traits>
+
+#include "modes_core.h"
 
 namespace qgw {
 
@@ -102,42 +98,23 @@ template <typename F> __device__ __forceinline__ void q_case(const StepArgs<doub
   else f(std::integral_constant<int, 2>{});
 }
 
-__device__ __forceinline__ int modes_exp(unsigned int hmax, int ce) {
-  return hmax >= 0x7ff00000u ? FX_NAN : hmax == 0 ? FX_ZERO : fx_scale(hmax) - 1083 + ce + 4;
+// the terms of GO outputs for one value
+template <int GO, bool ODD> __device__ __forceinline__ void modes_add(ModeAcc* s, fx_t x, const Q2* c) {
+  const ModeValue v = modes_value<ODD>(x);
+#pragma unroll
+  for (int g = 0; g < GO; g += 2) {
+    const Q4 cc = *reinterpret_cast<const Q4*>(c + g);
+    modes_term<ODD>(s[g], v, cc.x);
+    if (g + 1 < GO) modes_term<ODD>(s[g + 1 < GO ? g + 1 : g], v, cc.y);
+  }
 }
-// the terms of GO outputs for one value: acc (64 bits) and its part t in
-// units of 2^32, which holds four values' terms
-template <int GO> struct ModeAcc {
-  fx_t acc[GO];
-  int t[GO];
-  __device__ __forceinline__ void init(int nl) {
-#pragma unroll
-    for (int g = 0; g < GO; ++g) {
-      acc[g] = nl;  // 2 nl truncations of half a unit
-      t[g] = 0;
-    }
-  }
-  __device__ __forceinline__ void add(fx_t x, const Q2* c) {
-    const Q2 v = q2_split(x);
-#pragma unroll
-    for (int g = 0; g < GO; g += 2) {
-      const Q4 cc = *reinterpret_cast<const Q4*>(c + g);
-      acc[g] += (fx_t)v.h * cc.x.h;
-      t[g] += fx_mh(v.h, cc.x.l) + fx_mh(v.l, cc.x.h);
-      if (g + 1 < GO) {
-        acc[g + 1 < GO ? g + 1 : g] += (fx_t)v.h * cc.y.h;
-        t[g + 1 < GO ? g + 1 : g] += fx_mh(v.h, cc.y.l) + fx_mh(v.l, cc.y.h);
-      }
-    }
-  }
-  __device__ __forceinline__ void carry() {
-#pragma unroll
-    for (int g = 0; g < GO; ++g) {
-      acc[g] += t[g];
-      t[g] = 0;
-    }
-  }
-};
+__device__ __forceinline__ fx_t modes_in(double v, int E, unsigned int turn) {
+  return fx_from_bits<8>(modes_turned((unsigned long long)__double_as_longlong(v), turn), E);
+}
+__device__ __forceinline__ double modes_out(const ModeAcc& s, int ex, unsigned int turn) {
+  const double v = fx_out(s.acc, ex);
+  return __longlong_as_double((long long)modes_turned((unsigned long long)__double_as_longlong(v), turn));
+}
 
 // One point of a run of NL layers; cs: the constants as [group][l][GE], GE =
 // GO rounded up to even.
@@ -174,22 +151,26 @@ __device__ __forceinline__ void modes_point(const StepArgs<double>& a, const Mod
     load([&](int, size_t ol) { return src[ol]; });
   grid_next();
   const int E = fx_scale(h);
+  const unsigned int turn = modes_turn(i, j);
   fx_t x[NL];
 #pragma unroll
-  for (int l = 0; l < NL; ++l) x[l] = fx_from_bits<8>(__double_as_longlong(v[l]), E);
+  for (int l = 0; l < NL; ++l) x[l] = modes_in(v[l], E, turn);
 #pragma unroll
   for (int n = 0; n < S::NG; ++n) {
-    ModeAcc<S::GO> s;
-    s.init(NL);
+    ModeAcc s[S::GO] = {};
 #pragma unroll
     for (int l = 0; l < NL; ++l) {
-      s.add(x[l], cs + (n * NL + l) * S::GE);
-      if ((l & 3) == 3 || l == NL - 1) s.carry();
+      if (l & 1) modes_add<S::GO, true>(s, x[l], cs + (n * NL + l) * S::GE);
+      else modes_add<S::GO, false>(s, x[l], cs + (n * NL + l) * S::GE);
+      if ((l & 3) == 3 || l == NL - 1) {
+#pragma unroll
+        for (int g = 0; g < S::GO; ++g) modes_carry(s[g]);
+      }
     }
 #pragma unroll
     for (int g = 0; g < S::GO; ++g) {
       const int m = n * S::GO + g;
-      if (m < NL) dst[o + (size_t)m * a.lstride] = fx_out(s.acc[g], modes_exp(h, tb.e[m]));
+      if (m < NL) dst[o + (size_t)m * a.lstride] = modes_out(s[g], modes_exp(h, tb.e[m]), turn);
     }
   }
 }
@@ -215,6 +196,7 @@ __device__ __forceinline__ void modes_point_any(const StepArgs<double>& a, const
       load([&](int, size_t ol) { return src[ol]; });
   }
   const int E = fx_scale(h);
+  const unsigned int turn = modes_turn(i, j);
   const double* mat = FWD ? a.cl2m : a.cm2l;
   double* cd = (double*)cs;
   for (int m0 = 0; m0 < nl; m0 += GO) {
@@ -227,15 +209,19 @@ __device__ __forceinline__ void modes_point_any(const StepArgs<double>& a, const
     __syncthreads();
     if (!on) continue;
     if (a.modes_fx) {
-      ModeAcc<GO> s;
-      s.init(nl);
+      ModeAcc s[GO] = {};
       for (int l = 0; l < nl; ++l) {
-        s.add(fx_from_bits<8>(__double_as_longlong(src[o + (size_t)l * a.lstride]), E), cs + l * GO);
-        if ((l & 3) == 3) s.carry();
+        const fx_t x = modes_in(src[o + (size_t)l * a.lstride], E, turn);
+        if (l & 1) modes_add<GO, true>(s, x, cs + l * GO);
+        else modes_add<GO, false>(s, x, cs + l * GO);
+        if ((l & 3) == 3 || l == nl - 1) {
+#pragma unroll
+          for (int g = 0; g < GO; ++g) modes_carry(s[g]);
+        }
       }
-      s.carry();
-      for (int g = 0; g < GO && m0 + g < nl; ++g)
-        dst[o + (size_t)(m0 + g) * a.lstride] = fx_out(s.acc[g], modes_exp(h, tb.e[m0 + g]));
+#pragma unroll
+      for (int g = 0; g < GO; ++g)
+        if (m0 + g < nl) dst[o + (size_t)(m0 + g) * a.lstride] = modes_out(s[g], modes_exp(h, tb.e[m0 + g]), turn);
     } else {
       double acc[GO] = {};
       for (int l = 0; l < nl; ++l) {

@@ -7,6 +7,7 @@
 #include "../../qgw_gb300/csrc/dst_tables.h"
 #include "../../qgw_gb300/csrc/dst_warp.h"
 #include "../../qgw_gb300/csrc/dst_blue.h"
+#include "../../qgw_gb300/csrc/modes_core.h"
 
 using namespace qgw;
 
@@ -329,4 +330,54 @@ extern "C" void dst_fx_errors(int M, const double* x, double* err) {
 }
 extern "C" void dst_fx_run(int M, int howmany, double* data) {
   transform_length_ok(M) ? run_fx(M, howmany, data) : run_fx_blue(M, howmany, data);
+}
+
+static unsigned long long bits_of(double v) {
+  unsigned long long b;
+  std::memcpy(&b, &v, 8);
+  return b;
+}
+static double double_of(unsigned long long b) {
+  double v;
+  std::memcpy(&v, &b, 8);
+  return v;
+}
+static double fx_double(fx_t v, int e) {
+  return e == FX_NAN ? std::nan("") : fx_exp_ok(e) ? double_of(fx_to_bits(v, e)) : std::ldexp((double)v, e);
+}
+// The projection of a field x (nl layers of ny x nx) by mat: the errors of the
+// FP64 sums and of the fixed-point ones (modes_core.h) against sums in long
+// double, and those sums.
+extern "C" void modes_errors(int nl, int ny, int nx, const double* mat, const double* x, double* err64, double* errfx,
+                             double* exact) {
+  std::vector<Q2> c((size_t)nl * nl);
+  std::vector<int> e(nl);
+  fill_mode_table(nl, mat, c.data(), e.data());
+  const size_t n = (size_t)ny * nx;
+  std::vector<fx_t> v(nl);
+  for (size_t p = 0; p < n; ++p) {
+    const unsigned int turn = modes_turn((int)(p % nx), (int)(p / nx));
+    unsigned int h = 0;
+    for (int l = 0; l < nl; ++l) {
+      const unsigned int hi = (unsigned int)(bits_of(x[l * n + p]) >> 32) & 0x7fffffffu;
+      h = hi > h ? hi : h;
+    }
+    for (int l = 0; l < nl; ++l) v[l] = fx_from_bits<8>(modes_turned(bits_of(x[l * n + p]), turn), fx_scale(h));
+    for (int m = 0; m < nl; ++m) {
+      long double t = 0;
+      double f = 0;
+      ModeAcc s = {};
+      for (int l = 0; l < nl; ++l) {
+        t += (long double)mat[m * nl + l] * x[l * n + p];
+        f = std::fma(mat[m * nl + l], x[l * n + p], f);
+        if (l & 1) modes_term<true>(s, modes_value<true>(v[l]), c[m * nl + l]);
+        else modes_term<false>(s, modes_value<false>(v[l]), c[m * nl + l]);
+        if ((l & 3) == 3 || l == nl - 1) modes_carry(s);
+      }
+      const double r = double_of(modes_turned(bits_of(fx_double(s.acc, modes_exp(h, e[m]))), turn));
+      err64[m * n + p] = (double)(f - t);
+      errfx[m * n + p] = (double)(r - t);
+      exact[m * n + p] = (double)t;
+    }
+  }
 }

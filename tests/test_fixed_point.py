@@ -51,6 +51,64 @@ def test_rows_of_zeros_and_non_finite_rows(dstcore):  # noqa: F811
     assert np.all(x[[0, 3]] == 0) and np.all(np.isnan(x[[1, 2]]))
 
 
+def q_field(kind, nl, N):
+    """noise or eddies, in all layers, in the top one alone (top), in the
+    bottom one (bottom), weaker in each layer down (decay), or of single
+    precision (single)."""
+    rng, n = np.random.default_rng(nl), N - 1
+    q = 1e-7 * rng.standard_normal((nl, n, n))
+    if "eddies" in kind:
+        x = 2 * np.pi * np.arange(n) / n
+        for _ in range(8):
+            a, b, c, d, e = rng.random(5)
+            wave = np.outer(np.sin((1 + int(12 * a)) * x + 6 * b), np.sin((1 + int(12 * c)) * x + 6 * d))
+            q += 2e-6 * e * wave * 0.6 ** np.arange(nl)[:, None, None]
+    if "single" in kind:
+        q = q.astype(np.float32).astype(float)
+    if "decay" in kind:
+        q *= 0.6 ** np.arange(nl)[:, None, None]
+    if "top" in kind:
+        q[1:] = 0
+    if "bottom" in kind:
+        q[:-1] = 0
+    return q
+
+
+def projection_errors(lib, modes, q, N):
+    """Of psi (a row a layer: FP64 sums, fixed point), from the projections of
+    an inversion alone, in units of 2^-53 of the layer's norm: layers to modes
+    at the points, modes to layers at the rows' wave numbers."""
+    l2m, m2l, ird = modes
+    nl, k = len(ird), np.pi / 4e6 * np.arange(1, N)
+
+    def project(mat, f):
+        out = [np.empty((nl, N - 1, N - 1)) for _ in range(3)]
+        mat, f = np.ascontiguousarray(mat), np.ascontiguousarray(f)
+        lib.modes_errors.argtypes = [ctypes.c_int] * 3 + [ctypes.c_void_p] * 5
+        lib.modes_errors(nl, N - 1, N - 1, mat.ctypes.data, f.ctypes.data, *(o.ctypes.data for o in out))
+        return out
+
+    def spectral(m):
+        s = sf.dstn(m, type=1, axes=(1, 2)) / -(k[None, :, None] ** 2 + k[None, None] ** 2 + ird[:, None, None])
+        return sf.idst(s, type=1, axis=1)
+    *fwd, m = project(l2m, q)
+    *back, psi = project(m2l, spectral(m))
+    norm = np.linalg.norm(sf.idst(psi, type=1, axis=2), axis=(1, 2))
+    return np.stack([np.linalg.norm(sf.idst(np.tensordot(m2l, spectral(f), 1) + b, type=1, axis=2), axis=(1, 2))
+                     for f, b in zip(fwd, back)], 1) / norm[:, None] * 2.0 ** 53
+
+
+@pytest.mark.parametrize("kind", ["noise", "noise top", "eddies top", "noise bottom", "noise single", "eddies single"])
+@pytest.mark.parametrize("nl", [3, 8, 10])
+def test_projection_error_no_larger_than_fp64(dstcore, qgwlib, nl, kind):  # noqa: F811
+    """What the projections' rounding gives psi, also where products are
+    exact (rest below the top layer, single precision), is no larger than
+    with FP64 sums (or 2 units, the rounding of the results themselves)."""
+    N = 128
+    f64, fx = np.sqrt((projection_errors(dstcore, qgwlib.eigmode(C.cfg2(N, nl)), q_field(kind, nl, N), N) ** 2).mean(0))
+    assert fx <= max(f64, 2.0), (f64, fx)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("NX,NY", [(4, 6), (10, 14), (128, 16), (16, 256), (256, 128), (512, 30), (30, 512),
                                    (1024, 12), (96, 1024), (2048, 64), (64, 2048), (2430, 8), (4096, 10)])
@@ -67,6 +125,26 @@ def test_inversion_at_transform_lengths(qgwlib, NX, NY):
     m = np.tensordot(l2m, q[:, 1:-1, 1:-1], 1)
     k, l = np.pi * np.arange(1, NX) / p["Lx"], np.pi * np.arange(1, NY) / p["Lx"]
     s = sf.dstn(m, type=1, axes=(1, 2)) / -(k[None, None] ** 2 + l[None, :, None] ** 2 + ird[:, None, None])
+    ref = np.tensordot(m2l, sf.idstn(s, type=1, axes=(1, 2)), 1)
+    assert np.linalg.norm(psi[:, 1:-1, 1:-1] - ref) <= 2e-14 * np.linalg.norm(ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nl", [8, 10, 16])
+def test_inversion_of_one_layer(qgwlib, nl):
+    """psi of a q in the top layer alone, whose other layers' products are
+    exact, against scipy's transforms."""
+    N = 256
+    p = C.cfg2(N, nl)
+    q = np.pad(q_field("noise top", nl, N), ((0, 0), (1, 1), (1, 1)))
+    r = qgwlib.Run(p)
+    r.set_q(q)
+    psi, _ = r.get()
+    r.close()
+    l2m, m2l, ird = qgwlib.eigmode(p)
+    k = np.pi * np.arange(1, N) / p["Lx"]
+    s = sf.dstn(np.tensordot(l2m, q[:, 1:-1, 1:-1], 1), type=1, axes=(1, 2))
+    s /= -(k[None, None] ** 2 + k[None, :, None] ** 2 + ird[:, None, None])
     ref = np.tensordot(m2l, sf.idstn(s, type=1, axes=(1, 2)), 1)
     assert np.linalg.norm(psi[:, 1:-1, 1:-1] - ref) <= 2e-14 * np.linalg.norm(ref)
 

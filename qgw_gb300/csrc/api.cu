@@ -91,10 +91,10 @@ int upload_fx(qgw_run* r, qgw::FxTables* out, const qgw::DstGeom& g) {
   return cudaStreamSynchronize(r->stream) == cudaSuccess ? QGW_OK : QGW_ERR_CUDA;
 }
 
-// a projection matrix in fixed point, in one allocation (c | e)
+// a projection matrix in fixed point, in one allocation (c | e | k)
 int upload_modes(qgw_run* r, qgw::ModeTable* out, const std::vector<double>& mat) {
   const size_t nc = (size_t)r->nl * r->nl;
-  std::vector<qgw::Q2> h(nc + ((size_t)r->nl + 1) / 2);
+  std::vector<qgw::Q2> h(nc + (size_t)r->nl);
   qgw::fill_mode_table(r->nl, mat.data(), h.data(), (int*)(h.data() + nc));
   qgw::Q2* d;
   int rc = dalloc(r, &d, h.size());

@@ -48,11 +48,11 @@ QGW_HD Q2 q2_const(fx_t w) { return q2_split((int)w == (int)0x80000000 ? w + 1 :
 // Tables: twq the pass twiddles (cos, -sin) scaled by 2^62, in the order of
 // fill_pass_twiddles; nsj -s_j scaled by 2^63, j <= H (s_H = 1 has no
 // positive 2^63); spq (cos, -sin)(2 pi k / M) scaled by 2^63, 1 <= k <= H/2.
-// A projection's constants (modes_fx.cuh): c = (h 2^32 + l) 2^(e - 60) < 2^e,
-// e per row of the matrix.
+// A projection's constants (modes_core.h): c 2^-k = (h 2^32 + l) 2^(e - 60) <
+// 2^e, e per row of the matrix, k <= 0 per column.
 struct ModeTable {
   const Q2* c;   // nl x nl, row m: output m
-  const int* e;  // nl
+  const int* e;  // e (nl), k (nl)
 };
 // Chirp-z lengths (dst_blue.h): twq of the L-point FFT, bc the chirp c_m
 // scaled by 2^62, m < M, bz the transform of its conjugate scaled by 2^(62 - be).

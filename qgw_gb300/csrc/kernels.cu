@@ -502,7 +502,7 @@ template <bool FWD> static void launch_modes(const StepArgs<double>& a, int step
   const dim3 grid((unsigned int)((n + NT - 1) / NT));
   switch (a.modes_fx ? a.nl : 0) {
 #define QGW_MODES(N) \
-  case N: launch(k_modes<N, FWD>, grid, dim3(NT), sizeof(Q2) * ModeShape<N>::len, s, pdl, a, step_mode); break;
+  case N: launch(k_modes<N, FWD>, grid, dim3(NT), ModeShape<N>::bytes, s, pdl, a, step_mode); break;
     QGW_MODES(1) QGW_MODES(2) QGW_MODES(3) QGW_MODES(4) QGW_MODES(5) QGW_MODES(6) QGW_MODES(7) QGW_MODES(8)
     QGW_MODES(9) QGW_MODES(10) QGW_MODES(11) QGW_MODES(12) QGW_MODES(13) QGW_MODES(14) QGW_MODES(15) QGW_MODES(16)
 #undef QGW_MODES

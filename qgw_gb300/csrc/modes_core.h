@@ -1,10 +1,15 @@
 // modes_core.h -- the arithmetic of the FP64 path's vertical projections
 // (modes_fx.cuh), for the kernels and for checks on the host.
 //
-// A point's values become integers below 2^61 by the largest of them, the
-// coefficients integers below 2^60 by the largest of their row of the
-// matrix; products keep their high words and sums are exact, so the result
-// does not depend on how outputs are grouped.
+// The columns of the matrix are brought to like size by powers of two, which
+// go to the values (thin layers' coefficients are small and their vorticity
+// large).  A point's values then become integers below 2^61 by the largest of
+// them, the coefficients integers below 2^60 by the largest of their row;
+// products keep their high words and sums are exact, so the result does not
+// depend on how outputs are grouped.  The error is about 2^-56 of the largest
+// coefficient of the row times the largest value of the point, both as scaled.
+// No term of an output need reach that: what columns of too unlike size lose
+// by it is the reason for modes_fixed_ok's limits (dst_tables.h).
 //
 // Of a product's two cross terms one is truncated down and the other, of the
 // negated value, up, the two taking turns from layer to layer.  Where one of
@@ -24,9 +29,24 @@ namespace qgw {
 QGW_HD unsigned int modes_turn(int i, int j) { return (unsigned int)(i + j) << 31; }
 QGW_HD unsigned long long modes_turned(unsigned long long b, unsigned int turn) { return b ^ ((unsigned long long)turn << 32); }
 
-// exponent of the results of a point whose largest high word is hmax
-QGW_HD int modes_exp(unsigned int hmax, int ce) {
-  return hmax >= 0x7ff00000u ? FX_NAN : hmax == 0 ? FX_ZERO : fx_scale(hmax) - 1083 + ce + 4;
+// A point's largest high words, of the values as they are (which shows a
+// non-finite one) and as scaled by 2^k (below zero: as good as none).
+struct ModeMax {
+  unsigned int raw;
+  int hi;
+};
+QGW_HD void modes_max(ModeMax& h, unsigned int hi, int k) {
+  const int s = (int)hi + k * (1 << 20);
+  h.raw = hi > h.raw ? hi : h.raw;
+  h.hi = s > h.hi ? s : h.hi;
+}
+// the value of bits b of a column scaled by 2^k
+QGW_HD fx_t modes_in(unsigned long long b, const ModeMax& h, int k, unsigned int turn) {
+  return fx_from_bits<8>(modes_turned(b, turn), fx_scale((unsigned int)h.hi) - k);
+}
+// exponent of the point's results
+QGW_HD int modes_exp(const ModeMax& h, int ce) {
+  return h.raw >= 0x7ff00000u ? FX_NAN : h.hi == 0 ? FX_ZERO : fx_scale((unsigned int)h.hi) - 1083 + ce + 4;
 }
 // A value as its halves and the negated one of the half whose cross term is
 // truncated up: the low one (never -2^31) in even layers, the high one in odd

@@ -11,12 +11,9 @@
 // each pair of modes read the row's layers again.)  The extra pass over the
 // spectral field mostly stays in L2.
 //
-// The arithmetic is modes_core.h's.  It holds FP64's precision while the
-// inputs' columns of the matrix are of similar size: a value is kept to 2^-61
-// of the point's largest, and a coefficient 2^k times the others multiplies
-// that.  So runs whose columns' largest entries differ by more than 64
-// (strongly graded profiles of many layers, whose trapped modes reach 1e6), or
-// with more than 32 layers (the sums' headroom), keep FP64 sums (a.modes_fx = 0).
+// The arithmetic is modes_core.h's.  Runs of strongly graded profiles, whose
+// matrix columns differ by more than it takes, or of more than 20 layers
+// (modes_fixed_ok, dst_tables.h) keep FP64 sums (a.modes_fx = 0).
 #pragma once
 
 #include <type_traits>
@@ -108,9 +105,6 @@ template <int GO, bool ODD> __device__ __forceinline__ void modes_add(ModeAcc* s
     if (g + 1 < GO) modes_term<ODD>(s[g + 1 < GO ? g + 1 : g], v, cc.y);
   }
 }
-__device__ __forceinline__ fx_t modes_in(double v, int E, unsigned int turn) {
-  return fx_from_bits<8>(modes_turned((unsigned long long)__double_as_longlong(v), turn), E);
-}
 __device__ __forceinline__ double modes_out(const ModeAcc& s, int ex, unsigned int turn) {
   const double v = fx_out(s.acc, ex);
   return __longlong_as_double((long long)modes_turned((unsigned long long)__double_as_longlong(v), turn));
@@ -121,6 +115,7 @@ __device__ __forceinline__ double modes_out(const ModeAcc& s, int ex, unsigned i
 template <int NL> struct ModeShape {
   static constexpr int NG = NL > 8 ? 2 : 1, GO = (NL + NG - 1) / NG, GE = (GO + 1) & ~1;
   static constexpr int len = NG * NL * GE;
+  static constexpr size_t bytes = len * sizeof(Q2) + NL * sizeof(int);  // and the columns' k
 };
 template <int NL> __device__ __forceinline__ void modes_stage(const ModeTable& tb, Q2* cs) {
   using S = ModeShape<NL>;
@@ -128,6 +123,7 @@ template <int NL> __device__ __forceinline__ void modes_stage(const ModeTable& t
     const int g = w % S::GE, l = w / S::GE % NL, n = w / (S::GE * NL), m = n * S::GO + g;
     cs[w] = g < S::GO && m < NL ? tb.c[m * NL + l] : Q2{0, 0};
   }
+  if (threadIdx.x < NL) ((int*)(cs + S::len))[threadIdx.x] = tb.e[NL + threadIdx.x];
 }
 template <int NL, bool FWD>
 __device__ __forceinline__ void modes_point(const StepArgs<double>& a, const ModeTable& tb, const QUpdate& u, int j,
@@ -136,13 +132,14 @@ __device__ __forceinline__ void modes_point(const StepArgs<double>& a, const Mod
   const size_t o = (size_t)j * a.pitch + i;
   const double* src = FWD ? a.q : a.spec;
   double* dst = FWD ? a.spec : a.psi;
+  const int* k = (const int*)(cs + S::len);
   double v[NL];
-  unsigned int h = 0;
+  ModeMax h = {};
   auto load = [&](auto value) {
 #pragma unroll
     for (int l = 0; l < NL; ++l) {
       v[l] = value(l, o + (size_t)l * a.lstride);
-      h = max(h, fx_hi(v[l]));
+      modes_max(h, fx_hi(v[l]), k[l]);
     }
   };
   if constexpr (FWD)
@@ -150,11 +147,10 @@ __device__ __forceinline__ void modes_point(const StepArgs<double>& a, const Mod
   else
     load([&](int, size_t ol) { return src[ol]; });
   grid_next();
-  const int E = fx_scale(h);
   const unsigned int turn = modes_turn(i, j);
   fx_t x[NL];
 #pragma unroll
-  for (int l = 0; l < NL; ++l) x[l] = modes_in(v[l], E, turn);
+  for (int l = 0; l < NL; ++l) x[l] = modes_in((unsigned long long)__double_as_longlong(v[l]), h, k[l], turn);
 #pragma unroll
   for (int n = 0; n < S::NG; ++n) {
     ModeAcc s[S::GO] = {};
@@ -185,9 +181,10 @@ __device__ __forceinline__ void modes_point_any(const StepArgs<double>& a, const
   const size_t o = (size_t)j * a.pitch + i;
   const double* src = FWD ? a.q : a.spec;
   double* dst = FWD ? a.spec : a.psi;
-  unsigned int h = 0;
+  const int* k = tb.e + nl;
+  ModeMax h = {};
   auto load = [&](auto value) {
-    for (int l = 0; l < nl; ++l) h = max(h, fx_hi(value(l, o + (size_t)l * a.lstride)));
+    for (int l = 0; l < nl; ++l) modes_max(h, fx_hi(value(l, o + (size_t)l * a.lstride)), k[l]);
   };
   if (on) {
     if constexpr (FWD)
@@ -195,7 +192,6 @@ __device__ __forceinline__ void modes_point_any(const StepArgs<double>& a, const
     else
       load([&](int, size_t ol) { return src[ol]; });
   }
-  const int E = fx_scale(h);
   const unsigned int turn = modes_turn(i, j);
   const double* mat = FWD ? a.cl2m : a.cm2l;
   double* cd = (double*)cs;
@@ -211,7 +207,7 @@ __device__ __forceinline__ void modes_point_any(const StepArgs<double>& a, const
     if (a.modes_fx) {
       ModeAcc s[GO] = {};
       for (int l = 0; l < nl; ++l) {
-        const fx_t x = modes_in(src[o + (size_t)l * a.lstride], E, turn);
+        const fx_t x = modes_in((unsigned long long)__double_as_longlong(src[o + (size_t)l * a.lstride]), h, k[l], turn);
         if (l & 1) modes_add<GO, true>(s, x, cs + l * GO);
         else modes_add<GO, false>(s, x, cs + l * GO);
         if ((l & 3) == 3 || l == nl - 1) {

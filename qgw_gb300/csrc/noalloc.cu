@@ -49,8 +49,8 @@ constexpr size_t oCm = oCl + (size_t)kNlMax * kNlMax;
 constexpr size_t oClq = oCm + (size_t)kNlMax * kNlMax;
 constexpr size_t oCmq = oClq + (size_t)kNlMax * kNlMax;
 constexpr size_t oIrd = oCmq + (size_t)kNlMax * kNlMax;
-constexpr size_t oExp = oIrd + kNlMax;  // the projections' exponents (2 x kNlMax ints)
-constexpr size_t oLsq = oExp + kNlMax;
+constexpr size_t oExp = oIrd + kNlMax;  // the projections' exponents (2 x 2 kNlMax ints)
+constexpr size_t oLsq = oExp + 2 * kNlMax;
 constexpr size_t oKsq = oLsq + kMMax;
 constexpr size_t oState = oKsq + kMMax;
 constexpr size_t kTotal = oState + kStateD;
@@ -174,7 +174,7 @@ extern "C" int qgw_invert_pv_noalloc(const qgw_params* p, const double* cl2m, co
     std::memcpy(h_tab + (oCl - oTx), kcl, sizeof(double) * nl * nl);
     std::memcpy(h_tab + (oCm - oTx), kcm, sizeof(double) * nl * nl);
     qgw::fill_mode_table(nl, kcl, (qgw::Q2*)(h_tab + (oClq - oTx)), (int*)(h_tab + (oExp - oTx)));
-    qgw::fill_mode_table(nl, kcm, (qgw::Q2*)(h_tab + (oCmq - oTx)), (int*)(h_tab + (oExp - oTx)) + kNlMax);
+    qgw::fill_mode_table(nl, kcm, (qgw::Q2*)(h_tab + (oCmq - oTx)), (int*)(h_tab + (oExp - oTx)) + 2 * kNlMax);
     std::memcpy(h_tab + (oIrd - oTx), kir, sizeof(double) * nl);
     for (int k = 0; k < nx; ++k) { const double L = M_PI * (k + 1) / p->Lx; h_tab[oLsq - oTx + k] = L * L; }
     for (int j = 0; j < ny; ++j) { const double K = M_PI * (j + 1) / p->Lx; h_tab[oKsq - oTx + j] = K * K; }
@@ -203,7 +203,7 @@ extern "C" int qgw_invert_pv_noalloc(const qgw_params* p, const double* cl2m, co
   a.cm2l = base + oCm;
   a.modes_fx = qgw::modes_fixed_ok(nl, cl2m) && qgw::modes_fixed_ok(nl, cm2l);
   a.l2m = qgw::ModeTable{(const qgw::Q2*)(base + oClq), (const int*)(base + oExp)};
-  a.m2l = qgw::ModeTable{(const qgw::Q2*)(base + oCmq), (const int*)(base + oExp) + kNlMax};
+  a.m2l = qgw::ModeTable{(const qgw::Q2*)(base + oCmq), (const int*)(base + oExp) + 2 * kNlMax};
   a.iRd2 = base + oIrd;
   a.q = q_dev + pitch + 1;
   a.psi = psi_dev + pitch + 1;

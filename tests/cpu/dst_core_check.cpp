@@ -345,24 +345,23 @@ static double double_of(unsigned long long b) {
 static double fx_double(fx_t v, int e) {
   return e == FX_NAN ? std::nan("") : fx_exp_ok(e) ? double_of(fx_to_bits(v, e)) : std::ldexp((double)v, e);
 }
+extern "C" int modes_fixed(int nl, const double* mat) { return modes_fixed_ok(nl, mat) ? 1 : 0; }
 // The projection of a field x (nl layers of ny x nx) by mat: the errors of the
 // FP64 sums and of the fixed-point ones (modes_core.h) against sums in long
 // double, and those sums.
 extern "C" void modes_errors(int nl, int ny, int nx, const double* mat, const double* x, double* err64, double* errfx,
                              double* exact) {
   std::vector<Q2> c((size_t)nl * nl);
-  std::vector<int> e(nl);
+  std::vector<int> e(2 * (size_t)nl);
+  const int* k = e.data() + nl;
   fill_mode_table(nl, mat, c.data(), e.data());
   const size_t n = (size_t)ny * nx;
   std::vector<fx_t> v(nl);
   for (size_t p = 0; p < n; ++p) {
     const unsigned int turn = modes_turn((int)(p % nx), (int)(p / nx));
-    unsigned int h = 0;
-    for (int l = 0; l < nl; ++l) {
-      const unsigned int hi = (unsigned int)(bits_of(x[l * n + p]) >> 32) & 0x7fffffffu;
-      h = hi > h ? hi : h;
-    }
-    for (int l = 0; l < nl; ++l) v[l] = fx_from_bits<8>(modes_turned(bits_of(x[l * n + p]), turn), fx_scale(h));
+    ModeMax h = {};
+    for (int l = 0; l < nl; ++l) modes_max(h, (unsigned int)(bits_of(x[l * n + p]) >> 32) & 0x7fffffffu, k[l]);
+    for (int l = 0; l < nl; ++l) v[l] = modes_in(bits_of(x[l * n + p]), h, k[l], turn);
     for (int m = 0; m < nl; ++m) {
       long double t = 0;
       double f = 0;

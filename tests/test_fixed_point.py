@@ -109,6 +109,25 @@ def test_projection_error_no_larger_than_fp64(dstcore, qgwlib, nl, kind):  # noq
     assert fx <= max(f64, 2.0), (f64, fx)
 
 
+@pytest.mark.parametrize("kind", ["noise", "noise top", "noise decay", "noise bottom", "noise single", "eddies top",
+                                  "eddies decay single"])
+@pytest.mark.parametrize("nl,ratio", [(10, 1.3), (12, 1.5), (16, 1.3), (17, 1.3), (20, 1.3), (20, 1.5), (30, 1.3),
+                                      (32, 1.3)])
+def test_projection_error_of_every_layer(dstcore, qgwlib, nl, ratio, kind):  # noqa: F811
+    """The same layer by layer, for graded profiles of many layers wherever
+    the projections run in fixed point: their mean over the layers (each
+    layer's within 2 units more, a draw of the roundings)."""
+    dh = 4000 * (ratio - 1) / (ratio ** nl - 1) * ratio ** np.arange(nl)
+    gp = 0.02 * 0.1 ** (np.arange(nl - 1) / (nl - 2))
+    modes = qgwlib.eigmode(dict(C.cfg2(64, nl), dh=list(dh), N2=list(2 * gp / (dh[1:] + dh[:-1]))))
+    if not all(dstcore.modes_fixed(nl, np.ascontiguousarray(m).ctypes.data_as(ctypes.c_void_p)) for m in modes[:2]):
+        assert nl > 20 or ratio > 1.3
+        return
+    e = projection_errors(dstcore, modes, q_field(kind, nl, 64), 64)
+    f64, fx = np.sqrt((e ** 2).mean(0))
+    assert fx <= max(f64, 2.0) and np.all(e[:, 1] <= np.maximum(e[:, 0], 2.0) + 2.0), e
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("NX,NY", [(4, 6), (10, 14), (128, 16), (16, 256), (256, 128), (512, 30), (30, 512),
                                    (1024, 12), (96, 1024), (2048, 64), (64, 2048), (2430, 8), (4096, 10)])
@@ -130,7 +149,7 @@ def test_inversion_at_transform_lengths(qgwlib, NX, NY):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("nl", [8, 10, 16])
+@pytest.mark.parametrize("nl", [8, 10, 16, 20, 24])
 def test_inversion_of_one_layer(qgwlib, nl):
     """psi of a q in the top layer alone, whose other layers' products are
     exact, against scipy's transforms."""

@@ -42,6 +42,7 @@ QGW_HD Q2 q2_split(fx_t w) {
   q.h = (int)(w >> 32) - (q.l >> 31);
   return q;
 }
+QGW_HD fx_t q2_join(Q2 q) { return (fx_t)((unsigned long long)(unsigned int)q.h << 32) + q.l; }
 // of a constant: l is never -2^31 (fx_mul negates it)
 QGW_HD Q2 q2_const(fx_t w) { return q2_split((int)w == (int)0x80000000 ? w + 1 : w); }
 

@@ -4,16 +4,11 @@
 // The tile's psi and q become integers of one power of two each, taken from
 // the tile's own largest magnitudes.  The hyperviscosity sweeps, Laplacians
 // and differences are then exact integer additions, and the Arakawa Jacobian
-// (src/domain.h:17-27) is a sum over the eight neighbours of q,
-//   sum_n q_n C_n,  C_N = (psi_E - psi_W) + (psi_NE - psi_NW),
-//   C_NE = psi_E - psi_N, ...
-// whose C_n are differences of psi: shifted up to 2^59 (by the tile's
-// largest one-step difference) their products with q keep 2^-51 of |C q|,
-// where the floating-point form rounds at 2^-53 of |psi dq|, |psi| being tens
-// of |C| on any grid.  A point's few results become doubles at the end, for
-// the coefficients (3-4 FP64 operations a point instead of 34).  1024^2 x 10
-// with three sweeps: 0.767 -> 0.303 ms (FP64 pipe 86% busy before; now about
-// 740 instructions a point, mostly integer).
+// a sum of whole products (rhs_core.h).  A point's few results become doubles
+// at the end, for the coefficients (3-4 FP64 operations a point instead of
+// 34).  1024^2 x 10 with three sweeps: 0.767 -> 0.312 ms (FP64 pipe 86% busy
+// before; now integer instructions; with products cut to their high words
+// 0.303).
 //
 // What stays in FP64 (rhs_tile_compute): edge tiles at walls with bc_fac !=
 // 0, whose ghost values (2 bc_fac / Delta^2 psi at every sweep) exceed the
@@ -22,6 +17,8 @@
 // Every tile is TX x 16 points here; a taller tile runs as bands of 16 rows,
 // so that the scale of a point's tile does not depend on the tile shape.
 #pragma once
+
+#include "rhs_core.h"
 
 namespace qgw {
 
@@ -43,8 +40,8 @@ __device__ __forceinline__ unsigned long long rhs_tile_fx(const StepArgs<double>
   fx_t* L0 = (fx_t*)wk;
   fx_t* L1 = L0 + TS;
   fx_t* P = L1 + TS;  // HH x W, psi with halo R
-  fx_t* Q = P + TS;   // QH x W, q with halo 1
-  __shared__ unsigned int rmax[2][NT / 32], rmag[2][NT / 32];
+  Q2* Q = (Q2*)(P + TS);  // QH x W, q with halo 1
+  __shared__ unsigned int rmax[2][NT / 32], rmag[NT / 32];
   const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + ty * 32;
   const int nx = a.nx, ny = a.ny, pitch = a.pitch;
   const bool walls = EDGE && !a.periodic;
@@ -83,24 +80,16 @@ __device__ __forceinline__ unsigned long long rhs_tile_fx(const StepArgs<double>
 #pragma unroll
   for (int u = 0; u < NQ; ++u) {
     const int w = tid + u * NT, y = w / QW, o = y * W + w - y * QW - 1 + XO;
-    if (w < QW * QH) Q[o] = fx_from_bits(__double_as_longlong(in.qs[o]), Eq);
+    if (w < QW * QH) Q[o] = q2_split(fx_from_bits(__double_as_longlong(in.qs[o]), Eq));
   }
   const int ep = Ep - FX_EOFF, eq = Eq - FX_EOFF;  // exponents of P and Q
   __syncthreads();
 
-  // one-step differences' magnitude and the Laplacian sweeps (calc_diff,
-  // src/dynamics.h:13-44) with a shrinking halo, unscaled; at walls
-  // (bc_fac = 0 here) values outside the domain are zero
-  unsigned int dmag = 0, lmag = 0;
+  // the Laplacian sweeps (calc_diff, src/dynamics.h:13-44) with a shrinking
+  // halo, unscaled; at walls (bc_fac = 0 here) values outside the domain are
+  // zero
+  unsigned int lmag = 0;
   const int ksweep = a.nsweep;  // 0 or R
-  if (R == 1) {
-    for (int w = tid; w < QW * QH; w += NT) {
-      const int y = w / QW, x = w - y * QW, o = y * W + x - 1 + XO;
-      const fx_t c = P[o];
-      if (x < QW - 1) dmag |= fx_mag(P[o + 1] - c);
-      if (y < QH - 1) dmag |= fx_mag(P[o + W] - c);
-    }
-  }
   const fx_t* Lp = P;
   fx_t* Lc = L0;
   int lsh = 0;  // the sweeps' right shift
@@ -120,10 +109,7 @@ __device__ __forceinline__ unsigned long long rhs_tile_fx(const StepArgs<double>
         const int gi = i0 + xr + s - R, gj = j0 + yr + s - R;
         if (gi < 0 || gi >= nx || gj < 0 || gj >= ny) v = 0;
       }
-      if (s == 1 && R > 1) {
-        dmag |= fx_mag(Lp[o + 1] - c) | fx_mag(Lp[o + W] - c);
-        lmag |= fx_mag(v);
-      }
+      if (s == 1 && R > 1) lmag |= fx_mag(v);
       Lc[o] = v;
     };
     // the region's first 32 columns one row per warp, the rest after them
@@ -137,12 +123,12 @@ __device__ __forceinline__ unsigned long long rhs_tile_fx(const StepArgs<double>
     if (s < R) {
       if (s == 1) {
         lmag = __reduce_or_sync(0xffffffffu, lmag);
-        if (tx == 0) rmag[1][ty] = lmag;
+        if (tx == 0) rmag[ty] = lmag;
       }
       __syncthreads();
       if (s == 1) {
 #pragma unroll
-        for (int w = 0; w < NT / 32; ++w) lmag |= rmag[1][w];
+        for (int w = 0; w < NT / 32; ++w) lmag |= rmag[w];
         // each further sweep grows a value at most eightfold: room for them
         // (a rough psi only; a smooth one's Laplacian is far below it)
         lsh = 32 - fx_clz(lmag) + 32 + 3 * (R - 1) - 62;
@@ -160,17 +146,12 @@ __device__ __forceinline__ unsigned long long rhs_tile_fx(const StepArgs<double>
     Lp = Lc;
     Lc = Lc == L0 ? L1 : L0;
   }
-  dmag = __reduce_or_sync(0xffffffffu, dmag);
-  if (tx == 0) rmag[0][ty] = dmag;
-  __syncthreads();
-#pragma unroll
-  for (int w = 0; w < NT / 32; ++w) dmag |= rmag[0][w];
-  // |C| <= 4 differences: below 2^59 after the shift
-  const int sc = max(0, 25 - (32 - fx_clz(dmag)));
+  // (a thread reads back the last sweep's values it wrote: that region is one
+  // row of 32 points per warp, as below)
   // non-finite tiles and tiles of zeros, as the transforms mark them
   const bool bad = max(hp, hq) >= 0x7ff00000u;
   const int ed = bad ? FX_NAN : ep, el = bad ? FX_NAN : ep + lsh;
-  const int ej = bad ? FX_NAN : (hp == 0 || hq == 0) ? FX_ZERO : ep + eq + 64 - sc;
+  const int ej = bad ? FX_NAN : (hp == 0 || hq == 0) ? FX_ZERO : ep + eq + 64;
 
   const size_t fs = (size_t)a.nl * a.lstride;
   int s0, s1, s2;
@@ -183,39 +164,24 @@ __device__ __forceinline__ unsigned long long rhs_tile_fx(const StepArgs<double>
     const int gi = i0 + tx, gj = j0 + y;
     if (EDGE && (gi >= nx || gj >= ny)) continue;
     const fx_t* p = P + (y + R) * W + tx + XO;
-    const fx_t* q = Q + (y + 1) * W + tx + XO;
-    fx_t J = 0;
-    int t = 8;  // the sixteen truncations below, half a unit each
-    auto mac = [&](fx_t c, fx_t v) {
-      const Q2 b = q2_split(fx_shl(c, sc)), d = q2_split(v);
-      J += (fx_t)b.h * d.h;
-      t += fx_mh(b.h, d.l) + fx_mh(b.l, d.h);
-    };
-    const fx_t pc = p[0], pe = p[1], pw = p[-1], pn = p[W], ps = p[-W];
-    const fx_t pne = p[W + 1], pnw = p[W - 1], pse = p[-W + 1], psw = p[-W - 1];
-    const fx_t dx = pe - pw, dy = pn - ps;
-    mac(dx + (pne - pnw), q[W]);
-    mac((psw - pse) - dx, q[-W]);
-    mac((pse - pne) - dy, q[1]);
-    mac(dy + (pnw - psw), q[-1]);
-    mac(pe - pn, q[W + 1]);
-    mac(ps - pe, q[-W + 1]);
-    mac(pn - pw, q[W - 1]);
-    mac(pw - ps, q[-W - 1]);
-    J += t;
+    const Q2* q = Q + (y + 1) * W + tx + XO;
+    const FxNine ps = fx_nine(p, W);
+    int jn;
+    const fx_t J = fx_sum_value(fx_jacobian(ps, q, W), jn);
+    const fx_t dx = ps.e - ps.w;
     // rhs, src/dynamics.h:55-58
-    double f = fmaT(-a.inv12d2, fx_out(J, ej), -(a.b2d * fx_out(dx, ed)));
+    double f = fmaT(-a.inv12d2, fx_out(J, fx_exp_add(ej, -jn)), -(a.b2d * fx_out(dx, ed)));
     if (a.has_nu) {
-      const fx_t lq = ((q[1] + q[-1]) + (q[W] + q[-W])) - 4 * q[0];
+      const fx_t lq = ((q2_join(q[1]) + q2_join(q[-1])) + (q2_join(q[W]) + q2_join(q[-W]))) - 4 * q2_join(q[0]);
       f = fmaT(a.nu_d2, fx_out(lq, bad ? FX_NAN : eq), f);
     }
     if (ksweep > 0) f = fmaT(a.nuh_scaled, fx_out(Lp[(y + R) * W + tx + XO], el), f);
     // surface wind (src/dynamics.h:66) and bottom drag (:67-69)
     if (k == 0 && a.has_wind) f += a.wind[gj];
-    if (bottom && a.has_drag) f = fmaT(a.drag_d2, fx_out(((pe + pw) + (pn + ps)) - 4 * pc, ed), f);
+    if (bottom && a.has_drag) f = fmaT(a.drag_d2, fx_out(((ps.e + ps.w) + (ps.n + ps.s)) - 4 * ps.c, ed), f);
     fout[(size_t)gj * pitch + gi] = f;
     // CFL (src/timestep.h:74-87): one-sided differences
-    const fx_t du = pe - pc, dv = pn - pc;
+    const fx_t du = ps.e - ps.c, dv = ps.n - ps.c;
     cfl = max(cfl, max(du < 0 ? -du : du, dv < 0 ? -dv : dv));
   }
   return absbits(fx_out(cfl, ed));

@@ -1,6 +1,7 @@
 // CPU check of the device DST-I building blocks (qgw_gb300/csrc/dst_core.h):
 // runs every phase's work items in a plain loop, exactly as the kernels
 // spread them over threads, and exposes the result through a C function.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 #include <cstring>
@@ -8,6 +9,7 @@
 #include "../../qgw_gb300/csrc/dst_warp.h"
 #include "../../qgw_gb300/csrc/dst_blue.h"
 #include "../../qgw_gb300/csrc/modes_core.h"
+#include "../../qgw_gb300/csrc/rhs_core.h"
 
 using namespace qgw;
 
@@ -379,4 +381,58 @@ extern "C" void modes_errors(int nl, int ny, int nx, const double* mat, const do
       exact[m * n + p] = (double)t;
     }
   }
+}
+
+// The Arakawa Jacobian (times 12 Delta^2) of a field of ny x nx points with a
+// ring around it, in tiles of 32 x 16: the errors of the floating-point form
+// and of the fixed-point one (rhs_core.h) against long double, and the latter.
+extern "C" void jacobian_errors(int ny, int nx, const double* psi, const double* q, double* err64, double* errfx,
+                                double* exact) {
+  const int W = nx + 2;
+  std::vector<fx_t> P((size_t)W * (ny + 2));
+  std::vector<Q2> Q(P.size());
+  auto hi = [](double v) { return (unsigned int)(bits_of(v) >> 32) & 0x7fffffffu; };
+  for (int j0 = 0; j0 < ny; j0 += 16)
+    for (int i0 = 0; i0 < nx; i0 += 32) {
+      const int jn = std::min(ny, j0 + 16), in = std::min(nx, i0 + 32);
+      unsigned int hp = 0, hq = 0;
+      for (int y = j0; y < jn + 2; ++y)
+        for (int x = i0; x < in + 2; ++x) {
+          hp = std::max(hp, hi(psi[y * W + x]));
+          hq = std::max(hq, hi(q[y * W + x]));
+        }
+      const int Ep = fx_scale(hp) + 2, Eq = fx_scale(hq);
+      for (int y = j0; y < jn + 2; ++y)
+        for (int x = i0; x < in + 2; ++x) {
+          P[y * W + x] = fx_from_bits(bits_of(psi[y * W + x]), Ep);
+          Q[y * W + x] = q2_split(fx_from_bits(bits_of(q[y * W + x]), Eq));
+        }
+      for (int j = j0; j < jn; ++j)
+        for (int i = i0; i < in; ++i) {
+          const int o = (j + 1) * W + i + 1;
+          const double *p = psi + o, *z = q + o;
+          int n;
+          const fx_t v = fx_sum_value(fx_jacobian(fx_nine(P.data() + o, W), Q.data() + o, W), n);
+          const double r = fx_double(v, Ep + Eq - 2 * FX_EOFF + 64 - n);
+          double J = (p[1] - p[-1]) * (z[W] - z[-W]);
+          J = std::fma(-(p[W] - p[-W]), z[1] - z[-1], J);
+          J = std::fma(p[1], z[W + 1] - z[-W + 1], J);
+          J = std::fma(-p[-1], z[W - 1] - z[-W - 1], J);
+          J = std::fma(-p[W], z[W + 1] - z[W - 1], J);
+          J = std::fma(p[-W], z[-W + 1] - z[-W - 1], J);
+          J = std::fma(z[W], p[W + 1] - p[W - 1], J);
+          J = std::fma(-z[-W], p[-W + 1] - p[-W - 1], J);
+          J = std::fma(-z[1], p[W + 1] - p[-W + 1], J);
+          J = std::fma(z[-1], p[W - 1] - p[-W - 1], J);
+          auto d = [](const double* f, int a, int b) { return (long double)f[a] - f[b]; };
+          // the coefficients of q sum to zero: of its differences
+          const long double t = d(z, W, 0) * (d(p, 1, -1) + d(p, W + 1, W - 1)) - d(z, -W, 0) * (d(p, 1, -1) + d(p, -W + 1, -W - 1)) -
+                                d(z, 1, 0) * (d(p, W, -W) + d(p, W + 1, -W + 1)) + d(z, -1, 0) * (d(p, W, -W) + d(p, W - 1, -W - 1)) +
+                                d(z, W + 1, 0) * d(p, 1, W) + d(z, -W + 1, 0) * d(p, -W, 1) + d(z, W - 1, 0) * d(p, W, -1) +
+                                d(z, -W - 1, 0) * d(p, -1, -W);
+          err64[j * nx + i] = (double)(J - t);
+          errfx[j * nx + i] = (double)(r - t);
+          exact[j * nx + i] = (double)t;
+        }
+    }
 }

@@ -128,6 +128,70 @@ def test_projection_error_of_every_layer(dstcore, qgwlib, nl, ratio, kind):  # n
     assert fx <= max(f64, 2.0) and np.all(e[:, 1] <= np.maximum(e[:, 0], 2.0) + 2.0), e
 
 
+def vorticity(kind, N):
+    rng, (Y, X) = np.random.default_rng(11), np.mgrid[1:N, 1:N]
+    if kind == "front":
+        return 1e-5 + 1e-6 * np.tanh((X - N / 2 + N / 16 * np.sin(12 * Y / N)) / 3)
+    if kind == "vortex":
+        return 1e-5 * np.exp(-((X - N / 3) ** 2 + (Y - N / 2) ** 2) / 50) + 1e-12 * rng.standard_normal(X.shape)
+    q = sum(2e-6 * a * np.sin(2 * np.pi * int(1 + 4 * b) * X / N + 6 * c) * np.sin(2 * np.pi * int(1 + 4 * d) * Y / N + 6 * e)
+            for a, b, c, d, e in rng.random((8, 5)))
+    if kind == "single":
+        return q.astype(np.float32).astype(float)
+    return 1e-7 * rng.standard_normal(X.shape) + q * (kind == "eddies and noise") if "noise" in kind else q
+
+
+@pytest.mark.parametrize("kind", ["noise", "eddies", "eddies and noise", "single", "front", "vortex"])
+def test_jacobian_error_no_larger_than_fp64(dstcore, kind):  # noqa: F811
+    N = 160
+    q, k = vorticity(kind, N), np.pi / 4e6 * np.arange(1, N)
+    psi = sf.idstn(sf.dstn(q, type=1) / -(k[:, None] ** 2 + k ** 2 + 1e-10), type=1)
+    q, psi = (np.ascontiguousarray(np.pad(f, 1)) for f in (q, psi))
+    e64, efx, exact = (np.empty((N - 1, N - 1)) for _ in range(3))
+    dstcore.jacobian_errors.argtypes = [ctypes.c_int] * 2 + [ctypes.c_void_p] * 5
+    dstcore.jacobian_errors(N - 1, N - 1, psi.ctypes.data, q.ctypes.data, *(e.ctypes.data for e in (e64, efx, exact)))
+    f64, fx = (np.linalg.norm(e) / np.linalg.norm(exact) * 2.0 ** 53 for e in (e64, efx))
+    assert fx <= max(f64, 2.0), (f64, fx)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bc", [0.0, -1.0])
+@pytest.mark.parametrize("kind", ["eddies", "single", "half"])
+def test_jacobian_of_a_step(qgwlib, kind, bc):
+    """A step of nothing but the Jacobian, so long that q itself is all but
+    lost in it, against long double: to 4 units of 2^-53 (its own rounding, the
+    coefficient's, the update's and the comparison's), and exactly zero where
+    q is."""
+    N = 96
+    p = dict(C.cfg1(N), nl=1, dh=[4000.0], N2=[1.0], beta=0.0, tau0=0.0, nu=0.0, hEkb=0.0, bc_fac=bc, cfl=1e30)
+    r = qgwlib.Run(p)
+    q = np.zeros(r.shape)
+    n = r.shape[2] - 2
+    q[0, 1:-1, 1:-1] = vorticity("single" if kind == "single" else "eddies", n + 1)
+    if kind == "half":
+        q[0, :, : N // 2] = 0
+    r.set_q(q)
+    psi, q = r.get()
+    dt = 1e18
+    r.fix_dt(dt)
+    r.step(1)
+    q1 = r.get()[1][0, 1:-1, 1:-1]
+    r.close()
+    P, Q = (f[0].astype(np.longdouble) for f in (psi, q))
+
+    def d(f, a, b):
+        return (f[1 + a[1]:1 + a[1] + n, 1 + a[0]:1 + a[0] + n] - f[1 + b[1]:1 + b[1] + n, 1 + b[0]:1 + b[0] + n])
+    o, E, W, S, T = (0, 0), (1, 0), (-1, 0), (0, -1), (0, 1)
+    NE, NW, SE, SW = (1, 1), (-1, 1), (1, -1), (-1, -1)
+    J = (d(Q, T, o) * (d(P, E, W) + d(P, NE, NW)) - d(Q, S, o) * (d(P, E, W) + d(P, SE, SW))
+         - d(Q, E, o) * (d(P, T, S) + d(P, NE, SE)) + d(Q, W, o) * (d(P, T, S) + d(P, NW, SW))
+         + d(Q, NE, o) * d(P, E, T) + d(Q, SE, o) * d(P, S, E) + d(Q, NW, o) * d(P, T, W) + d(Q, SW, o) * d(P, W, S))
+    ref = Q[1:-1, 1:-1] - np.longdouble(dt) * 23 / 12 * J / (12 * np.longdouble(p["Lx"] / N) ** 2)
+    assert np.linalg.norm((q1 - ref).astype(float)) <= 4 * 2.0 ** -53 * np.linalg.norm(ref.astype(float))
+    if kind == "half":
+        assert np.all(q1[:, 2: N // 2 - 2] == 0)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("NX,NY", [(4, 6), (10, 14), (128, 16), (16, 256), (256, 128), (512, 30), (30, 512),
                                    (1024, 12), (96, 1024), (2048, 64), (64, 2048), (2430, 8), (4096, 10)])

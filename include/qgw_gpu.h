@@ -254,7 +254,9 @@ int qgw_profile_kernels(qgw_run* run, int nsteps, float* ms4);
  * in FP32 and 2 or 1 in FP64); row_group_fwd and row_group_inv, rows per
  * block of the forward and inverse row kernels (1..16; FP32: modes (layers) of
  * one grid row, balanced over the run's, and at most 8 in an inverse kernel
- * that also transforms zeta; FP64: rows of any layer).  0 keeps a value.  No choice changes the arithmetic: a run's
+ * that also transforms zeta; FP64: rows of any layer, as many of them as the
+ * device's shared memory holds, and in ensembles layers of one grid row).  0
+ * keeps a value.  No choice changes the arithmetic: a run's
  * results are bitwise the same for every shape.  QGW_ERR_PARAM when a value
  * is not one of these or the shape needs more shared memory than the
  * device has (the run keeps its shape). */

@@ -592,13 +592,13 @@ int set_shape(qgw_run* r, StepArgs<T>& a, const qgw_shape& sh) {
   if (sh.row_group_fwd) {
     if (sh.row_group_fwd < 1 || sh.row_group_fwd > 16) return QGW_ERR_PARAM;
     b.G1 = mode_group(r->nl, Mx, sizeof(T), any, 1, 16, sh.row_group_fwd, bufs_x);
-    b.RB1 = b.G1;
+    if constexpr (sizeof(T) == 8) b.RB1 = qgw::rows_fit_f64(b, sh.row_group_fwd);
   }
   if (sh.row_group_inv) {
     if (sh.row_group_inv < 1 || sh.row_group_inv > 16) return QGW_ERR_PARAM;
     const bool zm = a.zeta_mode != 0;
     b.G3 = mode_group(r->nl, Mx, sizeof(T), any, zm ? 2 : 1, zm ? 8 : 16, sh.row_group_inv, bufs_x);
-    b.RB3 = b.G3;
+    if constexpr (sizeof(T) == 8) b.RB3 = qgw::rows_fit_f64(b, sh.row_group_inv);
   }
   if (b.rhs_ty != a.rhs_ty) encode_rhs_maps<T>(r, b);
   cudaError_t e;
@@ -616,8 +616,8 @@ template <typename T>
 void get_shape(const StepArgs<T>& a, qgw_shape* sh) {
   sh->rhs_tile_rows = a.rhs_ty == 32 ? 32 : 16;
   sh->col_tile = a.CT1 ? a.CT1 : a.CT ? a.CT : 32 / (int)sizeof(T);
-  sh->row_group_fwd = a.G1;
-  sh->row_group_inv = a.G3;
+  sh->row_group_fwd = sizeof(T) == 8 ? a.RB1 : a.G1;
+  sh->row_group_inv = sizeof(T) == 8 ? a.RB3 : a.G3;
 }
 
 }  // namespace

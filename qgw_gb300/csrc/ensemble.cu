@@ -359,17 +359,33 @@ int qgw_ensemble_step(qgw_ensemble* ens, int nsteps, const int* max_steps, int u
   return bad ? QGW_ERR_NAN : QGW_OK;
 }
 
+// A member's shape in the batched kernels, whose FP64 row kernels take rows of
+// one grid row (G1, G3) where a single run's take rows of any layer.
+static void member_shape(qgw_run* r, qgw_shape* sh) {
+  qgw_get_shape(r, sh);
+  if (r->precision != QGW_FP64) return;
+  sh->row_group_fwd = r->a64.G1;
+  sh->row_group_inv = r->a64.G3;
+}
+
 // The same work-tile shape for every member (qgw_set_shape), then the
 // member table rebuilt; a member that refuses the shape leaves every member
 // at its previous one.
 static int ensemble_set_shape(qgw::EnsembleCore* e, const qgw_shape& sh) {
   const int n = (int)e->members.size();
-  std::vector<qgw_shape> old(n);
-  for (int i = 0; i < n; ++i) qgw_get_shape(e->members[i], &old[i]);
+  std::vector<qgw::StepArgs<double>> a64(n);
+  std::vector<qgw::StepArgs<float>> a32(n);
+  for (int i = 0; i < n; ++i) {
+    a64[i] = e->members[i]->a64;
+    a32[i] = e->members[i]->a32;
+  }
   for (int i = 0; i < n; ++i) {
     const int rc = qgw_set_shape(e->members[i], &sh);
     if (rc) {
-      for (int j = 0; j < i; ++j) qgw_set_shape(e->members[j], &old[j]);
+      for (int j = 0; j < i; ++j) {
+        e->members[j]->a64 = a64[j];
+        e->members[j]->a32 = a32[j];
+      }
       return rc;
     }
   }
@@ -418,7 +434,7 @@ int qgw_ensemble_tune(qgw_ensemble* ens, int trial_steps, float* best_ms) {
     const int ctd = e->precision == QGW_FP64 ? 4 : 8;
     const std::vector<int> cand[4] = {{16, 32}, {ctd, ctd / 2}, {2, 4, 8, 16}, {2, 3, 4, 5}};
     qgw_shape cur{};
-    qgw_get_shape(e->members[0], &cur);
+    member_shape(e->members[0], &cur);
     int* field[4] = {&cur.rhs_tile_rows, &cur.col_tile, &cur.row_group_fwd, &cur.row_group_inv};
     for (int f = 0; f < 4; ++f) {
       float best = 1e30f;
@@ -514,7 +530,8 @@ int qgw_ensemble_set_shape(qgw_ensemble* ens, const qgw_shape* sh) {
 int qgw_ensemble_shape(qgw_ensemble* ens, int i, qgw_shape* sh) {
   qgw::EnsembleCore* e = ens ? &ens->core : nullptr;
   if (!e || !sh || i < 0 || i >= (int)e->members.size()) return QGW_ERR_PARAM;
-  return qgw_get_shape(e->members[i], sh);
+  member_shape(e->members[i], sh);
+  return QGW_OK;
 }
 
 int qgw_ensemble_grids(qgw_ensemble* ens, int* bps4) {

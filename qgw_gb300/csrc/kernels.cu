@@ -425,6 +425,9 @@ static __global__ void k_budget_final(const double* part, int nblk, double scale
 // maximum (never lowered) so that runs of different sizes can coexist.
 [[maybe_unused]] static size_t rows_bytes(const StepArgs<double>& a) { return smem_rows_f64(a, std::max(a.RB1, a.RB3)); }
 [[maybe_unused]] static size_t rows_bytes(const StepArgs<float>&) { return 0; }
+// static shared memory of the row and column kernels, at most
+template <typename T> constexpr size_t static_tot = sizeof(T) * GMAX * 32 + 64;
+static_assert(sizeof(double) * tot_len<double, -1> <= static_tot<double>, "the chirp-z kernels' scratch");
 template <typename T, bool COMP>
 static cudaError_t set_attrs(const StepArgs<T>& a) {
   int dev = 0, optin = 0;
@@ -432,13 +435,12 @@ static cudaError_t set_attrs(const StepArgs<T>& a) {
   if (e != cudaSuccess) return e;
   e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e != cudaSuccess) return e;
-  const size_t static_tot = sizeof(T) * GMAX * 32 + 64;
-  if (smem_rows<T, COMP>(a) + static_tot > (size_t)optin || smem_cols<T, COMP>(a) + static_tot > (size_t)optin ||
-      smem_rows_inv<T, COMP>(a) + static_tot > (size_t)optin || rhs_halo(a) > RHS_RMAX ||
-      (sizeof(T) == 8 && rows_bytes(a) + static_tot > (size_t)optin) ||
+  if (smem_rows<T, COMP>(a) + static_tot<T> > (size_t)optin || smem_cols<T, COMP>(a) + static_tot<T> > (size_t)optin ||
+      smem_rows_inv<T, COMP>(a) + static_tot<T> > (size_t)optin || rhs_halo(a) > RHS_RMAX ||
+      (sizeof(T) == 8 && rows_bytes(a) + static_tot<T> > (size_t)optin) ||
       smem_rhs<T>(a) + 1024 > (size_t)optin || smem_rhs_tiles<T>(a) + 1024 > (size_t)optin)
     return cudaErrorInvalidValue;
-  const int lim = optin - (int)static_tot;
+  const int lim = optin - (int)static_tot<T>;
   const void* columns[] = {
       (const void*)k_cols<T, COMP, false, CTD<T>, 0>,     (const void*)k_cols<T, COMP, false, CTD<T>, 512>,
       (const void*)k_cols<T, COMP, false, CTD<T> / 2, 0>, (const void*)k_cols<T, COMP, false, CTD<T> / 2, 512>,
@@ -677,6 +679,15 @@ int rhs_tile_x() { return TX; }
 int rhs_box_width() { return TW; }
 
 cudaError_t prepare_f64(const StepArgs<double>& a) { return set_attrs<double, false>(a); }
+
+int rows_fit_f64(const StepArgs<double>& a, int want) {
+  int dev = 0, optin = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+    return 1;
+  while (want > 1 && smem_rows_f64(a, want) + static_tot<double> > (size_t)optin) --want;
+  return want;
+}
 
 int rhs_grid_f64(const StepArgs<double>&) { return 0; }  // one block per tile
 

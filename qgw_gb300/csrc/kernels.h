@@ -14,6 +14,9 @@ cudaError_t prepare_f32c(const StepArgs<float>& a);
 // one block per tile, as the FP64 path runs); after prepare_*
 int rhs_grid_f64(const StepArgs<double>& a);
 int rhs_grid_f32c(const StepArgs<float>& a);
+// rows per block of the FP64 row kernels: want, or as many as the device's
+// shared memory holds
+int rows_fit_f64(const StepArgs<double>& a, int want);
 
 void enqueue_begin(DevState* st, double t_out, double tend, cudaStream_t s);
 void enqueue_step_f64(const StepArgs<double>& a, cudaStream_t s);

@@ -122,6 +122,34 @@ def test_tall_rhs_tiles_by_default(qgwlib, p):
     assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][0], out[1][0])
 
 
+def test_fp64_shape_is_the_one_the_row_kernels_take(qgwlib):
+    """FP64 rows per block: setting the shape that was read changes nothing,
+    a request above the layer count is taken, one beyond the shared memory
+    cut to what it holds, and an ensemble that refuses a shape at its last
+    member keeps every member's."""
+    for p, most in ((C.basin_params(1024, 1), 16), (C.cfg1(256), 16), (dict(C.cfg2(2048, 3), NY=64), 12)):
+        q0 = C.noise_ic(p, 47)
+        r = qgwlib.Run(p, 0)
+        before = r.get_shape()
+        r.set_shape(**before)
+        assert r.get_shape() == before
+        r.set_q(q0)
+        psi = r.get()[0]
+        r.set_shape(row_group_fwd=16, row_group_inv=16)
+        sh = r.get_shape()
+        assert sh["row_group_fwd"] == sh["row_group_inv"] == most, sh
+        assert np.array_equal(r.get()[0], psi)
+        r.close()
+    ens = qgwlib.Ensemble([C.cfg2(64, 5), dict(C.cfg2(2048, 16), NY=64)], 0)
+    before = [ens.get_shape(i) for i in range(2)]
+    with pytest.raises(qgwlib.QgwError):
+        ens.set_shape(row_group_fwd=16)
+    assert [ens.get_shape(i) for i in range(2)] == before
+    ens.set_shape(row_group_fwd=2)
+    assert [ens.get_shape(i)["row_group_fwd"] for i in range(2)] == [2, 2]
+    ens.close()
+
+
 def test_shape_refuses_unknown_values(qgwlib):
     r = qgwlib.Run(C.cfg1(64), 1)
     before = r.get_shape()

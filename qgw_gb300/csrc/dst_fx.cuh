@@ -450,19 +450,22 @@ __device__ __forceinline__ fx_t* dst_fx_blue(double* A, double* B, int nrows, in
 // they were written, their largest high words noted), B the second buffer:
 // returns the buffer that holds Y_k at index k as integers of the rows'
 // exponents sc->ex.  HL: the half-length whose transform alone the kernel
-// holds, 0, or -1 for the chirp-z lengths.
+// holds, 0 for those without a kernel of their own, -1 for the chirp-z lengths,
+// -2 for all but these (the batched kernels, two buffers).
 template <int HL>
 __device__ __forceinline__ fx_t* dst_fx(double* A, double* B, int nrows, int ld, const DstGeom& g, const FxTables& tb,
                                         FxScratch* sc) {
   if constexpr (HL == 512) return dst_fx_fixed<9, true>(A, B, nrows, ld, tb, sc);
   if constexpr (HL == 1024) return dst_fx_fixed<10, true>(A, B, nrows, ld, tb, sc);
   if constexpr (HL == -1) return dst_fx_blue(A, B, nrows, ld, g, tb, sc);
+  if constexpr (HL == -2) {
+    if (g.H == 512) return dst_fx_fixed<9>(A, B, nrows, ld, tb, sc);
+    if (g.H == 1024) return dst_fx_fixed<10>(A, B, nrows, ld, tb, sc);
+  }
   switch (g.H) {
     case 64: return dst_fx_fixed<6>(A, B, nrows, ld, tb, sc);
     case 128: return dst_fx_fixed<7>(A, B, nrows, ld, tb, sc);
     case 256: return dst_fx_fixed<8>(A, B, nrows, ld, tb, sc);
-    case 512: return dst_fx_fixed<9>(A, B, nrows, ld, tb, sc);
-    case 1024: return dst_fx_fixed<10>(A, B, nrows, ld, tb, sc);
     default: return dst_fx_any(A, B, nrows, ld, g, tb, sc);
   }
 }

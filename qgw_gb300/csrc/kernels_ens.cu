@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 3 : 2) k_cols_ens(EnsArgs
     const int ntx = PER ? (sa.gx.H + 2) / 2 : (sa.nx + CT - 1) / CT;
     if constexpr (PER && sizeof(T) == 8) body_cols_per_fx<2>(sa, step_mode, local % ntx, local / ntx, smem_raw, tot);
     else if constexpr (PER) body_cols_per<T, COMP>(sa, step_mode, local % ntx, local / ntx, smem_raw);
-    else body_cols<T, COMP, CT>(sa, step_mode, local % ntx, local / ntx, smem_raw, tot);
+    else body_cols<T, COMP, CT, -2>(sa, step_mode, local % ntx, local / ntx, smem_raw, tot);
     __syncthreads();
   }
 }

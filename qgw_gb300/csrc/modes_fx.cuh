@@ -294,7 +294,7 @@ __device__ __forceinline__ void body_rows_f64(const StepArgs<double>& a, int ste
   for (int i0 = 0; i0 < np; i0 += NT)
     modes_point_any<!INV>(a, INV ? a.m2l : a.l2m, u, j, i0 + threadIdx.x, i0 + (int)threadIdx.x < np, (Q2*)smem_raw);
   __syncthreads();
-  for (int l = 0; l < a.nl; l += G) rows_f64<PER, 0, INV>(a, INV ? a.psi : a.spec, l, min(G, a.nl - l), j, A, B, tot);
+  for (int l = 0; l < a.nl; l += G) rows_f64<PER, -2, INV>(a, INV ? a.psi : a.spec, l, min(G, a.nl - l), j, A, B, tot);
 }
 
 }  // namespace qgw

@@ -141,9 +141,8 @@ __device__ __forceinline__ T* dst_block_blue(T* A, T* B, int nrows, int ld, cons
 template <typename T, int HL = 0>
 __device__ __forceinline__ T* dst_block(T* A, T* B, int nrows, int ld, const DstGeom& g, const DstTables<T>& tb,
                                         T* tot) {
-  if constexpr (sizeof(T) == 8) {
-    return A;  // (never: body_cols has left through body_cols_fx)
-  } else if constexpr (HL == -1) {
+  static_assert(sizeof(T) == 4, "FP64 rows go through dst_fx");
+  if constexpr (HL == -1) {
     return dst_block_blue<T>(A, B, nrows, ld, g, tb);
   } else if constexpr (HL == 512) {
     return dst_block_warp_f32<9>(A, nrows, ld, tb);
@@ -639,6 +638,98 @@ __device__ __forceinline__ void body_cols_fx(const StepArgs<double>& a, int k0, 
   }
 }
 
+// The rest of body_cols in FP32: forward DST of the tile in A, divide, second
+// field, inverse DST, store.  The block is synchronised.
+template <int CT, int HL>
+__device__ __forceinline__ void body_cols_f32(const StepArgs<float>& a, int k0, int CTb, int m, float* A, float* B,
+                                              int ld, bool vec, float* tot) {
+  const int ny = a.ny;
+  const bool zm = a.zeta_mode != 0;
+  constexpr int RB = 2;  // rows per pass (body_cols)
+  float* O = dst_block<float, HL>(A, B, CT, ld, a.gy, a.ty, tot);
+  float* C = O + (size_t)CT * ld;  // the second field's rows (zeta mode)
+  const double iRd2 = a.iRd2[m];
+  // power of the 5-point symbol in the second field: L psi (zeta mode 1) or
+  // the whole hyperviscosity chain L^nsweep psi (zeta mode 2)
+  const int zpow = a.zeta_mode == 2 ? a.nsweep : 1;
+  const float ird2f = a.iRd2f[m];
+  const float normf = a.fc[FC_NORM], lx2f = a.fc[FC_LX2], ly2f = a.fc[FC_LY2];
+  // the tile's per-column table values, the same for every row
+  float lsqc[CT], sxc[CT];
+#pragma unroll
+  for (int c = 0; c < CT; ++c) {
+    const int k = min(k0 + c, a.nx - 1);
+    lsqc[c] = a.Lsqf[k];
+    sxc[c] = zm ? a.sx2f[k] : 0.f;
+  }
+  // RB rows per pass, their per-row loads issued before any is used
+  for (int j0 = threadIdx.x - 1; j0 < ny; j0 += RB * NT) {
+    float ksq4[RB], sy4[RB];
+#pragma unroll
+    for (int u = 0; u < RB; ++u) {
+      const int jj = j0 + u * NT;
+      if (jj < 0 || jj >= ny) continue;
+      ksq4[u] = a.Ksqf[jj];
+      sy4[u] = zm ? a.sy2f[jj] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < RB; ++u) {
+      const int jj = j0 + u * NT;
+      if (jj < 0 || jj >= ny) continue;
+      const int pj = pr<float>(jj + 1);
+#pragma unroll
+      for (int c = 0; c < CT; ++c) {
+        const int k = min(k0 + c, a.nx - 1);
+        float x;
+        if (m == 0 && jj < a.low_k64 && k < a.low_k64) {
+          // barotropic mode, lowest wavenumbers: divide in FP64
+          const double fact = -(a.Lsq[k] + a.Ksq[jj] + iRd2);
+          x = (float)((double)O[c * ld + pj] / fact / a.norm);
+        } else {
+          const float fact = -((lsqc[c] + ksq4[u]) + ird2f);
+          x = O[c * ld + pj] / (fact * normf);
+        }
+        O[c * ld + pj] = x;
+        if (zm) {
+          // spectral discrete Laplacian of psi: lambda(k, j) * psi_hat with
+          // lambda = -4/Delta^2 (sin^2 kx + sin^2 ky), the exact symbol of
+          // the 5-point Laplacian with zero ghosts in the DST basis; applied
+          // zpow times, one factor after the other (no underflow of
+          // lambda^zpow at the lowest wavenumbers)
+          const float lam = lx2f * sxc[c] + ly2f * sy4[u];
+          float z = lam * x;
+          for (int s = 1; s < zpow; ++s) z = z * lam;
+          C[c * ld + pj] = z;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  float* Oth = (O == A) ? B : A;
+  float* O2 = dst_block<float, HL>(O, Oth, zm ? 2 * CT : CT, ld, a.gy, a.ty, tot);
+  float *S = a.spec + (size_t)m * a.lstride, *S2 = zm ? a.spec2 + (size_t)m * a.lstride : nullptr;
+  grid_next();
+  float v[CT];
+  for (int jj = threadIdx.x - 1; jj < ny; jj += NT) {
+    if (jj < 0) continue;
+    const int pj = pr<float>(jj + 1);
+#pragma unroll
+    for (int c = 0; c < CT; ++c) v[c] = c < CTb ? O2[c * ld + pj] : 0.f;
+    float* dst = S + (size_t)jj * a.pitch + k0;
+    if (vec) store_cols<float, CT>(dst, v);
+    else
+      for (int c = 0; c < CTb; ++c) dst[c] = v[c];
+    if (zm) {
+#pragma unroll
+      for (int c = 0; c < CT; ++c) v[c] = c < CTb ? O2[(CT + c) * ld + pj] : 0.f;
+      float* dst2 = S2 + (size_t)jj * a.pitch + k0;
+      if (vec) store_cols<float, CT>(dst2, v);
+      else
+        for (int c = 0; c < CTb; ++c) dst2[c] = v[c];
+    }
+  }
+}
+
 template <typename T, bool COMP, int CT, int HL = 0>
 __device__ __forceinline__ void body_cols(const StepArgs<T>& a, int step_mode, int bx, int m, unsigned char* smem_raw,
                                           T* tot) {
@@ -714,109 +805,8 @@ __device__ __forceinline__ void body_cols(const StepArgs<T>& a, int step_mode, i
     for (int c = 0; c < CT; ++c) fx_note_max(&sc[0], c, hmax[c]);
   }
   __syncthreads();
-  if constexpr (FX) {
-    body_cols_fx<CT, HL>(a, k0, CTb, m, A, B, ld, vec, sc);
-    return;
-  }
-  T* O = dst_block<T, HL>(A, B, CT, ld, a.gy, a.ty, tot);
-  T* C = O + (size_t)CT * ld;  // the second field's rows (zeta mode)
-  const double iRd2 = a.iRd2[m];
-  // power of the 5-point symbol in the second field: L psi (zeta mode 1) or
-  // the whole hyperviscosity chain L^nsweep psi (zeta mode 2)
-  const int zpow = (COMP && a.zeta_mode == 2) ? a.nsweep : 1;
-  const float ird2f = COMP ? a.iRd2f[m] : 0.f;
-  const float normf = a.fc[FC_NORM], lx2f = a.fc[FC_LX2], ly2f = a.fc[FC_LY2];
-  // the tile's per-column table values, the same for every row
-  float lsqc[CT], sxc[CT];
-#pragma unroll
-  for (int c = 0; c < CT; ++c) {
-    const int k = min(k0 + c, a.nx - 1);
-    lsqc[c] = COMP ? a.Lsqf[k] : 0.f;
-    sxc[c] = zm ? a.sx2f[k] : 0.f;
-  }
-  // RB rows per pass, their per-row loads issued before any is used
-  for (int j0 = threadIdx.x - 1; j0 < ny; j0 += RB * NT) {
-    T h4[RB][CT];
-    float ksq4[RB], sy4[RB];
-#pragma unroll
-    for (int u = 0; u < RB; ++u) {
-      const int jj = j0 + u * NT;
-      if (jj < 0 || jj >= ny) continue;
-      if (!COMP) {
-        const T* hrow = (const T*)(a.hinv + (size_t)m * a.lstride + (size_t)jj * a.pitch + k0);
-        if constexpr (VEC) {
-          if (vec) {
-            load_cols<T, CT>(hrow, h4[u]);
-            continue;
-          }
-        }
-        for (int c = 0; c < CT; ++c) h4[u][c] = c < CTb ? hrow[c] : T(0);
-      } else {
-        ksq4[u] = a.Ksqf[jj];
-        sy4[u] = zm ? a.sy2f[jj] : 0.f;
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < RB; ++u) {
-      const int jj = j0 + u * NT;
-      if (jj < 0 || jj >= ny) continue;
-      const int pj = pr<T>(jj + 1);
-      if (!COMP) {
-#pragma unroll
-        for (int c = 0; c < CT; ++c) O[c * ld + pj] *= h4[u][c];
-      } else {
-#pragma unroll
-        for (int c = 0; c < CT; ++c) {
-          const int k = min(k0 + c, a.nx - 1);
-          float x;
-          if (m == 0 && jj < a.low_k64 && k < a.low_k64) {
-            // barotropic mode, lowest wavenumbers: divide in FP64
-            const double fact = -(a.Lsq[k] + a.Ksq[jj] + iRd2);
-            x = (float)((double)O[c * ld + pj] / fact / a.norm);
-          } else {
-            const float fact = -((lsqc[c] + ksq4[u]) + ird2f);
-            x = (float)O[c * ld + pj] / (fact * normf);
-          }
-          O[c * ld + pj] = (T)x;
-          if (zm) {
-            // spectral discrete Laplacian of psi: lambda(k, j) * psi_hat with
-            // lambda = -4/Delta^2 (sin^2 kx + sin^2 ky), the exact symbol of
-            // the 5-point Laplacian with zero ghosts in the DST basis; applied
-            // zpow times, one factor after the other (no underflow of
-            // lambda^zpow at the lowest wavenumbers)
-            const float lam = lx2f * sxc[c] + ly2f * sy4[u];
-            float z = lam * x;
-            for (int s = 1; s < zpow; ++s) z = z * lam;
-            C[c * ld + pj] = (T)z;
-          }
-        }
-      }
-    }
-  }
-  __syncthreads();
-  T* Oth = (O == A) ? B : A;
-  T* O2 = dst_block<T, HL>(O, Oth, zm ? 2 * CT : CT, ld, a.gy, a.ty, tot);
-  T* S2 = zm ? a.spec2 + (size_t)m * a.lstride : nullptr;
-  grid_next();
-  T v[CT];
-  for (int jj = threadIdx.x - 1; jj < ny; jj += NT) {
-    if (jj < 0) continue;
-    const int pj = pr<T>(jj + 1);
-#pragma unroll
-    for (int c = 0; c < CT; ++c) v[c] = c < CTb ? O2[c * ld + pj] : T(0);
-    T* dst = S + (size_t)jj * a.pitch + k0;
-    if (vec) store_cols<T, CT>(dst, v);
-    else
-      for (int c = 0; c < CTb; ++c) dst[c] = v[c];
-    if (zm) {
-#pragma unroll
-      for (int c = 0; c < CT; ++c) v[c] = c < CTb ? O2[(CT + c) * ld + pj] : T(0);
-      T* dst2 = S2 + (size_t)jj * a.pitch + k0;
-      if (vec) store_cols<T, CT>(dst2, v);
-      else
-        for (int c = 0; c < CTb; ++c) dst2[c] = v[c];
-    }
-  }
+  if constexpr (FX) body_cols_fx<CT, HL>(a, k0, CTb, m, A, B, ld, vec, sc);
+  else body_cols_f32<CT, HL>(a, k0, CTb, m, A, B, ld, vec, tot);
 }
 
 // ------------------------------------------------------------- K2 periodic

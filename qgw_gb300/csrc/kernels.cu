@@ -68,12 +68,13 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 4) k_rhs(const __grid
 // FP64: the projections, one thread per point (NL: layers in registers, 0:
 // any number), and the row transforms (modes_fx.cuh).  The projections wait
 // on their loads: five blocks per SM below eight layers (48 registers, few
-// spills), four up to ten.  Both forward kernels at three, four and five
+// spills), four from there on.  Both forward kernels at three, four and five
 // blocks: 1024^2 x 10 0.265, 0.256 and 0.258 ms, 768^2 x 8 0.182, 0.173 and
-// 0.181, 1024^2 x 6 0.163, 0.157 and 0.155.  More layers need the registers
-// (any number, two and five blocks: 256^2 x 20 0.080 and 0.142).
+// 0.181, 1024^2 x 6 0.163, 0.157 and 0.155; at two to five, 512^2 x 12 0.124,
+// 0.113, 0.107 and 0.115, 512^2 x 16 0.162, 0.150, 0.147 and 0.181.  Any number
+// needs the registers (two and five: 256^2 x 20 0.081 and 0.141).
 template <int NL, bool FWD>
-__global__ void __launch_bounds__(NT, NL == 0 || NL > 10 ? 2 : NL >= 8 ? 4 : 5) k_modes(const __grid_constant__ StepArgs<double> a, int step_mode) {
+__global__ void __launch_bounds__(NT, NL == 0 ? 2 : NL >= 8 ? 4 : 5) k_modes(const __grid_constant__ StepArgs<double> a, int step_mode) {
   grid_wait();
   if (step_mode && !a.state->active) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -425,7 +426,8 @@ static __global__ void k_budget_final(const double* part, int nblk, double scale
 // maximum (never lowered) so that runs of different sizes can coexist.
 [[maybe_unused]] static size_t rows_bytes(const StepArgs<double>& a) { return smem_rows_f64(a, std::max(a.RB1, a.RB3)); }
 [[maybe_unused]] static size_t rows_bytes(const StepArgs<float>&) { return 0; }
-// static shared memory of the row and column kernels, at most
+// static shared memory of the row and column kernels, at most (with a margin
+// in FP64: the sizes a run takes or refuses go by this)
 template <typename T> constexpr size_t static_tot = sizeof(T) * GMAX * 32 + 64;
 static_assert(sizeof(double) * tot_len<double, -1> <= static_tot<double>, "the chirp-z kernels' scratch");
 template <typename T, bool COMP>

@@ -299,13 +299,15 @@ int qgw_probe_fp_rates(double* fp64_tflops, double* fp32_tflops);
 /* ---- ensembles: many runs, one launch per step stage --------------------
  * Members may differ in grid size and layer count (one precision per
  * ensemble).  qgw_ensemble_step advances every member by up to nsteps steps
- * (max_steps[i] > 0 caps member i), each stage as one persistent launch
- * over all members' work items, the four launches of a step captured once
- * as a CUDA graph (use_graph != 0) and replayed.  A member's result is
+ * (max_steps[i] > 0 caps member i), each stage as one launch over all
+ * members' work items (one block per item unless the tuner chose a
+ * persistent grid), the four launches of a step captured once as a CUDA
+ * graph (use_graph != 0) and replayed.  A member's result is
  * bitwise the same alone and in any ensemble.  qgw_ensemble_tune chooses
- * the members' work-tile shape (RHS tile height, column-tile width, modes
- * per row-kernel block; qgw_set_shape) and then each stage's persistent
- * grid size, one choice at a time, timing whole steps for every candidate;
+ * the members' work-tile shape (RHS tile height, column-tile width, layers
+ * per row-kernel block; qgw_set_shape) and then each stage's grid (one block
+ * per item, or a persistent grid of some blocks per SM), one choice at a
+ * time, timing whole steps for every candidate;
  * the trial steps advance the state, so set q afterwards.  No reference
  * counterpart: the reference runs one configuration per process. */
 typedef struct qgw_ensemble qgw_ensemble;

@@ -354,7 +354,8 @@ int setup_args(qgw_run* r, StepArgs<T>& a) {
   // reals per row buffer (the chirp-z form holds L complex values)
   const int Mrow = a.gx.blue ? 2 * a.gx.H : Mx;
   {
-    // QGW_ROW_GROUP overrides the modes per forward-rows block (tuning knob)
+    // QGW_ROW_GROUP overrides the modes per forward-rows block (FP32c, and
+    // FP64 ensembles; tuning knob)
     const char* e = std::getenv("QGW_ROW_GROUP");
     const int want = e ? std::atoi(e) : 0;
     const size_t budget = row_budget(sizeof(T), Mrow, r->nl);

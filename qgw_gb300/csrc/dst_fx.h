@@ -14,7 +14,7 @@
 // 62 bits.  The prefix sum of the odd outputs, which multiplies the
 // roundings before it by about sqrt(M) and in floating point adds one per
 // term, adds none.  The error against exact arithmetic is below the FP64
-// transform's (tests/test_host.py).
+// transform's (tests/test_fixed_point.py).
 //
 // A value v of a row stands for v 2^e, e the row's exponent.  A row whose
 // largest magnitude is infinite or NaN has every output NaN, a row of zeros

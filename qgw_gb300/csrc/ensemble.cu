@@ -1,7 +1,7 @@
 // ensemble.cu -- batches of independent runs (uneven grids and layer
-// counts) advanced together: one persistent launch per step stage over all
+// counts) advanced together: one launch per step stage over all
 // members, the four launches of a step captured once as a CUDA graph and
-// replayed, and a project autotuner for the persistent grid of each stage.
+// replayed, and a project autotuner for the grid of each stage.
 //
 // Each member is a full qgw_run (own fields, own device scalars, own CFL
 // counter); the batched kernels only change which block computes which
@@ -395,8 +395,8 @@ static int ensemble_set_shape(qgw::EnsembleCore* e, const qgw_shape& sh) {
 // Autotuner, coordinate descent timed over `trial_steps` whole steps per
 // candidate (each choice measured in the context of the others: caches,
 // the member states the step leaves behind): first the work-tile shape of
-// every member -- RHS tile height, column-tile width, modes per block of the
-// forward and of the inverse row kernels -- then the persistent grid of
+// every member -- RHS tile height, column-tile width, layers per block of the
+// forward and of the inverse row kernels -- then the grid of
 // each stage (blocks per SM).  Runs on the current state and then restores
 // the members' time scalars; the trial steps advance q, so callers re-set
 // q before the time loop.  best_ms[4] (optional) receives the step time

@@ -54,7 +54,7 @@ void enqueue_budget_f64(const StepArgs<double>& a, const double* wts, double* pa
 void enqueue_budget_f32c(const StepArgs<float>& a, const double* wts, double* part, int nblk, double scale,
                          double* out, cudaStream_t s);
 
-// ensembles (one persistent launch per stage over all members)
+// ensembles (one launch per stage over all members)
 // dynamic shared memory per stage; the RHS stage per halo radius R (rhs_bytes[R], 0: no member)
 // and the (ensemble-wide) RHS tile height and column-tile width
 struct EnsSmem { size_t bytes[4]; size_t rhs_bytes[5]; int rhs_ty; int ct; };

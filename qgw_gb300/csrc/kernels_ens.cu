@@ -1,4 +1,4 @@
-// kernels_ens.cu -- the ensemble step kernels: one persistent launch per
+// kernels_ens.cu -- the ensemble step kernels: one launch per
 // stage over all members of a batch, and their launchers; the device side
 // they share with the single-run kernels is step_device.cuh.
 #include "step_device.cuh"
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(NT) k_flush_ens(EnsArgs<T> e) {
   }
 }
 
-// ---- ensembles: one persistent launch per stage over all members
+// ---- ensembles: one launch per stage over all members
 template <typename T, bool COMP>
 static cudaError_t set_attrs_ens() {
   int dev = 0, optin = 0;

@@ -119,7 +119,7 @@ template <typename T> struct StepArgs {
   int nsweep;                      // hyperviscosity Laplacian sweeps (0: off)
   int has_nu, has_topo, has_wind, has_drag;
   // grouping
-  int G1;                          // modes per block in the row passes
+  int G1;                          // modes per block in the row passes (FP64: ensembles alone)
   int G3;                          // modes per block in K3 (zeta doubles the rows)
   // compensated path: a second spectral field formed in K2, transformed by
   // K3 into `zeta`, read by K4.  0: none.  1: zeta = L psi (the 5-point

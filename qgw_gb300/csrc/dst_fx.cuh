@@ -11,8 +11,8 @@
 // Measured at 1024^2 x 10 against the floating-point transforms (FP64 pipe
 // 83-88% busy): columns 0.784 -> 0.227 ms; forward rows 0.640 -> 0.34 and
 // inverse rows 0.551 -> 0.28, and with the projections in kernels of their own
-// (modes_fx.cuh) 0.249 and 0.191 for both kernels; rel-L2 error of q after 10
-// steps 1.7e-13 -> 2.3e-14.  Bound by integer instructions: a product is six
+// (modes_fx.cuh) 0.249 and 0.195 for both kernels; rel-L2 error of q after 10
+// steps 2.3e-13 -> 3.3e-14.  Bound by integer instructions: a product is six
 // (three multiplies, of which the wide one issues at 16 a clock and SM), a
 // double to fixed point and back a dozen each.
 #pragma once

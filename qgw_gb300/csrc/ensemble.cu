@@ -236,7 +236,8 @@ void ens_core_free_tables(EnsembleCore* e) {
 // A new member's shape: FP32c RHS tiles of 32 rows.  The batched kernel holds
 // one tile a block, so the taller tile's smaller halo costs no residency (the
 // single run's ring of two tiles does lose blocks at radius 3): 16 members of
-// 64^2 to 512^2, 482 -> 446 us a step.  QGW_RHS_TILE_ROWS overrides.
+// 64^2 to 512^2, three draws, 480, 452 and 583 -> 444, 418 and 542 us a step
+// (runs of one side within 0.3).  QGW_RHS_TILE_ROWS overrides.
 void ens_member_shape(qgw_run* r) {
   if (r->precision == QGW_FP64 || std::getenv("QGW_RHS_TILE_ROWS")) return;
   qgw_shape sh{};

@@ -81,11 +81,11 @@ __global__ void __launch_bounds__(NT, NL == 0 ? 2 : NL >= 8 ? 4 : 5) k_modes(con
   Q2* cs = (Q2*)smem_raw;
   const ModeTable& tb = FWD ? a.l2m : a.m2l;
   __shared__ QUpdate u;
-  if (FWD && threadIdx.x == 0) u = q_update(a, step_mode);
+  if (FWD && threadIdx.x == 0 && (NL > 0 || threadIdx.y == 0)) u = q_update(a, step_mode);
   if constexpr (NL > 0) modes_stage<NL>(tb, cs);
   __syncthreads();
   const int np = !FWD && a.periodic ? a.nx + 2 : a.nx;
-  const int w = blockIdx.x * NT + threadIdx.x, j = w / np, i = w - j * np;
+  const int w = blockIdx.x * (NL > 0 ? NT : blockDim.x) + threadIdx.x, j = w / np, i = w - j * np;
   if constexpr (NL == 0) modes_point_any<FWD>(a, tb, u, j, i, j < a.ny, cs);
   else if (j < a.ny) modes_point<NL, FWD>(a, tb, u, j, i, cs);
 }
@@ -458,7 +458,8 @@ static cudaError_t set_attrs(const StepArgs<T>& a) {
                           (const void*)k_rows_f64<false, 0, false>,   (const void*)k_rows_f64<false, 0, true>,
                           (const void*)k_rows_f64<false, 512, false>, (const void*)k_rows_f64<false, 512, true>,
                           (const void*)k_rows_f64<false, -1, false>,  (const void*)k_rows_f64<false, -1, true>,
-                          (const void*)k_rows_f64<true, 0, false>,    (const void*)k_rows_f64<true, 0, true>};
+                          (const void*)k_rows_f64<true, 0, false>,    (const void*)k_rows_f64<true, 0, true>,
+                          (const void*)k_modes<0, true>,              (const void*)k_modes<0, false>};
     for (const void* f : rows)
       if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, lim))) return e;
   } else {
@@ -500,6 +501,24 @@ static void launch(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStre
   cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
 }
 
+// Threads that share a point in the projections of any number of layers, which
+// read the layers again for every MODES_GO outputs: more of them where the
+// points alone fill few blocks, as long as each has outputs and two blocks'
+// constants fit an SM (or the blocks are fewer than the SMs).  In FP64 up to
+// three blocks per SM, in fixed point, whose values each thread converts
+// again, up to one and a half.  Forward and inverse stage in ms, with one
+// thread a point and as chosen: 64^2 x 128 2.24 and 0.40, 128^2 x 128 2.31 and
+// 1.21, 256^2 x 64 1.26 and 1.11, 128^2 x 24 0.129 and 0.088, 64^2 x 17 0.093
+// and 0.065; beyond the lines 384^2 x 24 0.517 with one and 0.523 with two,
+// 256^2 x 17 0.136 and 0.141.
+static inline int modes_any_split(const StepArgs<double>& a, size_t n) {
+  const size_t few = (size_t)(a.modes_fx ? 228 : 512) * NT;
+  int GY = 1;
+  while (GY < 8 && GY * MODES_GO < a.nl && n * GY < few &&
+         (modes_any_bytes(a.nl, 2 * GY) <= (size_t)110 * 1024 || 2 * GY * n <= (size_t)152 * NT))
+    GY *= 2;
+  return GY;
+}
 // FP64: a projection and the row transforms after it
 template <bool FWD> static void launch_modes(const StepArgs<double>& a, int step_mode, bool pdl, cudaStream_t s) {
   const size_t n = (size_t)a.ny * (!FWD && a.periodic ? a.nx + 2 : a.nx);
@@ -510,7 +529,12 @@ template <bool FWD> static void launch_modes(const StepArgs<double>& a, int step
     QGW_MODES(1) QGW_MODES(2) QGW_MODES(3) QGW_MODES(4) QGW_MODES(5) QGW_MODES(6) QGW_MODES(7) QGW_MODES(8)
     QGW_MODES(9) QGW_MODES(10) QGW_MODES(11) QGW_MODES(12) QGW_MODES(13) QGW_MODES(14) QGW_MODES(15) QGW_MODES(16)
 #undef QGW_MODES
-    default: launch(k_modes<0, FWD>, grid, dim3(NT), sizeof(Q2) * 8 * a.nl, s, pdl, a, step_mode); break;
+    default: {
+      const int GY = modes_any_split(a, n), pts = NT / GY;
+      launch(k_modes<0, FWD>, dim3((unsigned int)((n + pts - 1) / pts)), dim3(pts, GY), modes_any_bytes(a.nl, GY), s,
+             pdl, a, step_mode);
+      break;
+    }
   }
 }
 template <bool INV> static void launch_rows(const StepArgs<double>& a, int step_mode, bool pdl, cudaStream_t s) {

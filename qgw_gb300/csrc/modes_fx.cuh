@@ -171,20 +171,26 @@ __device__ __forceinline__ void modes_point(const StepArgs<double>& a, const Mod
   }
 }
 // The same for any nl, by the whole block (on: the thread has a point), in
-// fixed point or, where a.modes_fx is 0, in FP64; cs: nl x 8 constants of
-// shared memory.
+// fixed point or, where a.modes_fx is 0, in FP64.  A block of GY = blockDim.y
+// > 1 gives each of its points to GY threads, which take the layers in turns
+// as q is brought up to date and then every GY-th group of outputs.  cs:
+// shared memory, modes_any_bytes(nl, GY).
+constexpr int MODES_GO = 8;  // outputs a thread forms at a time
+constexpr size_t modes_any_bytes(int nl, int GY) {
+  return sizeof(Q2) * MODES_GO * (size_t)nl * GY + (GY > 1 ? NT * sizeof(ModeMax) : 0);
+}
 template <bool FWD>
 __device__ __forceinline__ void modes_point_any(const StepArgs<double>& a, const ModeTable& tb, const QUpdate& u,
                                                 int j, int i, bool on, Q2* cs) {
-  constexpr int GO = 8;
-  const int nl = a.nl;
+  constexpr int GO = MODES_GO;
+  const int nl = a.nl, y = threadIdx.y, GY = blockDim.y, tid = threadIdx.x + y * blockDim.x;
   const size_t o = (size_t)j * a.pitch + i;
   const double* src = FWD ? a.q : a.spec;
   double* dst = FWD ? a.spec : a.psi;
   const int* k = tb.e + nl;
   ModeMax h = {};
   auto load = [&](auto value) {
-    for (int l = 0; l < nl; ++l) modes_max(h, fx_hi(value(l, o + (size_t)l * a.lstride)), k[l]);
+    for (int l = y; l < nl; l += GY) modes_max(h, fx_hi(value(l, o + (size_t)l * a.lstride)), k[l]);
   };
   if (on) {
     if constexpr (FWD)
@@ -192,24 +198,35 @@ __device__ __forceinline__ void modes_point_any(const StepArgs<double>& a, const
     else
       load([&](int, size_t ol) { return src[ol]; });
   }
+  if (GY > 1) {
+    ModeMax* hs = (ModeMax*)(cs + (size_t)nl * GO * GY);
+    hs[tid] = h;
+    __syncthreads();
+    for (int g = 0; g < GY; ++g) {
+      const ModeMax v = hs[g * blockDim.x + threadIdx.x];
+      h.raw = max(h.raw, v.raw);
+      h.hi = max(h.hi, v.hi);
+    }
+  }
   const unsigned int turn = modes_turn(i, j);
   const double* mat = FWD ? a.cl2m : a.cm2l;
   double* cd = (double*)cs;
-  for (int m0 = 0; m0 < nl; m0 += GO) {
+  for (int b0 = 0; b0 < nl; b0 += GO * GY) {
     __syncthreads();
-    for (int w = threadIdx.x; w < nl * GO; w += NT) {
-      const int g = w % GO, l = w / GO, e = (m0 + g) * nl + l;
-      if (a.modes_fx) cs[w] = m0 + g < nl ? tb.c[e] : Q2{0, 0};
-      else cd[w] = m0 + g < nl ? mat[e] : 0.0;
+    for (int w = tid; w < nl * GO * GY; w += NT) {
+      const int g = w % GO, l = w / GO % nl, m = b0 + w / (GO * nl) * GO + g, e = m * nl + l;
+      if (a.modes_fx) cs[w] = m < nl ? tb.c[e] : Q2{0, 0};
+      else cd[w] = m < nl ? mat[e] : 0.0;
     }
     __syncthreads();
-    if (!on) continue;
+    const int m0 = b0 + y * GO, c0 = y * nl;
+    if (!on || m0 >= nl) continue;
     if (a.modes_fx) {
       ModeAcc s[GO] = {};
       for (int l = 0; l < nl; ++l) {
         const fx_t x = modes_in((unsigned long long)__double_as_longlong(src[o + (size_t)l * a.lstride]), h, k[l], turn);
-        if (l & 1) modes_add<GO, true>(s, x, cs + l * GO);
-        else modes_add<GO, false>(s, x, cs + l * GO);
+        if (l & 1) modes_add<GO, true>(s, x, cs + (c0 + l) * GO);
+        else modes_add<GO, false>(s, x, cs + (c0 + l) * GO);
         if ((l & 3) == 3 || l == nl - 1) {
 #pragma unroll
           for (int g = 0; g < GO; ++g) modes_carry(s[g]);
@@ -223,7 +240,7 @@ __device__ __forceinline__ void modes_point_any(const StepArgs<double>& a, const
       for (int l = 0; l < nl; ++l) {
         const double v = src[o + (size_t)l * a.lstride];
         double c[GO];
-        ld_coefs<GO, double>(cd + l * GO, c);
+        ld_coefs<GO, double>(cd + (c0 + l) * GO, c);
 #pragma unroll
         for (int g = 0; g < GO; ++g) acc[g] = fmaT(c[g], v, acc[g]);
       }

@@ -47,6 +47,35 @@ def test_ensemble_members_equal_alone(qgwlib, prec, graph):
     ens.close()
 
 
+@pytest.mark.parametrize("N,nl,bc", [(4, 17, 0.0), (16, 9, 0.0), (64, 20, -1.0), (48, 24, 0.0), (128, 17, 1.0),
+                                     (128, 40, 0.0), (64, 65, -1.0), (32, 256, 0.0), (160, 130, 0.0), (384, 24, 0.0)])
+def test_layers_beyond_a_threads_registers(qgwlib, N, nl, bc):
+    """A single run's projections give a point to one, two, four or eight
+    threads, an ensemble's to one: bitwise the same, q in from the host and
+    forced runs included."""
+    p = dict(C.cfg2(N, nl), bc_fac=bc)
+    if nl == 9:  # strongly graded: FP64 sums
+        p.update(dh=[30.0 * 2 ** k for k in range(nl)])
+    if nl == 65:
+        p.update(k_f=8 * np.pi / p["Lx"], sigma_f=1e-12)
+    q0 = C.noise_ic(p, 61)
+    psi_a, q_a = alone(qgwlib, p, 0, q0, 3)
+    ens = qgwlib.Ensemble([p], 0)
+    ens.set_q(0, q0)
+    ens.fix_dt(0, p["dt"])
+    ens.step(3)
+    psi, q = ens.get(0)
+    ens.close()
+    assert np.array_equal(q, q_a) and np.array_equal(psi, psi_a) and np.all(np.isfinite(q)) and np.any(psi)
+    r = qgwlib.Run(p, 0)
+    r.set_q(np.zeros_like(q0))
+    r.fix_dt(p["dt"])
+    out = np.empty_like(q0)
+    r.step_host(3, q0, out)
+    r.close()
+    assert np.array_equal(out[:, 1:-1, 1:-1], q_a[:, 1:-1, 1:-1])
+
+
 def test_ensemble_tune_then_run(qgwlib):
     ps = members()
     ens = qgwlib.Ensemble(ps, 1)

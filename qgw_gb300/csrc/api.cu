@@ -365,17 +365,24 @@ int setup_args(qgw_run* r, StepArgs<T>& a) {
   a.G3 = mode_group(r->nl, Mrow, sizeof(T), 110 * 1024, 1, 16, inv_group(0, Mrow, r->nl, bufs_x), bufs_x);
   if (sizeof(T) == 8) {
     // FP64 row kernels take rows of any layer: as many as the budget holds,
-    // but on small grids no more than leave every SM a few blocks
+    // but on small grids no more than leave every SM a few blocks -- two (four
+    // for transforms of 256 points and more, whose phases fill a block with
+    // fewer rows) -- rounded down to a power of two, whose phases end in whole
+    // rounds of the block's threads.  384^2 x 8: ten rows 0.061 / 0.054 ms
+    // forward / inverse, eight 0.055 / 0.046; 512^2 x 5: eight 0.048 / 0.041,
+    // four 0.044 / 0.038.
     a.G3 = a.G1;
-    // -- two blocks per SM (four for transforms of 256 points and more, whose
-    // phases fill a block with fewer rows) -- rounded down to a power of two,
-    // whose phases end in whole rounds of the block's threads.  384^2 x 8:
-    // ten rows 0.061 / 0.054 ms forward / inverse, eight 0.055 / 0.046; 512^2
-    // x 5: eight 0.048 / 0.041, four 0.044 / 0.038.
     const int fit = mode_group(1 << 20, Mrow, sizeof(T), row_budget(sizeof(T), Mrow, r->nl), 1, 16, 16);
     const int want = std::max(1, std::min(fit, r->nl * r->ny / (a.gx.H >= 256 ? 608 : 304)));
     a.RB1 = 1;
     while (2 * a.RB1 <= want) a.RB1 *= 2;
+    // Up to eight rows the shorter transforms are a block's latency, and the
+    // blocks that are resident at once, three per SM, take all rows where they
+    // can: 200^2 x 3 one row (597 blocks) 0.030 / 0.029 ms, two 0.023 / 0.021;
+    // 200^2 x 5 two 0.033 / 0.031, three 0.027 / 0.025, four the same; 384^2 x
+    // 5 four 0.045 / 0.042, five 0.036 / 0.033, six 0.040 / 0.037.
+    const int wave = (r->nl * r->ny + 455) / 456;
+    if (a.gx.H < 256 && wave <= std::min(fit, 8)) a.RB1 = wave;
     a.RB3 = a.RB1;
   }
   a.CT = a.CT1 = 0;

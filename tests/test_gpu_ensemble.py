@@ -179,6 +179,26 @@ def test_fp64_shape_is_the_one_the_row_kernels_take(qgwlib):
     ens.close()
 
 
+@pytest.mark.parametrize("N,nl,bc,rows", [(36, 12, 0.0, 1), (72, 7, 0.0, 2), (64, 15, -1.0, 3), (46, 40, 0.0, 4),
+                                          (200, 10, 0.0, 5), (96, 26, -1.0, 6), (256, 12, 0.0, 7), (300, 12, 0.0, 8)])
+def test_fp64_rows_per_block_by_default(qgwlib, N, nl, bc, rows):
+    """The fewest rows per block that leave three blocks per SM, bitwise the
+    result of one row."""
+    p = dict(C.cfg2(N, nl), bc_fac=bc)
+    q0 = C.noise_ic(p, 53)
+    psi_a, q_a = alone(qgwlib, p, 0, q0, 2)
+    r = qgwlib.Run(p, 0)
+    sh = r.get_shape()
+    assert sh["row_group_fwd"] == sh["row_group_inv"] == rows, sh
+    r.set_shape(row_group_fwd=1, row_group_inv=1)
+    r.set_q(q0)
+    r.fix_dt(p["dt"])
+    r.step(2)
+    psi, q = r.get()
+    r.close()
+    assert np.array_equal(q, q_a) and np.array_equal(psi, psi_a)
+
+
 def test_shape_refuses_unknown_values(qgwlib):
     r = qgwlib.Run(C.cfg1(64), 1)
     before = r.get_shape()

@@ -892,9 +892,10 @@ __device__ __forceinline__ void body_cols_per_fx(const StepArgs<double>& a, int 
   }
 }
 // complex columns per tile of a single FP64 run: as many as leave three
-// blocks per SM
+// blocks per SM, and fewer where those blocks are not one and a half
 static inline int per_cols(const StepArgs<double>& a) {
-  return (size_t)8 * row_len<double>(a.gy) * sizeof(double) <= (size_t)74 * 1024 ? 4 : 2;
+  const bool fits = (size_t)8 * row_len<double>(a.gy) * sizeof(double) <= (size_t)74 * 1024;
+  return fits && (a.gx.H + 4) / 4 * a.nl >= 228 ? 4 : 2;
 }
 
 template <typename T, bool COMP>

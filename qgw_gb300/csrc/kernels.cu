@@ -615,6 +615,15 @@ template <typename T, bool COMP>
 static void launch_rhs(const StepArgs<T>& a, bool pdl, cudaStream_t s) {
   const int ntx = rhs_ntx(a), nty = rhs_nty(a), ntiles = ntx * nty * a.nl;
   const int grid = (a.rhs_grid > 0 && a.rhs_grid < ntiles) ? a.rhs_grid : ntiles;
+  // Tiles that stay in FP64 take several times as long as the others.  Placed
+  // while the kernel before drains, all of a small grid's blocks crowd the SMs
+  // that come free first and wait on their FP64 pipes: such a grid launches
+  // plainly.  72^2 x 13 no-slip (195 tiles) a step of 99 -> 90 us, 192^2 x 3
+  // with topography 95 -> 76, 384x240x3 120 -> 101; below 100 tiles (64^2 x 3:
+  // 58 against 61) and above four blocks per SM (256^2 x 6: 89 against 92) the
+  // overlap is worth more.
+  if constexpr (sizeof(T) == 8)
+    if ((a.cbc > 0 || a.has_topo) && ntiles >= 100 && ntiles < 608) pdl = false;
   const dim3 blk(32, 8);
   const size_t sm = smem_rhs_tiles(a);
   const bool t32 = rhs_ty(a) == 32;

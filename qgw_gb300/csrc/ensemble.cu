@@ -193,7 +193,6 @@ int qgw_ensemble_create(int n, const qgw_params* params, int precision, qgw_ense
   for (int i = 0; i < n; ++i) {
     qgw_run* r = nullptr;
     if ((rc = qgw_create(&params[i], nullptr, nullptr, nullptr, nullptr, precision, &r))) return fail(rc);
-    qgw::ens_member_shape(r);
     e->members.push_back(r);
   }
   if ((rc = qgw::ens_core_build(e))) return fail(rc);
@@ -233,16 +232,30 @@ void ens_core_free_tables(EnsembleCore* e) {
   e->d_maxsteps = nullptr;
 }
 
-// A new member's shape: FP32c RHS tiles of 32 rows.  The batched kernel holds
-// one tile a block, so the taller tile's smaller halo costs no residency (the
-// single run's ring of two tiles does lose blocks at radius 3): 16 members of
-// 64^2 to 512^2, three draws, 480, 452 and 583 -> 444, 418 and 542 us a step
-// (runs of one side within 0.3).  QGW_RHS_TILE_ROWS overrides.
-void ens_member_shape(qgw_run* r) {
-  if (r->precision == QGW_FP64 || std::getenv("QGW_RHS_TILE_ROWS")) return;
-  qgw_shape sh{};
-  sh.rhs_tile_rows = 32;
-  (void)qgw_set_shape(r, &sh);  // refused: it keeps 16
+// The members' RHS tile height in FP32c, unless a call chose one
+// (rhs_rows_set): 32 rows where there are 16-row tiles for more than one wave
+// of five blocks per SM.  The batched kernel holds one tile a block, so the
+// taller tile's smaller halo costs no residency (the single run's ring of two
+// tiles does lose blocks at radius 3): 16 members of 64^2 to 512^2, three
+// draws, 480, 452 and 583 -> 444, 418 and 542 us a step (runs of one side
+// within 0.3).  A single wave waits for its longest block: 8 members of 64^2 x
+// 5 (320 tiles) 83.3 us in 32 rows, 81.4 in 16, one of 256^2 x 5 (640) 55.1
+// and 53.0; 16 of 128^2 x 2 (1024) 108 and 111.  QGW_RHS_TILE_ROWS overrides.
+static int default_rhs_rows(EnsembleCore* e) {
+  if (e->precision == QGW_FP64 || e->rhs_rows_set || std::getenv("QGW_RHS_TILE_ROWS")) return QGW_OK;
+  long long tiles = 0;
+  for (const qgw_run* r : e->members)
+    tiles += (long long)((r->nx + rhs_tile_x() - 1) / rhs_tile_x()) * ((r->ny + 15) / 16) * r->nl;
+  qgw_shape want{};
+  want.rhs_tile_rows = tiles > 5 * e->nsm ? 32 : 16;
+  for (qgw_run* r : e->members) {
+    qgw_shape sh{};
+    qgw_get_shape(r, &sh);
+    if (sh.rhs_tile_rows == want.rhs_tile_rows) continue;
+    const int rc = qgw_set_shape(r, &want);
+    if (rc && rc != QGW_ERR_PARAM) return rc;  // refused: it keeps 16
+  }
+  return QGW_OK;
 }
 
 // The batched kernels take the column-tile width and the RHS tile height
@@ -284,8 +297,8 @@ int ens_core_build(EnsembleCore* e) {
     const bool blue = e->precision == QGW_FP64 ? (r->a64.gx.blue || r->a64.gy.blue) : (r->a32.gx.blue || r->a32.gy.blue);
     if (blue) return QGW_ERR_UNSUPPORTED;
   }
-  const int rc = uniform_shape(e);
-  if (rc) return rc;
+  int rc = default_rhs_rows(e);
+  if (rc || (rc = uniform_shape(e))) return rc;
   return build_tables(e);
 }
 
@@ -390,6 +403,7 @@ static int ensemble_set_shape(qgw::EnsembleCore* e, const qgw_shape& sh) {
       return rc;
     }
   }
+  if (sh.rhs_tile_rows) e->rhs_rows_set = true;
   return qgw::ens_core_build(e);
 }
 

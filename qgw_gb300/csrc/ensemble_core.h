@@ -38,13 +38,13 @@ struct EnsembleCore {
   int bps[4] = {0, 0, 0, 0};
   int grid[4] = {0, 0, 0, 0};
   int rhs_grid[5] = {0, 0, 0, 0, 0};
+  bool rhs_rows_set = false;  // a call chose the RHS tile height
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   std::vector<DevState> h_states;
 };
 
 // (re)build the device member table and work lists from e->members
-void ens_member_shape(qgw_run* r);  // the default shape of a new member
 int ens_core_build(EnsembleCore* e);
 void ens_core_free_tables(EnsembleCore* e);
 // enqueue up to nsteps steps for every member (max_steps[i] > 0 caps member

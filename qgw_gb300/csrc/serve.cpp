@@ -95,7 +95,6 @@ int admit_one(qgw_pool* pl, const std::shared_ptr<Request>& r) {
     qgw_destroy(run);
     return QGW_ERR_UNSUPPORTED;
   }
-  qgw::ens_member_shape(run);
   if ((rc = qgw_set_q(run, r->q0.data()))) {
     qgw_destroy(run);
     return rc;

@@ -230,6 +230,18 @@ def test_ensemble_nondefault_shape_equals_alone(qgwlib, prec):
     ens.close()
 
 
+def test_ensemble_rhs_rows_by_default(qgwlib):
+    """FP32c members take 16-row RHS tiles up to 760 of them in all and 32-row
+    ones from there on; a height that was set stays."""
+    for n, rows in ((18, 16), (19, 32)):  # 2 x 4 x 5 tiles each, and 16
+        ens = qgwlib.Ensemble([C.cfg2(64, 5)] * n + [C.cfg2(64, 2)], 1)
+        assert all(ens.get_shape(i)["rhs_tile_rows"] == rows for i in (0, n))
+        ens.set_shape(rhs_tile_rows=48 - rows)
+        ens.set_shape(col_tile=4)
+        assert all(ens.get_shape(i)["rhs_tile_rows"] == 48 - rows for i in (0, n))
+        ens.close()
+
+
 def test_ensemble_tuner_picks_a_shape(qgwlib):
     """The tuner's shape is one of its candidates, and the tuned ensemble
     still matches each run alone bitwise."""

@@ -315,6 +315,10 @@ static __global__ void __launch_bounds__(256) k_reset(DevState* st, unsigned int
 // Boundary copies: the reference layout (nl, ny+2, nx+2) in one contiguous
 // device buffer (or the caller's host array) <-> the interior-only run
 // layout, a row at a time.
+// Four waves of blocks, so that the last one's rows even out: a stored q of
+// 2048^2 x 6 from host memory 1.078 -> 1.055 ms, from the device 0.185 -> 0.168;
+// q of 1024^2 x 10 into host memory 0.606 -> 0.597.
+static inline int pack_blocks(int rows) { return std::min(rows, 152 * 32); }
 template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(256) k_unpack(const double* __restrict__ full, T* __restrict__ dst,
                                                 T* __restrict__ lo, int nx, int ny, int nl, int pitch) {
@@ -701,12 +705,12 @@ void enqueue_begin(DevState* st, double t_out, double tend, cudaStream_t s) {
 
 void enqueue_unpack_split(const double* full, float* hi, float* lo, int nx, int ny, int nl, int pitch,
                           cudaStream_t s) {
-  k_unpack<float, true><<<std::min(nl * ny, 152 * 8), 256, 0, s>>>(full, hi, lo, nx, ny, nl, pitch);
+  k_unpack<float, true><<<pack_blocks(nl * ny), 256, 0, s>>>(full, hi, lo, nx, ny, nl, pitch);
 }
 
 void enqueue_pack_join(const float* hi, const float* lo, const float* psi, double c, int periodic, double* full, int nx,
                        int ny, int nl, int pitch, cudaStream_t s) {
-  k_pack<float><<<std::min(nl * (ny + 2), 152 * 8), 256, 0, s>>>(hi, lo, psi, c, periodic, full, nx, ny, nl, pitch);
+  k_pack<float><<<pack_blocks(nl * (ny + 2)), 256, 0, s>>>(hi, lo, psi, c, periodic, full, nx, ny, nl, pitch);
 }
 
 int rhs_tile_x() { return TX; }
@@ -745,12 +749,12 @@ void enqueue_reset(DevState* st, void* fab, size_t bytes, cudaStream_t s) {
   k_reset<<<(int)std::min(blocks, (size_t)152 * 8), 256, 0, s>>>(st, (unsigned int*)fab, bytes / 4);
 }
 void enqueue_unpack_f64(const double* full, double* q, int nx, int ny, int nl, int pitch, cudaStream_t s) {
-  k_unpack<double, false><<<std::min(nl * ny, 152 * 8), 256, 0, s>>>(full, q, nullptr, nx, ny, nl, pitch);
+  k_unpack<double, false><<<pack_blocks(nl * ny), 256, 0, s>>>(full, q, nullptr, nx, ny, nl, pitch);
 }
 
 void enqueue_pack_f64(const double* src, const double* psi, double c, int periodic, double* full, int nx, int ny, int nl,
                       int pitch, cudaStream_t s) {
-  k_pack<double><<<std::min(nl * (ny + 2), 152 * 8), 256, 0, s>>>(src, nullptr, psi, c, periodic, full, nx, ny, nl, pitch);
+  k_pack<double><<<pack_blocks(nl * (ny + 2)), 256, 0, s>>>(src, nullptr, psi, c, periodic, full, nx, ny, nl, pitch);
 }
 
 void enqueue_split_f64(const double* src, float* hi, float* lo, size_t n, cudaStream_t s) {

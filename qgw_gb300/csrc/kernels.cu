@@ -65,8 +65,8 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 4) k_rhs(const __grid
   body_rhs_tiles<T, COMP, R, TY, rhs_nbuf<T>()>(a, ntx, nty, base, a.use_tma ? &a.tm[0] : nullptr, bar);
 }
 
-// FP64: the projections, one thread per point (NL: layers in registers, 0:
-// any number), and the row transforms (modes_fx.cuh).  The projections wait
+// FP64: the projections, one thread per point (NL: layers in registers; 0:
+// any number, blockDim.y threads per point), and the row transforms (modes_fx.cuh).  The projections wait
 // on their loads: five blocks per SM below eight layers (48 registers, few
 // spills), four from there on.  Both forward kernels at three, four and five
 // blocks: 1024^2 x 10 0.265, 0.256 and 0.258 ms, 768^2 x 8 0.182, 0.173 and
@@ -508,10 +508,10 @@ static void launch(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStre
 // Threads that share a point in the projections of any number of layers, which
 // read the layers again for every MODES_GO outputs: more of them where the
 // points alone fill few blocks, as long as each has outputs and two blocks'
-// constants fit an SM (or the blocks are fewer than the SMs).  In FP64 up to
-// three blocks per SM, in fixed point, whose values each thread converts
-// again, up to one and a half.  Forward and inverse stage in ms, with one
-// thread a point and as chosen: 64^2 x 128 2.24 and 0.40, 128^2 x 128 2.31 and
+// constants fit an SM (or the blocks are fewer than the SMs).  Doubled up to 512
+// blocks in FP64, up to one and a half per SM in fixed point, whose values each
+// thread converts again.  Forward and inverse stage in ms, with one thread a
+// point and as chosen: 64^2 x 128 2.24 and 0.40, 128^2 x 128 2.31 and
 // 1.21, 256^2 x 64 1.26 and 1.11, 128^2 x 24 0.129 and 0.088, 64^2 x 17 0.093
 // and 0.065; beyond the lines 384^2 x 24 0.517 with one and 0.523 with two,
 // 256^2 x 17 0.136 and 0.141.
@@ -523,6 +523,7 @@ static inline int modes_any_split(const StepArgs<double>& a, size_t n) {
     GY *= 2;
   return GY;
 }
+
 // FP64: a projection and the row transforms after it
 template <bool FWD> static void launch_modes(const StepArgs<double>& a, int step_mode, bool pdl, cudaStream_t s) {
   const size_t n = (size_t)a.ny * (!FWD && a.periodic ? a.nx + 2 : a.nx);

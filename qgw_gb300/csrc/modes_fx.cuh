@@ -5,7 +5,7 @@
 // point by point and are linear, so each runs as a kernel of its own beside
 // the row transforms: a thread holds one point's nl values, so every value is
 // loaded and turned into fixed point once for all nl outputs, and the row
-// kernel takes rows of any layer, four at a time.  (Inside the row kernels
+// kernel takes rows of any layer, several at a time.  (Inside the row kernels
 // the projection cost nl FP64 multiply-adds a point, two thirds of their
 // FP64-pipe-bound time, and shared memory held the rows of two modes only, so
 // each pair of modes read the row's layers again.)  The extra pass over the

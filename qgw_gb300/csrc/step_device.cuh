@@ -892,7 +892,9 @@ __device__ __forceinline__ void body_cols_per_fx(const StepArgs<double>& a, int 
   }
 }
 // complex columns per tile of a single FP64 run: as many as leave three
-// blocks per SM, and fewer where those blocks are not one and a half
+// blocks per SM, and two where tiles of four are not one and a half per SM:
+// 512^2 x 3 (195 of them) 0.035 -> 0.024 ms, 72^2 x 7 (70) 0.0202 -> 0.0165;
+// 256^2 x 6 (198) 0.0225 -> 0.0184, x 10 (330) 0.025 with four
 static inline int per_cols(const StepArgs<double>& a) {
   const bool fits = (size_t)8 * row_len<double>(a.gy) * sizeof(double) <= (size_t)74 * 1024;
   return fits && (a.gx.H + 4) / 4 * a.nl >= 228 ? 4 : 2;
